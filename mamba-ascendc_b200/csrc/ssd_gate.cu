@@ -8,6 +8,10 @@
 // The reference fuses these into its state-epilogue and gate kernels (mamba2_ssd_state_epilogue.cpp:413-482,
 // bwd_gate/design.md:8-13).  Element-wise and bandwidth bound: the tensors are walked as [tokens, H*P] with
 // float4 accesses along the row; dD is reduced in two phases in a fixed order (fp64 in the second phase).
+//
+// What bounds these kernels is how many loads are in flight, so both dimensions of a CTA follow the shape: `ct`
+// threads along a row and `rt` rows side by side (a row of a few hundred channels otherwise leaves most of
+// the CTA idle), kGateUnroll rows per thread at once, and row blocks small enough to give every SM several CTAs.
 #include "ssd_host.h"
 
 namespace ssd {
@@ -15,7 +19,30 @@ namespace ssd {
 namespace {
 
 constexpr int kGateThreads = 256;
-constexpr int kGateRows = 128;  // tokens per CTA in the backward pass (one dD partial per CTA and column)
+constexpr int kGateUnroll = 4;        // rows of one thread in flight together
+constexpr int kGateMaxRows = 128;     // tokens per CTA in the backward pass (one dD partial per CTA and column) ...
+constexpr int kGateCtasWanted = 1184; // ... fewer when that leaves less than eight CTAs per SM of 148, ...
+constexpr int kGateMinRows = 32;      // ... but there not so few that adding up the partials takes longer than forming them
+
+// How [rows, cols / 4] float4s are laid over CTAs: `colblocks` blocks of `ct` threads along a row, `rt` rows side by
+// side in a CTA.  ct * rt <= kGateThreads, and ct is as even a share of the row as the block count allows.
+struct GateGrid {
+    int ct, rt, colblocks, rows_per_cta;
+    long long rowblocks;
+};
+GateGrid gate_grid(long long rows, int cols, int min_rows) {
+    GateGrid g;
+    const int c4 = cols / 4;
+    g.colblocks = (c4 + kGateThreads - 1) / kGateThreads;
+    g.ct = (c4 + g.colblocks - 1) / g.colblocks;
+    g.rt = kGateThreads / g.ct;
+    const int least = g.rt * kGateUnroll > min_rows ? g.rt * kGateUnroll : min_rows;
+    g.rows_per_cta = kGateMaxRows > least ? kGateMaxRows : least;
+    while (g.rows_per_cta / 2 >= least && (rows + g.rows_per_cta - 1) / g.rows_per_cta * g.colblocks < kGateCtasWanted)
+        g.rows_per_cta /= 2;
+    g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
+    return g;
+}
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -31,94 +58,154 @@ __device__ __forceinline__ float4 load_d(const float* D, int d_mode, int c, int 
     return make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+template <bool HAS_D, bool HAS_Z>
 __global__ void __launch_bounds__(kGateThreads)
 gate_skip_fwd_kernel(const float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ D, int d_mode,
-                     const float* __restrict__ z, float* __restrict__ out, long long rows, int cols, int p_dim) {
-    const int c = (blockIdx.x * kGateThreads + threadIdx.x) * 4;
-    if (c >= cols) return;
+                     const float* __restrict__ z, float* __restrict__ out, long long rows, int cols, int p_dim, int ct,
+                     int rt, int rows_per_cta) {
+    const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
+    const int c = (blockIdx.x * ct + tx) * 4;
+    if (c >= cols || ty >= rt) return;
     const float4 d = load_d(D, d_mode, c, p_dim);
-    for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
-        const size_t o = static_cast<size_t>(r) * cols + c;
-        float4 v = ld4(y + o);
-        if (d_mode) {
-            const float4 xv = ld4(x + o);
-            v.x += d.x * xv.x;
-            v.y += d.y * xv.y;
-            v.z += d.z * xv.z;
-            v.w += d.w * xv.w;
+    const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_cta;
+    const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
+    for (long long r = r0 + ty; r < r1; r += kGateUnroll * rt) {
+        float4 v[kGateUnroll], xv[kGateUnroll], zv[kGateUnroll];
+#pragma unroll
+        for (int u = 0; u < kGateUnroll; ++u) {
+            const long long ru = r + u * rt;
+            if (ru < r1) {
+                const size_t o = static_cast<size_t>(ru) * cols + c;
+                v[u] = ld4(y + o);
+                if (HAS_D) xv[u] = ld4(x + o);
+                if (HAS_Z) zv[u] = ld4(z + o);
+            }
         }
-        if (z) {
-            const float4 zv = ld4(z + o);
-            v.x *= zv.x * sigmoidf_(zv.x);
-            v.y *= zv.y * sigmoidf_(zv.y);
-            v.z *= zv.z * sigmoidf_(zv.z);
-            v.w *= zv.w * sigmoidf_(zv.w);
+#pragma unroll
+        for (int u = 0; u < kGateUnroll; ++u) {
+            const long long ru = r + u * rt;
+            if (ru >= r1) break;
+            if (HAS_D) {
+                v[u].x += d.x * xv[u].x;
+                v[u].y += d.y * xv[u].y;
+                v[u].z += d.z * xv[u].z;
+                v[u].w += d.w * xv[u].w;
+            }
+            if (HAS_Z) {
+                v[u].x *= zv[u].x * sigmoidf_(zv[u].x);
+                v[u].y *= zv[u].y * sigmoidf_(zv[u].y);
+                v[u].z *= zv[u].z * sigmoidf_(zv[u].z);
+                v[u].w *= zv[u].w * sigmoidf_(zv[u].w);
+            }
+            st4(out + static_cast<size_t>(ru) * cols + c, v[u]);
         }
-        st4(out + o, v);
     }
 }
 
-// Backward, one CTA per (1024 columns, kGateRows tokens).  dy and dz may be null (no z: dy equals dout and the
-// caller uses dout itself).  part[row_block][cols] receives this CTA's sum over its tokens of dy .* x.
+// Backward.  dy and dz are written only with z (without, dy equals dout and the caller uses dout itself).
+// part[row_block][cols] receives this CTA's sum over its tokens of dy .* x: each thread over its own rows, then the
+// `rt` rows that stand side by side in order.
+template <bool HAS_D, bool HAS_Z>
 __global__ void __launch_bounds__(kGateThreads)
 gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y, const float* __restrict__ x,
                      const float* __restrict__ D, int d_mode, const float* __restrict__ z, float* __restrict__ dy,
-                     float* __restrict__ dz, float* __restrict__ part, long long rows, int cols, int p_dim) {
-    const int c = (blockIdx.x * kGateThreads + threadIdx.x) * 4;
-    if (c >= cols) return;
-    const float4 d = load_d(D, d_mode, c, p_dim);
-    const long long r0 = static_cast<long long>(blockIdx.y) * kGateRows;
-    const long long r1 = r0 + kGateRows < rows ? r0 + kGateRows : rows;
+                     float* __restrict__ dz, float* __restrict__ part, long long rows, int cols, int p_dim, int ct, int rt,
+                     int rows_per_cta) {
+    __shared__ float4 sums[kGateThreads];
+    const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
+    const int c = (blockIdx.x * ct + tx) * 4;
+    const bool active = c < cols && ty < rt;
+    const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_cta;
+    const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
+    constexpr int kUnroll = HAS_Z ? 2 : kGateUnroll;  // four tensors a row with z: eight float4 in flight
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (long long r = r0; r < r1; ++r) {
-        const size_t o = static_cast<size_t>(r) * cols + c;
-        const float4 g = ld4(dout + o);
-        float4 gy = g;
-        float4 xv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (d_mode) xv = ld4(x + o);
-        if (z) {
-            const float4 zv = ld4(z + o);
-            const float4 yv = ld4(y + o);
-            const float zz[4] = {zv.x, zv.y, zv.z, zv.w};
-            const float pre[4] = {yv.x + d.x * xv.x, yv.y + d.y * xv.y, yv.z + d.z * xv.z, yv.w + d.w * xv.w};
-            const float gg[4] = {g.x, g.y, g.z, g.w};
-            float oy[4], oz[4];
+    if (active) {
+        const float4 d = load_d(D, d_mode, c, p_dim);
+        for (long long r = r0 + ty; r < r1; r += kUnroll * rt) {
+            float4 g[kUnroll], xv[kUnroll], zv[kUnroll], yv[kUnroll];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float s = sigmoidf_(zz[i]);
-                oy[i] = gg[i] * zz[i] * s;
-                oz[i] = gg[i] * pre[i] * s * (1.f + zz[i] * (1.f - s));
+            for (int u = 0; u < kUnroll; ++u) {
+                const long long ru = r + u * rt;
+                if (ru < r1) {
+                    const size_t o = static_cast<size_t>(ru) * cols + c;
+                    g[u] = ld4(dout + o);
+                    xv[u] = HAS_D ? ld4(x + o) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (HAS_Z) {
+                        zv[u] = ld4(z + o);
+                        yv[u] = ld4(y + o);
+                    }
+                }
             }
-            gy = make_float4(oy[0], oy[1], oy[2], oy[3]);
-            st4(dy + o, gy);
-            st4(dz + o, make_float4(oz[0], oz[1], oz[2], oz[3]));
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const long long ru = r + u * rt;
+                if (ru >= r1) break;
+                float4 gy = g[u];
+                if (HAS_Z) {
+                    const size_t o = static_cast<size_t>(ru) * cols + c;
+                    const float zz[4] = {zv[u].x, zv[u].y, zv[u].z, zv[u].w};
+                    const float pre[4] = {yv[u].x + d.x * xv[u].x, yv[u].y + d.y * xv[u].y, yv[u].z + d.z * xv[u].z,
+                                          yv[u].w + d.w * xv[u].w};
+                    const float gg[4] = {gy.x, gy.y, gy.z, gy.w};
+                    float oy[4], oz[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float s = sigmoidf_(zz[i]);
+                        oy[i] = gg[i] * zz[i] * s;
+                        oz[i] = gg[i] * pre[i] * s * (1.f + zz[i] * (1.f - s));
+                    }
+                    gy = make_float4(oy[0], oy[1], oy[2], oy[3]);
+                    st4(dy + o, gy);
+                    st4(dz + o, make_float4(oz[0], oz[1], oz[2], oz[3]));
+                }
+                acc.x += gy.x * xv[u].x;
+                acc.y += gy.y * xv[u].y;
+                acc.z += gy.z * xv[u].z;
+                acc.w += gy.w * xv[u].w;
+            }
         }
-        acc.x += gy.x * xv.x;
-        acc.y += gy.y * xv.y;
-        acc.z += gy.z * xv.z;
-        acc.w += gy.w * xv.w;
     }
-    if (d_mode) st4(part + static_cast<size_t>(blockIdx.y) * cols + c, acc);
+    if (!HAS_D) return;
+    sums[threadIdx.x] = acc;
+    __syncthreads();
+    if (active && ty == 0) {
+        for (int i = 1; i < rt; ++i) {
+            const float4 o = sums[i * ct + tx];
+            acc.x += o.x;
+            acc.y += o.y;
+            acc.z += o.z;
+            acc.w += o.w;
+        }
+        st4(part + static_cast<size_t>(blockIdx.y) * cols + c, acc);
+    }
 }
 
-// Second phase of dD: block per head, thread per channel; row blocks in order, then (per-head D) the channels.
+// Second phase of dD: a CTA per head, `lanes` threads per channel that take the row blocks in turn; their fp64 sums
+// are added in order, then (per-head D) the channels.
 __global__ void gate_dd_reduce_kernel(const float* __restrict__ part, int row_blocks, int cols, int p_dim, int d_mode,
-                                      float* __restrict__ dD) {
+                                      int lanes, float* __restrict__ dD) {
     extern __shared__ double red[];
-    const int h = blockIdx.x, p = threadIdx.x;
+    const int h = blockIdx.x, p = threadIdx.x % p_dim, l = threadIdx.x / p_dim;
     double s = 0.0;
-    if (p < p_dim)
-        for (int rb = 0; rb < row_blocks; ++rb) s += part[static_cast<size_t>(rb) * cols + h * p_dim + p];
-    if (d_mode == 2) {
-        if (p < p_dim) dD[h * p_dim + p] = static_cast<float>(s);
-        return;
-    }
-    red[p] = p < p_dim ? s : 0.0;
+    if (l < lanes)
+#pragma unroll 8
+        for (int rb = l; rb < row_blocks; rb += lanes) s += part[static_cast<size_t>(rb) * cols + h * p_dim + p];
+    red[threadIdx.x] = s;
     __syncthreads();
-    if (p == 0) {
+    if (l == 0) {
+        for (int i = 1; i < lanes; ++i) s += red[i * p_dim + p];
+        if (d_mode == 2) dD[h * p_dim + p] = static_cast<float>(s);
+    }
+    if (d_mode == 2) return;
+    __syncthreads();
+    if (l == 0) red[p] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
         double t = 0.0;
-        for (int i = 0; i < p_dim; ++i) t += red[i];
-        dD[h] = static_cast<float>(t);
+        for (int i = threadIdx.x; i < p_dim; i += 32) t += red[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) dD[h] = static_cast<float>(t);
     }
 }
 
@@ -139,7 +226,7 @@ extern "C" size_t ssd_gate_partial_floats(const SsdShape* shape) {
     long long rows = 0;
     int cols = 0;
     if (ssd::gate_dims(shape, &rows, &cols) != SSD_OK) return 0;
-    return static_cast<size_t>((rows + ssd::kGateRows - 1) / ssd::kGateRows) * cols;
+    return static_cast<size_t>(ssd::gate_grid(rows, cols, kGateMinRows).rowblocks) * cols;
 }
 
 extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const float* x, const float* D, int d_mode,
@@ -151,9 +238,20 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     if (rc != SSD_OK) return rc;
     if (!y || !out || (d_mode != 0 && (!D || !x))) return SSD_ERR_NULL;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
-    const dim3 grid((cols / 4 + kGateThreads - 1) / kGateThreads, static_cast<unsigned>(rows < 1024 ? rows : 1024));
-    gate_skip_fwd_kernel<<<grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(y, x, D, d_mode, z, out, rows,
-                                                                                            cols, shape->headdim);
+    GateGrid g = gate_grid(rows, cols, 1);
+    while (g.rowblocks > 65535) {
+        g.rows_per_cta *= 2;
+        g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
+    }
+    const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
+    auto launch = [&](auto kernel) {
+        kernel<<<grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+            y, x, D, d_mode, z, out, rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta);
+    };
+    if (d_mode != 0)
+        z ? launch(gate_skip_fwd_kernel<true, true>) : launch(gate_skip_fwd_kernel<true, false>);
+    else
+        z ? launch(gate_skip_fwd_kernel<false, true>) : launch(gate_skip_fwd_kernel<false, false>);
     return launch_status();
 }
 
@@ -168,16 +266,24 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!dout || (z && (!y || !dy || !dz)) || (d_mode != 0 && (!D || !x || !dD_partial || !dD))) return SSD_ERR_NULL;
     if (!z && d_mode == 0) return SSD_OK;  // nothing to do
-    const long long row_blocks = (rows + kGateRows - 1) / kGateRows;
-    if (row_blocks > 65535) return SSD_ERR_UNSUPPORTED;
+    const GateGrid g = gate_grid(rows, cols, kGateMinRows);
+    if (g.rowblocks > 65535) return SSD_ERR_UNSUPPORTED;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const dim3 grid((cols / 4 + kGateThreads - 1) / kGateThreads, static_cast<unsigned>(row_blocks));
-    gate_skip_bwd_kernel<<<grid, kGateThreads, 0, st>>>(dout, y, x, D, d_mode, z, dy, dz, dD_partial, rows, cols,
-                                                        shape->headdim);
+    const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
+    auto launch = [&](auto kernel) {
+        kernel<<<grid, kGateThreads, 0, st>>>(dout, y, x, D, d_mode, z, dy, dz, dD_partial, rows, cols, shape->headdim,
+                                              g.ct, g.rt, g.rows_per_cta);
+    };
+    if (d_mode != 0)
+        z ? launch(gate_skip_bwd_kernel<true, true>) : launch(gate_skip_bwd_kernel<true, false>);
+    else
+        launch(gate_skip_bwd_kernel<false, true>);
     if (d_mode != 0) {
-        const int threads = (shape->headdim + 31) / 32 * 32;
+        const int p = shape->headdim;
+        const int lanes = 1024 / p;
+        const int threads = (lanes * p + 31) / 32 * 32;
         gate_dd_reduce_kernel<<<shape->nheads, threads, threads * sizeof(double), st>>>(
-            dD_partial, static_cast<int>(row_blocks), cols, shape->headdim, d_mode, dD);
+            dD_partial, static_cast<int>(g.rowblocks), cols, p, d_mode, lanes, dD);
     }
     return launch_status();
 }
