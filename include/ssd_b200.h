@@ -200,6 +200,10 @@ int ssd_chunk_dbc_bwd(const SsdShape* shape, const float* x, const float* bm, co
  * phase of mamba2_ssd_dt_bwd (op_kernel :1013-1068). */
 int ssd_dt_finalize_bwd(const SsdShape* shape, const float* ddt_t, const double* dA_partial, float* ddt, float* dA,
                         ssd_stream_t stream);
+/* The same launch with d(dt_bias)[H], the sum of ddt over batch and tokens (mamba2_ssd_dt_bwd/design.md:63-77), formed on
+ * the way; null leaves it out. */
+int ssd_dt_finalize_bias_bwd(const SsdShape* shape, const float* ddt_t, const double* dA_partial, float* ddt, float* dA,
+                             float* ddt_bias, ssd_stream_t stream);
 
 /* ---------------------------------------------------------------- D skip connection and SiLU(z) gate
  *

@@ -75,6 +75,7 @@ SIGNATURES = {
     "ssd_chunk_dx_bwd": (ctypes.c_int, [_shape_p] + [_p] * 15 + [_p, ctypes.c_int, _p, _p]),
     "ssd_chunk_dbc_bwd": (ctypes.c_int, [_shape_p] + [_p] * 13),
     "ssd_dt_finalize_bwd": (ctypes.c_int, [_shape_p] + [_p] * 5),
+    "ssd_dt_finalize_bias_bwd": (ctypes.c_int, [_shape_p] + [_p] * 6),
     "ssd_gate_partial_floats": (ctypes.c_size_t, [_shape_p]),
     "ssd_gate_skip_fwd": (ctypes.c_int, [_shape_p, _p, _p, _p, ctypes.c_int, _p, _p, _p]),
     "ssd_gate_skip_bwd": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, ctypes.c_int, _p, _p, _p, _p, _p, _p]),

@@ -225,7 +225,7 @@ def forward_stages(x, dt, A, B, C, dt_softplus: bool, want_final: bool = True, i
 
 
 def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplus: bool, want_dinitial: bool = False,
-                    dt_bias=None, dt_limit=(0.0, float("inf")), valid_len: int = 0, outflow=None, D=None):
+                    dt_bias=None, dt_limit=(0.0, float("inf")), valid_len: int = 0, outflow=None, D=None, ddt_bias=None):
     """Run the backward stages; returns (dx, ddt, dA, dB, dC, d_initial_states or None).
 
     ``outflow(d_initial0) -> extra dfinal or None`` (sequence-parallel mode): called once the local state
@@ -233,7 +233,9 @@ def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplu
     its successors; what it returns is added to ``dfinal`` before the reverse recurrence runs.
 
     ``D``: the skip connection of the gated node; then ``dout`` / ``out`` are the gradient / value of the SSD
-    output before skip and gate, and ``D * dout`` is added to dx by the dx kernel."""
+    output before skip and gate, and ``D * dout`` is added to dx by the dx kernel.
+
+    ``ddt_bias`` [H]: receives the sum of ddt over batch and tokens."""
     shape = make_shape(x, B, dt_softplus, dt_limit, valid_len)
     b, l, h, p = x.shape
     n = B.shape[3]
@@ -275,7 +277,8 @@ def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplu
     _call("mamba2_ssd_chunk_dx_bwd", lib.ssd_chunk_dx_bwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(dout), _ptr(out), _ptr(dstates), _ptr(q),
                                      _ptr(cs), _ptr(dt), _ptr(dt_bias), _ptr(A), _ptr(g_last), _ptr(dx), _ptr(ddt_t),
                                      _ptr(dA_part), _ptr(D), _d_mode(D), _ptr(status), st)
-    _call("mamba2_ssd_dt_bwd", lib.ssd_dt_finalize_bwd, sp, _ptr(ddt_t), _ptr(dA_part), _ptr(ddt), _ptr(dA), st)
+    _call("mamba2_ssd_dt_bwd", lib.ssd_dt_finalize_bias_bwd, sp, _ptr(ddt_t), _ptr(dA_part), _ptr(ddt), _ptr(dA),
+          _ptr(ddt_bias), st)
     return dx, ddt, dA, dB, dC, d_initial
 
 
@@ -317,11 +320,11 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
                 out, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
                                                        initial_states=initial_states, dt_bias=dt_bias,
                                                        dt_limit=ctx.dt_limit, valid_len=ctx.valid_len)
+            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
             dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal,
                                                          ctx.dt_softplus, want_dinitial=ctx.has_initial,
                                                          dt_bias=dt_bias, dt_limit=ctx.dt_limit,
-                                                         valid_len=ctx.valid_len)
-        dbias = ddt.sum(dim=(0, 1)) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
+                                                         valid_len=ctx.valid_len, ddt_bias=dbias)
         return dx, ddt, dA, dB, dC, None, dinit, dbias, None, None, None
 
 
@@ -392,11 +395,12 @@ class _Mamba2SsdGatedAutograd(torch.autograd.Function):
                 y, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
                                                      initial_states=initial_states, dt_bias=dt_bias,
                                                      dt_limit=ctx.dt_limit)
+            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None
             dy, dz, dD = gate_backward(dout, y, x, B, D, z)
             dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, y, q, cs, states, dy, dfinal,
                                                          ctx.dt_softplus, want_dinitial=ctx.has_initial,
-                                                         dt_bias=dt_bias, dt_limit=ctx.dt_limit, D=D)
-        dbias = ddt.sum(dim=(0, 1)) if dt_bias is not None else None
+                                                         dt_bias=dt_bias, dt_limit=ctx.dt_limit, D=D,
+                                                         ddt_bias=dbias)
         return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
 
 
