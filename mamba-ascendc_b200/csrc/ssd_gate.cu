@@ -226,7 +226,7 @@ extern "C" size_t ssd_gate_partial_floats(const SsdShape* shape) {
     long long rows = 0;
     int cols = 0;
     if (ssd::gate_dims(shape, &rows, &cols) != SSD_OK) return 0;
-    return static_cast<size_t>(ssd::gate_grid(rows, cols, kGateMinRows).rowblocks) * cols;
+    return static_cast<size_t>(ssd::gate_grid(rows, cols, ssd::kGateMinRows).rowblocks) * cols;
 }
 
 extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const float* x, const float* D, int d_mode,
