@@ -143,7 +143,7 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     // ---- warp 16: issues every tensor-core instruction of the CTA.  Its warp group hands most of its
     // registers to the four computing groups.
     if (warp >= kThreads / 32) {
-        reg_release<kIssuerRegs>();
+        reg_release<kProducerRegs>();
         if (warp == kThreads / 32 && lane == 0) {
             const uint32_t ss = smem_u32(smem + L::kS), su = smem_u32(smem + L::kU), sb = smem_u32(smem + L::kB),
                            sc = smem_u32(smem + L::kC);
@@ -307,7 +307,7 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         return;
     }
 
-    reg_acquire<kComputeRegs>();
+    reg_acquire<kProducedComputeRegs>();
 
     const int t_row = (warp & 3) * 32 + lane;  // this thread's row of the accumulators (TMEM lane)
     const int qr = warp & 3;                   // its block of 32 rows

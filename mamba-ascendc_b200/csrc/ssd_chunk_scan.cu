@@ -129,7 +129,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 
     // ---- warp 16: issues every tensor-core instruction of the CTA
     if (warp >= kThreads / 32) {
-        reg_release<kIssuerRegs>();  // this warp group hands most of its registers to the computing groups
+        reg_release<kProducerRegs>();  // this warp group hands most of its registers to the computing groups
         if (warp == kThreads / 32 && lane == 0) {
             const Operand bm{smem_u32(smem + L::kB), smem_u32(smem + L::kB) + kHalf, kTile, false, 2 * kHalf};
             uint32_t pcb = 0, ps = 0, pw = 0;  // ps: one parity bit per S-ready barrier
@@ -268,7 +268,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         }
         return;
     }
-    reg_acquire<kComputeRegs>();
+    reg_acquire<kProducedComputeRegs>();
 
     auto x_tile = [&](int it) { return smem + L::kX + (it % NB) * L::kXTile; };
     auto s_tile = [&](int it) { return smem + L::kS + (it % NB) * L::kSTile; };

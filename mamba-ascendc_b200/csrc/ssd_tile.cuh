@@ -19,10 +19,16 @@ constexpr int kThreads = 512;              // compute threads (16 warps)
 // publishes the per-head rows (the remaining warps leave at once).  A whole group, because register trading
 // (reg_release / reg_acquire) works on groups of four warps: a 17th warp alone would cap every thread at
 // 96 registers (five warps on one scheduler share its 512 registers per lane).  The registers traded are the
-// CTA's own (640 x 96 at launch): with 112 for the compute groups the fifth group cannot keep more than 32.
+// CTA's own (640 x 96 at launch): with 112 for the compute groups the fifth group cannot keep more than 32, with 104
+// it keeps 64.  The persistent kernels take the second split: at 32 registers their producer and issuing warps
+// spilled 88 to 208 bytes a thread on the way from a freed buffer to the next load.
 constexpr int kLaunchThreadsGroups = kThreads + 128;
 constexpr uint32_t kIssuerRegs = 32;    // 96 at launch (640 threads): the issuing group keeps 32 ...
 constexpr uint32_t kComputeRegs = 112;  // ... and each of the four computing groups takes 16 more
+constexpr uint32_t kProducerRegs = 64;         // the split of the persistent kernels
+constexpr uint32_t kProducedComputeRegs = 104;
+static_assert(128 * kIssuerRegs + 512 * kComputeRegs <= 640 * 96 && 128 * kProducerRegs + 512 * kProducedComputeRegs <= 640 * 96,
+              "the registers traded are those of the launch");
 
 // Barrier over the 512 compute threads only (named barrier 1); the MMA-issuing warp never joins it.
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
