@@ -108,6 +108,15 @@ size_t ssd_buffer_bytes(const SsdShape* shape, int which);
 int ssd_dt_cumsum(const SsdShape* shape, const float* dt, const float* dt_bias, const float* A, float* q, float* cs,
                   ssd_stream_t stream);
 
+/* A whole forward call on a short sequence: the recurrence itself, token by token in fp32, with the D skip connection
+ * (D: d_mode 1 [H], 2 [H,P], 0 none) and the z gate [B,L,H,P] (null = none) in the same launch.  Any seqlen and headdim, dstate a multiple of 4
+ * up to 128; `tile` and `valid_len` play no part (valid_len must be 0).  initial_state / final_state [B,H,P,N], either may be null, and
+ * bm, cm need 16-byte aligned base addresses.  Stands in for the same entry point of the reference
+ * as the stages below (mamba2_ssd_fwd.cpp:49-136). */
+int ssd_recurrent_fwd(const SsdShape* shape, const float* x, const float* dt, const float* dt_bias, const float* A,
+                      const float* bm, const float* cm, const float* D, int d_mode, const float* z,
+                      const float* initial_state, float* out, float* final_state, ssd_stream_t stream);
+
 /* states[b,h,k,p,n] = sum_t w_t X[t,p] M[t,n] on tcgen05.
  * mode 0: X = x, M = B, w_t = q_t exp(cs_last - cs_t): the chunk-state product of
  *         mamba2_ssd_chunk_mix (mamba_ascendc/csrc/aclnn/mamba2_ssd_chunk_mix.cpp:7-69).

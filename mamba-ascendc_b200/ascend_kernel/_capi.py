@@ -65,6 +65,7 @@ SIGNATURES = {
     "ssd_selftest_tile_walk": (ctypes.c_int, [_shape_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, _p]),
     "ssd_selftest_umma": (ctypes.c_int, [_p, _p, _p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _p, _p]),
     "ssd_dt_cumsum": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p, _p]),
+    "ssd_recurrent_fwd": (ctypes.c_int, [_shape_p] + [_p] * 7 + [ctypes.c_int] + [_p] * 5),
     "ssd_chunk_state": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p, ctypes.c_int, _p, _p]),
     "ssd_state_passing_fwd": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p]),
     "ssd_chunk_scan_fwd": (ctypes.c_int, [_shape_p] + [_p] * 9),

@@ -451,6 +451,37 @@ def _device_guard(device: torch.device):
     return torch.cuda.device(device)
 
 
+# Longest sequence that takes the recurrence kernel instead of the tile kernels (which treat 128 tokens at a time and so
+# cost the same for 1 token as for 128).  Device time of both, us, with D, z and an initial state:
+#   [batch, heads, P, N, G]     1 token      16 tokens    64 tokens    100 tokens
+#   [ 1,   4, 64,  64, 1]     3.4 /  47     8.7 /  47     29 /  47     45 /   47
+#   [16,  24, 64, 128, 1]     7.0 / 165      26 / 180     90 / 198    139 /  192
+#   [64, 128, 64,  64, 8]      49 / 397     208 / 516    753 / 875   1171 / 1083
+SHORT_SEQUENCE = 64
+
+
+def _short_sequence(x, B, C, D, z, initial_states) -> bool:
+    """Whether a call without gradients runs as one recurrence launch (ssd_recurrent_fwd)."""
+    n = B.shape[3]
+    if not (0 < x.shape[1] <= SHORT_SEQUENCE and 0 < n <= 128 and n % 4 == 0 and min(x.shape) > 0 and B.shape[2] > 0):
+        return False
+    if torch.autograd.forward_ad._current_level >= 0:  # tangents of D and z come from the framework's operations
+        return False
+    return not any(t is not None and t.data_ptr() & 15 for t in (B, C, initial_states))
+
+
+def recurrent_forward(x, dt, A, B, C, dt_softplus: bool, want_final: bool, initial_states, dt_bias, dt_limit, D, z):
+    b, l, h, p = x.shape
+    g, n = B.shape[2], B.shape[3]
+    shape = _capi.SsdShape(b, l, h, p, n, TILE, g, _capi.SSD_FLAG_DT_SOFTPLUS if dt_softplus else 0, dt_limit[0],
+                           dt_limit[1], 0)
+    out = torch.empty_like(x)
+    final = torch.empty(b, h, p, n, device=x.device, dtype=torch.float32) if want_final else None
+    _call("mamba2_ssd_recurrent", _capi.lib.ssd_recurrent_fwd, ctypes.byref(shape), _ptr(x), _ptr(dt), _ptr(dt_bias),
+          _ptr(A), _ptr(B), _ptr(C), _ptr(D), _d_mode(D), _ptr(z), _ptr(initial_states), _ptr(out), _ptr(final), _stream())
+    return out, final
+
+
 def _requires_grad(*tensors) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
@@ -488,6 +519,10 @@ def mamba2_ssd_fwd(
         return out_k, final_k
 
     with _device_guard(x.device):
+        if not _requires_grad(x, dt, A, B, C, D, z, initial_states, dt_bias) and _short_sequence(x, B, C, D, z, initial_states):
+            out, final = recurrent_forward(x, dt, A, B, C, bool(dt_softplus), return_final_state, initial_states, dt_bias,
+                                           lim, D, z)
+            return (out, final) if return_final_state else out
         p, n = x.shape[3], B.shape[3]
         native = p == 64 and x.shape[1] % TILE == 0
         if native and n == 64 and (D is not None or z is not None) and _requires_grad(
