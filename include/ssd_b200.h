@@ -204,6 +204,13 @@ int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const float* bm, con
 int ssd_chunk_dbc_bwd(const SsdShape* shape, const float* x, const float* bm, const float* cm, const float* dout,
                       const float* states_start, const float* dstates, const float* q, const float* cs, float* dB,
                       float* dC, float* g_last, int* status, ssd_stream_t stream);
+/* The same with the heads of a group dealt to `split` work items (a divisor of H/G), for shapes with fewer (batch, group,
+ * tile) items than SMs: each item leaves a partial dB and dC in `partial` (2 * split * B*L*G*N floats, null with split 1) and a second
+ * launch adds them in order.  ssd_dbc_split is the split that pays for `shape` (1: none). */
+int ssd_dbc_split(const SsdShape* shape);
+int ssd_chunk_dbc_split_bwd(const SsdShape* shape, const float* x, const float* bm, const float* cm, const float* dout,
+                            const float* states_start, const float* dstates, const float* q, const float* cs, float* dB,
+                            float* dC, float* g_last, int split, float* partial, int* status, ssd_stream_t stream);
 
 /* ddt[B,L,H] from ddt_t and dA[H] from dA_partial (fixed-order sums).  Stands in for the reduce
  * phase of mamba2_ssd_dt_bwd (op_kernel :1013-1068). */

@@ -75,6 +75,8 @@ SIGNATURES = {
     "ssd_state_fold": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, ctypes.c_int, _p]),
     "ssd_chunk_dx_bwd": (ctypes.c_int, [_shape_p] + [_p] * 15 + [_p, ctypes.c_int, _p, _p]),
     "ssd_chunk_dbc_bwd": (ctypes.c_int, [_shape_p] + [_p] * 13),
+    "ssd_dbc_split": (ctypes.c_int, [_shape_p]),
+    "ssd_chunk_dbc_split_bwd": (ctypes.c_int, [_shape_p] + [_p] * 11 + [ctypes.c_int, _p, _p, _p]),
     "ssd_dt_finalize_bwd": (ctypes.c_int, [_shape_p] + [_p] * 5),
     "ssd_dt_finalize_bias_bwd": (ctypes.c_int, [_shape_p] + [_p] * 6),
     "ssd_gate_partial_floats": (ctypes.c_size_t, [_shape_p]),

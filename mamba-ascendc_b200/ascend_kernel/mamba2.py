@@ -272,8 +272,10 @@ def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplu
     if not fused:
         _call("mamba2_ssd_state_passing_bwd", lib.ssd_state_passing_bwd, sp, _ptr(dstates), None, _ptr(cs), _ptr(dfinal),
               None, _ptr(d_initial), st)
-    _call("mamba2_ssd_chunk_dbc_bwd", lib.ssd_chunk_dbc_bwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(dout), _ptr(states), _ptr(dstates),
-                                      _ptr(q), _ptr(cs), _ptr(dB), _ptr(dC), _ptr(g_last), _ptr(status), st)
+    split = lib.ssd_dbc_split(sp)  # > 1: few work items, the heads of a group are dealt to several
+    part = torch.empty(2 * split * B.numel(), device=dev, dtype=torch.float32) if split > 1 else None
+    _call("mamba2_ssd_chunk_dbc_bwd", lib.ssd_chunk_dbc_split_bwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(dout), _ptr(states),
+          _ptr(dstates), _ptr(q), _ptr(cs), _ptr(dB), _ptr(dC), _ptr(g_last), split, _ptr(part), _ptr(status), st)
     _call("mamba2_ssd_chunk_dx_bwd", lib.ssd_chunk_dx_bwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(dout), _ptr(out), _ptr(dstates), _ptr(q),
                                      _ptr(cs), _ptr(dt), _ptr(dt_bias), _ptr(A), _ptr(g_last), _ptr(dx), _ptr(ddt_t),
                                      _ptr(dA_part), _ptr(D), _d_mode(D), _ptr(status), st)

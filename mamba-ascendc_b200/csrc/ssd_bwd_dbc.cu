@@ -66,7 +66,7 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_du,
                const __grid_constant__ CUtensorMap map_db, const __grid_constant__ CUtensorMap map_dc,
                const float* __restrict__ q, const float* __restrict__ cs, float* __restrict__ g_last, SsdShape s,
-               int* status) {
+               int split, int* status) {
     using L = BwdDbcSmem;
     constexpr int N = L::N;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -88,16 +88,17 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int heads_per_group = s.nheads / s.ngroups;
+    const int groups = s.ngroups * split;  // of work items; `split` of them share a group and leave a partial sum each
+    const int heads_per_group = s.nheads / groups;
     const int nchunks = s.seqlen / kTile;
     // Work list of this CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the (batch, group, token
     // tile) grid, token tile fastest; the heads of all its tiles form one flat sequence of iterations,
     // so the loads, splits and products of a tile's first head overlap the previous tile's last head.
-    const int num_tiles = s.batch * s.ngroups * nchunks;
+    const int num_tiles = s.batch * groups * nchunks;
     const int my_tiles = (num_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                          static_cast<int>(gridDim.x);
     const int total = my_tiles * heads_per_group;
-    const TileWalk walk(s, static_cast<int>(gridDim.x));
+    const TileWalk walk(s, static_cast<int>(gridDim.x), split);
     using Where = HeadPos;
     auto first_tile = [&]() { return walk.first(static_cast<int>(blockIdx.x)); };
     auto advance = [&](TilePos& t) { walk.advance(t); };
@@ -198,12 +199,13 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 tma_tile_2d(smem + L::kS, 64, &map_s, full_su, 0, w.tile_index * 64, false);
                 tma_tile_2d(smem + L::kU, 64, &map_du, full_su, 0, w.tile_index * 64, false);
             };
-            auto load_bc = [&](int g, int tok0) {
+            auto load_bc = [&](int item_group, int tok0) {
+                const int g = walk.group_of(item_group);
                 mbar_arrive_expect_tx(full_bc, 2 * L::kPTile);
                 tma_tile_3d(smem + L::kB, kTile, &map_b, full_bc, 0, g, tok0, false);
                 tma_tile_3d(smem + L::kC, kTile, &map_c, full_bc, 0, g, tok0, false);
             };
-            // Finished tile of group g at token tok0, staged by the compute warps in the region of the tile's
+            // Finished tile of (work item) group g at token tok0, staged by the compute warps in the region of the tile's
             // last head, iteration `j` (named barrier 4 says so).
             auto store_tile = [&](int j, int g, int tok0) {
                 asm volatile("bar.sync 4, 544;" ::: "memory");
@@ -574,14 +576,52 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+// Sum of the partial gradients [B,L,G,split,N] of the work items of a group, in order: dB, then dC.
+__global__ void __launch_bounds__(256)
+dbc_sum_kernel(const float* __restrict__ partial, float* __restrict__ dB, float* __restrict__ dC, size_t quads, int split,
+               int row_quads) {
+    const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
+    if (i >= 2 * quads) return;
+    const bool second = i >= quads;
+    const size_t e = second ? i - quads : i;
+    const size_t row = e / row_quads;
+    const float4* src = reinterpret_cast<const float4*>(partial) + (second ? quads * split : 0) +
+                        row * split * row_quads + (e - row * row_quads);
+    float4 sum = src[0];
+#pragma unroll 4
+    for (int j = 1; j < split; ++j) {
+        const float4 v = src[static_cast<size_t>(j) * row_quads];
+        sum.x += v.x;
+        sum.y += v.y;
+        sum.z += v.z;
+        sum.w += v.w;
+    }
+    reinterpret_cast<float4*>(second ? dC : dB)[e] = sum;
+}
+
 }  // namespace
 
 }  // namespace ssd
+
+extern "C" int ssd_dbc_split(const SsdShape* shape) {
+    using namespace ssd;
+    if (ssd_check_shape(shape) != SSD_OK) return 1;
+    const int64_t items = static_cast<int64_t>(shape->seqlen / kTile) * shape->ngroups * shape->batch;
+    return choose_head_split(items, shape->nheads / shape->ngroups, sm_count(), 1, 5);
+}
 
 extern "C" int ssd_chunk_dbc_bwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
                                  const float* dout, const float* states_start, const float* dstates, const float* q,
                                  const float* cs, float* dB, float* dC, float* g_last, int* status,
                                  ssd_stream_t stream) {
+    return ssd_chunk_dbc_split_bwd(shape, x, bm, cm, dout, states_start, dstates, q, cs, dB, dC, g_last, 1, nullptr, status,
+                                   stream);
+}
+
+extern "C" int ssd_chunk_dbc_split_bwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
+                                       const float* dout, const float* states_start, const float* dstates,
+                                       const float* q, const float* cs, float* dB, float* dC, float* g_last, int split,
+                                       float* partial, int* status, ssd_stream_t stream) {
     using namespace ssd;
     const int rc0 = ssd_check_shape(shape);
     if (rc0 != SSD_OK) return rc0;
@@ -589,14 +629,21 @@ extern "C" int ssd_chunk_dbc_bwd(const SsdShape* shape, const float* x, const fl
         return SSD_ERR_NULL;
     const SsdShape& s = *shape;
     if (s.dstate != 64) return SSD_ERR_UNSUPPORTED;
+    if (split < 1 || (s.nheads / s.ngroups) % split != 0) return SSD_ERR_SHAPE;
+    if (split > 1 && !partial) return SSD_ERR_NULL;
+    if ((reinterpret_cast<uintptr_t>(partial) & 15u) != 0) return SSD_ERR_ALIGN;
+    const int groups = s.ngroups * split;
+    const size_t elems = static_cast<size_t>(s.batch) * s.seqlen * s.ngroups * s.dstate;  // of dB, and of dC
+    float* out_db = split > 1 ? partial : dB;
+    float* out_dc = split > 1 ? partial + elems * split : dC;
     CUtensorMap map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc;
     const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
     int rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
     if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_b, bm, tokens, s.ngroups, s.dstate, kTile);
     if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, tokens, s.ngroups, s.dstate, kTile);
     if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dout, dout, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_db, dB, tokens, s.ngroups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dc, dC, tokens, s.ngroups, s.dstate, kTile);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_db, out_db, tokens, groups, s.dstate, kTile);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dc, out_dc, tokens, groups, s.dstate, kTile);
     const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
     if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_s, states_start, state_rows, s.dstate, 64);
     if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_du, dstates, state_rows, s.dstate, 64);
@@ -605,11 +652,17 @@ extern "C" int ssd_chunk_dbc_bwd(const SsdShape* shape, const float* x, const fl
     static std::atomic<uint64_t> smem_set{0};
     rc = set_max_smem_once(reinterpret_cast<const void*>(bwd_dbc_kernel), smem, smem_set);
     if (rc != SSD_OK) return rc;
-    const int tiles = (s.seqlen / kTile) * s.ngroups * s.batch;
+    const int64_t tiles = static_cast<int64_t>(s.seqlen / kTile) * groups * s.batch;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
-    const dim3 grid(tiles < sms ? tiles : sms);  // persistent: one CTA per SM walks its share of the tiles
+    if (tiles * split > 0x7fffffff) return SSD_ERR_RANGE;
+    const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
     bwd_dbc_kernel<<<grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, status);
+        map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, status);
+    rc = launch_status();
+    if (rc != SSD_OK || split == 1) return rc;
+    const size_t quads = 2 * elems / 4;
+    dbc_sum_kernel<<<static_cast<unsigned>((quads + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        partial, dB, dC, elems / 4, split, s.dstate / 4);
     return launch_status();
 }

@@ -60,7 +60,7 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
               const __grid_constant__ CUtensorMap map_x, const float* __restrict__ q, const float* __restrict__ cs,
               const float* __restrict__ dt, const float* __restrict__ dt_bias, const float* __restrict__ A,
               const float* __restrict__ g_last, float* __restrict__ ddt_t, double* __restrict__ dA_part,
-              const float* __restrict__ dy_raw, const float* __restrict__ dskip, int d_mode, SsdShape s, int* status) {
+              const float* __restrict__ dy_raw, const float* __restrict__ dskip, int d_mode, SsdShape s, int split, int* status) {
     using L = BwdDxSmem;
     constexpr int N = L::N;
     extern __shared__ uint8_t smem_raw[];
@@ -85,11 +85,12 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-    const int heads_per_group = s.nheads / s.ngroups;
+    const int k = blockIdx.x, b = blockIdx.z;
+    const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
+    const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
     const int tok0 = b * s.seqlen + k * kTile;
-    const int h_first = g * heads_per_group;
+    const int h_first = blockIdx.y * heads_per_group;
     const bool softplus = (s.flags & SSD_FLAG_DT_SOFTPLUS) != 0;
 
 
@@ -480,7 +481,11 @@ extern "C" int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const flo
     if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_du, dstates, state_rows, s.dstate, 64);
     if (rc != SSD_OK) return rc;
     const size_t smem = BwdDxSmem::kTotal + 1024;
-    const dim3 grid(s.seqlen / kTile, s.ngroups, s.batch);
+    const int sms = sm_count();
+    if (sms <= 0) return SSD_ERR_LAUNCH;
+    const int64_t items = static_cast<int64_t>(s.seqlen / kTile) * s.ngroups * s.batch;
+    const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 3);
+    const dim3 grid(s.seqlen / kTile, s.ngroups * split, s.batch);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (d_mode == 0) {
         static std::atomic<uint64_t> smem_set{0};
@@ -488,14 +493,14 @@ extern "C" int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const flo
         if (rc != SSD_OK) return rc;
         bwd_dx_kernel<false><<<grid, kLaunchThreadsGroups, smem, st>>>(
             map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial,
-            nullptr, nullptr, 0, s, status);
+            nullptr, nullptr, 0, s, split, status);
     } else {
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(bwd_dx_kernel<true>), smem, smem_set);
         if (rc != SSD_OK) return rc;
         bwd_dx_kernel<true><<<grid, kLaunchThreadsGroups, smem, st>>>(
             map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial,
-            dout, D, d_mode, s, status);
+            dout, D, d_mode, s, split, status);
     }
     return launch_status();
 }

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kLaunchThreadsGroups, 1)
 chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_s,
                   const __grid_constant__ CUtensorMap map_out, const float* __restrict__ q,
-                  const float* __restrict__ cs, SsdShape s, int* status) {
+                  const float* __restrict__ cs, SsdShape s, int split, int* status) {
     using L = ChunkScanSmem<N>;
     constexpr int NB = L::kBuf;
     constexpr int NOFF = L::kOffBuf;
@@ -80,15 +80,16 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                                        //     the compute warps may run up to two heads ahead of the producer warp)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int heads_per_group = s.nheads / s.ngroups;
+    const int groups = s.ngroups * split;  // of work items; `split` of them share a group's B and C
+    const int heads_per_group = s.nheads / groups;
     const int nchunks = s.seqlen / kTile;
     // Work list of this CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the (batch, group, token tile)
     // grid, token tile fastest; the heads of all its tiles form one flat sequence of iterations.
-    const int num_tiles = s.batch * s.ngroups * nchunks;
+    const int num_tiles = s.batch * groups * nchunks;
     const int my_tiles = (num_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                          static_cast<int>(gridDim.x);
     const int total = my_tiles * heads_per_group;
-    const TileWalk walk(s, static_cast<int>(gridDim.x));
+    const TileWalk walk(s, static_cast<int>(gridDim.x), split);
 
     if (total <= 0) return;  // no work item for this CTA: leave before anything is allocated
     // An earlier kernel or CTA gave up on a bounded wait: leave without doing work.  Thread 0 alone reads the
@@ -175,9 +176,10 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             };
             auto load_cb = [&](const HeadPos& w) {  // C and B of a tile
                 mbar_arrive_expect_tx(full_c, 2 * L::kCTile);
+                const int g = walk.group_of(w.g);
                 for (int cb = 0; cb < kBlocks; ++cb) {
-                    tma_tile_3d(smem + L::kC + cb * 2 * kHalf, kTile, &map_c, full_c, 64 * cb, w.g, w.tok0, false);
-                    tma_tile_3d(smem + L::kB + cb * 2 * kHalf, kTile, &map_b, full_c, 64 * cb, w.g, w.tok0, false);
+                    tma_tile_3d(smem + L::kC + cb * 2 * kHalf, kTile, &map_c, full_c, 64 * cb, g, w.tok0, false);
+                    tma_tile_3d(smem + L::kB + cb * 2 * kHalf, kTile, &map_b, full_c, 64 * cb, g, w.tok0, false);
                 }
             };
             TilePos cur = walk.first(static_cast<int>(blockIdx.x));
@@ -455,11 +457,14 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
     static std::atomic<uint64_t> smem_set{0};  // one per instantiation
     rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_scan_kernel<N>), smem, smem_set);
     if (rc != SSD_OK) return rc;
-    const int tiles = (s.seqlen / kTile) * s.ngroups * s.batch;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
-    const dim3 grid(tiles < sms ? tiles : sms);  // persistent: one CTA per SM walks its share of the tiles
-    chunk_scan_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_b, map_c, map_s, map_out, q, cs, s, status);
+    const int64_t items = static_cast<int64_t>(s.seqlen / kTile) * s.ngroups * s.batch;
+    const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 2);
+    const int64_t tiles = items * split;
+    const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
+    chunk_scan_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_b, map_c, map_s, map_out, q, cs, s, split,
+                                                                       status);
     return launch_status();
 }
 

@@ -47,7 +47,7 @@ template <int N>
 __global__ void __launch_bounds__(kCsLaunch, (N == 64 ? 2 : 1))
 chunk_state_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_m,
                    const __grid_constant__ CUtensorMap map_st, const float* __restrict__ q,
-                   const float* __restrict__ cs, SsdShape s, int mode, int* status) {
+                   const float* __restrict__ cs, SsdShape s, int split, int mode, int* status) {
     using L = ChunkStateSmem<N>;
     constexpr int kBlocks = N / 64;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -60,11 +60,12 @@ chunk_state_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-    const int heads_per_group = s.nheads / s.ngroups;
+    const int k = blockIdx.x, b = blockIdx.z;
+    const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
+    const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
     const int tok0 = b * s.seqlen + k * kTile;
-    const int h_first = g * heads_per_group;
+    const int h_first = blockIdx.y * heads_per_group;
     const int npairs = (heads_per_group + 1) / 2;
 
     if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need the declared alignment
@@ -239,7 +240,7 @@ template <int N>
 __global__ void __launch_bounds__(kLaunchThreadsGroups, 1)
 chunk_state_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_m,
                    const __grid_constant__ CUtensorMap map_st, const float* __restrict__ q,
-                   const float* __restrict__ cs, SsdShape s, int mode, int* status) {
+                   const float* __restrict__ cs, SsdShape s, int split, int mode, int* status) {
     using L = ChunkStateWideSmem<N>;
     constexpr int kBlocks = N / 64;
     extern __shared__ uint8_t smem_raw[];
@@ -253,11 +254,12 @@ chunk_state_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-    const int heads_per_group = s.nheads / s.ngroups;
+    const int k = blockIdx.x, b = blockIdx.z;
+    const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
+    const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
     const int tok0 = b * s.seqlen + k * kTile;
-    const int h_first = g * heads_per_group;
+    const int h_first = blockIdx.y * heads_per_group;
     const int npairs = (heads_per_group + 1) / 2;
 
 
@@ -434,20 +436,24 @@ int launch_chunk_state(const SsdShape& s, const float* x, const float* m, const 
     const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
     rc = make_tmap_f32_2d(&map_st, states, state_rows, s.dstate, 64);
     if (rc != SSD_OK) return rc;
-    const dim3 grid(s.seqlen / kTile, s.ngroups, s.batch);
+    const int sms = sm_count();
+    if (sms <= 0) return SSD_ERR_LAUNCH;
+    const int64_t items = static_cast<int64_t>(s.seqlen / kTile) * s.ngroups * s.batch;
+    const int split = choose_head_split(items, s.nheads / s.ngroups, N == 64 ? 2 * sms : sms, 2, 1);
+    const dim3 grid(s.seqlen / kTile, s.ngroups * split, s.batch);
     if constexpr (N == 64) {
         const size_t smem = ChunkStateSmem<N>::kTotal;
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_kernel<N>), smem, smem_set);
         if (rc != SSD_OK) return rc;
-        chunk_state_kernel<N><<<grid, kCsLaunch, smem, stream>>>(map_x, map_m, map_st, q, cs, s, mode, status);
+        chunk_state_kernel<N><<<grid, kCsLaunch, smem, stream>>>(map_x, map_m, map_st, q, cs, s, split, mode, status);
     } else {
         const size_t smem = ChunkStateWideSmem<N>::kTotal + 1024;
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_wide_kernel<N>), smem, smem_set);
         if (rc != SSD_OK) return rc;
-        chunk_state_wide_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_m, map_st, q, cs, s, mode,
-                                                                                 status);
+        chunk_state_wide_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_m, map_st, q, cs, s, split,
+                                                                                 mode, status);
     }
     return launch_status();
 }

@@ -143,6 +143,23 @@ int sm_count() {
     return n;
 }
 
+int choose_head_split(int64_t items, int heads_per_group, int slots, int unit, int overhead_halves) {
+    if (slots <= 0 || items >= 16ll * slots) return 1;  // the last round is a small part of the whole
+    int best = 1;
+    int64_t best_cost = 0;
+    for (int d = 1; d <= heads_per_group; ++d) {
+        if (items * d > 32ll * slots && d > 1) break;
+        if (heads_per_group % d != 0) continue;
+        const int units = (heads_per_group / d + unit - 1) / unit;
+        const int64_t cost = (items * d + slots - 1) / slots * (2 * units + overhead_halves);
+        if (d == 1 || cost * 20 < best_cost * 19) {
+            best = d;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 int set_max_smem_once(const void* func, size_t bytes, std::atomic<uint64_t>& done) {
     const int dev = current_device();
     if (dev < 0) return SSD_ERR_LAUNCH;

@@ -49,6 +49,14 @@ int sm_count();
 // each device's context); `done` is the launcher's own bit set, one bit per device.
 int set_max_smem_once(const void* func, size_t bytes, std::atomic<uint64_t>& done);
 
+// Into how many work items the heads of a group are dealt, for a kernel whose `items` = batch * ngroups * tiles work
+// items take `slots` CTAs at a time.  An item treats `unit` heads at once and costs `overhead_halves` half units besides
+// (its B and C tiles and their product); a round costs as much as one item.  Few groups and a short sequence leave SMs
+// without an item, and a split gives them one at the price of the overhead: 8192 tokens of 32 heads in one group (64 items
+// on 148 SMs) take 44 instead of 75 us in the output kernel and 27 instead of 64 us in the state kernel, with two and
+// four items per group.  A split has to promise 5% to be taken.
+int choose_head_split(int64_t items, int heads_per_group, int slots, int unit, int overhead_halves);
+
 inline int launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SSD_OK : SSD_ERR_LAUNCH;

@@ -50,6 +50,10 @@ constexpr uint32_t kSlabBytes = 128 * 128;  // one staged box: 128 rows x 32 flo
 // c + gridDim.x, ... and, inside a tile, the heads of the group in sequence.  Positions are advanced without
 // divisions (three at kernel start), so that the warp that issues the loads has the next coordinates ready
 // before the barrier that frees their memory flips.
+//
+// `split` > 1: the heads of a group are dealt to that many work items (choose_head_split says when that is
+// worth it).  The walk then runs over groups of heads_per_group / split heads; the group whose B and C a work item
+// reads is group_of(g).
 struct TilePos {
     int b, g, k;
 };
@@ -59,9 +63,11 @@ struct HeadPos {
 };
 struct TileWalk {
     int nchunks, ngroups, nheads, seqlen, heads_per_group, step_k, step_g, step_b;
-    __host__ __device__ __forceinline__ TileWalk(const SsdShape& s, int grid)
-        : nchunks(s.seqlen / 128), ngroups(s.ngroups), nheads(s.nheads), seqlen(s.seqlen),
-          heads_per_group(s.nheads / s.ngroups) {
+    unsigned split_inverse;  // 0: no split, else ceil(2^32 / split)
+    __host__ __device__ __forceinline__ TileWalk(const SsdShape& s, int grid, int split = 1)
+        : nchunks(s.seqlen / 128), ngroups(s.ngroups * split), nheads(s.nheads), seqlen(s.seqlen),
+          heads_per_group(s.nheads / (s.ngroups * split)),
+          split_inverse(split > 1 ? static_cast<unsigned>((0x100000000ull + split - 1) / split) : 0u) {
         step_k = grid % nchunks;
         step_g = (grid / nchunks) % ngroups;
         step_b = grid / (nchunks * ngroups);
@@ -85,6 +91,11 @@ struct TileWalk {
             ++t.b;
         }
         t.b += step_b;
+    }
+    // g / split without a division; exact while g * split < 2^32
+    __host__ __device__ __forceinline__ int group_of(int g) const {
+        if (split_inverse == 0) return g;
+        return static_cast<int>((static_cast<unsigned long long>(static_cast<unsigned>(g)) * split_inverse) >> 32);
     }
     // The head `ahead` heads after head `hi` of tile `t` in the CTA's sequence.
     __host__ __device__ __forceinline__ HeadPos locate(TilePos t, int hi, int ahead) const {
