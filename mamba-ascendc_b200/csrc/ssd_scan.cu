@@ -1,7 +1,7 @@
 // Bandwidth-bound scan kernels of the SSD path (no tensor cores):
 //   dt_cumsum_kernel        q = softplus(dt), cs = in-tile inclusive cumsum of A*q   (warp scan)
-//   state_passing_fwd       S_{k+1} = exp(cs_last,k) * S_k + U_k, in place over the chunk states
-//   state_passing_bwd       reverse recurrence, in place over the local dS; also d(cs_last)
+//   state_walk              S_{k+1} = exp(cs_last,k) * S_k + U_k, in place over the chunk states, or the reverse recurrence
+//   state_passing_bwd       reverse recurrence, in place over the local dS, with d(cs_last) as well
 //   dt_finalize             [B,H,L] -> [B,L,H] transpose of ddt, fixed-order reductions of dA and d(dt_bias)
 #include "ssd_host.h"
 #include "ssd_tile.cuh"
@@ -72,34 +72,75 @@ dt_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ dt_bias
     }
 }
 
-// ------------------------------------------------------------------ forward state passing
-// One thread owns four consecutive state elements of one (b,h) and walks the
-// chunks; the buffer holds U_k on entry and S_k (state at the START of chunk
-// k) on exit.  final receives S_K.
-__global__ void __launch_bounds__(256)
-state_passing_fwd_kernel(float* __restrict__ states, const float* __restrict__ cs,
-                         const float* __restrict__ initial_state, float* __restrict__ final_state, int nchunks,
-                         int pn4, int seqlen, size_t total) {
-    const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+// ------------------------------------------------------------------ state passing, either direction
+// One thread owns four consecutive state elements of one (b,h) and walks the tiles, ascending (forward: the buffer holds
+// U_k on entry and S_k, the state at the START of tile k, on exit) or descending (backward: dS_k on entry, dU_k on exit);
+// the recurrence is the same:  v = states[k] ; states[k] = st ; st = exp(cs_last,k) * st + v.  `end` receives the last st.
+//
+// Bound by HBM, and by the loads in flight where there are few (b,h) chains to walk: kWalkTiles tiles are requested ahead of
+// the kWalkTiles being worked on, and CTAs are small so that few chains still reach every SM.  32 chains of 64 tiles
+// (67 MB): 9.8 us = 6.8 TB/s partly from L2, against 26 us with one load ahead and CTAs of 256; 256 chains of 32 tiles (268 MB): 40.2
+// us = 6.7 TB/s, against 52.
+constexpr int kWalkTiles = 8;
+constexpr int kWalkThreads = 64;
+template <bool REVERSE>
+__global__ void __launch_bounds__(kWalkThreads)
+state_walk_kernel(float* __restrict__ states, const float* __restrict__ cs, const float* __restrict__ start,
+                  float* __restrict__ end, int nchunks, int pn4, int seqlen, size_t total) {
+    const size_t idx = static_cast<size_t>(blockIdx.x) * kWalkThreads + threadIdx.x;
     if (idx >= total) return;
     const size_t bh = idx / pn4;
     const int e = static_cast<int>(idx % pn4);
     float4* p = reinterpret_cast<float4*>(states) + bh * nchunks * pn4 + e;
     const float* csl = cs + bh * seqlen + (kTile - 1);
-    float4 st = initial_state ? reinterpret_cast<const float4*>(initial_state)[bh * pn4 + e]
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 u = p[0];
-    for (int k = 0; k < nchunks; ++k) {
-        const float4 cur = u;
-        if (k + 1 < nchunks) u = p[static_cast<size_t>(k + 1) * pn4];  // next load in flight before the store
-        const float alpha = expf(csl[static_cast<size_t>(k) * kTile]);
-        p[static_cast<size_t>(k) * pn4] = st;
-        st.x = alpha * st.x + cur.x;
-        st.y = alpha * st.y + cur.y;
-        st.z = alpha * st.z + cur.z;
-        st.w = alpha * st.w + cur.w;
+    auto tile_of = [&](int i) { return static_cast<size_t>(REVERSE ? nchunks - 1 - i : i); };
+    float4 st = start ? reinterpret_cast<const float4*>(start)[bh * pn4 + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 u[kWalkTiles];
+    float c[kWalkTiles];
+#pragma unroll
+    for (int i = 0; i < kWalkTiles; ++i)
+        if (i < nchunks) {
+            u[i] = p[tile_of(i) * pn4];
+            c[i] = csl[tile_of(i) * kTile];
+        }
+    for (int k = 0; k < nchunks; k += kWalkTiles) {
+        float4 un[kWalkTiles];
+        float cn[kWalkTiles];
+#pragma unroll
+        for (int i = 0; i < kWalkTiles; ++i)
+            if (k + kWalkTiles + i < nchunks) {
+                un[i] = p[tile_of(k + kWalkTiles + i) * pn4];
+                cn[i] = csl[tile_of(k + kWalkTiles + i) * kTile];
+            }
+#pragma unroll
+        for (int i = 0; i < kWalkTiles; ++i) {
+            if (k + i >= nchunks) break;
+            const float alpha = expf(c[i]);
+            p[tile_of(k + i) * pn4] = st;
+            st.x = alpha * st.x + u[i].x;
+            st.y = alpha * st.y + u[i].y;
+            st.z = alpha * st.z + u[i].z;
+            st.w = alpha * st.w + u[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < kWalkTiles; ++i) {
+            u[i] = un[i];
+            c[i] = cn[i];
+        }
     }
-    if (final_state != nullptr) reinterpret_cast<float4*>(final_state)[bh * pn4 + e] = st;
+    if (end != nullptr) reinterpret_cast<float4*>(end)[bh * pn4 + e] = st;
+}
+
+template <bool REVERSE>
+int launch_state_walk(const SsdShape& s, float* states, const float* cs, const float* start, float* end,
+                      cudaStream_t stream) {
+    const int pn4 = s.headdim * s.dstate / 4;
+    const size_t total = static_cast<size_t>(s.batch) * s.nheads * pn4;
+    const size_t blocks = (total + kWalkThreads - 1) / kWalkThreads;
+    if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
+    state_walk_kernel<REVERSE><<<static_cast<unsigned>(blocks), kWalkThreads, 0, stream>>>(
+        states, cs, start, end, s.seqlen / kTile, pn4, s.seqlen, total);
+    return launch_status();
 }
 
 // ------------------------------------------------------------------ read-only fold of the recurrence
@@ -131,7 +172,7 @@ state_fold_kernel(const float* __restrict__ terms, const float* __restrict__ cs,
     reinterpret_cast<float4*>(result)[bh * pn4 + e] = acc;
 }
 
-// ------------------------------------------------------------------ backward state passing
+// ------------------------------------------------------------------ backward state passing with g_last
 // CTA = one (b,h); thread owns ELEMS float4 of the [P,N] state.  dstates holds
 // the local dS_k on entry and dU_k (gradient reaching chunk k's own state
 // contribution, i.e. d loss / d S_{k+1}) on exit.  g_last[b,h,k] =
@@ -150,14 +191,13 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
     float4* dp = reinterpret_cast<float4*>(dstates) + bh * nchunks * pn4;
     const float4* sp = reinterpret_cast<const float4*>(states_start) + bh * nchunks * pn4;
     const float* csl = cs + bh * seqlen + (kTile - 1);
-    const bool want_g = g_last != nullptr;  // without it the forward's states are not read at all
     float4 g[ELEMS], ds_n[ELEMS], st_n[ELEMS];
 #pragma unroll
     for (int i = 0; i < ELEMS; ++i) {
         g[i] = dfinal ? reinterpret_cast<const float4*>(dfinal)[bh * pn4 + i * 1024 + tid] : make_float4(0, 0, 0, 0);
         const size_t o = static_cast<size_t>(nchunks - 1) * pn4 + i * 1024 + tid;
         ds_n[i] = dp[o];
-        st_n[i] = want_g ? sp[o] : make_float4(0, 0, 0, 0);
+        st_n[i] = sp[o];
     }
     if constexpr (!LONG) {
         // No block-wide barrier inside the walk over the tiles: each warp reduces its own products and
@@ -172,7 +212,7 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
                 const float4 st = st_n[i];
                 if (k > 0) {
                     ds_n[i] = dp[o - pn4];
-                    if (want_g) st_n[i] = sp[o - pn4];
+                    st_n[i] = sp[o - pn4];
                 }
                 dp[o] = g[i];
                 dot += g[i].x * st.x + g[i].y * st.y + g[i].z * st.z + g[i].w * st.w;
@@ -190,7 +230,7 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
             float v = part[k * 32 + lane];
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-            if (lane == 0 && want_g) g_last[bh * nchunks + k] = expf(csl[static_cast<size_t>(k) * kTile]) * v;
+            if (lane == 0) g_last[bh * nchunks + k] = expf(csl[static_cast<size_t>(k) * kTile]) * v;
         }
     } else {
         // More tiles than partials fit the shared memory (sequences beyond 49152 tokens): the same walk in
@@ -207,7 +247,7 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
                     const float4 st = st_n[i];
                     if (k > 0) {
                         ds_n[i] = dp[o - pn4];
-                        if (want_g) st_n[i] = sp[o - pn4];
+                        st_n[i] = sp[o - pn4];
                     }
                     dp[o] = g[i];
                     dot += g[i].x * st.x + g[i].y * st.y + g[i].z * st.z + g[i].w * st.w;
@@ -225,7 +265,7 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
                 float v = part[(k - k_lo) * 32 + lane];
 #pragma unroll
                 for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-                if (lane == 0 && want_g) g_last[bh * nchunks + k] = expf(csl[static_cast<size_t>(k) * kTile]) * v;
+                if (lane == 0) g_last[bh * nchunks + k] = expf(csl[static_cast<size_t>(k) * kTile]) * v;
             }
             if (k_lo > 0) __syncthreads();  // the partials are read before the next block overwrites them
         }
@@ -334,12 +374,7 @@ extern "C" int ssd_state_passing_fwd(const SsdShape* shape, float* states, const
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!states || !cs) return SSD_ERR_NULL;
-    const int pn4 = shape->headdim * shape->dstate / 4;
-    const size_t total = static_cast<size_t>(shape->batch) * shape->nheads * pn4;
-    const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    state_passing_fwd_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        states, cs, initial_state, final_state, shape->seqlen / kTile, pn4, shape->seqlen, total);
-    return launch_status();
+    return launch_state_walk<false>(*shape, states, cs, initial_state, final_state, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ssd_state_fold(const SsdShape* shape, const float* terms, const float* cs, const float* start,
@@ -362,8 +397,9 @@ extern "C" int ssd_state_passing_bwd(const SsdShape* shape, float* dstates, cons
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!dstates || !cs || (g_last && !states_start)) return SSD_ERR_NULL;
-    const unsigned blocks = static_cast<unsigned>(shape->batch) * shape->nheads;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (!g_last) return launch_state_walk<true>(*shape, dstates, cs, dfinal, d_initial, st);
+    const unsigned blocks = static_cast<unsigned>(shape->batch) * shape->nheads;
     const int nchunks = shape->seqlen / kTile;
     const size_t part_bytes = static_cast<size_t>(nchunks < kPartTiles ? nchunks : kPartTiles) * 32 * sizeof(float);
     const bool lng = nchunks > kPartTiles;
