@@ -37,7 +37,19 @@ enum {
     SSD_ERR_STATIC_SCRATCH = -8 /* problem too large for ssd_forward_static's built-in scratch */
 };
 
-enum { SSD_FLAG_DT_SOFTPLUS = 1u };
+enum {
+    SSD_FLAG_DT_SOFTPLUS = 1u,
+    /* The caller's tensors have their real extents, nothing is padded: `headdim` (a multiple of 4, up to 64) and `dstate` (a
+     * multiple of 4, up to 128) are theirs, and x, dt, B, C, out and their gradients hold `valid_len` tokens per
+     * sequence when valid_len is not 0 (then seqlen is valid_len rounded up to the tile).  Only the internal buffers are
+     * laid out for the kernels' own sizes: states [B,H,K,64,N'] with N' = 64 or 128, rows of `seqlen` tokens.  The tile
+     * loads fill with zeros what lies outside a tensor, and the stores leave it out.  With this flag the backward stages
+     * take dstate 128 as well; g_last then has two halves [2,B,H,K], one per 64 columns. */
+    SSD_FLAG_EXTENTS = 2u
+};
+/* With SSD_FLAG_EXTENTS: `parts` heads of 64 channels stand for one head of 64 * parts.  nheads counts the former; dt, A,
+ * dt_bias, D[H], ddt, dA, d(dt_bias) have nheads / parts heads. */
+#define SSD_FLAG_HEAD_PARTS(parts) ((uint32_t)((parts)-1) << 8)
 
 /* Problem shape.  `tile` is the number of tokens one CTA treats as a chunk
  * (the results do not depend on it mathematically); the kernels need
@@ -138,6 +150,11 @@ int ssd_state_passing_fwd(const SsdShape* shape, float* states, const float* cs,
 int ssd_chunk_scan_fwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
                        const float* states_start, const float* q, const float* cs, float* out, int* status,
                        ssd_stream_t stream);
+/* The same with the output written a second time to out_copy (null = not): for a caller that hands `out` on, to be modified in
+ * place, and needs the values for backward. */
+int ssd_chunk_scan_copy_fwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
+                            const float* states_start, const float* q, const float* cs, float* out, float* out_copy,
+                            int* status, ssd_stream_t stream);
 
 /* ---------------------------------------------------------------- backward stages (dstate == 64)
  *

@@ -14,6 +14,12 @@ LIB_NAME = "libssd_b200.so"
 
 SSD_OK = 0
 SSD_FLAG_DT_SOFTPLUS = 1
+SSD_FLAG_EXTENTS = 2
+
+
+def head_parts_flag(parts: int) -> int:
+    """SSD_FLAG_HEAD_PARTS of the header."""
+    return (parts - 1) << 8
 
 
 class SsdShape(ctypes.Structure):
@@ -69,6 +75,7 @@ SIGNATURES = {
     "ssd_chunk_state": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p, ctypes.c_int, _p, _p]),
     "ssd_state_passing_fwd": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p]),
     "ssd_chunk_scan_fwd": (ctypes.c_int, [_shape_p] + [_p] * 9),
+    "ssd_chunk_scan_copy_fwd": (ctypes.c_int, [_shape_p] + [_p] * 10),
     "ssd_state_passing_bwd": (ctypes.c_int, [_shape_p] + [_p] * 7),
     "ssd_chunk_state_scan_supported": (ctypes.c_int, [_shape_p]),
     "ssd_chunk_state_scan": (ctypes.c_int, [_shape_p] + [_p] * 7 + [ctypes.c_int, _p, _p]),

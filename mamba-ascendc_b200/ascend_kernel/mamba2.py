@@ -77,6 +77,18 @@ def make_shape(x: torch.Tensor, B: torch.Tensor, dt_softplus: bool,
                           float(dt_limit[0]), float(dt_limit[1]), int(valid_len))
 
 
+def extents_shape(x: torch.Tensor, B: torch.Tensor, heads: int, dt_softplus: bool,
+                  dt_limit: Tuple[float, float]) -> _capi.SsdShape:
+    """The shape of a call whose tensors keep their real extents (SSD_FLAG_EXTENTS): any length, headdim up to 64 or (as
+    ``x`` [B,L,heads * parts,64]) a multiple of 64, state size up to 128."""
+    b, l, h, p = x.shape
+    g, n = B.shape[2], B.shape[3]
+    tiles = (l + TILE - 1) // TILE
+    flags = (_capi.SSD_FLAG_EXTENTS | (_capi.SSD_FLAG_DT_SOFTPLUS if dt_softplus else 0) |
+             _capi.head_parts_flag(h // heads))
+    return _capi.SsdShape(b, tiles * TILE, h, p, n, TILE, g, flags, dt_limit[0], dt_limit[1], l if l % TILE else 0)
+
+
 # ----------------------------------------------------------------------------- validation
 def _check_tensor(t: torch.Tensor, name: str) -> None:
     # mamba_ascendc/csrc/ops/mamba2_ssd_fwd/op_host/mamba2_ssd_fwd.cpp:15-23
@@ -165,6 +177,11 @@ def _use_state_scan(shape: "_capi.SsdShape", device: torch.device) -> bool:
     return 2 * shape.batch * shape.ngroups >= 3 * sms
 
 
+def _state_cols(shape: "_capi.SsdShape") -> int:
+    """State columns of the internal buffers."""
+    return 64 if shape.dstate <= 64 else 128
+
+
 # ----------------------------------------------------------------------------- stage drivers
 # When set to a list, every stage launch is bracketed by CUDA events on the launching stream and
 # (name, start, end) is appended; used by bench.py to time individual kernels inside a step.
@@ -184,48 +201,52 @@ def _call(name: str, fn, *args) -> None:
 
 
 def forward_stages(x, dt, A, B, C, dt_softplus: bool, want_final: bool = True, initial_states=None, dt_bias=None,
-                   dt_limit=(0.0, float("inf")), valid_len: int = 0, inflow=None):
+                   dt_limit=(0.0, float("inf")), valid_len: int = 0, inflow=None, shape=None, copy=None):
     """Run the four forward stages; returns (out, final_state, q, cs, states_start).
 
     ``inflow(final0, log_decay) -> initial_states`` (sequence-parallel mode): called once the per-tile states
     exist, with the state this block of tokens would hand on from a zero start ([B,H,P,N]) and the logarithm
-    of its total decay ([B,H]); what it returns seeds the recurrence."""
-    shape = make_shape(x, B, dt_softplus, dt_limit, valid_len)
+    of its total decay ([B,H]); what it returns seeds the recurrence.
+
+    ``shape``: from ``extents_shape``; the default is the kernels' own sizes, whole tiles.  ``copy``: like ``out``, receives its
+    values as well."""
+    if shape is None:
+        shape = make_shape(x, B, dt_softplus, dt_limit, valid_len)
     _capi.check(_capi.lib.ssd_check_shape(ctypes.byref(shape)), "mamba2_ssd_fwd")
-    b, l, h, p = x.shape
-    n = B.shape[3]
+    b, l, h = shape.batch, shape.seqlen, shape.nheads
     k = l // TILE
     dev = x.device
     status = _status(dev)
     st = _stream()
     q = torch.empty(b, h, l, device=dev, dtype=torch.float32)
     cs = torch.empty_like(q)
-    states = torch.empty(b, h, k, p, n, device=dev, dtype=torch.float32)
+    states = torch.empty(b, h, k, 64, _state_cols(shape), device=dev, dtype=torch.float32)
     out = torch.empty_like(x)
-    final = torch.empty(b, h, p, n, device=dev, dtype=torch.float32) if want_final else None
+    final = torch.empty(b, h, shape.headdim, shape.dstate, device=dev, dtype=torch.float32) if want_final else None
     lib = _capi.lib
     sp = ctypes.byref(shape)
     _call("mamba2_ssd_dt_cumsum", lib.ssd_dt_cumsum, sp, _ptr(dt), _ptr(dt_bias), _ptr(A), _ptr(q), _ptr(cs), st)
     if inflow is None and _use_state_scan(shape, dev):
         _call("mamba2_ssd_chunk_state_scan", lib.ssd_chunk_state_scan, sp, _ptr(x), _ptr(B), _ptr(q), _ptr(cs),
               _ptr(initial_states), _ptr(states), _ptr(final), 0, _ptr(status), st)
-        _call("mamba2_ssd_chunk_scan", lib.ssd_chunk_scan_fwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(states), _ptr(q), _ptr(cs),
-              _ptr(out), _ptr(status), st)
+        _call("mamba2_ssd_chunk_scan", lib.ssd_chunk_scan_copy_fwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(states), _ptr(q),
+              _ptr(cs), _ptr(out), _ptr(copy), _ptr(status), st)
         return out, final, q, cs, states
     _call("mamba2_ssd_chunk_state", lib.ssd_chunk_state, sp, _ptr(x), _ptr(B), _ptr(q), _ptr(cs), _ptr(states), 0, _ptr(status), st)
     if inflow is not None:
-        final0 = torch.empty(b, h, p, n, device=dev, dtype=torch.float32)
+        final0 = torch.empty(b, h, shape.headdim, shape.dstate, device=dev, dtype=torch.float32)
         _call("mamba2_ssd_state_fold", lib.ssd_state_fold, sp, _ptr(states), _ptr(cs), None, _ptr(final0), 0, st)
         initial_states = inflow(final0, cs.view(b, h, k, TILE)[..., -1].sum(-1))
     _call("mamba2_ssd_state_passing", lib.ssd_state_passing_fwd, sp, _ptr(states), _ptr(cs), _ptr(initial_states),
           _ptr(final), st)
-    _call("mamba2_ssd_chunk_scan", lib.ssd_chunk_scan_fwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(states), _ptr(q), _ptr(cs), _ptr(out),
-                                       _ptr(status), st)
+    _call("mamba2_ssd_chunk_scan", lib.ssd_chunk_scan_copy_fwd, sp, _ptr(x), _ptr(B), _ptr(C), _ptr(states), _ptr(q), _ptr(cs),
+          _ptr(out), _ptr(copy), _ptr(status), st)
     return out, final, q, cs, states
 
 
 def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplus: bool, want_dinitial: bool = False,
-                    dt_bias=None, dt_limit=(0.0, float("inf")), valid_len: int = 0, outflow=None, D=None, ddt_bias=None):
+                    dt_bias=None, dt_limit=(0.0, float("inf")), valid_len: int = 0, outflow=None, D=None, ddt_bias=None,
+                    shape=None):
     """Run the backward stages; returns (dx, ddt, dA, dB, dC, d_initial_states or None).
 
     ``outflow(d_initial0) -> extra dfinal or None`` (sequence-parallel mode): called once the local state
@@ -236,17 +257,18 @@ def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplu
     output before skip and gate, and ``D * dout`` is added to dx by the dx kernel.
 
     ``ddt_bias`` [H]: receives the sum of ddt over batch and tokens."""
-    shape = make_shape(x, B, dt_softplus, dt_limit, valid_len)
-    b, l, h, p = x.shape
-    n = B.shape[3]
+    if shape is None:
+        shape = make_shape(x, B, dt_softplus, dt_limit, valid_len)
+    b, l, h, p, n = shape.batch, shape.seqlen, shape.nheads, shape.headdim, shape.dstate
     k = l // TILE
     dev = x.device
     status = _status(dev)
     st = _stream()
     lib = _capi.lib
     sp = ctypes.byref(shape)
-    dstates = torch.empty(b, h, k, p, n, device=dev, dtype=torch.float32)
-    g_last = torch.empty(b, h, k, device=dev, dtype=torch.float32)
+    n_state = _state_cols(shape)
+    dstates = torch.empty(b, h, k, 64, n_state, device=dev, dtype=torch.float32)
+    g_last = torch.empty(n_state // 64, b, h, k, device=dev, dtype=torch.float32)
     ddt_t = torch.empty(b, h, l, device=dev, dtype=torch.float32)
     dA_part = torch.empty(b, h, k, device=dev, dtype=torch.float64)
     dx = torch.empty_like(x)
@@ -284,11 +306,102 @@ def backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal, dt_softplu
     return dx, ddt, dA, dB, dC, d_initial
 
 
+# ----------------------------------------------------------------------------- D skip and z gate
+def _d_mode(D: Optional[torch.Tensor]) -> int:
+    return 0 if D is None else D.dim()  # 1: [H], 2: [H,P]
+
+
+def _gate_shape(x, heads: Optional[int]) -> "_capi.SsdShape":
+    b, l, h, p = x.shape
+    heads = heads or h  # of D; x may hold several heads of 64 channels for each
+    return _capi.SsdShape(b, l, heads, p * (h // heads), 64, TILE, 1, 0, 0.0, 0.0, 0)
+
+
+def gate_forward(y, x, B, D, z, heads: Optional[int] = None):
+    """out = (y + D .* x) .* silu(z) in one pass (ssd_gate_skip_fwd)."""
+    shape = _gate_shape(x, heads)
+    out = torch.empty_like(y)
+    _call("mamba2_ssd_gate", _capi.lib.ssd_gate_skip_fwd, ctypes.byref(shape), _ptr(y), _ptr(x), _ptr(D), _d_mode(D),
+          _ptr(z), _ptr(out), _stream())
+    return out
+
+
+def gate_backward(dout, y, x, B, D, z, heads: Optional[int] = None):
+    """(dy, dz, dD) of the gate / skip epilogue in one pass; without z, dy is dout itself."""
+    shape = _gate_shape(x, heads)
+    sp = ctypes.byref(shape)
+    dy = torch.empty_like(dout) if z is not None else dout
+    dz = torch.empty_like(dout) if z is not None else None
+    dD = part = None
+    if D is not None:
+        dD = torch.empty_like(D)
+        part = torch.empty(_capi.lib.ssd_gate_partial_floats(sp), device=dout.device, dtype=torch.float32)
+    _call("mamba2_ssd_bwd_gate", _capi.lib.ssd_gate_skip_bwd, sp, _ptr(dout), _ptr(y), _ptr(x), _ptr(D), _d_mode(D),
+          _ptr(z), _ptr(dy) if z is not None else None, _ptr(dz), _ptr(part), _ptr(dD), _stream())
+    return dy, dz, dD
+
+
 # ----------------------------------------------------------------------------- autograd
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous fp32 at an address the tile loads take (a gradient may be a slice of a larger one)."""
+    t = t.contiguous().float()
+    return t.clone() if t.data_ptr() & 15 else t
+
+
 class _Mamba2SsdAutograd(torch.autograd.Function):
-    """Counterpart of ``_Mamba2SsdAutogradM1`` (mamba2.py:1661-1838): saves the inputs plus, under the
-    default policy, q, cs, the tile-start states and the output; backward returns gradients for x, dt, A, B, C, the initial states and
-    dt_bias, and None for the non-tensor arguments."""
+    """Counterpart of ``_Mamba2SsdAutogradM1`` (mamba2.py:1661-1838), with the D skip connection and the z gate inside the node:
+    the epilogue runs as one fused pass forward and one backward (the reference fuses them into its state-epilogue and
+    gate kernels, mamba2_ssd_state_epilogue.cpp:413-482, bwd_gate/design.md:8-13), and the skip connection's share of dx
+    is added in the epilogue of the dx kernel.  Saves the inputs plus, under the default policy, q, cs, the tile-start states and
+    the SSD output before the epilogue.  ``x`` is [B,L,H * parts,64] for a headdim of 64 * parts."""
+
+    @staticmethod
+    def forward(ctx, x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, dt_min, dt_max):
+        ctx.shape = extents_shape(x, B, A.shape[0], dt_softplus, (dt_min, dt_max))
+        ctx.gated = D is not None or z is not None
+        ctx.recompute = _save_policy == "recompute"
+        # Without an epilogue the output is what backward needs.  At the kernels' own sizes it is saved itself, so that
+        # changing it in place is an error in backward; elsewhere the caller may change it, and a copy is saved.
+        own_sizes = x.shape[3] == 64 and B.shape[3] == 64 and x.shape[1] % TILE == 0 and x.shape[2] == A.shape[0]
+        copy = None if ctx.gated or ctx.recompute or own_sizes else torch.empty_like(x)
+        y, final, q, cs, states = forward_stages(x, dt, A, B, C, dt_softplus, want_final=True, initial_states=initial_states,
+                                                 dt_bias=dt_bias, shape=ctx.shape, copy=copy)
+        out = gate_forward(y, x, B, D, z, A.shape[0]) if ctx.gated else y
+        if ctx.recompute:  # inputs only; y, q, cs and the tile-start states are rebuilt in backward
+            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, initial_states)
+        else:
+            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, y if copy is None else copy, q, cs, states)
+        ctx.dt_softplus = dt_softplus
+        ctx.has_initial = initial_states is not None
+        return out, final
+
+    @staticmethod
+    def backward(ctx, dout, dfinal):
+        if ctx.recompute:
+            x, dt, A, B, C, dt_bias, D, z, initial_states = ctx.saved_tensors
+        else:
+            x, dt, A, B, C, dt_bias, D, z, y, q, cs, states = ctx.saved_tensors
+        if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
+            dout = torch.zeros_like(x)
+        dout = _aligned(dout)
+        if dfinal is not None:
+            dfinal = _aligned(dfinal)
+        with _device_guard(x.device):
+            if ctx.recompute:
+                y, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
+                                                     initial_states=initial_states, dt_bias=dt_bias, shape=ctx.shape)
+            dy, dz, dD = gate_backward(dout, y, x, B, D, z, A.shape[0]) if ctx.gated else (dout, None, None)
+            if not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9)):  # D and z alone
+                return None, None, None, None, None, dD, dz, None, None, None, None, None
+            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
+            dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, y, q, cs, states, dy, dfinal, ctx.dt_softplus,
+                                                         want_dinitial=ctx.has_initial, dt_bias=dt_bias, D=D,
+                                                         ddt_bias=dbias, shape=ctx.shape)
+        return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
+
+
+class _Mamba2SsdPadded(torch.autograd.Function):
+    """The plain SSD node on the kernels' own sizes, for the calls that ``shapes.run_general`` pads or cuts into blocks."""
 
     @staticmethod
     def forward(ctx, x, dt, A, B, C, dt_softplus, initial_states, dt_bias, dt_min, dt_max, valid_len):
@@ -297,7 +410,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
                                                    dt_limit=(dt_min, dt_max), valid_len=valid_len)
         ctx.valid_len = valid_len
         ctx.recompute = _save_policy == "recompute"
-        if ctx.recompute:  # inputs only; out, q, cs and the tile-start states are rebuilt in backward
+        if ctx.recompute:
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, initial_states)
         else:
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, out, q, cs, states)
@@ -312,7 +425,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
             x, dt, A, B, C, dt_bias, initial_states = ctx.saved_tensors
         else:
             x, dt, A, B, C, dt_bias, out, q, cs, states = ctx.saved_tensors
-        if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
+        if dout is None:
             dout = torch.zeros_like(x)
         dout = dout.contiguous().float()
         if dfinal is not None:
@@ -322,88 +435,12 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
                 out, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
                                                        initial_states=initial_states, dt_bias=dt_bias,
                                                        dt_limit=ctx.dt_limit, valid_len=ctx.valid_len)
-            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
+            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None
             dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, out, q, cs, states, dout, dfinal,
                                                          ctx.dt_softplus, want_dinitial=ctx.has_initial,
                                                          dt_bias=dt_bias, dt_limit=ctx.dt_limit,
                                                          valid_len=ctx.valid_len, ddt_bias=dbias)
         return dx, ddt, dA, dB, dC, None, dinit, dbias, None, None, None
-
-
-# ----------------------------------------------------------------------------- D skip and z gate
-def _d_mode(D: Optional[torch.Tensor]) -> int:
-    return 0 if D is None else D.dim()  # 1: [H], 2: [H,P]
-
-
-def gate_forward(y, x, B, D, z):
-    """out = (y + D .* x) .* silu(z) in one pass (ssd_gate_skip_fwd)."""
-    shape = make_shape(x, B, False)
-    out = torch.empty_like(y)
-    _call("mamba2_ssd_gate", _capi.lib.ssd_gate_skip_fwd, ctypes.byref(shape), _ptr(y), _ptr(x), _ptr(D), _d_mode(D),
-          _ptr(z), _ptr(out), _stream())
-    return out
-
-
-def gate_backward(dout, y, x, B, D, z):
-    """(dy, dz, dD) of the gate / skip epilogue in one pass; without z, dy is dout itself."""
-    shape = make_shape(x, B, False)
-    sp = ctypes.byref(shape)
-    dy = torch.empty_like(dout) if z is not None else dout
-    dz = torch.empty_like(dout) if z is not None else None
-    dD = part = None
-    if D is not None:
-        dD = torch.empty_like(D)
-        part = torch.empty(_capi.lib.ssd_gate_partial_floats(sp), device=dout.device, dtype=torch.float32)
-    _call("mamba2_ssd_bwd_gate", _capi.lib.ssd_gate_skip_bwd, sp, _ptr(dout), _ptr(y), _ptr(x), _ptr(D), _d_mode(D),
-          _ptr(z), _ptr(dy) if z is not None else None, _ptr(dz), _ptr(part), _ptr(dD), _stream())
-    return dy, dz, dD
-
-
-class _Mamba2SsdGatedAutograd(torch.autograd.Function):
-    """The SSD with its D skip connection and z gate as one autograd node: the epilogue runs as one fused pass
-    forward and one backward (the reference fuses them into its state-epilogue and gate kernels,
-    mamba2_ssd_state_epilogue.cpp:413-482, bwd_gate/design.md:8-13), and the skip connection's share of dx is
-    added in the epilogue of the dx kernel."""
-
-    @staticmethod
-    def forward(ctx, x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, dt_min, dt_max):
-        y, final, q, cs, states = forward_stages(x, dt, A, B, C, dt_softplus, want_final=True,
-                                                 initial_states=initial_states, dt_bias=dt_bias,
-                                                 dt_limit=(dt_min, dt_max))
-        out = gate_forward(y, x, B, D, z)
-        ctx.recompute = _save_policy == "recompute"
-        if ctx.recompute:
-            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, initial_states)
-        else:
-            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, y, q, cs, states)
-        ctx.dt_softplus = dt_softplus
-        ctx.has_initial = initial_states is not None
-        ctx.dt_limit = (dt_min, dt_max)
-        return out, final
-
-    @staticmethod
-    def backward(ctx, dout, dfinal):
-        if ctx.recompute:
-            x, dt, A, B, C, dt_bias, D, z, initial_states = ctx.saved_tensors
-        else:
-            x, dt, A, B, C, dt_bias, D, z, y, q, cs, states = ctx.saved_tensors
-        if dout is None:
-            dout = torch.zeros_like(x)
-        dout = dout.contiguous().float()
-        if dfinal is not None:
-            dfinal = dfinal.contiguous().float()
-        with _device_guard(x.device):
-            if ctx.recompute:
-                y, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
-                                                     initial_states=initial_states, dt_bias=dt_bias,
-                                                     dt_limit=ctx.dt_limit)
-            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None
-            dy, dz, dD = gate_backward(dout, y, x, B, D, z)
-            dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, y, q, cs, states, dy, dfinal,
-                                                         ctx.dt_softplus, want_dinitial=ctx.has_initial,
-                                                         dt_bias=dt_bias, dt_limit=ctx.dt_limit, D=D,
-                                                         ddt_bias=dbias)
-        return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
 
 
 # What the autograd function keeps between forward and backward (mamba2_ssd_bwd/design.md:207-223 lists the
@@ -472,6 +509,43 @@ def _short_sequence(x, B, C, D, z, initial_states) -> bool:
     return not any(t is not None and t.data_ptr() & 15 for t in (B, C, initial_states))
 
 
+def _tile_extents(x, B, C, D, z, initial_states) -> bool:
+    """Whether the tile kernels read and write the caller's tensors as they are: their tile loads and stores cut a tile off
+    at the end of a sequence, of a head's channels and of the state's columns, in steps of four floats from 16-byte
+    aligned addresses.  What this leaves (other headdims and state sizes) is padded or cut into blocks by shapes.py."""
+    p, n = x.shape[3], B.shape[3]
+    if min(x.shape) <= 0 or min(B.shape) <= 0 or n % 4 or n > 128 or p > 1024 or (p % 64 if p > 64 else p % 4):
+        return False
+    if torch.autograd.forward_ad._current_level >= 0 and (p != 64 or x.shape[1] % TILE):
+        return False  # tangents of D and z come from the framework's operations
+    if p == 64 and x.shape[1] % TILE == 0 and n in (64, 128):
+        return True  # the kernels' own sizes: nothing to fall back to
+    return not any(t is not None and t.data_ptr() & 15 for t in (x, B, C, D, z, initial_states))
+
+
+def _tile_call(x, dt, A, B, C, D, z, dt_bias, dt_softplus, lim, initial_states, return_final_state, grad):
+    b, l, h, p = x.shape
+    parts = p // 64 if p > 64 else 1
+    if parts > 1:  # a head of 64 * parts channels is that many heads of 64 that share dt, A and the group
+        x = x.view(b, l, h * parts, 64)
+        z = z.view(x.shape) if z is not None else None
+        D = D.view(h * parts, 64) if D is not None and D.dim() == 2 else D
+        if initial_states is not None:
+            initial_states = initial_states.view(b, h * parts, 64, -1)
+    if grad:
+        out, final = _Mamba2SsdAutograd.apply(x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, lim[0], lim[1])
+    else:
+        out, final, *_ = forward_stages(x, dt, A, B, C, dt_softplus, want_final=return_final_state,
+                                        initial_states=initial_states, dt_bias=dt_bias,
+                                        shape=extents_shape(x, B, h, dt_softplus, lim))
+        if D is not None or z is not None:
+            out = gate_forward(out, x, B, D, z, h)
+    if parts > 1:
+        out = out.view(b, l, h, p)
+        final = final.view(b, h, p, -1) if final is not None else None
+    return (out, final) if return_final_state else out
+
+
 def recurrent_forward(x, dt, A, B, C, dt_softplus: bool, want_final: bool, initial_states, dt_bias, dt_limit, D, z):
     b, l, h, p = x.shape
     g, n = B.shape[2], B.shape[3]
@@ -515,33 +589,22 @@ def mamba2_ssd_fwd(
     def core(xk, dtk, Ak, Bk, Ck, init, bias, valid):
         # the fixed-shape call: headdim 64, state size 64 (128 without gradients), whole tiles
         if needs_grad:
-            return _Mamba2SsdAutograd.apply(xk, dtk, Ak, Bk, Ck, bool(dt_softplus), init, bias, lim[0], lim[1], valid)
+            return _Mamba2SsdPadded.apply(xk, dtk, Ak, Bk, Ck, bool(dt_softplus), init, bias, lim[0], lim[1], valid)
         out_k, final_k, *_ = forward_stages(xk, dtk, Ak, Bk, Ck, bool(dt_softplus), want_final=return_final_state,
                                             initial_states=init, dt_bias=bias, dt_limit=lim, valid_len=valid)
         return out_k, final_k
 
     with _device_guard(x.device):
-        if not _requires_grad(x, dt, A, B, C, D, z, initial_states, dt_bias) and _short_sequence(x, B, C, D, z, initial_states):
+        grad_anywhere = needs_grad or _requires_grad(D, z)
+        if not grad_anywhere and _short_sequence(x, B, C, D, z, initial_states):
             out, final = recurrent_forward(x, dt, A, B, C, bool(dt_softplus), return_final_state, initial_states, dt_bias,
                                            lim, D, z)
             return (out, final) if return_final_state else out
-        p, n = x.shape[3], B.shape[3]
-        native = p == 64 and x.shape[1] % TILE == 0
-        if native and n == 64 and (D is not None or z is not None) and _requires_grad(
-                x, dt, A, B, C, initial_states, dt_bias, D, z):
-            # the kernels' own shapes with a D skip or z gate under autograd: one node, fused epilogue
-            out, final = _Mamba2SsdGatedAutograd.apply(x, dt, A, B, C, D, z, bool(dt_softplus), initial_states,
-                                                       dt_bias, lim[0], lim[1])
-            return (out, final) if return_final_state else out
-        if native and (n == 64 or (n == 128 and not needs_grad)):
-            out, final = core(x, dt, A, B, C, initial_states, dt_bias, 0)  # the kernels' own shapes
-            if not _requires_grad(D, z, out):
-                if D is not None or z is not None:  # no gradients anywhere: the fused epilogue pass
-                    out = gate_forward(out, x, B, D, z)
-                return (out, final) if return_final_state else out
-        else:
-            # any sequence length, headdim and state size: see shapes.py
-            out, final = run_general(core, x, dt, A, B, C, initial_states, dt_bias, needs_grad)
+        if _tile_extents(x, B, C, D, z, initial_states):
+            return _tile_call(x, dt, A, B, C, D, z, dt_bias, bool(dt_softplus), lim, initial_states, return_final_state,
+                              grad_anywhere)
+        # any other headdim and state size, unaligned addresses: see shapes.py
+        out, final = run_general(core, x, dt, A, B, C, initial_states, dt_bias, needs_grad)
         # D skip connection and z gate (ssd_reference.py:300-318) as element-wise epilogue; under autograd
         # their gradients (dD, dz and the extra term of dx) come from these same operations
         if D is not None:

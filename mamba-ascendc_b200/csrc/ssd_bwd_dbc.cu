@@ -66,7 +66,7 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_du,
                const __grid_constant__ CUtensorMap map_db, const __grid_constant__ CUtensorMap map_dc,
                const float* __restrict__ q, const float* __restrict__ cs, float* __restrict__ g_last, SsdShape s,
-               int split, int* status) {
+               int split, int blocks, int* status) {
     using L = BwdDbcSmem;
     constexpr int N = L::N;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -88,8 +88,11 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int groups = s.ngroups * split;  // of work items; `split` of them share a group and leave a partial sum each
-    const int heads_per_group = s.nheads / groups;
+    // groups of work items: `split` of them share a group and leave a partial sum each; with state size 128 every one of
+    // these is two work items, one per block of 64 columns (dB, dC and the state terms are separate by columns, D0 is not
+    // and is formed for both)
+    const int groups = s.ngroups * split * blocks;
+    const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
     // Work list of this CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the (batch, group, token
     // tile) grid, token tile fastest; the heads of all its tiles form one flat sequence of iterations,
@@ -98,7 +101,7 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     const int my_tiles = (num_tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
                          static_cast<int>(gridDim.x);
     const int total = my_tiles * heads_per_group;
-    const TileWalk walk(s, static_cast<int>(gridDim.x), split);
+    const TileWalk walk(s, static_cast<int>(gridDim.x), split, blocks);
     using Where = HeadPos;
     auto first_tile = [&]() { return walk.first(static_cast<int>(blockIdx.x)); };
     auto advance = [&](TilePos& t) { walk.advance(t); };
@@ -191,38 +194,39 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 uint8_t* r = smem + (it & 1) * L::kRegion;
                 uint64_t* bar = &full_gx[it & 1];
                 mbar_arrive_expect_tx(bar, 2 * L::kPTile);
-                tma_tile_3d(r + L::kG, kTile, &map_dout, bar, 0, w.h, w.tok0, false);
-                tma_tile_3d(r + L::kX, kTile, &map_x, bar, 0, w.h, w.tok0, false);
+                tma_tile_tokens(r + L::kG, &map_dout, bar, 0, w.h, w.tok, w.b, false);
+                tma_tile_tokens(r + L::kX, &map_x, bar, 0, w.h, w.tok, w.b, false);
             };
             auto load_su = [&](const Where& w) {
                 mbar_arrive_expect_tx(full_su, 2 * L::kSTile);
-                tma_tile_2d(smem + L::kS, 64, &map_s, full_su, 0, w.tile_index * 64, false);
-                tma_tile_2d(smem + L::kU, 64, &map_du, full_su, 0, w.tile_index * 64, false);
+                const int col0 = 64 * walk.column_block(w.g);
+                tma_tile_2d(smem + L::kS, 64, &map_s, full_su, col0, w.tile_index * 64, false);
+                tma_tile_2d(smem + L::kU, 64, &map_du, full_su, col0, w.tile_index * 64, false);
             };
-            auto load_bc = [&](int item_group, int tok0) {
-                const int g = walk.group_of(item_group);
+            auto load_bc = [&](const Where& w) {
+                const int g = walk.group_of(w.g), col0 = 64 * walk.column_block(w.g);
                 mbar_arrive_expect_tx(full_bc, 2 * L::kPTile);
-                tma_tile_3d(smem + L::kB, kTile, &map_b, full_bc, 0, g, tok0, false);
-                tma_tile_3d(smem + L::kC, kTile, &map_c, full_bc, 0, g, tok0, false);
+                tma_tile_tokens(smem + L::kB, &map_b, full_bc, col0, g, w.tok, w.b, false);
+                tma_tile_tokens(smem + L::kC, &map_c, full_bc, col0, g, w.tok, w.b, false);
             };
-            // Finished tile of (work item) group g at token tok0, staged by the compute warps in the region of the tile's
+            // Finished tile of a work item, staged by the compute warps in the region of the tile's
             // last head, iteration `j` (named barrier 4 says so).
-            auto store_tile = [&](int j, int g, int tok0) {
+            auto store_tile = [&](int j, const TilePos& at) {
                 asm volatile("bar.sync 4, 544;" ::: "memory");
                 if (lane == 0 && *reinterpret_cast<volatile int*>(status) == 0) {
                     const uint8_t* stage = smem + (j & 1) * L::kRegion;
-                    tma_store_3d(&map_dc, stage, 0, g, tok0);
-                    tma_store_3d(&map_dc, stage + kSlabBytes, 32, g, tok0);
-                    tma_store_3d(&map_db, stage + 2 * kSlabBytes, 0, g, tok0);
-                    tma_store_3d(&map_db, stage + 3 * kSlabBytes, 32, g, tok0);
+                    const int g = at.g >> walk.block_bits, col0 = 64 * walk.column_block(at.g);
+                    tma_store_tokens(&map_dc, stage, col0, g, at.k * kTile, at.b, s.dstate);
+                    tma_store_tokens(&map_db, stage + 2 * kSlabBytes, col0, g, at.k * kTile, at.b, s.dstate);
                     tma_store_commit();
                 }
             };
             TilePos cur = first_tile();
-            int hi = 0, prev_g = 0, prev_tok0 = 0;
+            TilePos prev = cur;
+            int hi = 0;
             if (lane == 0) {
                 const Where w0 = locate(cur, 0, 0);
-                load_bc(w0.g, w0.tok0);
+                load_bc(w0);
                 load_gx(0, w0);
                 load_su(w0);
                 if (total > 1) load_gx(1, locate(cur, 0, 1));
@@ -237,8 +241,8 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     mbar_wait(bar_g2, p_g2, status, kStatusMmaTimeout | wait_site(5, 11));
                     p_g2 ^= 1;
                     tc_fence_after_sync();
-                    if (lane == 0) load_bc(w0.g, w0.tok0);
-                    store_tile(it - 1, prev_g, prev_tok0);
+                    if (lane == 0) load_bc(w0);
+                    store_tile(it - 1, prev);
                     if (lane == 0 && it + 1 < total) {  // the next head's dout / x tiles, once the store has read
                         tma_store_wait_read();
                         load_gx(it + 1, w1);
@@ -256,13 +260,12 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                 }
                 if (++hi == heads_per_group) {
                     hi = 0;
-                    prev_g = cur.g;
-                    prev_tok0 = cur.b * s.seqlen + cur.k * kTile;
+                    prev = cur;
                     advance(cur);
                 }
             }
             if (total > 0) {
-                store_tile(total - 1, prev_g, prev_tok0);
+                store_tile(total - 1, prev);
                 if (lane == 0) tma_store_wait_all();
             }
         }
@@ -287,7 +290,8 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     set[32 * j + lane] = c[j];
                     set[kTile + 32 * j + lane] = qv[j];
                 }
-                if (lane == 0) set[2 * kTile] = __int_as_float(w.tile_index);
+                if (lane == 0)  // where g_last of this head goes (one half of it per column block)
+                    set[2 * kTile] = __int_as_float(w.tile_index + walk.column_block(w.g) * (s.batch * s.nheads * nchunks));
                 mbar_arrive(&rows_ready[it & 1]);
             };
             for (int it = 0; it < 2 && it < total; ++it) {
@@ -606,7 +610,7 @@ dbc_sum_kernel(const float* __restrict__ partial, float* __restrict__ dB, float*
 extern "C" int ssd_dbc_split(const SsdShape* shape) {
     using namespace ssd;
     if (ssd_check_shape(shape) != SSD_OK) return 1;
-    const int64_t items = static_cast<int64_t>(shape->seqlen / kTile) * shape->ngroups * shape->batch;
+    const int64_t items = static_cast<int64_t>(shape->seqlen / kTile) * shape->ngroups * shape->batch * (state_cols(*shape) / 64);
     return choose_head_split(items, shape->nheads / shape->ngroups, sm_count(), 1, 5);
 }
 
@@ -628,37 +632,36 @@ extern "C" int ssd_chunk_dbc_split_bwd(const SsdShape* shape, const float* x, co
     if (!x || !bm || !cm || !dout || !states_start || !dstates || !q || !cs || !dB || !dC || !status)
         return SSD_ERR_NULL;
     const SsdShape& s = *shape;
-    if (s.dstate != 64) return SSD_ERR_UNSUPPORTED;
+    if (s.dstate != 64 && !has_extents(s)) return SSD_ERR_UNSUPPORTED;
     if (split < 1 || (s.nheads / s.ngroups) % split != 0) return SSD_ERR_SHAPE;
     if (split > 1 && !partial) return SSD_ERR_NULL;
     if ((reinterpret_cast<uintptr_t>(partial) & 15u) != 0) return SSD_ERR_ALIGN;
     const int groups = s.ngroups * split;
-    const size_t elems = static_cast<size_t>(s.batch) * s.seqlen * s.ngroups * s.dstate;  // of dB, and of dC
+    const size_t elems = static_cast<size_t>(s.batch) * row_tokens(s) * s.ngroups * s.dstate;  // of dB, and of dC
     float* out_db = split > 1 ? partial : dB;
     float* out_dc = split > 1 ? partial + elems * split : dC;
     CUtensorMap map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc;
-    const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
-    int rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_b, bm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dout, dout, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_db, out_db, tokens, groups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dc, out_dc, tokens, groups, s.dstate, kTile);
-    const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
-    if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_s, states_start, state_rows, s.dstate, 64);
-    if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_du, dstates, state_rows, s.dstate, 64);
+    int rc = make_tmap_f32_tokens(&map_x, x, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_b, bm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dout, dout, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_db, out_db, s, groups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dc, out_dc, s, groups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_s, states_start, s);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_du, dstates, s);
     if (rc != SSD_OK) return rc;
     const size_t smem = BwdDbcSmem::kTotal;
     static std::atomic<uint64_t> smem_set{0};
     rc = set_max_smem_once(reinterpret_cast<const void*>(bwd_dbc_kernel), smem, smem_set);
     if (rc != SSD_OK) return rc;
-    const int64_t tiles = static_cast<int64_t>(s.seqlen / kTile) * groups * s.batch;
+    const int blocks = state_cols(s) / 64;
+    const int64_t tiles = static_cast<int64_t>(s.seqlen / kTile) * groups * blocks * s.batch;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
     if (tiles * split > 0x7fffffff) return SSD_ERR_RANGE;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
     bwd_dbc_kernel<<<grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, status);
+        map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, blocks, status);
     rc = launch_status();
     if (rc != SSD_OK || split == 1) return rc;
     const size_t quads = 2 * elems / 4;

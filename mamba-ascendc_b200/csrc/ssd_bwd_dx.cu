@@ -28,11 +28,13 @@ namespace ssd {
 
 namespace {
 
-// dstate N = 64 only
+// With state size 128 the second 64 columns of B and C arrive where the first dout tile and the first output tile go
+// once CB^T exists (kG0 and kO), dU is two tiles, and B fills the tensor memory that is left.
+template <int N>
 struct BwdDxSmem {
-    static constexpr int N = 64;
     static constexpr uint32_t kPTile = kTile * 128 * 2;  // [128 x 64] hi + lo (= the fp32 tile)
-    static constexpr uint32_t kUTile = 64 * 128 * 2;     // dU [64 x 64] hi + lo
+    static constexpr uint32_t kUBlock = 64 * 128 * 2;    // 64 columns of dU [64 x 64], hi + lo
+    static constexpr uint32_t kUTile = kUBlock * (N / 64);
     static constexpr uint32_t kB = 0;               // fp32 B as it landed (it goes to tensor memory), then the x tiles
     static constexpr uint32_t kG0 = kB + kPTile;    // dout of even heads, then their fp32 dx slabs
     static constexpr uint32_t kG1 = kG0 + kPTile;   // C (for CB only), then dout / dx of odd heads
@@ -46,13 +48,13 @@ struct BwdDxSmem {
     static constexpr uint32_t kBars = kRows + kRowFloats * 4;
     static constexpr uint32_t kTotal = kBars + 128;
 };
-static_assert(BwdDxSmem::kTotal + 1024 <= 232448, "dx kernel exceeds the shared memory of one SM");
-static_assert((BwdDxSmem::kRows + (2 * BwdDxSmem::kRowSet + 24 * kTile) * 4) % 8 == 0, "double scratch alignment");
+static_assert(BwdDxSmem<128>::kTotal + 1024 <= 232448, "dx kernel exceeds the shared memory of one SM");
+static_assert((BwdDxSmem<64>::kRows + (2 * BwdDxSmem<64>::kRowSet + 24 * kTile) * 4) % 8 == 0, "double scratch alignment");
 
 // SKIP: the D skip connection's share of dx, D .* dy, is added in the epilogue (dy is what this kernel is
 // given as dout; the thread reads its 16 values again from global memory, where the tile load of a moment
 // ago has left them in L2).  d_mode 1: D[H], 2: D[H,P].
-template <bool SKIP>
+template <int N, bool SKIP>
 __global__ void __launch_bounds__(kLaunchThreadsGroups, 1)
 bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
               const __grid_constant__ CUtensorMap map_dout, const __grid_constant__ CUtensorMap map_out,
@@ -61,8 +63,8 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
               const float* __restrict__ dt, const float* __restrict__ dt_bias, const float* __restrict__ A,
               const float* __restrict__ g_last, float* __restrict__ ddt_t, double* __restrict__ dA_part,
               const float* __restrict__ dy_raw, const float* __restrict__ dskip, int d_mode, SsdShape s, int split, int* status) {
-    using L = BwdDxSmem;
-    constexpr int N = L::N;
+    using L = BwdDxSmem<N>;
+    constexpr int kBlocks = N / 64;  // of 64 state columns
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     float* rows = reinterpret_cast<float*>(smem + L::kRows);
@@ -89,7 +91,8 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
     const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
-    const int tok0 = b * s.seqlen + k * kTile;
+    const int tok = k * kTile, tokens = row_tokens(s);
+    const int parts = head_parts(s);
     const int h_first = blockIdx.y * heads_per_group;
     const bool softplus = (s.flags & SSD_FLAG_DT_SOFTPLUS) != 0;
 
@@ -114,9 +117,10 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
         return;
     }
     // CB^T [128], D1 [64], D2 [64]; A operands (row in lane, two bf16 contraction elements per column):
-    // B hi [32] | lo [32] for CB^T and D2, W^T hi [64] | lo [64] for D1
-    const uint32_t tm_cb = tmem, tm_d1 = tmem + 128, tm_d2 = tmem + 192, tm_bhi = tmem + 256, tm_blo = tmem + 288;
-    const uint32_t tm_whi = tmem + 320, tm_wlo = tmem + 384;
+    // B hi [N/2] | lo [N/2] for CB^T and D2, W^T hi [64] | lo [64] for D1
+    const uint32_t tm_cb = tmem, tm_d1 = tmem + 128, tm_d2 = tmem + 192, tm_bhi = tmem + 256, tm_blo = tm_bhi + N / 2;
+    const uint32_t tm_whi = tmem + 256 + N, tm_wlo = tm_whi + 64;
+    static_assert(256 + N + 128 <= 512, "tensor memory columns");
     bool ok = true;
     constexpr uint32_t kHalf = kTile * 128;  // hi -> lo distance of a [128 x 64] tile
 
@@ -124,8 +128,10 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     if (warp >= kThreads / 32) {
         reg_release<kIssuerRegs>();  // this warp group hands most of its registers to the computing groups
         if (warp == kThreads / 32 && lane == 0) {
-            const Operand c{smem_u32(smem + L::kG1), smem_u32(smem + L::kG1) + kHalf, kTile, false};
-            const Operand du{smem_u32(smem + L::kU), smem_u32(smem + L::kU) + 64 * 128, 64, false};
+            // the column blocks of C are neighbours (kG1, kO), as are those of dU
+            const Operand c{smem_u32(smem + L::kG1), smem_u32(smem + L::kG1) + kHalf, kTile, false, L::kPTile};
+            const Operand du{smem_u32(smem + L::kU), smem_u32(smem + L::kU) + 64 * 128, 64, false, L::kUBlock};
+            static_assert(L::kO == L::kG1 + L::kPTile, "the second column block of C");
             mbar_wait(bar_rcb, 0, status, kStatusMmaTimeout | wait_site(4, 1));
             tc_fence_after_sync();
             issue_gemm_split_ta<N / 16>(tm_cb, tm_bhi, tm_blo, c, 0, make_idesc_bf16(128, 128, false, false), false);
@@ -144,7 +150,7 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
                 tc_fence_after_sync();
                 // every warp has consumed the forward-output tile of this head: the next head's may land
                 if (hi + 1 < heads_per_group)
-                    tma_tile_3d(smem + L::kO, kTile, &map_out, full_o, 0, h_first + hi + 1, tok0);
+                    tma_tile_tokens(smem + L::kO, &map_out, full_o, 0, h_first + hi + 1, tok, b);
                 issue_gemm_split_ta<kTile / 16>(tm_d1, tm_whi, tm_wlo, gy, 0, make_idesc_bf16(128, 64, false, true), false);
                 umma_commit(bar_d1);
             }
@@ -156,12 +162,28 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     // ---- loads.  One thread issues them; each lands in its operand tile's own memory.
     auto srow_of = [&](int h) { return ((b * s.nheads + h) * nchunks + k) * 64; };
     auto g_tile = [&](int hi) { return smem + ((hi & 1) ? L::kG1 : L::kG0); };
+    auto load_u = [&](int h) {
+        mbar_arrive_expect_tx(full_u, L::kUTile);
+        for (int cb = 0; cb < kBlocks; ++cb)
+            tma_tile_2d(smem + L::kU + cb * L::kUBlock, 64, &map_du, full_u, 64 * cb, srow_of(h), false);
+    };
+    auto split_u = [&]() {  // warps 0-7 the first 64 columns, warps 8-15 the others
+        split_tile_inplace(smem + L::kU, 64, nullptr, warp, lane);
+        if (kBlocks == 2 && warp >= 8) split_tile_inplace(smem + L::kU + L::kUBlock, 64, nullptr, warp - 8, lane);
+    };
     if (tid == 0) {
-        tma_tile_3d(smem + L::kB, kTile, &map_b, full_b, 0, g, tok0);
-        tma_tile_3d(smem + L::kG1, kTile, &map_c, &full_g[1], 0, g, tok0);
-        tma_tile_3d(smem + L::kG0, kTile, &map_dout, &full_g[0], 0, h_first, tok0);
-        tma_tile_3d(smem + L::kO, kTile, &map_out, full_o, 0, h_first, tok0);
-        tma_tile_2d(smem + L::kU, 64, &map_du, full_u, 0, srow_of(h_first));
+        mbar_arrive_expect_tx(full_b, kBlocks * L::kPTile);
+        mbar_arrive_expect_tx(&full_g[1], kBlocks * L::kPTile);
+        tma_tile_tokens(smem + L::kB, &map_b, full_b, 0, g, tok, b, false);
+        tma_tile_tokens(smem + L::kG1, &map_c, &full_g[1], 0, g, tok, b, false);
+        if (kBlocks == 2) {
+            tma_tile_tokens(smem + L::kG0, &map_b, full_b, 64, g, tok, b, false);
+            tma_tile_tokens(smem + L::kO, &map_c, &full_g[1], 64, g, tok, b, false);
+        } else {
+            tma_tile_tokens(smem + L::kG0, &map_dout, &full_g[0], 0, h_first, tok, b);
+            tma_tile_tokens(smem + L::kO, &map_out, full_o, 0, h_first, tok, b);
+        }
+        load_u(h_first);
     }
 
     // rows (cs, q, decay references, dt) and per-head scalars are fetched one head ahead into registers
@@ -174,9 +196,12 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
             r_q = q[o + tid];
             r_ref = cs[o + (tid & ~31)];
         } else if (tid >= 384) {  // warps 12-15 run the dt stage
-            r_dt = dt[(static_cast<size_t>(tok0) + (tid - 384)) * s.nheads + h] + (dt_bias ? dt_bias[h] : 0.f);
-            r_a = A[h];
+            const int t = tok + tid - 384, source = parts > 1 ? h / parts : h, sources = parts > 1 ? s.nheads / parts : s.nheads;
+            r_dt = (t < tokens ? dt[(static_cast<size_t>(b) * tokens + t) * sources + source] : 0.f) +
+                   (dt_bias ? dt_bias[source] : 0.f);
+            r_a = A[source];
             r_gl = g_last[bh * nchunks + k];
+            if (kBlocks == 2) r_gl += g_last[static_cast<size_t>(s.batch) * s.nheads * nchunks + bh * nchunks + k];
         }
     };
     auto publish_rows = [&](int set) {
@@ -193,9 +218,9 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     ok = mbar_wait(full_b, 0, status, kStatusTmaTimeout | wait_site(4, 4)) && ok;
     // B is an A operand only (of CB^T = B * C^T and D2 = B * dU^T): it goes to tensor memory (row t in lane t)
     // from the fp32 tile as it landed and never needs a shared-memory operand tile
-    if (warp < 8) {
+    if (warp < 8 * kBlocks) {
         const uint32_t row = (warp & 3) * 32 + lane, kq = warp >> 2;
-        const uint8_t* src = smem + L::kB + kq * kHalf;
+        const uint8_t* src = smem + (kq >> 1 ? L::kG0 : L::kB) + (kq & 1) * kHalf;
         float v[32];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -213,22 +238,28 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     }
     ok = mbar_wait(&full_g[1], (pg >> 1) & 1u, status, kStatusTmaTimeout | wait_site(4, 5)) && ok;  // C
     pg ^= 2u;
-    split_tile_inplace(smem + L::kG1, kTile, nullptr, warp, lane);
+    for (int cb = 0; cb < kBlocks; ++cb) split_tile_inplace(smem + L::kG1 + cb * L::kPTile, kTile, nullptr, warp, lane);
     signal_issuer(bar_rcb, lane);
     publish_rows(0);
     ok = mbar_wait(full_u, pu, status, kStatusTmaTimeout | wait_site(4, 6)) && ok;  // dU of the first head
     pu ^= 1;
-    split_tile_inplace(smem + L::kU, 64, nullptr, warp, lane);
+    split_u();
     ok = mbar_wait(bar_cb, 0, status, kStatusMmaTimeout | wait_site(4, 7)) && ok;  // CB^T ready; the C tile is dead
     tc_fence_after_sync();
     if (tid == 0) {
-        if (heads_per_group > 1) tma_tile_3d(smem + L::kG1, kTile, &map_dout, &full_g[1], 0, h_first + 1, tok0);
-        tma_tile_3d(smem + L::kB, kTile, &map_x, full_x, 0, h_first, tok0);  // B is in TMEM: x takes its memory
+        if (kBlocks == 2) {  // B and C have left these
+            tma_tile_tokens(smem + L::kG0, &map_dout, &full_g[0], 0, h_first, tok, b);
+            tma_tile_tokens(smem + L::kO, &map_out, full_o, 0, h_first, tok, b);
+        }
+        if (heads_per_group > 1) tma_tile_tokens(smem + L::kG1, &map_dout, &full_g[1], 0, h_first + 1, tok, b);
+        tma_tile_tokens(smem + L::kB, &map_x, full_x, 0, h_first, tok, b);  // B is in TMEM: x takes its memory
     }
     cta_sync();  // rows of the first head are visible
 
     const int t_row = (warp & 3) * 32 + lane;
     const int cg = warp >> 2;  // 32-column chunk of the W pass, 16-column group of the accumulators
+    // of this thread's four quads of a row, those inside the tensor
+    const int skip_quads = tok + t_row < tokens ? min(4, (s.headdim - cg * 16) / 4) : 0;
     constexpr int kIoThread = 256;  // issues the dx stores (not one of the dt-stage threads)
     // ---- the dt stage of head `hp` of the group (warps 12-15, whose share of the W pass is the lightest; one
     // thread per row, own barrier), in fp64 so that the long sums feeding dA add no rounding error of their
@@ -347,20 +378,22 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
         // before it starts, and the tile still has a whole head to arrive.
         if (tid == kIoThread && hi > 0 && hi + 1 < heads_per_group) {
             tma_store_wait_read();
-            tma_tile_3d(g_tile(hi + 1), kTile, &map_dout, &full_g[gb ^ 1], 0, h + 1, tok0);
+            tma_tile_tokens(g_tile(hi + 1), &map_dout, &full_g[gb ^ 1], 0, h + 1, tok, b);
         }
         if (warp >= 12 && hi > 0) dt_stage(hi - 1);
         float4 dyv[4];
+        float d_head = 0.f;
         if constexpr (SKIP) {  // this thread's 16 values of dy, in flight under the products
             const float4* src = reinterpret_cast<const float4*>(
-                dy_raw + (static_cast<size_t>(tok0 + t_row) * s.nheads + h) * 64 + cg * 16);
+                dy_raw + ((static_cast<size_t>(b) * tokens + tok + t_row) * s.nheads + h) * s.headdim + cg * 16);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) dyv[i] = __ldg(src + i);
+            for (int i = 0; i < 4; ++i) dyv[i] = i < skip_quads ? __ldg(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (d_mode == 1) d_head = __ldg(dskip + (parts > 1 ? h / parts : h));
         }
         ok = mbar_wait(bar_d2, d2_parity, status, kStatusMmaTimeout | wait_site(4, 10)) && ok;
         d2_parity ^= 1;
         // D2 no longer reads the dU tile: the next head's may land
-        if (tid == 0 && hi + 1 < heads_per_group) tma_tile_2d(smem + L::kU, 64, &map_du, full_u, 0, srow_of(h + 1));
+        if (tid == 0 && hi + 1 < heads_per_group) load_u(h + 1);
         ok = mbar_wait(bar_d1, d1_parity, status, kStatusMmaTimeout | wait_site(4, 11)) && ok;
         d1_parity ^= 1;
         tc_fence_after_sync();
@@ -391,11 +424,10 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
                                        qt * (a[2] + decay * bb[2]), qt * (a[3] + decay * bb[3]));
                 if constexpr (SKIP) {
                     float4 dv;
-                    if (d_mode == 2) {
-                        dv = __ldg(reinterpret_cast<const float4*>(dskip + h * 64 + cg * 16 + 4 * c4));
+                    if (d_mode == 2 && c4 < skip_quads) {
+                        dv = __ldg(reinterpret_cast<const float4*>(dskip + h * s.headdim + cg * 16) + c4);
                     } else {
-                        const float d1v = __ldg(dskip + h);
-                        dv = make_float4(d1v, d1v, d1v, d1v);
+                        dv = make_float4(d_head, d_head, d_head, d_head);
                     }
                     o.x = fmaf(dv.x, dyv[c4].x, o.x);
                     o.y = fmaf(dv.y, dyv[c4].y, o.y);
@@ -411,18 +443,17 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
             publish_rows(gb ^ 1);  // next head's rows, other buffer
             ok = mbar_wait(full_u, pu, status, kStatusTmaTimeout | wait_site(4, 13)) && ok;  // next head's dU tile
             pu ^= 1;
-            split_tile_inplace(smem + L::kU, 64, nullptr, warp, lane);
+            split_u();
         }
         fence_proxy_async_smem();
         tc_fence_before_sync();
         cta_sync();
         if (tid == kIoThread && ok) {  // the dout tile of head hi + 2 follows once the store has read the memory: see above
-            tma_store_3d(&map_dx, g_tile(hi), 0, h, tok0);
-            tma_store_3d(&map_dx, g_tile(hi) + kHalf, 32, h, tok0);
+            tma_store_tokens(&map_dx, g_tile(hi), 0, h, tok, b, s.headdim);
             tma_store_commit();
         }
         // everyone has read x: the next head's x tile may land in its place
-        if (tid == 0 && hi + 1 < heads_per_group) tma_tile_3d(smem + L::kB, kTile, &map_x, full_x, 0, h + 1, tok0);
+        if (tid == 0 && hi + 1 < heads_per_group) tma_tile_tokens(smem + L::kB, &map_x, full_x, 0, h + 1, tok, b);
 
         // the dt stage of this head runs later, under the next head's D1 product.  Its inputs are gathered into
         // registers now, while no product competes for shared memory (under a product each of these reads
@@ -466,41 +497,37 @@ extern "C" int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const flo
         !dA_partial || !status)
         return SSD_ERR_NULL;
     const SsdShape& s = *shape;
-    if (s.dstate != 64) return SSD_ERR_UNSUPPORTED;
+    if (s.dstate != 64 && !has_extents(s)) return SSD_ERR_UNSUPPORTED;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (d_mode != 0 && !D) return SSD_ERR_NULL;
     CUtensorMap map_b, map_c, map_dout, map_out, map_du, map_dx, map_x;
-    const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
-    int rc = make_tmap_f32_tokens(&map_b, bm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dout, dout, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_out, out, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dx, dx, tokens, s.nheads, s.headdim, kTile);
-    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
-    const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
-    if (rc == SSD_OK) rc = make_tmap_f32_2d(&map_du, dstates, state_rows, s.dstate, 64);
+    if (d_mode == 2 && (reinterpret_cast<uintptr_t>(D) & 15u) != 0) return SSD_ERR_ALIGN;
+    int rc = make_tmap_f32_tokens(&map_b, bm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dout, dout, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_out, out, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_dx, dx, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_x, x, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_du, dstates, s);
     if (rc != SSD_OK) return rc;
-    const size_t smem = BwdDxSmem::kTotal + 1024;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
     const int64_t items = static_cast<int64_t>(s.seqlen / kTile) * s.ngroups * s.batch;
     const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 3);
     const dim3 grid(s.seqlen / kTile, s.ngroups * split, s.batch);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (d_mode == 0) {
-        static std::atomic<uint64_t> smem_set{0};
-        rc = set_max_smem_once(reinterpret_cast<const void*>(bwd_dx_kernel<false>), smem, smem_set);
-        if (rc != SSD_OK) return rc;
-        bwd_dx_kernel<false><<<grid, kLaunchThreadsGroups, smem, st>>>(
-            map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial,
-            nullptr, nullptr, 0, s, split, status);
-    } else {
-        static std::atomic<uint64_t> smem_set{0};
-        rc = set_max_smem_once(reinterpret_cast<const void*>(bwd_dx_kernel<true>), smem, smem_set);
-        if (rc != SSD_OK) return rc;
-        bwd_dx_kernel<true><<<grid, kLaunchThreadsGroups, smem, st>>>(
-            map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial,
-            dout, D, d_mode, s, split, status);
-    }
-    return launch_status();
+    auto launch = [&](auto kernel, size_t smem, std::atomic<uint64_t>& smem_set) {
+        const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), smem, smem_set);
+        if (r != SSD_OK) return r;
+        kernel<<<grid, kLaunchThreadsGroups, smem, st>>>(map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt,
+                                                         dt_bias, A, g_last, ddt_t, dA_partial, dout, D, d_mode, s, split,
+                                                         status);
+        return launch_status();
+    };
+    static std::atomic<uint64_t> smem_set[4];
+    if (state_cols(s) == 64)
+        return d_mode == 0 ? launch(bwd_dx_kernel<64, false>, BwdDxSmem<64>::kTotal + 1024, smem_set[0])
+                           : launch(bwd_dx_kernel<64, true>, BwdDxSmem<64>::kTotal + 1024, smem_set[1]);
+    return d_mode == 0 ? launch(bwd_dx_kernel<128, false>, BwdDxSmem<128>::kTotal + 1024, smem_set[2])
+                       : launch(bwd_dx_kernel<128, true>, BwdDxSmem<128>::kTotal + 1024, smem_set[3]);
 }

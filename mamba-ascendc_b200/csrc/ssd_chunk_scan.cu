@@ -45,8 +45,8 @@ template <int N>
 __global__ void __launch_bounds__(kLaunchThreadsGroups, 1)
 chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_s,
-                  const __grid_constant__ CUtensorMap map_out, const float* __restrict__ q,
-                  const float* __restrict__ cs, SsdShape s, int split, int* status) {
+                  const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_copy, bool copy,
+                  const float* __restrict__ q, const float* __restrict__ cs, SsdShape s, int split, int* status) {
     using L = ChunkScanSmem<N>;
     constexpr int NB = L::kBuf;
     constexpr int NOFF = L::kOffBuf;
@@ -166,7 +166,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // tile; the coordinates of the next loads are ready before the wait.
         if (warp == kThreads / 32 + 1) {
             auto load_x = [&](int it, const HeadPos& w) {
-                tma_tile_3d(smem + L::kX + (it % NB) * L::kXTile, kTile, &map_x, &full_x[it % NB], 0, w.h, w.tok0);
+                tma_tile_tokens(smem + L::kX + (it % NB) * L::kXTile, &map_x, &full_x[it % NB], 0, w.h, w.tok, w.b);
             };
             auto load_s = [&](int it, const HeadPos& w) {
                 mbar_arrive_expect_tx(&full_s[it % NB], L::kSTile);
@@ -178,8 +178,8 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 mbar_arrive_expect_tx(full_c, 2 * L::kCTile);
                 const int g = walk.group_of(w.g);
                 for (int cb = 0; cb < kBlocks; ++cb) {
-                    tma_tile_3d(smem + L::kC + cb * 2 * kHalf, kTile, &map_c, full_c, 64 * cb, g, w.tok0, false);
-                    tma_tile_3d(smem + L::kB + cb * 2 * kHalf, kTile, &map_b, full_c, 64 * cb, g, w.tok0, false);
+                    tma_tile_tokens(smem + L::kC + cb * 2 * kHalf, &map_c, full_c, 64 * cb, g, w.tok, w.b, false);
+                    tma_tile_tokens(smem + L::kB + cb * 2 * kHalf, &map_b, full_c, 64 * cb, g, w.tok, w.b, false);
                 }
             };
             TilePos cur = walk.first(static_cast<int>(blockIdx.x));
@@ -214,8 +214,8 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 if (lane == 0) {
                     if (*reinterpret_cast<volatile int*>(status) == 0) {
                         const uint8_t* stage = smem + L::kX + (it % NB) * L::kXTile;
-                        tma_store_3d(&map_out, stage, 0, w0.h, w0.tok0);
-                        tma_store_3d(&map_out, stage + kHalf, 32, w0.h, w0.tok0);
+                        tma_store_tokens(&map_out, stage, 0, w0.h, w0.tok, w0.b, s.headdim);
+                        if (copy) tma_store_tokens(&map_copy, stage, 0, w0.h, w0.tok, w0.b, s.headdim);
                         tma_store_commit();
                     }
                     if (it + NB < total) {  // then the buffer can take the next x tile that maps to it
@@ -439,19 +439,14 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 
 template <int N>
 int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const float* cm, const float* states,
-                      const float* q, const float* cs, float* out, int* status, cudaStream_t stream) {
-    CUtensorMap map_x, map_b, map_c, map_s, map_out;
-    const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
-    int rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
-    if (rc != SSD_OK) return rc;
-    rc = make_tmap_f32_tokens(&map_b, bm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc != SSD_OK) return rc;
-    rc = make_tmap_f32_tokens(&map_c, cm, tokens, s.ngroups, s.dstate, kTile);
-    if (rc != SSD_OK) return rc;
-    const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
-    rc = make_tmap_f32_2d(&map_s, states, state_rows, s.dstate, 64);
-    if (rc != SSD_OK) return rc;
-    rc = make_tmap_f32_tokens(&map_out, out, tokens, s.nheads, s.headdim, kTile);
+                      const float* q, const float* cs, float* out, float* out_copy, int* status, cudaStream_t stream) {
+    CUtensorMap map_x, map_b, map_c, map_s, map_out, map_copy;
+    int rc = make_tmap_f32_tokens(&map_x, x, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_b, bm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_c, cm, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_s, states, s);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_out, out, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_copy, out_copy ? out_copy : out, s, s.nheads, s.headdim);
     if (rc != SSD_OK) return rc;
     const size_t smem = ChunkScanSmem<N>::kTotal + 1024;
     static std::atomic<uint64_t> smem_set{0};  // one per instantiation
@@ -463,8 +458,8 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
     const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 2);
     const int64_t tiles = items * split;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
-    chunk_scan_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_b, map_c, map_s, map_out, q, cs, s, split,
-                                                                       status);
+    chunk_scan_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_b, map_c, map_s, map_out, map_copy,
+                                                                       out_copy != nullptr, q, cs, s, split, status);
     return launch_status();
 }
 
@@ -475,11 +470,17 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
 extern "C" int ssd_chunk_scan_fwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
                                   const float* states_start, const float* q, const float* cs, float* out, int* status,
                                   ssd_stream_t stream) {
+    return ssd_chunk_scan_copy_fwd(shape, x, bm, cm, states_start, q, cs, out, nullptr, status, stream);
+}
+
+extern "C" int ssd_chunk_scan_copy_fwd(const SsdShape* shape, const float* x, const float* bm, const float* cm,
+                                       const float* states_start, const float* q, const float* cs, float* out,
+                                       float* out_copy, int* status, ssd_stream_t stream) {
     using namespace ssd;
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!x || !bm || !cm || !states_start || !q || !cs || !out || !status) return SSD_ERR_NULL;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    return shape->dstate == 64 ? launch_chunk_scan<64>(*shape, x, bm, cm, states_start, q, cs, out, status, st)
-                               : launch_chunk_scan<128>(*shape, x, bm, cm, states_start, q, cs, out, status, st);
+    return state_cols(*shape) == 64 ? launch_chunk_scan<64>(*shape, x, bm, cm, states_start, q, cs, out, out_copy, status, st)
+                                    : launch_chunk_scan<128>(*shape, x, bm, cm, states_start, q, cs, out, out_copy, status, st);
 }

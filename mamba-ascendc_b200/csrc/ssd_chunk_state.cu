@@ -64,7 +64,7 @@ chunk_state_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
     const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
-    const int tok0 = b * s.seqlen + k * kTile;
+    const int tok = k * kTile;
     const int h_first = blockIdx.y * heads_per_group;
     const int npairs = (heads_per_group + 1) / 2;
 
@@ -121,12 +121,12 @@ chunk_state_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const int nh = heads_in(pair);
         mbar_arrive_expect_tx(full_x, nh * L::kXTile);
         for (int hh = 0; hh < nh; ++hh)
-            tma_tile_3d(buf + hh * L::kXTile, kTile, &map_x, full_x, 0, h_first + 2 * pair + hh, tok0, false);
+            tma_tile_tokens(buf + hh * L::kXTile, &map_x, full_x, 0, h_first + 2 * pair + hh, tok, b, false);
     };
     if (tid == 0) {
         mbar_arrive_expect_tx(full_m, L::kMTile);
         for (int cb = 0; cb < kBlocks; ++cb)
-            tma_tile_3d(smem + L::kM + cb * 2 * kHalf, kTile, &map_m, full_m, 64 * cb, g, tok0, false);
+            tma_tile_tokens(smem + L::kM + cb * 2 * kHalf, &map_m, full_m, 64 * cb, g, tok, b, false);
         load_pair(0);
     }
 
@@ -258,7 +258,7 @@ chunk_state_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     const int g = blockIdx.y / split;  // `split` work items share a group (choose_head_split)
     const int heads_per_group = s.nheads / (s.ngroups * split);
     const int nchunks = s.seqlen / kTile;
-    const int tok0 = b * s.seqlen + k * kTile;
+    const int tok = k * kTile;
     const int h_first = blockIdx.y * heads_per_group;
     const int npairs = (heads_per_group + 1) / 2;
 
@@ -314,13 +314,13 @@ chunk_state_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         const int nh = heads_in(pair);
         mbar_arrive_expect_tx(&full_x[pair & 1], nh * L::kXTile);
         for (int hh = 0; hh < nh; ++hh)
-            tma_tile_3d(pair_buf(pair) + hh * L::kXTile, kTile, &map_x, &full_x[pair & 1], 0, h_first + 2 * pair + hh,
-                        tok0, false);
+            tma_tile_tokens(pair_buf(pair) + hh * L::kXTile, &map_x, &full_x[pair & 1], 0, h_first + 2 * pair + hh, tok, b,
+                            false);
     };
     if (tid == 0) {
         mbar_arrive_expect_tx(full_m, L::kMTile);
         for (int cb = 0; cb < kBlocks; ++cb)
-            tma_tile_3d(smem + L::kM + cb * 2 * kHalf, kTile, &map_m, full_m, 64 * cb, g, tok0, false);
+            tma_tile_tokens(smem + L::kM + cb * 2 * kHalf, &map_m, full_m, 64 * cb, g, tok, b, false);
         load_pair(0);
         if (npairs > 1) load_pair(1);
     }
@@ -428,13 +428,9 @@ template <int N>
 int launch_chunk_state(const SsdShape& s, const float* x, const float* m, const float* q, const float* cs,
                        float* states, int mode, int* status, cudaStream_t stream) {
     CUtensorMap map_x, map_m, map_st;
-    const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
-    int rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
-    if (rc != SSD_OK) return rc;
-    rc = make_tmap_f32_tokens(&map_m, m, tokens, s.ngroups, s.dstate, kTile);
-    if (rc != SSD_OK) return rc;
-    const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
-    rc = make_tmap_f32_2d(&map_st, states, state_rows, s.dstate, 64);
+    int rc = make_tmap_f32_tokens(&map_x, x, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_m, m, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_st, states, s);
     if (rc != SSD_OK) return rc;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
@@ -470,6 +466,6 @@ extern "C" int ssd_chunk_state(const SsdShape* shape, const float* x, const floa
     if (!x || !m || !q || !cs || !states || !status) return SSD_ERR_NULL;
     if (mode != 0 && mode != 1) return SSD_ERR_UNSUPPORTED;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    return shape->dstate == 64 ? launch_chunk_state<64>(*shape, x, m, q, cs, states, mode, status, st)
-                               : launch_chunk_state<128>(*shape, x, m, q, cs, states, mode, status, st);
+    return state_cols(*shape) == 64 ? launch_chunk_state<64>(*shape, x, m, q, cs, states, mode, status, st)
+                                    : launch_chunk_state<128>(*shape, x, m, q, cs, states, mode, status, st);
 }

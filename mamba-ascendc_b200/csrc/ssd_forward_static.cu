@@ -64,6 +64,7 @@ extern "C" int ssd_forward_static(const SsdShape* shape, const float* x, const f
     if (rc0 != SSD_OK) return rc0;
     if (!x || !dt || !A || !bm || !cm || !out || !status) return SSD_ERR_NULL;
     const SsdShape& s = *shape;
+    if ((s.flags & SSD_FLAG_EXTENTS) != 0) return SSD_ERR_UNSUPPORTED;
     const size_t row_bytes = align256(sizeof(float) * s.batch * s.nheads * static_cast<size_t>(s.seqlen));
     const size_t state_bytes =
         sizeof(float) * s.batch * s.nheads * static_cast<size_t>(s.seqlen / s.tile) * s.headdim * s.dstate;

@@ -46,7 +46,7 @@ GateGrid gate_grid(long long rows, int cols, int min_rows) {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + __expf(-v)); }
+__device__ __forceinline__ float sigmoidf_(float v) { return 1.f / (1.f + expf(-v)); }
 
 // D for the four columns c..c+3 of a row (c % 4 == 0): d_mode 0 none, 1 per head [H], 2 per channel [H,P].
 __device__ __forceinline__ float4 load_d(const float* D, int d_mode, int c, int p_dim) {

@@ -39,14 +39,14 @@ namespace {
 struct TmapKey {
     const void* base;
     uint32_t rank;
-    uint64_t dims[3];
-    uint64_t strides[2];
-    uint32_t box[3];
+    uint64_t dims[4];
+    uint64_t strides[3];
+    uint32_t box[4];
     bool operator==(const TmapKey& o) const {
         if (base != o.base || rank != o.rank) return false;
-        for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 4; ++i)
             if (dims[i] != o.dims[i] || box[i] != o.box[i]) return false;
-        return strides[0] == o.strides[0] && strides[1] == o.strides[1];
+        return strides[0] == o.strides[0] && strides[1] == o.strides[1] && strides[2] == o.strides[2];
     }
 };
 struct TmapSlot {
@@ -61,7 +61,7 @@ std::mutex g_tmap_mutex;
 size_t tmap_hash(const TmapKey& k) {
     uint64_t h = reinterpret_cast<uintptr_t>(k.base) >> 4;
     h = h * 0x9E3779B97F4A7C15ull + k.dims[0];
-    h = h * 0x9E3779B97F4A7C15ull + k.dims[1] + (k.dims[2] << 20);
+    h = h * 0x9E3779B97F4A7C15ull + k.dims[1] + (k.dims[2] << 20) + (k.dims[3] << 44);
     h = h * 0x9E3779B97F4A7C15ull + k.box[1] + (static_cast<uint64_t>(k.box[2]) << 12) + k.rank;
     return static_cast<size_t>((h >> 17) % kTmapSlots);
 }
@@ -73,7 +73,7 @@ int make_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t* 
     EncodeTiledFn fn = encode_tiled();
     if (fn == nullptr) return SSD_ERR_TENSORMAP;
     if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return SSD_ERR_ALIGN;
-    if (rank < 2 || rank > 3) return SSD_ERR_TENSORMAP;
+    if (rank < 2 || rank > 4) return SSD_ERR_TENSORMAP;
     TmapKey key{};
     key.base = base;
     key.rank = static_cast<uint32_t>(rank);
@@ -111,10 +111,10 @@ int make_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t* 
         // SSD_B200_DEBUG=1: say what the driver answered (an error left behind by an earlier asynchronous fault
         // comes back from this call as well, with a code of its own)
         if (const char* dbg = std::getenv("SSD_B200_DEBUG"); dbg != nullptr && dbg[0] == '1')
-            std::fprintf(stderr, "ssd_b200: cuTensorMapEncodeTiled -> %d (base %p, rank %d, dims %llu %llu %llu, box %u %u %u)\n",
+            std::fprintf(stderr, "ssd_b200: cuTensorMapEncodeTiled -> %d (base %p, rank %d, dims %llu %llu %llu %llu, box %u %u %u %u)\n",
                          static_cast<int>(r), base, rank, static_cast<unsigned long long>(key.dims[0]),
                          static_cast<unsigned long long>(key.dims[1]), static_cast<unsigned long long>(key.dims[2]),
-                         key.box[0], key.box[1], key.box[2]);
+                         static_cast<unsigned long long>(key.dims[3]), key.box[0], key.box[1], key.box[2], key.box[3]);
         return SSD_ERR_TENSORMAP;
     }
     slot.used = true;
@@ -205,13 +205,21 @@ extern "C" int ssd_check_shape(const SsdShape* s) {
     if (s->nheads % s->ngroups != 0) return SSD_ERR_SHAPE;
     if (!(s->dt_min <= s->dt_max)) return SSD_ERR_SHAPE;
     if (s->valid_len < 0 || s->valid_len > s->seqlen) return SSD_ERR_SHAPE;
-    if (s->headdim != 64) return SSD_ERR_UNSUPPORTED;
-    if (s->dstate != 64 && s->dstate != 128) return SSD_ERR_UNSUPPORTED;
     if (s->tile != 128 || s->seqlen % s->tile != 0) return SSD_ERR_UNSUPPORTED;
+    if (ssd::has_extents(*s)) {
+        if (s->headdim > 64 || s->headdim % 4 != 0 || s->dstate > 128 || s->dstate % 4 != 0) return SSD_ERR_UNSUPPORTED;
+        if (s->valid_len != 0 && s->valid_len <= s->seqlen - s->tile) return SSD_ERR_SHAPE;
+        const int parts = ssd::head_parts(*s);
+        if (parts > 1 && (s->headdim != 64 || s->nheads % parts != 0 || s->nheads / parts % s->ngroups != 0))
+            return SSD_ERR_SHAPE;
+    } else {
+        if (s->headdim != 64) return SSD_ERR_UNSUPPORTED;
+        if (s->dstate != 64 && s->dstate != 128) return SSD_ERR_UNSUPPORTED;
+    }
     // grid.y / grid.z of the tile kernels, and the int32 coordinates of the TMA tile loads
     if (s->batch > 65535 || s->ngroups > 65535) return SSD_ERR_RANGE;
     const int64_t tokens = static_cast<int64_t>(s->batch) * s->seqlen;
-    const int64_t state_rows = static_cast<int64_t>(s->batch) * s->nheads * (s->seqlen / s->tile) * s->headdim;
+    const int64_t state_rows = static_cast<int64_t>(s->batch) * s->nheads * (s->seqlen / s->tile) * ssd::kStateRows;
     if (tokens >= (int64_t(1) << 31) || state_rows >= (int64_t(1) << 31)) return SSD_ERR_RANGE;
     return SSD_OK;
 }
@@ -220,14 +228,15 @@ extern "C" size_t ssd_buffer_bytes(const SsdShape* s, int which) {
     if (ssd_check_shape(s) != SSD_OK) return 0;
     const size_t bh = static_cast<size_t>(s->batch) * s->nheads;
     const size_t k = static_cast<size_t>(s->seqlen / s->tile);
-    const size_t pn = static_cast<size_t>(s->headdim) * s->dstate;
+    const size_t pn = static_cast<size_t>(ssd::kStateRows) * ssd::state_cols(*s);
     switch (which) {
         case SSD_BUF_Q:
         case SSD_BUF_CS:
         case SSD_BUF_DDT_T: return sizeof(float) * bh * s->seqlen;
         case SSD_BUF_STATES: return sizeof(float) * bh * k * pn;
-        case SSD_BUF_FINAL_STATE: return sizeof(float) * bh * pn;
-        case SSD_BUF_G_LAST: return sizeof(float) * bh * k;
+        case SSD_BUF_FINAL_STATE: return sizeof(float) * bh * s->headdim * s->dstate;
+        case SSD_BUF_G_LAST:
+            return sizeof(float) * bh * k * (ssd::has_extents(*s) ? ssd::state_cols(*s) / 64 : 1);
         case SSD_BUF_DA_PARTIAL: return sizeof(double) * bh * k;
         case SSD_BUF_GATE_PARTIAL: return sizeof(float) * ssd_gate_partial_floats(s);
         case SSD_BUF_STATUS: return sizeof(int32_t);

@@ -12,6 +12,19 @@
 
 namespace ssd {
 
+// ---- what the caller's tensors and the internal buffers look like (see SSD_FLAG_EXTENTS)
+inline __host__ __device__ bool has_extents(const SsdShape& s) { return (s.flags & SSD_FLAG_EXTENTS) != 0; }
+// tokens per sequence of the token-major tensors
+inline __host__ __device__ int row_tokens(const SsdShape& s) {
+    return has_extents(s) && s.valid_len > 0 ? s.valid_len : s.seqlen;
+}
+// heads of the kernels per head of dt, A, dt_bias and D[H]
+inline __host__ __device__ int head_parts(const SsdShape& s) {
+    return has_extents(s) ? static_cast<int>((s.flags >> 8) & 0xFFFFu) + 1 : 1;
+}
+constexpr int kStateRows = 64;  // headdim of the internal state buffers
+inline __host__ __device__ int state_cols(const SsdShape& s) { return s.dstate <= 64 ? 64 : 128; }
+
 // Tensor map over fp32 data for TMA tile loads with 128-byte swizzle.
 // dims/box are innermost first; strides_bytes has rank-1 entries (stride of
 // dims[1], dims[2], ...).  The innermost box extent must be 32 floats.
@@ -29,14 +42,20 @@ inline int make_tmap_f32_2d(CUtensorMap* map, const void* base, uint64_t rows, u
     return make_tmap_f32(map, base, 2, dims, strides, box);
 }
 
-// Token-major activation [tokens, heads, width] (x, dout, out: width = P; B, C:
-// heads = G, width = N); box = 32 floats of one head for `box_rows` tokens.
-inline int make_tmap_f32_tokens(CUtensorMap* map, const void* base, uint64_t tokens, uint64_t heads, uint64_t width,
-                                uint32_t box_rows) {
-    const uint64_t dims[3] = {width, heads, tokens};
-    const uint64_t strides[2] = {width * sizeof(float), heads * width * sizeof(float)};
-    const uint32_t box[3] = {32u, 1u, box_rows};
-    return make_tmap_f32(map, base, 3, dims, strides, box);
+// Token-major activation [batch, tokens, heads, width] (x, dout, out: width = P; B, C: heads = G, width = N); box = 32
+// floats of one head for 128 tokens.  Batch is a dimension of its own, so that a tile that runs over the end of a
+// sequence is filled with zeros (load) or cut off (store) instead of reaching into the next one.
+inline int make_tmap_f32_tokens(CUtensorMap* map, const void* base, const SsdShape& s, uint64_t heads, uint64_t width) {
+    const uint64_t tokens = row_tokens(s), row = width * sizeof(float);
+    const uint64_t dims[4] = {width, heads, tokens, static_cast<uint64_t>(s.batch)};
+    const uint64_t strides[3] = {row, heads * row, tokens * heads * row};
+    const uint32_t box[4] = {32u, 1u, 128u, 1u};
+    return make_tmap_f32(map, base, 4, dims, strides, box);
+}
+// The state buffers [B,H,K,64,N'] as rows; box = 32 floats of 64 rows.
+inline int make_tmap_f32_states(CUtensorMap* map, const void* base, const SsdShape& s) {
+    const uint64_t rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / s.tile) * kStateRows;
+    return make_tmap_f32_2d(map, base, rows, state_cols(s), 64);
 }
 
 // Index of the current device, or -1.

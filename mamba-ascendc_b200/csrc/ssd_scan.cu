@@ -23,17 +23,19 @@ dt_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ dt_bias
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int k = blockIdx.x, h0 = blockIdx.y * 32, b = blockIdx.z;
     const int heads = min(32, s.nheads - h0);  // <= 1 << head_bits
+    const int parts = head_parts(s), tokens = row_tokens(s) - k * kTile;  // tokens of dt from this tile on
     const bool softplus = (s.flags & SSD_FLAG_DT_SOFTPLUS) != 0;
     {
         const int hh = tid & ((1 << head_bits) - 1), t_first = tid >> head_bits, t_step = 256 >> head_bits;
         if (hh < heads) {
-            const float bias = dt_bias != nullptr ? dt_bias[h0 + hh] : 0.f;
-            const float* src = dt + (static_cast<size_t>(b) * s.seqlen + k * kTile) * s.nheads + h0 + hh;
+            const int source = (h0 + hh) / parts, sources = s.nheads / parts;
+            const float bias = dt_bias != nullptr ? dt_bias[source] : 0.f;
+            const float* src = dt + (static_cast<size_t>(b) * row_tokens(s) + k * kTile) * sources + source;
             float v[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int t = t_first + i * t_step;
-                if (t < kTile) v[i] = src[static_cast<size_t>(t) * s.nheads];
+                v[i] = t < kTile && t < tokens ? src[static_cast<size_t>(t) * sources] : 0.f;
             }
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -50,7 +52,7 @@ dt_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ dt_bias
     __syncthreads();
     for (int hh = warp; hh < heads; hh += 8) {
         const int head = h0 + hh;
-        const float a = A[head];
+        const float a = A[head / parts];
         float qv[4], c[4];
         float run = 0.f;
 #pragma unroll
@@ -86,15 +88,19 @@ constexpr int kWalkThreads = 64;
 template <bool REVERSE>
 __global__ void __launch_bounds__(kWalkThreads)
 state_walk_kernel(float* __restrict__ states, const float* __restrict__ cs, const float* __restrict__ start,
-                  float* __restrict__ end, int nchunks, int pn4, int seqlen, size_t total) {
+                  float* __restrict__ end, int nchunks, int n4, int seqlen, int headdim, int dstate4, size_t total) {
     const size_t idx = static_cast<size_t>(blockIdx.x) * kWalkThreads + threadIdx.x;
     if (idx >= total) return;
+    const int pn4 = kStateRows * n4;
     const size_t bh = idx / pn4;
     const int e = static_cast<int>(idx % pn4);
+    const int row = e / n4, col = e % n4;  // of the state; `start` and `end` are [headdim, dstate4]
+    const bool inside = row < headdim && col < dstate4;
+    const size_t edge = (bh * headdim + row) * dstate4 + col;
     float4* p = reinterpret_cast<float4*>(states) + bh * nchunks * pn4 + e;
     const float* csl = cs + bh * seqlen + (kTile - 1);
     auto tile_of = [&](int i) { return static_cast<size_t>(REVERSE ? nchunks - 1 - i : i); };
-    float4 st = start ? reinterpret_cast<const float4*>(start)[bh * pn4 + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 st = start && inside ? reinterpret_cast<const float4*>(start)[edge] : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 u[kWalkTiles];
     float c[kWalkTiles];
 #pragma unroll
@@ -128,18 +134,18 @@ state_walk_kernel(float* __restrict__ states, const float* __restrict__ cs, cons
             c[i] = cn[i];
         }
     }
-    if (end != nullptr) reinterpret_cast<float4*>(end)[bh * pn4 + e] = st;
+    if (end != nullptr && inside) reinterpret_cast<float4*>(end)[edge] = st;
 }
 
 template <bool REVERSE>
 int launch_state_walk(const SsdShape& s, float* states, const float* cs, const float* start, float* end,
                       cudaStream_t stream) {
-    const int pn4 = s.headdim * s.dstate / 4;
-    const size_t total = static_cast<size_t>(s.batch) * s.nheads * pn4;
+    const int n4 = state_cols(s) / 4;
+    const size_t total = static_cast<size_t>(s.batch) * s.nheads * kStateRows * n4;
     const size_t blocks = (total + kWalkThreads - 1) / kWalkThreads;
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
     state_walk_kernel<REVERSE><<<static_cast<unsigned>(blocks), kWalkThreads, 0, stream>>>(
-        states, cs, start, end, s.seqlen / kTile, pn4, s.seqlen, total);
+        states, cs, start, end, s.seqlen / kTile, n4, s.seqlen, s.headdim, s.dstate / 4, total);
     return launch_status();
 }
 
@@ -279,7 +285,8 @@ state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ 
 // ------------------------------------------------------------------ ddt transpose, dA and d(dt_bias)
 // One launch, two kinds of CTA.  The first batch * tiles * ceil(H / 32) CTAs turn ddt_t [B,H,L] into ddt [B,L,H], a
 // [128 tokens x up to 32 heads] patch each through shared memory.  The last H CTAs reduce one head each, in fp64 and
-// in a fixed order: dA[h] over the per-tile partials, d(dt_bias)[h] (if asked for) over the head's rows of ddt_t.
+// in a fixed order: dA[h] over the per-tile partials, d(dt_bias)[h] (if asked for) over the head's rows of ddt_t.  A head
+// that the kernels treat as `parts` heads has that many rows and partials, which are added up here.
 __device__ __forceinline__ double block_sum_256(double v, double* red, int tid) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
@@ -291,8 +298,8 @@ __device__ __forceinline__ double block_sum_256(double v, double* red, int tid) 
 
 __global__ void __launch_bounds__(256)
 dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ part, float* __restrict__ ddt,
-                   float* __restrict__ dA, float* __restrict__ ddt_bias, int batch, int nchunks, int nheads,
-                   int head_blocks, int head_bits) {
+                   float* __restrict__ dA, float* __restrict__ ddt_bias, int batch, int nchunks, int nheads, int parts,
+                   int tokens, int head_blocks, int head_bits) {
     __shared__ float patch[kTile][33];
     __shared__ double red[8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -305,9 +312,17 @@ dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ p
         float4 v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            if (warp + 8 * i < heads)
-                v[i] = *reinterpret_cast<const float4*>(ddt_t + (static_cast<size_t>(b) * nheads + h0 + warp + 8 * i) * seqlen +
-                                                        k * kTile + 4 * lane);
+            if (warp + 8 * i < heads) {
+                const float* src = ddt_t + (static_cast<size_t>(b) * nheads + h0 + warp + 8 * i) * parts * seqlen + k * kTile + 4 * lane;
+                v[i] = *reinterpret_cast<const float4*>(src);
+                for (int j = 1; j < parts; ++j) {
+                    const float4 o = *reinterpret_cast<const float4*>(src + static_cast<size_t>(j) * seqlen);
+                    v[i].x += o.x;
+                    v[i].y += o.y;
+                    v[i].z += o.z;
+                    v[i].w += o.w;
+                }
+            }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (warp + 8 * i >= heads) break;
@@ -319,24 +334,26 @@ dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ p
         __syncthreads();
         const int hh = tid & ((1 << head_bits) - 1);
         if (hh >= heads) return;
-        float* dst = ddt + (static_cast<size_t>(b) * seqlen + k * kTile) * nheads + h0 + hh;
-        for (int t = tid >> head_bits; t < kTile; t += 256 >> head_bits) dst[static_cast<size_t>(t) * nheads] = patch[t][hh];
+        float* dst = ddt + (static_cast<size_t>(b) * tokens + k * kTile) * nheads + h0 + hh;
+        const int t_end = min(kTile, tokens - k * kTile);
+        for (int t = tid >> head_bits; t < t_end; t += 256 >> head_bits) dst[static_cast<size_t>(t) * nheads] = patch[t][hh];
         return;
     }
     const int h = blockIdx.x - turns;
     double acc = 0.0;
-    for (int i = tid; i < batch * nchunks; i += 256) {
-        const int b = i / nchunks, k = i - b * nchunks;
-        acc += part[(static_cast<size_t>(b) * nheads + h) * nchunks + k];
+    const int per_head = parts * nchunks;  // the parts of a head are neighbours
+    for (int i = tid; i < batch * per_head; i += 256) {
+        const int b = i / per_head, k = i - b * per_head;
+        acc += part[(static_cast<size_t>(b) * nheads + h) * per_head + k];
     }
     acc = block_sum_256(acc, red, tid);
     if (tid == 0) dA[h] = static_cast<float>(acc);
     if (ddt_bias == nullptr) return;
     acc = 0.0;
     for (int b = 0; b < batch; ++b) {
-        const float4* row = reinterpret_cast<const float4*>(ddt_t + (static_cast<size_t>(b) * nheads + h) * seqlen);
+        const float4* row = reinterpret_cast<const float4*>(ddt_t + (static_cast<size_t>(b) * nheads + h) * parts * seqlen);
 #pragma unroll 4
-        for (int i = tid; i < seqlen / 4; i += 256) {
+        for (int i = tid; i < parts * (seqlen / 4); i += 256) {
             const float4 f = row[i];
             acc += (static_cast<double>(f.x) + f.y) + (static_cast<double>(f.z) + f.w);
         }
@@ -383,6 +400,7 @@ extern "C" int ssd_state_fold(const SsdShape* shape, const float* terms, const f
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!terms || !cs || !result) return SSD_ERR_NULL;
+    if (has_extents(*shape)) return SSD_ERR_UNSUPPORTED;
     const int pn4 = shape->headdim * shape->dstate / 4;
     const size_t total = static_cast<size_t>(shape->batch) * shape->nheads * pn4;
     const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
@@ -397,6 +415,7 @@ extern "C" int ssd_state_passing_bwd(const SsdShape* shape, float* dstates, cons
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!dstates || !cs || (g_last && !states_start)) return SSD_ERR_NULL;
+    if (g_last && has_extents(*shape)) return SSD_ERR_UNSUPPORTED;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (!g_last) return launch_state_walk<true>(*shape, dstates, cs, dfinal, d_initial, st);
     const unsigned blocks = static_cast<unsigned>(shape->batch) * shape->nheads;
@@ -421,12 +440,13 @@ extern "C" int ssd_dt_finalize_bias_bwd(const SsdShape* shape, const float* ddt_
     const int rc = ssd_check_shape(shape);
     if (rc != SSD_OK) return rc;
     if (!ddt_t || !dA_partial || !ddt || !dA) return SSD_ERR_NULL;
-    const int nchunks = shape->seqlen / kTile, head_blocks = (shape->nheads + 31) / 32;
-    const int64_t blocks = static_cast<int64_t>(shape->batch) * nchunks * head_blocks + shape->nheads;
+    const int parts = head_parts(*shape), heads = shape->nheads / parts;
+    const int nchunks = shape->seqlen / kTile, head_blocks = (heads + 31) / 32;
+    const int64_t blocks = static_cast<int64_t>(shape->batch) * nchunks * head_blocks + heads;
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
     dt_finalize_kernel<<<static_cast<unsigned>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        ddt_t, dA_partial, ddt, dA, ddt_bias, shape->batch, nchunks, shape->nheads, head_blocks,
-        head_bits_of(shape->nheads));
+        ddt_t, dA_partial, ddt, dA, ddt_bias, shape->batch, nchunks, heads, parts, row_tokens(*shape), head_blocks,
+        head_bits_of(heads));
     return launch_status();
 }
 

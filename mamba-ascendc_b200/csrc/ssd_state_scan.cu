@@ -129,13 +129,13 @@ chunk_state_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     auto heads_in = [&](int pair) { return (2 * pair + 1 < heads_per_group) ? 2 : 1; };
     auto load_pair = [&](int step) {
         const int pair = step % npairs, nh = heads_in(pair);
-        const int tok0 = b * s.seqlen + tile_of(step) * kTile;
+        const int tok = tile_of(step) * kTile;
         mbar_arrive_expect_tx(full_x, nh * L::kXTile);
         for (int hh = 0; hh < nh; ++hh)
-            tma_tile_3d(buf + hh * L::kXTile, kTile, &map_x, full_x, 0, h_first + 2 * pair + hh, tok0, false);
+            tma_tile_tokens(buf + hh * L::kXTile, &map_x, full_x, 0, h_first + 2 * pair + hh, tok, b, false);
     };
     auto load_m = [&](int step) {
-        tma_tile_3d(smem + L::kM, kTile, &map_m, full_m, 0, g, b * s.seqlen + tile_of(step) * kTile);
+        tma_tile_tokens(smem + L::kM, &map_m, full_m, 0, g, tile_of(step) * kTile, b);
     };
     if (tid == 0) {
         load_m(0);
@@ -171,15 +171,16 @@ chunk_state_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     const int e_col = (warp >> 2) * 32;
     auto tm_state = [&](int pair) { return tmem + 64u + 64u * static_cast<uint32_t>(pair); };
     auto state_elem = [&](int pair) {  // offset of this thread's 32 values inside a [B,H,P,N] tensor
-        return ((static_cast<size_t>(b) * s.nheads + h_first + 2 * pair + e_hh) * 64 + e_p) * N + e_col;
+        return ((static_cast<size_t>(b) * s.nheads + h_first + 2 * pair + e_hh) * s.headdim + e_p) * s.dstate + e_col;
     };
+    const int e_quads = e_p < s.headdim ? min(8, max(0, (s.dstate - e_col) / 4)) : 0;  // of them inside the tensor
     for (int pair = 0; pair < npairs; ++pair) {
         float v[32];
         if (start != nullptr && e_hh < heads_in(pair)) {
             const float4* src = reinterpret_cast<const float4*>(start + state_elem(pair));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float4 f = src[i];
+                const float4 f = i < e_quads ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
                 v[4 * i] = f.x;
                 v[4 * i + 1] = f.y;
                 v[4 * i + 2] = f.z;
@@ -275,7 +276,8 @@ chunk_state_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             tmem_ld_wait();
             float4* dst = reinterpret_cast<float4*>(end + state_elem(pair));
 #pragma unroll
-            for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            for (int i = 0; i < 8; ++i)
+                if (i < e_quads) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
     }
     if (tid == kIoThread) tma_store_wait_all();
@@ -288,13 +290,9 @@ template <int MODE>
 int launch_state_scan(const SsdShape& s, const float* x, const float* m, const float* q, const float* cs,
                       const float* start, float* states, float* end, int* status, cudaStream_t stream) {
     CUtensorMap map_x, map_m, map_st;
-    const uint64_t tokens = static_cast<uint64_t>(s.batch) * s.seqlen;
-    int rc = make_tmap_f32_tokens(&map_x, x, tokens, s.nheads, s.headdim, kTile);
-    if (rc != SSD_OK) return rc;
-    rc = make_tmap_f32_tokens(&map_m, m, tokens, s.ngroups, s.dstate, kTile);
-    if (rc != SSD_OK) return rc;
-    const uint64_t state_rows = static_cast<uint64_t>(s.batch) * s.nheads * (s.seqlen / kTile) * s.headdim;
-    rc = make_tmap_f32_2d(&map_st, states, state_rows, s.dstate, 64);
+    int rc = make_tmap_f32_tokens(&map_x, x, s, s.nheads, s.headdim);
+    if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_m, m, s, s.ngroups, s.dstate);
+    if (rc == SSD_OK) rc = make_tmap_f32_states(&map_st, states, s);
     if (rc != SSD_OK) return rc;
     const size_t smem = StateScanSmem::kTotal;
     static std::atomic<uint64_t> smem_set{0};
@@ -312,7 +310,7 @@ int launch_state_scan(const SsdShape& s, const float* x, const float* m, const f
 extern "C" int ssd_chunk_state_scan_supported(const SsdShape* shape) {
     if (ssd_check_shape(shape) != SSD_OK) return 0;
     const int heads_per_group = shape->nheads / shape->ngroups;
-    return shape->dstate == 64 && (heads_per_group + 1) / 2 <= ssd::kSsMaxPairs ? 1 : 0;
+    return ssd::state_cols(*shape) == 64 && (heads_per_group + 1) / 2 <= ssd::kSsMaxPairs ? 1 : 0;
 }
 
 extern "C" int ssd_chunk_state_scan(const SsdShape* shape, const float* x, const float* m, const float* q,

@@ -9,6 +9,7 @@
 #pragma once
 
 #include "../../include/ssd_b200.h"
+#include "ssd_host.h"
 #include "ssd_umma.cuh"
 
 namespace ssd {
@@ -52,22 +53,25 @@ constexpr uint32_t kSlabBytes = 128 * 128;  // one staged box: 128 rows x 32 flo
 // before the barrier that frees their memory flips.
 //
 // `split` > 1: the heads of a group are dealt to that many work items (choose_head_split says when that is
-// worth it).  The walk then runs over groups of heads_per_group / split heads; the group whose B and C a work item
-// reads is group_of(g).
+// worth it).  `blocks` = 2: each of these is two work items, one per 64 columns of the state (column_block).  The walk
+// then runs over that many groups; the group whose B and C a work item reads is group_of(g).
 struct TilePos {
     int b, g, k;
 };
 struct HeadPos {
-    int g, h, tok0;
+    int g, h;
+    int tok, b;      // first token of the tile inside its sequence, and the sequence
+    int tok0;        // the same counted over all sequences of `seqlen` tokens
     int tile_index;  // (batch, head, token tile) index: first row of q / cs over 128, state row over 64
 };
 struct TileWalk {
     int nchunks, ngroups, nheads, seqlen, heads_per_group, step_k, step_g, step_b;
     unsigned split_inverse;  // 0: no split, else ceil(2^32 / split)
-    __host__ __device__ __forceinline__ TileWalk(const SsdShape& s, int grid, int split = 1)
-        : nchunks(s.seqlen / 128), ngroups(s.ngroups * split), nheads(s.nheads), seqlen(s.seqlen),
+    int block_bits;          // log2 of the column blocks
+    __host__ __device__ __forceinline__ TileWalk(const SsdShape& s, int grid, int split = 1, int blocks = 1)
+        : nchunks(s.seqlen / 128), ngroups(s.ngroups * split * blocks), nheads(s.nheads), seqlen(s.seqlen),
           heads_per_group(s.nheads / (s.ngroups * split)),
-          split_inverse(split > 1 ? static_cast<unsigned>((0x100000000ull + split - 1) / split) : 0u) {
+          block_bits(blocks == 2 ? 1 : 0), split_inverse(split > 1 ? static_cast<unsigned>((0x100000000ull + split - 1) / split) : 0u) {
         step_k = grid % nchunks;
         step_g = (grid / nchunks) % ngroups;
         step_b = grid / (nchunks * ngroups);
@@ -94,9 +98,11 @@ struct TileWalk {
     }
     // g / split without a division; exact while g * split < 2^32
     __host__ __device__ __forceinline__ int group_of(int g) const {
+        g >>= block_bits;
         if (split_inverse == 0) return g;
         return static_cast<int>((static_cast<unsigned long long>(static_cast<unsigned>(g)) * split_inverse) >> 32);
     }
+    __host__ __device__ __forceinline__ int column_block(int g) const { return g & ((1 << block_bits) - 1); }
     // The head `ahead` heads after head `hi` of tile `t` in the CTA's sequence.
     __host__ __device__ __forceinline__ HeadPos locate(TilePos t, int hi, int ahead) const {
         hi += ahead;
@@ -106,8 +112,10 @@ struct TileWalk {
         }
         HeadPos w;
         w.g = t.g;
-        w.h = t.g * heads_per_group + hi;
-        w.tok0 = t.b * seqlen + t.k * 128;
+        w.h = (t.g >> block_bits) * heads_per_group + hi;
+        w.tok = t.k * 128;
+        w.b = t.b;
+        w.tok0 = t.b * seqlen + w.tok;
         w.tile_index = (t.b * nheads + w.h) * nchunks + t.k;
         return w;
     }
@@ -120,11 +128,20 @@ struct TileWalk {
 // the threads split it in place: no staging buffer, and the load can be issued as soon as the tile's
 // previous consumer (an MMA) has finished, a whole head ahead of its use.
 // `expect` = false: the caller has already announced the bytes of several tiles on `bar` in one go.
-__device__ __forceinline__ void tma_tile_3d(uint8_t* tile, uint32_t rows, const CUtensorMap* m, uint64_t* bar, int col0,
-                                            int c1, int c2, bool expect = true) {
-    if (expect) mbar_arrive_expect_tx(bar, 2u * rows * 128u);
-    tma_load_3d(tile, m, bar, col0, c1, c2);
-    tma_load_3d(tile + rows * 128u, m, bar, col0 + 32, c1, c2);
+// 128 tokens from `tok` of sequence `b`, 64 columns from `col0` of head (or group) `head`; what lies beyond the tensor's
+// tokens or columns arrives as zeros and counts in full.
+__device__ __forceinline__ void tma_tile_tokens(uint8_t* tile, const CUtensorMap* m, uint64_t* bar, int col0, int head,
+                                                int tok, int b, bool expect = true) {
+    if (expect) mbar_arrive_expect_tx(bar, 2u * 128u * 128u);
+    tma_load_4d(tile, m, bar, col0, head, tok, b);
+    tma_load_4d(tile + 128u * 128u, m, bar, col0 + 32, head, tok, b);
+}
+// The same way back from two staged slabs; `width` = columns of the tensor (tokens beyond its end are left out by the
+// engine, a slab without any column is not stored at all).
+__device__ __forceinline__ void tma_store_tokens(const CUtensorMap* m, const uint8_t* stage, int col0, int head, int tok,
+                                                 int b, int width) {
+    if (col0 < width) tma_store_4d(m, stage, col0, head, tok, b);
+    if (col0 + 32 < width) tma_store_4d(m, stage + 128u * 128u, col0 + 32, head, tok, b);
 }
 __device__ __forceinline__ void tma_tile_2d(uint8_t* tile, uint32_t rows, const CUtensorMap* m, uint64_t* bar, int col0,
                                             int c1, bool expect = true) {

@@ -2,7 +2,8 @@
 every divisor class of the heads per group, against the fp64 oracle.
 
 Tolerance: that of the tensor-core path anywhere else (operands with 16 mantissa bits, fp32 sums): 3e-5 of the norm on every
-output and gradient but dA, whose sum over all tokens cancels (2e-3, as the parity tests allow)."""
+output and gradient but ddt, a suffix sum of up to 128 signed terms (sqrt(128) * 6e-6 of a term: 1e-4), and dA, whose sum over
+all tokens cancels (2e-3, as the parity tests allow)."""
 import pytest
 import torch
 
@@ -30,7 +31,7 @@ def test_forward_and_backward(shape):
     check_status()
     got = [out.detach(), final.detach()] + [t.grad for t in leaves]
     for g, w, name in zip(got, want, ["out", "final", "dx", "ddt", "dA", "dB", "dC"]):
-        assert O.rel_l2(g.cpu(), w) <= (2e-3 if name == "dA" else 3e-5), name
+        assert O.rel_l2(g.cpu(), w) <= (2e-3 if name == "dA" else 1e-4 if name == "ddt" else 3e-5), name
 
 
 @pytest.mark.parametrize("shape", [(1, 128, 6, 64, 128, 64, 1), (1, 384, 16, 64, 128, 64, 2)])
