@@ -333,6 +333,39 @@ int ssd_selftest_wait_expiry(int* status, int polls, ssd_stream_t stream);
  * No counterpart in the reference. */
 int ssd_selftest_tile_walk(const SsdShape* shape, int grid, int cta, int count, int* out);
 
+/* ---------------------------------------------------------------- whole calls
+ *
+ * One entry point per direction that runs the stages above in order: forward (dt_cumsum, states, output, then the D / z
+ * epilogue) and backward (epilogue, state gradients, dB / dC, dx and dt).  The internal buffers lie in one caller-allocated
+ * workspace, 256-byte aligned, of the size given by the query; backward reads the forward's (q, cs, states).  A
+ * rejected argument of a later stage is reported after the earlier ones have been launched.  `state_route`: 0 picks
+ * ssd_chunk_state_scan where it is the faster route, 1 wherever it takes the shape, 2 never. */
+typedef struct SsdForwardArgs {
+    const float *x, *dt, *dt_bias /* or null */, *A, *bm, *cm;
+    const float *D /* or null */, *z /* or null */, *initial_state /* or null */;
+    float* y;           /* the SSD output before the epilogue */
+    float* out;         /* with D or z the epilogue's output; without, a second copy of y or null */
+    float* final_state; /* or null */
+    void* work;         /* ssd_forward_work_bytes() */
+    int32_t* status;
+    int32_t d_mode;     /* of D: 1 [H], 2 [H,P] */
+} SsdForwardArgs;
+typedef struct SsdBackwardArgs {
+    const float *x, *dt, *dt_bias, *A, *bm, *cm, *D, *z, *y /* as the forward call left it */;
+    const float *dout, *dfinal /* or null */;
+    const void* forward_work;
+    float *dx, *ddt, *dA, *dB, *dC;
+    float *dD, *dz;     /* with D, with z */
+    float *d_dt_bias, *d_initial; /* or null */
+    void* work;         /* ssd_backward_work_bytes() */
+    int32_t* status;
+    int32_t d_mode;
+} SsdBackwardArgs;
+size_t ssd_forward_work_bytes(const SsdShape* shape);
+size_t ssd_backward_work_bytes(const SsdShape* shape, int has_d, int has_z);
+int ssd_forward(const SsdShape* shape, const SsdForwardArgs* args, int state_route, ssd_stream_t stream);
+int ssd_backward(const SsdShape* shape, const SsdBackwardArgs* args, int state_route, ssd_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

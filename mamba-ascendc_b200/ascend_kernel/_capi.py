@@ -40,6 +40,17 @@ class SsdShape(ctypes.Structure):
     ]
 
 
+def _args(name: str, pointers: str):
+    """Mirror of one of the header's argument records: pointers, then the mode of D."""
+    fields = [(f, ctypes.c_void_p) for f in pointers.split()] + [("d_mode", ctypes.c_int32)]
+    return type(name, (ctypes.Structure,), {"_fields_": fields})
+
+
+SsdForwardArgs = _args("SsdForwardArgs", "x dt dt_bias A bm cm D z initial_state y out final_state work status")
+SsdBackwardArgs = _args("SsdBackwardArgs", "x dt dt_bias A bm cm D z y dout dfinal forward_work dx ddt dA dB dC dD dz "
+                                           "d_dt_bias d_initial work status")
+
+
 def library_path() -> Path:
     override = os.environ.get("SSD_B200_LIBRARY")
     if override:
@@ -93,6 +104,10 @@ SIGNATURES = {
                                             ctypes.c_int, ctypes.c_float, _p]),
     "ssd_block_conv_silu_fwd": (ctypes.c_int, [_p, ctypes.c_longlong, _p, _p, _p, _p, _p, ctypes.c_int, ctypes.c_int,
                                               ctypes.c_int, ctypes.c_int, _p]),
+    "ssd_forward_work_bytes": (ctypes.c_size_t, [_shape_p]),
+    "ssd_backward_work_bytes": (ctypes.c_size_t, [_shape_p, ctypes.c_int, ctypes.c_int]),
+    "ssd_forward": (ctypes.c_int, [_shape_p, ctypes.POINTER(SsdForwardArgs), ctypes.c_int, _p]),
+    "ssd_backward": (ctypes.c_int, [_shape_p, ctypes.POINTER(SsdBackwardArgs), ctypes.c_int, _p]),
     "ssd_static_scratch_bytes": (ctypes.c_size_t, []),
     "ssd_forward_static": (ctypes.c_int, [_shape_p] + [_p] * 9),
 }

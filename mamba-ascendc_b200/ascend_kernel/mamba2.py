@@ -66,7 +66,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def make_shape(x: torch.Tensor, B: torch.Tensor, dt_softplus: bool,
@@ -91,6 +91,8 @@ def extents_shape(x: torch.Tensor, B: torch.Tensor, heads: int, dt_softplus: boo
 
 # ----------------------------------------------------------------------------- validation
 def _check_tensor(t: torch.Tensor, name: str) -> None:
+    if t.is_cuda and t.dtype is torch.float32 and t.is_contiguous():
+        return
     # mamba_ascendc/csrc/ops/mamba2_ssd_fwd/op_host/mamba2_ssd_fwd.cpp:15-23
     if not t.is_cuda:
         raise RuntimeError(f"mamba2_ssd_fwd: {name} must be a CUDA tensor")
@@ -341,6 +343,65 @@ def gate_backward(dout, y, x, B, D, z, heads: Optional[int] = None):
     return dy, dz, dD
 
 
+# ----------------------------------------------------------------------------- whole calls
+# The stages of one direction as one foreign call (ssd_forward, ssd_backward).  While stage_events collects, the same
+# stages are launched one by one with events around them.
+_ROUTES = {"auto": 0, "on": 1, "off": 2}
+
+
+def forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, shape, want_final: bool, copy: bool = False):
+    """(out, final, y, work tensors): ``y`` is the SSD output before the D / z epilogue; without one it is ``out`` itself, or
+    with ``copy`` a tensor of its own."""
+    gated = D is not None or z is not None
+    dev = x.device
+    out = torch.empty_like(x)
+    if stage_events is not None:
+        y, final, *work = forward_stages(x, dt, A, B, C, False, want_final=want_final, initial_states=initial_states,
+                                         dt_bias=dt_bias, shape=shape, copy=out if copy else None)
+        if gated:
+            out = gate_forward(y, x, B, D, z, A.shape[0])
+        return (out if gated or copy else y), final, y, work
+    y = torch.empty_like(x) if gated or copy else out
+    sp = ctypes.byref(shape)
+    lib = _capi.lib
+    work = torch.empty(lib.ssd_forward_work_bytes(sp), device=dev, dtype=torch.uint8)
+    final = (torch.empty(shape.batch, shape.nheads, shape.headdim, shape.dstate, device=dev, dtype=torch.float32)
+             if want_final else None)
+    args = _capi.SsdForwardArgs(
+        x.data_ptr(), dt.data_ptr(), _ptr(dt_bias), A.data_ptr(), B.data_ptr(), C.data_ptr(), _ptr(D), _ptr(z),
+        _ptr(initial_states), y.data_ptr(), out.data_ptr() if gated or copy else None, _ptr(final), work.data_ptr(),
+        _status(dev).data_ptr(), _d_mode(D))
+    _capi.check(lib.ssd_forward(sp, ctypes.byref(args), _ROUTES[_state_scan], _stream()), "mamba2_ssd_fwd")
+    return out, final, y, (work,)
+
+
+def backward_call(x, dt, A, B, C, D, z, dt_bias, y, work, dout, dfinal, shape, want_dinitial: bool):
+    """(dx, ddt, dA, dB, dC, dD, dz, d_initial, d_dt_bias); ``work`` from ``forward_call``."""
+    gated = D is not None or z is not None
+    dbias = torch.empty_like(dt_bias) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
+    if len(work) == 3:  # launched one by one
+        dy, dz, dD = gate_backward(dout, y, x, B, D, z, A.shape[0]) if gated else (dout, None, None)
+        dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, y, *work, dy, dfinal, False, want_dinitial=want_dinitial,
+                                                     dt_bias=dt_bias, D=D, ddt_bias=dbias, shape=shape)
+        return dx, ddt, dA, dB, dC, dD, dz, dinit, dbias
+    dev = x.device
+    lib = _capi.lib
+    sp = ctypes.byref(shape)
+    scratch = torch.empty(lib.ssd_backward_work_bytes(sp, D is not None, z is not None), device=dev, dtype=torch.uint8)
+    dx, ddt, dA, dB, dC = (torch.empty_like(t) for t in (x, dt, A, B, C))
+    dD = torch.empty_like(D) if D is not None else None
+    dz = torch.empty_like(z) if z is not None else None
+    dinit = (torch.empty(shape.batch, shape.nheads, shape.headdim, shape.dstate, device=dev, dtype=torch.float32)
+             if want_dinitial else None)
+    args = _capi.SsdBackwardArgs(
+        x.data_ptr(), dt.data_ptr(), _ptr(dt_bias), A.data_ptr(), B.data_ptr(), C.data_ptr(), _ptr(D), _ptr(z), y.data_ptr(),
+        dout.data_ptr(), _ptr(dfinal), work[0].data_ptr(), dx.data_ptr(), ddt.data_ptr(), dA.data_ptr(), dB.data_ptr(),
+        dC.data_ptr(), _ptr(dD), _ptr(dz), _ptr(dbias), _ptr(dinit), scratch.data_ptr(), _status(dev).data_ptr(),
+        _d_mode(D))
+    _capi.check(lib.ssd_backward(sp, ctypes.byref(args), _ROUTES[_state_scan], _stream()), "mamba2_ssd_bwd")
+    return dx, ddt, dA, dB, dC, dD, dz, dinit, dbias
+
+
 # ----------------------------------------------------------------------------- autograd
 def _aligned(t: torch.Tensor) -> torch.Tensor:
     """Contiguous fp32 at an address the tile loads take (a gradient may be a slice of a larger one)."""
@@ -358,21 +419,17 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, dt_min, dt_max):
         ctx.shape = extents_shape(x, B, A.shape[0], dt_softplus, (dt_min, dt_max))
-        ctx.gated = D is not None or z is not None
         ctx.recompute = _save_policy == "recompute"
+        ctx.has_initial = initial_states is not None
         # Without an epilogue the output is what backward needs.  At the kernels' own sizes it is saved itself, so that
         # changing it in place is an error in backward; elsewhere the caller may change it, and a copy is saved.
         own_sizes = x.shape[3] == 64 and B.shape[3] == 64 and x.shape[1] % TILE == 0 and x.shape[2] == A.shape[0]
-        copy = None if ctx.gated or ctx.recompute or own_sizes else torch.empty_like(x)
-        y, final, q, cs, states = forward_stages(x, dt, A, B, C, dt_softplus, want_final=True, initial_states=initial_states,
-                                                 dt_bias=dt_bias, shape=ctx.shape, copy=copy)
-        out = gate_forward(y, x, B, D, z, A.shape[0]) if ctx.gated else y
+        copy = D is None and z is None and not ctx.recompute and not own_sizes
+        out, final, y, work = forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, ctx.shape, True, copy=copy)
         if ctx.recompute:  # inputs only; y, q, cs and the tile-start states are rebuilt in backward
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, initial_states)
         else:
-            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, y if copy is None else copy, q, cs, states)
-        ctx.dt_softplus = dt_softplus
-        ctx.has_initial = initial_states is not None
+            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, y, *work)
         return out, final
 
     @staticmethod
@@ -380,7 +437,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         if ctx.recompute:
             x, dt, A, B, C, dt_bias, D, z, initial_states = ctx.saved_tensors
         else:
-            x, dt, A, B, C, dt_bias, D, z, y, q, cs, states = ctx.saved_tensors
+            x, dt, A, B, C, dt_bias, D, z, y, *work = ctx.saved_tensors
         if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
             dout = torch.zeros_like(x)
         dout = _aligned(dout)
@@ -388,15 +445,12 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
             dfinal = _aligned(dfinal)
         with _device_guard(x.device):
             if ctx.recompute:
-                y, _, q, cs, states = forward_stages(x, dt, A, B, C, ctx.dt_softplus, want_final=False,
-                                                     initial_states=initial_states, dt_bias=dt_bias, shape=ctx.shape)
-            dy, dz, dD = gate_backward(dout, y, x, B, D, z, A.shape[0]) if ctx.gated else (dout, None, None)
+                y, _, _, work = forward_call(x, dt, A, B, C, None, None, dt_bias, initial_states, ctx.shape, False)
             if not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9)):  # D and z alone
+                _, dz, dD = gate_backward(dout, y, x, B, D, z, A.shape[0])
                 return None, None, None, None, None, dD, dz, None, None, None, None, None
-            dbias = torch.empty_like(dt_bias) if dt_bias is not None else None  # mamba2_ssd_dt_bwd/design.md:63-77
-            dx, ddt, dA, dB, dC, dinit = backward_stages(x, dt, A, B, C, y, q, cs, states, dy, dfinal, ctx.dt_softplus,
-                                                         want_dinitial=ctx.has_initial, dt_bias=dt_bias, D=D,
-                                                         ddt_bias=dbias, shape=ctx.shape)
+            dx, ddt, dA, dB, dC, dD, dz, dinit, dbias = backward_call(x, dt, A, B, C, D, z, dt_bias, y, work, dout, dfinal,
+                                                                      ctx.shape, ctx.has_initial)
         return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
 
 
@@ -535,11 +589,8 @@ def _tile_call(x, dt, A, B, C, D, z, dt_bias, dt_softplus, lim, initial_states, 
     if grad:
         out, final = _Mamba2SsdAutograd.apply(x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, lim[0], lim[1])
     else:
-        out, final, *_ = forward_stages(x, dt, A, B, C, dt_softplus, want_final=return_final_state,
-                                        initial_states=initial_states, dt_bias=dt_bias,
-                                        shape=extents_shape(x, B, h, dt_softplus, lim))
-        if D is not None or z is not None:
-            out = gate_forward(out, x, B, D, z, h)
+        out, final, _, _ = forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, extents_shape(x, B, h, dt_softplus, lim),
+                                        return_final_state)
     if parts > 1:
         out = out.view(b, l, h, p)
         final = final.view(b, h, p, -1) if final is not None else None

@@ -238,6 +238,7 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     if (rc != SSD_OK) return rc;
     if (!y || !out || (d_mode != 0 && (!D || !x))) return SSD_ERR_NULL;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
+    if (!aligned16(y, x, z, out, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     GateGrid g = gate_grid(rows, cols, 1);
     while (g.rowblocks > 65535) {
         g.rows_per_cta *= 2;
@@ -266,6 +267,7 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!dout || (z && (!y || !dy || !dz)) || (d_mode != 0 && (!D || !x || !dD_partial || !dD))) return SSD_ERR_NULL;
     if (!z && d_mode == 0) return SSD_OK;  // nothing to do
+    if (!aligned16(dout, y, x, z, dy, dz, dD_partial, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(rows, cols, kGateMinRows);
     if (g.rowblocks > 65535) return SSD_ERR_UNSUPPORTED;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);

@@ -76,6 +76,12 @@ int set_max_smem_once(const void* func, size_t bytes, std::atomic<uint64_t>& don
 // four items per group.  A split has to promise 5% to be taken.
 int choose_head_split(int64_t items, int heads_per_group, int slots, int unit, int overhead_halves);
 
+// Whether every pointer (null ones aside) takes 16-byte accesses.
+template <class... P>
+inline bool aligned16(const P*... p) {
+    return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0;
+}
+
 inline int launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SSD_OK : SSD_ERR_LAUNCH;

@@ -140,6 +140,7 @@ state_walk_kernel(float* __restrict__ states, const float* __restrict__ cs, cons
 template <bool REVERSE>
 int launch_state_walk(const SsdShape& s, float* states, const float* cs, const float* start, float* end,
                       cudaStream_t stream) {
+    if (!aligned16(states, start, end)) return SSD_ERR_ALIGN;
     const int n4 = state_cols(s) / 4;
     const size_t total = static_cast<size_t>(s.batch) * s.nheads * kStateRows * n4;
     const size_t blocks = (total + kWalkThreads - 1) / kWalkThreads;
