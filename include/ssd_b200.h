@@ -272,6 +272,14 @@ int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const float* y, 
  *   bias [C] may be null. */
 int ssd_block_rmsnorm_fwd(const float* x, long long x_stride, const float* z, long long z_stride, const float* w,
                           float* out, long long rows, int d, float eps, ssd_stream_t stream);
+/* The norm of (x + D .* skip) with D[h] of the head h = column / headdim (skip [rows,d], null = none), and the convolution that
+ * also copies dt [B,L,heads] from the columns behind the convolved ones and forms A = -exp(A_log) [heads]. */
+int ssd_block_skip_rmsnorm_fwd(const float* x, long long x_stride, const float* skip, const float* D, int headdim,
+                               const float* z, long long z_stride, const float* w, float* out, long long rows, int d,
+                               float eps, ssd_stream_t stream);
+int ssd_block_conv_split_fwd(const float* xbc, long long row_stride, const float* weight, const float* bias,
+                             const float* a_log, float* x_out, float* b_out, float* c_out, float* dt_out, float* a_out,
+                             int batch, int seqlen, int d_in, int gn, int heads, ssd_stream_t stream);
 int ssd_block_conv_silu_fwd(const float* xbc, long long row_stride, const float* weight, const float* bias,
                             float* x_out, float* b_out, float* c_out, int batch, int seqlen, int d_in, int gn,
                             ssd_stream_t stream);

@@ -68,11 +68,12 @@ def _fast(t: torch.Tensor) -> bool:
 
 
 def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: torch.Tensor, eps: float, rows: int,
-                    d: int) -> torch.Tensor:
+                    d: int, skip=None, D=None, headdim: int = 0) -> torch.Tensor:
     capi = _kernels()
     out = torch.empty(rows, d, device=weight.device, dtype=torch.float32)
-    capi.check(capi.lib.ssd_block_rmsnorm_fwd(x2d, x_stride, z, z_stride, weight.data_ptr(), out.data_ptr(), rows, d,
-                                              eps, torch.cuda.current_stream().cuda_stream), "vmamba2_rmsnorm")
+    capi.check(capi.lib.ssd_block_skip_rmsnorm_fwd(x2d, x_stride, skip, D, headdim, z, z_stride, weight.data_ptr(),
+                                                   out.data_ptr(), rows, d, eps,
+                                                   torch.cuda.current_stream().cuda_stream), "vmamba2_rmsnorm")
     return out
 
 
@@ -113,7 +114,8 @@ class Mamba2Block(nn.Module):
         b, l, _ = u.shape
         d_in, g, n, h, p = cfg.d_inner, cfg.ngroups, cfg.d_state, cfg.nheads, cfg.headdim
         zxbcdt = self.in_proj(self.norm(u))
-        if _fast(zxbcdt) and zxbcdt.is_contiguous() and cfg.d_conv == 4 and d_in <= 512:
+        if (_fast(zxbcdt) and zxbcdt.is_contiguous() and cfg.d_conv == 4 and d_in <= 512 and
+                all(t.dtype == torch.float32 and t.is_contiguous() for t in (self.A_log, self.D))):
             return u + self.out_proj(self._fused_inner(zxbcdt, b, l))
         z, xbc, dt = torch.split(zxbcdt, [d_in, d_in + 2 * g * n, h], dim=-1)
         xbc = F.silu(self.conv1d(xbc.transpose(1, 2))[..., :l].transpose(1, 2))
@@ -137,16 +139,17 @@ class Mamba2Block(nn.Module):
         cm = torch.empty(b, l, g, n, device=dev, dtype=torch.float32)
         w = self.conv1d.weight.view(-1, cfg.d_conv)
         bias = self.conv1d.bias
-        capi.check(capi.lib.ssd_block_conv_silu_fwd(zxbcdt.data_ptr() + 4 * d_in, width, w.data_ptr(),
-                                                    None if bias is None else bias.data_ptr(), x.data_ptr(),
-                                                    bm.data_ptr(), cm.data_ptr(), b, l, d_in, g * n,
-                                                    torch.cuda.current_stream().cuda_stream), "vmamba2_conv1d")
-        dt = zxbcdt[..., d_in + d_in + 2 * g * n:].contiguous()
-        y = self.ssd_fn(x, dt, -torch.exp(self.A_log), bm, cm, cfg.chunk_size, D=self.D, dt_bias=self.dt_bias,
-                        dt_softplus=True)
-        y = y.contiguous()
+        dt = torch.empty(b, l, h, device=dev, dtype=torch.float32)
+        A = torch.empty(h, device=dev, dtype=torch.float32)
+        capi.check(capi.lib.ssd_block_conv_split_fwd(zxbcdt.data_ptr() + 4 * d_in, width, w.data_ptr(),
+                                                     None if bias is None else bias.data_ptr(), self.A_log.data_ptr(),
+                                                     x.data_ptr(), bm.data_ptr(), cm.data_ptr(), dt.data_ptr(),
+                                                     A.data_ptr(), b, l, d_in, g * n, h,
+                                                     torch.cuda.current_stream().cuda_stream), "vmamba2_conv1d")
+        # the skip connection is added where the gated norm reads y anyway
+        y = self.ssd_fn(x, dt, A, bm, cm, cfg.chunk_size, dt_bias=self.dt_bias, dt_softplus=True).contiguous()
         return _rmsnorm_kernel(y.data_ptr(), d_in, zxbcdt.data_ptr(), width, self.out_norm.weight, self.out_norm.eps,
-                               b * l, d_in).view(b, l, d_in)
+                               b * l, d_in, x.data_ptr(), self.D.data_ptr(), p).view(b, l, d_in)
 
 
 class VisionMamba2(nn.Module):

@@ -80,3 +80,47 @@ def test_dt_stages_take_any_number_of_heads(b, l, h):
     assert torch.equal(ddt, ddt_t.transpose(1, 2))
     assert (dA.double() - part.sum((0, 2))).abs().max() < 1e-6 * part.abs().sum()
     assert (dbias.double() - ddt_t.double().sum((0, 2))).abs().max() < 1e-6 * ddt_t.double().norm()
+
+
+@pytest.mark.parametrize("offset", [0, 1])  # 1: rows that are not 8-byte aligned
+@pytest.mark.parametrize("with_z,with_skip", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("rows,d", [(1, 1), (9, 64), (5, 192), (17, 194), (3, 384), (8, 385), (4, 512)])
+def test_norm_with_gate_and_skip(rows, d, with_z, with_skip, offset):
+    from ascend_kernel import _capi
+
+    gen = torch.Generator(device="cuda").manual_seed(rows + d)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    headdim = 32 if d % 32 == 0 else 1
+    wide, x, skip, w = rnd(rows, d + 7), rnd(rows * d + 1)[offset:offset + rows * d].view(rows, d), rnd(rows, d), rnd(d)
+    D = rnd(d // headdim)
+    out = torch.empty(rows, d, device="cuda")
+    _capi.check(_capi.lib.ssd_block_skip_rmsnorm_fwd(
+        x.data_ptr(), d, skip.data_ptr() if with_skip else None, D.data_ptr() if with_skip else None, headdim,
+        wide.data_ptr() if with_z else None, d + 7, w.data_ptr(), out.data_ptr(), rows, d, 1e-5,
+        torch.cuda.current_stream().cuda_stream), "norm")
+    t = x.double()
+    if with_skip:
+        t = t + skip.double() * D.double().repeat_interleave(headdim)
+    if with_z:
+        t = t * torch.nn.functional.silu(wide[:, :d].double())
+    assert _rel(out, t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()) <= REL
+
+
+@pytest.mark.parametrize("batch,l,d_in,gn,heads", [(1, 1, 4, 4, 0), (2, 15, 64, 32, 3), (1, 16, 130, 7, 130), (3, 67, 384, 64, 6)])
+def test_convolution_and_split(batch, l, d_in, gn, heads):
+    from ascend_kernel import _capi
+
+    gen = torch.Generator(device="cuda").manual_seed(l + d_in)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    ch = d_in + 2 * gn
+    src, weight, bias, a_log = rnd(batch, l, ch + heads + 5), rnd(ch, 4), rnd(ch), rnd(max(heads, 1))
+    x, bm, cm, dt = (torch.empty(batch, l, n, device="cuda") for n in (d_in, gn, gn, heads))
+    A = torch.empty(heads, device="cuda")
+    _capi.check(_capi.lib.ssd_block_conv_split_fwd(
+        src.data_ptr(), ch + heads + 5, weight.data_ptr(), bias.data_ptr(), a_log.data_ptr(), x.data_ptr(), bm.data_ptr(),
+        cm.data_ptr(), dt.data_ptr(), A.data_ptr(), batch, l, d_in, gn, heads,
+        torch.cuda.current_stream().cuda_stream), "conv")
+    padded = torch.nn.functional.pad(src[..., :ch].double(), (0, 0, 3, 0))
+    want = bias.double() + sum(padded[:, k:k + l] * weight[:, k].double() for k in range(4))
+    assert _rel(torch.cat([x, bm, cm], -1), torch.nn.functional.silu(want)) <= REL
+    assert torch.equal(dt, src[..., ch:ch + heads]) and torch.allclose(A, -torch.exp(a_log[:heads]), rtol=1e-6)
