@@ -107,6 +107,9 @@ SIGNATURES = {
     "ssd_block_skip_rmsnorm_fwd": (ctypes.c_int, [_p, ctypes.c_longlong, _p, _p, ctypes.c_int, _p, ctypes.c_longlong, _p, _p,
                                                  ctypes.c_longlong, ctypes.c_int, ctypes.c_float, _p]),
     "ssd_block_conv_split_fwd": (ctypes.c_int, [_p, ctypes.c_longlong] + [_p] * 8 + [ctypes.c_int] * 5 + [_p]),
+    "ssd_linear_work_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
+    "ssd_linear_pays": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]),
+    "ssd_linear_fwd": (ctypes.c_int, [_p, _p, _p, _p, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, _p, _p, _p]),
     "ssd_forward_work_bytes": (ctypes.c_size_t, [_shape_p]),
     "ssd_backward_work_bytes": (ctypes.c_size_t, [_shape_p, ctypes.c_int, ctypes.c_int]),
     "ssd_forward": (ctypes.c_int, [_shape_p, ctypes.POINTER(SsdForwardArgs), ctypes.c_int, _p]),

@@ -77,6 +77,36 @@ def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: 
     return out
 
 
+def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``layer(x)`` (+ residual).  A plain bias-free fp32 projection in inference runs as ``ssd_linear_fwd`` (tensor cores at
+    fp32 accuracy); anything else about the layer, the precision the caller chose or the sizes goes to the layer itself."""
+    capi = _kernels()
+    if (type(layer) is nn.Linear and layer.bias is None and _fast(x) and x.is_contiguous() and x.data_ptr() % 16 == 0 and
+            layer.weight.dtype == torch.float32 and layer.weight.is_contiguous() and layer.weight.is_cuda and
+            not torch.is_autocast_enabled() and torch.get_float32_matmul_precision() == "highest" and
+            not (layer._forward_hooks or layer._forward_pre_hooks or _global_hooks()) and
+            (residual is None or (residual.is_contiguous() and residual.dtype == torch.float32))):
+        n, k = layer.weight.shape
+        rows = x.numel() // k if k else 0
+        if capi.lib.ssd_linear_pays(rows, n, k):
+            from .mamba2 import _status
+
+            work = torch.empty(capi.lib.ssd_linear_work_bytes(n, k), device=x.device, dtype=torch.uint8)
+            out = torch.empty(*x.shape[:-1], n, device=x.device, dtype=torch.float32)
+            capi.check(capi.lib.ssd_linear_fwd(x.data_ptr(), layer.weight.data_ptr(),
+                                               None if residual is None else residual.data_ptr(), out.data_ptr(), rows, n,
+                                               k, work.data_ptr(), _status(x.device).data_ptr(),
+                                               torch.cuda.current_stream().cuda_stream), "vmamba2_linear")
+            return out
+    y = layer(x)
+    return y if residual is None else residual + y
+
+
+def _global_hooks() -> bool:
+    m = torch.nn.modules.module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float = 1e-5):
         super().__init__()
@@ -113,10 +143,10 @@ class Mamba2Block(nn.Module):
         cfg = self.cfg
         b, l, _ = u.shape
         d_in, g, n, h, p = cfg.d_inner, cfg.ngroups, cfg.d_state, cfg.nheads, cfg.headdim
-        zxbcdt = self.in_proj(self.norm(u))
+        zxbcdt = _linear(self.in_proj, self.norm(u))
         if (_fast(zxbcdt) and zxbcdt.is_contiguous() and cfg.d_conv == 4 and d_in <= 512 and
                 all(t.dtype == torch.float32 and t.is_contiguous() for t in (self.A_log, self.D))):
-            return u + self.out_proj(self._fused_inner(zxbcdt, b, l))
+            return _linear(self.out_proj, self._fused_inner(zxbcdt, b, l), residual=u)
         z, xbc, dt = torch.split(zxbcdt, [d_in, d_in + 2 * g * n, h], dim=-1)
         xbc = F.silu(self.conv1d(xbc.transpose(1, 2))[..., :l].transpose(1, 2))
         x, bm, cm = torch.split(xbc, [d_in, g * n, g * n], dim=-1)
