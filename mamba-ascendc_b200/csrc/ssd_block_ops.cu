@@ -14,6 +14,7 @@
 // 8-byte aligned) with lanes along the channels (coalesced).  The reference's demo network applies the same operations with framework calls
 // (mamba_torch/vmamba2_network.py:197-302).
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 
 namespace ssd {
 
@@ -37,6 +38,8 @@ struct NormArgs {
 template <int VEC, int ITERS, bool GATE, bool SKIP>
 __global__ void __launch_bounds__(256)
 block_rmsnorm_kernel(const NormArgs a) {
+    after_previous();
+    allow_next();
     const int lane = threadIdx.x & 31;
     const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= a.rows) return;
@@ -97,7 +100,7 @@ template <int VEC, int ITERS>
 int launch_norm(const NormArgs& a, cudaStream_t stream) {
     const long long blocks = (a.rows + 7) / 8;
     if (blocks > 0x7fffffffLL) return SSD_ERR_RANGE;
-    auto launch = [&](auto kernel) { kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(a); };
+    auto launch = [&](auto kernel) { launch_plain(kernel, static_cast<unsigned>(blocks), 256, 0, stream, a); };
     if (a.skip != nullptr)
         a.z ? launch(block_rmsnorm_kernel<VEC, ITERS, true, true>) : launch(block_rmsnorm_kernel<VEC, ITERS, false, true>);
     else
@@ -120,6 +123,8 @@ struct ConvArgs {
 
 __global__ void __launch_bounds__(128)
 block_conv_silu_kernel(const ConvArgs a) {
+    after_previous();
+    allow_next();
     const int channels = a.d_in + 2 * a.gn;
     const int c = blockIdx.x * 128 + threadIdx.x;
     if (c >= channels + a.heads) return;
@@ -201,7 +206,7 @@ extern "C" int ssd_block_conv_split_fwd(const float* xbc, long long row_stride, 
     if (batch > 65535 || (seqlen + kConvTokens - 1) / kConvTokens > 65535) return SSD_ERR_RANGE;
     const ConvArgs a{xbc, weight, bias, a_log, x_out, b_out, c_out, dt_out, a_out, row_stride, seqlen, d_in, gn, heads};
     const dim3 grid((d_in + 2 * gn + heads + 127) / 128, (seqlen + kConvTokens - 1) / kConvTokens, batch);
-    block_conv_silu_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+    launch_plain(block_conv_silu_kernel, grid, 128, 0, reinterpret_cast<cudaStream_t>(stream), a);
     return launch_status();
 }
 

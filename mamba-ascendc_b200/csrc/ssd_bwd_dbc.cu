@@ -28,6 +28,7 @@
 // by TMA while the next tile's first head is already being worked on.
 #include "ssd_decay.cuh"
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -116,7 +117,6 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
     // left waiting on a barrier that departed warps will not reach.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 7; ++i) mbar_init(&bars[i], 1);
         mbar_init(bar_rdy0, kThreads / 32);
         mbar_init(bar_rdy1, kThreads / 32);
@@ -128,10 +128,13 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 512);
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, 512);
         return;
@@ -584,6 +587,8 @@ bwd_dbc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 __global__ void __launch_bounds__(256)
 dbc_sum_kernel(const float* __restrict__ partial, float* __restrict__ dB, float* __restrict__ dC, size_t quads, int split,
                int row_quads) {
+    after_previous();
+    allow_next();
     const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
     if (i >= 2 * quads) return;
     const bool second = i >= quads;
@@ -660,12 +665,12 @@ extern "C" int ssd_chunk_dbc_split_bwd(const SsdShape* shape, const float* x, co
     if (sms <= 0) return SSD_ERR_LAUNCH;
     if (tiles * split > 0x7fffffff) return SSD_ERR_RANGE;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
-    bwd_dbc_kernel<<<grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        map_x, map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, blocks, status);
+    launch_chained(bwd_dbc_kernel, grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream), map_x,
+                   map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, blocks, status);
     rc = launch_status();
     if (rc != SSD_OK || split == 1) return rc;
     const size_t quads = 2 * elems / 4;
-    dbc_sum_kernel<<<static_cast<unsigned>((quads + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        partial, dB, dC, elems / 4, split, s.dstate / 4);
+    launch_plain(dbc_sum_kernel, static_cast<unsigned>((quads + 255) / 256), 256, 0,
+                 reinterpret_cast<cudaStream_t>(stream), partial, dB, dC, elems / 4, split, s.dstate / 4);
     return launch_status();
 }

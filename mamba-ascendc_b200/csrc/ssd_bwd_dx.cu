@@ -22,6 +22,7 @@
 // dout tile is double buffered, so all loads of head h+1 are in flight while head h computes.
 #include "ssd_decay.cuh"
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -101,17 +102,19 @@ bwd_dx_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
     // left waiting on a barrier that departed warps will not reach.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
         for (int i = 8; i < 11; ++i) mbar_init(&bars[i], kThreads / 32);
         mbar_init(full_x, 1);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 512);
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, 512);
         return;
@@ -519,9 +522,8 @@ extern "C" int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const flo
     auto launch = [&](auto kernel, size_t smem, std::atomic<uint64_t>& smem_set) {
         const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), smem, smem_set);
         if (r != SSD_OK) return r;
-        kernel<<<grid, kLaunchThreadsGroups, smem, st>>>(map_b, map_c, map_dout, map_out, map_du, map_dx, map_x, q, cs, dt,
-                                                         dt_bias, A, g_last, ddt_t, dA_partial, dout, D, d_mode, s, split,
-                                                         status);
+        launch_chained(kernel, grid, kLaunchThreadsGroups, smem, st, map_b, map_c, map_dout, map_out, map_du, map_dx,
+                       map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial, dout, D, d_mode, s, split, status);
         return launch_status();
     };
     static std::atomic<uint64_t> smem_set[4];

@@ -16,6 +16,7 @@
 // as S is split and runs under the W pass; the output tile is staged in the dead x tile and written by TMA.
 #include "ssd_decay.cuh"
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -96,7 +97,6 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
     // left waiting on a barrier that departed warps will not reach.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 9; ++i) mbar_init(&bars[i], 1);
         for (int i = 0; i < 3; ++i) mbar_init(&bar_yp[i], 1);
         for (int i = 9; i < 12; ++i) mbar_init(&bars[i], kThreads / 32);
@@ -109,10 +109,13 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 512);
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, 512);
         return;
@@ -458,8 +461,8 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
     const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 2);
     const int64_t tiles = items * split;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
-    chunk_scan_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_b, map_c, map_s, map_out, map_copy,
-                                                                       out_copy != nullptr, q, cs, s, split, status);
+    launch_chained(chunk_scan_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_b, map_c, map_s, map_out,
+                   map_copy, out_copy != nullptr, q, cs, s, split, status);
     return launch_status();
 }
 

@@ -15,6 +15,7 @@
 // are serial (load, split, product, write-out); the overlap comes from the other CTA on the SM being in a
 // different phase, which also hides each CTA's start-up and load latency.
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -77,16 +78,18 @@ chunk_state_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
     // left waiting on a barrier that departed warps will not reach.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
         mbar_init(bar_rdy, kCsWarps);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, N);  // one accumulator [128 x N]
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, N);
         return;
@@ -267,17 +270,19 @@ chunk_state_wide_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
     // left waiting on a barrier that departed warps will not reach.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 5; ++i) mbar_init(&bars[i], 1);
         mbar_init(&bar_rdy[0], kThreads / 32);
         mbar_init(&bar_rdy[1], kThreads / 32);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 2 * N);  // two accumulators [128 x N], by pair parity
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, 2 * N);
         return;
@@ -442,14 +447,14 @@ int launch_chunk_state(const SsdShape& s, const float* x, const float* m, const 
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_kernel<N>), smem, smem_set);
         if (rc != SSD_OK) return rc;
-        chunk_state_kernel<N><<<grid, kCsLaunch, smem, stream>>>(map_x, map_m, map_st, q, cs, s, split, mode, status);
+        launch_plain(chunk_state_kernel<N>, grid, kCsLaunch, smem, stream, map_x, map_m, map_st, q, cs, s, split, mode, status);
     } else {
         const size_t smem = ChunkStateWideSmem<N>::kTotal + 1024;
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_wide_kernel<N>), smem, smem_set);
         if (rc != SSD_OK) return rc;
-        chunk_state_wide_kernel<N><<<grid, kLaunchThreadsGroups, smem, stream>>>(map_x, map_m, map_st, q, cs, s, split,
-                                                                                 mode, status);
+        launch_chained(chunk_state_wide_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_m, map_st, q,
+                       cs, s, split, mode, status);
     }
     return launch_status();
 }

@@ -13,6 +13,7 @@
 // threads along a row and `rt` rows side by side (a row of a few hundred channels otherwise leaves most of
 // the CTA idle), kGateUnroll rows per thread at once, and row blocks small enough to give every SM several CTAs.
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 
 namespace ssd {
 
@@ -63,6 +64,8 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_skip_fwd_kernel(const float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ D, int d_mode,
                      const float* __restrict__ z, float* __restrict__ out, long long rows, int cols, int p_dim, int ct,
                      int rt, int rows_per_cta) {
+    after_previous();
+    allow_next();
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
     const int c = (blockIdx.x * ct + tx) * 4;
     if (c >= cols || ty >= rt) return;
@@ -111,6 +114,8 @@ gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y
                      const float* __restrict__ D, int d_mode, const float* __restrict__ z, float* __restrict__ dy,
                      float* __restrict__ dz, float* __restrict__ part, long long rows, int cols, int p_dim, int ct, int rt,
                      int rows_per_cta) {
+    after_previous();
+    allow_next();
     __shared__ float4 sums[kGateThreads];
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
     const int c = (blockIdx.x * ct + tx) * 4;
@@ -184,6 +189,8 @@ gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y
 // are added in order, then (per-head D) the channels.
 __global__ void gate_dd_reduce_kernel(const float* __restrict__ part, int row_blocks, int cols, int p_dim, int d_mode,
                                       int lanes, float* __restrict__ dD) {
+    after_previous();
+    allow_next();
     extern __shared__ double red[];
     const int h = blockIdx.x, p = threadIdx.x % p_dim, l = threadIdx.x / p_dim;
     double s = 0.0;
@@ -246,8 +253,8 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     }
     const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
     auto launch = [&](auto kernel) {
-        kernel<<<grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-            y, x, D, d_mode, z, out, rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta);
+        launch_plain(kernel, grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out,
+                     rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta);
     };
     if (d_mode != 0)
         z ? launch(gate_skip_fwd_kernel<true, true>) : launch(gate_skip_fwd_kernel<true, false>);
@@ -273,8 +280,8 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
     auto launch = [&](auto kernel) {
-        kernel<<<grid, kGateThreads, 0, st>>>(dout, y, x, D, d_mode, z, dy, dz, dD_partial, rows, cols, shape->headdim,
-                                              g.ct, g.rt, g.rows_per_cta);
+        launch_plain(kernel, grid, kGateThreads, 0, st, dout, y, x, D, d_mode, z, dy, dz, dD_partial, rows, cols,
+                     shape->headdim, g.ct, g.rt, g.rows_per_cta);
     };
     if (d_mode != 0)
         z ? launch(gate_skip_bwd_kernel<true, true>) : launch(gate_skip_bwd_kernel<true, false>);
@@ -284,8 +291,8 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
         const int p = shape->headdim;
         const int lanes = 1024 / p;
         const int threads = (lanes * p + 31) / 32 * 32;
-        gate_dd_reduce_kernel<<<shape->nheads, threads, threads * sizeof(double), st>>>(
-            dD_partial, static_cast<int>(g.rowblocks), cols, p, d_mode, lanes, dD);
+        launch_plain(gate_dd_reduce_kernel, shape->nheads, threads, threads * sizeof(double), st, dD_partial,
+                     static_cast<int>(g.rowblocks), cols, p, d_mode, lanes, dD);
     }
     return launch_status();
 }

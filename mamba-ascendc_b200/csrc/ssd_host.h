@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/ssd_b200.h"
 
@@ -75,6 +76,36 @@ int set_max_smem_once(const void* func, size_t bytes, std::atomic<uint64_t>& don
 // on 148 SMs) take 44 instead of 75 us in the output kernel and 27 instead of 64 us in the state kernel, with two and
 // four items per group.  A split has to promise 5% to be taken.
 int choose_head_split(int64_t items, int heads_per_group, int slots, int unit, int overhead_halves);
+
+// Kernel launches.  launch_chained: programmatic stream order -- the kernel may start while the one before it in the stream is
+// still running its last CTAs, and waits (after_previous, ssd_pdl.cuh) before it touches global memory, so that its start-up
+// (launch, barriers, tensor memory) lies under the tail of that kernel.  For kernels that fill an SM with one CTA: forward of
+// [4,2048,16,64,128] 85 -> 81 us, Vision network 2540 -> 2497 us.  Not for kernels of small CTAs: placed early, they pile up on
+// the SMs that are free first and stay there (with all kernels chained, prefill went from 137 to 145 us and the training
+// step at [8,4096,32] from 1027 to 1052); those use launch_plain.
+template <class... Expected, class... Args>
+inline void launch_config(bool chained, void (*kernel)(Expected...), dim3 grid, unsigned block, size_t smem,
+                          cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = dim3(block);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = chained ? 1 : 0;
+    (void)cudaLaunchKernelEx(&config, kernel, static_cast<Expected>(args)...);  // launch_status() picks an error up
+}
+template <class Kernel, class... Args>
+inline void launch_chained(Kernel kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_config(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+template <class Kernel, class... Args>
+inline void launch_plain(Kernel kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_config(false, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
 
 // Whether every pointer (null ones aside) takes 16-byte accesses.
 template <class... P>

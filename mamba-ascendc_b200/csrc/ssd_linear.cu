@@ -19,6 +19,7 @@
 // [16384,192] x [902,192]: 41 us (132 in the library); [16384,384] x [192,384] + residual: 25 us (65).  Measured and dropped:
 // 64-column tiles in three stages (46 and 30 us), CTAs starting at different tiles (no change).
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -58,6 +59,8 @@ __device__ __forceinline__ void split3_pair(float a, float b, uint32_t& hi, uint
 // w [cols, k] -> parts [3][cols_padded][k] bf16 (rows beyond cols are zero); one thread per pair.
 __global__ void __launch_bounds__(256)
 linear_split_kernel(const float* __restrict__ w, uint32_t* __restrict__ parts, int cols, int cols_padded, int k) {
+    after_previous();
+    allow_next();
     const size_t pairs = static_cast<size_t>(cols_padded) * k / 2;
     const size_t i = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
     if (i >= pairs) return;
@@ -103,7 +106,6 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         return;
     }
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         mbar_init(full_x, 1);
         mbar_init(x_ready, kLinWarps);
         for (int i = 0; i < 2; ++i) {
@@ -115,10 +117,13 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 512);
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {  // an earlier kernel gave up on a bounded wait: leave without doing work
         if (warp == 0) tmem_dealloc(tmem, 512);
         return;
@@ -308,15 +313,16 @@ extern "C" int ssd_linear_fwd(const float* x, const float* w, const float* resid
     if (rc != SSD_OK) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const size_t pairs = static_cast<size_t>(a.cols_padded) * k / 2;
-    linear_split_kernel<<<static_cast<unsigned>((pairs + 255) / 256), 256, 0, st>>>(w, static_cast<uint32_t*>(work), cols,
-                                                                                   a.cols_padded, k);
+    launch_plain(linear_split_kernel, static_cast<unsigned>((pairs + 255) / 256), 256, 0, st, w,
+                 static_cast<uint32_t*>(work), cols, a.cols_padded, k);
     rc = launch_status();
     if (rc != SSD_OK) return rc;
     static std::atomic<uint64_t> smem_set[kLinMaxBlocks];
     auto launch = [&](auto kernel, int b) {
         const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), lin_smem_bytes(b), smem_set[b - 1]);
         if (r != SSD_OK) return r;
-        kernel<<<dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(b), st>>>(map_x, map_w, a, status);
+        launch_chained(kernel, dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(b), st,
+                       map_x, map_w, a, status);
         return launch_status();
     };
     return blocks == 3 ? launch(linear_kernel<3>, 3) : blocks == 2 ? launch(linear_kernel<2>, 2) : launch(linear_kernel<1>, 1);

@@ -14,6 +14,7 @@
 // memory sixteen at a time.  One token of [16, 24, 64, 128] (25 MB of state in and out): 7.0 us = 3.6 TB/s, where the
 // padded tile route spent 165 us; [64, 128, 64, 64], 268 MB: 49 us = 5.5 TB/s.
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -35,6 +36,8 @@ struct RecArgs {
 template <int LPR>
 __global__ void __launch_bounds__(kRecThreads)
 recurrent_kernel(const RecArgs a, const SsdShape s, int row_blocks, int tokens_staged) {
+    after_previous();
+    allow_next();
     constexpr int kGroups = kRecThreads / LPR;
     constexpr int kCtaRows = kGroups * kRecRows;
     extern __shared__ __align__(16) float rec_smem[];
@@ -146,7 +149,7 @@ int launch_recurrent(const RecArgs& a, const SsdShape& s, cudaStream_t stream) {
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
     const int tokens = s.seqlen < kRecTokens ? s.seqlen : kRecTokens;
     const size_t smem = sizeof(float) * tokens * (2 * s.dstate + (a.z != nullptr ? 2 : 1) * kCtaRows + 2);
-    recurrent_kernel<LPR><<<static_cast<unsigned>(blocks), kRecThreads, smem, stream>>>(a, s, row_blocks, tokens);
+    launch_plain(recurrent_kernel<LPR>, static_cast<unsigned>(blocks), kRecThreads, smem, stream, a, s, row_blocks, tokens);
     return launch_status();
 }
 static_assert(sizeof(float) * kRecTokens * (2 * kRecMaxState + 2 * (kRecThreads / 8 * kRecRows) + 2) <= 48 * 1024,

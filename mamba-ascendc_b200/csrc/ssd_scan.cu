@@ -4,6 +4,7 @@
 //   state_passing_bwd       reverse recurrence, in place over the local dS, with d(cs_last) as well
 //   dt_finalize             [B,H,L] -> [B,L,H] transpose of ddt, fixed-order reductions of dA and d(dt_bias)
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -19,6 +20,8 @@ namespace {
 __global__ void __launch_bounds__(256)
 dt_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ dt_bias, const float* __restrict__ A,
                  float* __restrict__ q, float* __restrict__ cs, SsdShape s, int head_bits) {
+    after_previous();
+    allow_next();
     __shared__ float patch[kTile][33];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int k = blockIdx.x, h0 = blockIdx.y * 32, b = blockIdx.z;
@@ -89,6 +92,8 @@ template <bool REVERSE>
 __global__ void __launch_bounds__(kWalkThreads)
 state_walk_kernel(float* __restrict__ states, const float* __restrict__ cs, const float* __restrict__ start,
                   float* __restrict__ end, int nchunks, int n4, int seqlen, int headdim, int dstate4, size_t total) {
+    after_previous();
+    allow_next();
     const size_t idx = static_cast<size_t>(blockIdx.x) * kWalkThreads + threadIdx.x;
     if (idx >= total) return;
     const int pn4 = kStateRows * n4;
@@ -145,8 +150,8 @@ int launch_state_walk(const SsdShape& s, float* states, const float* cs, const f
     const size_t total = static_cast<size_t>(s.batch) * s.nheads * kStateRows * n4;
     const size_t blocks = (total + kWalkThreads - 1) / kWalkThreads;
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
-    state_walk_kernel<REVERSE><<<static_cast<unsigned>(blocks), kWalkThreads, 0, stream>>>(
-        states, cs, start, end, s.seqlen / kTile, n4, s.seqlen, s.headdim, s.dstate / 4, total);
+    launch_plain(state_walk_kernel<REVERSE>, static_cast<unsigned>(blocks), kWalkThreads, 0, stream, states, cs, start,
+                 end, s.seqlen / kTile, n4, s.seqlen, s.headdim, s.dstate / 4, total);
     return launch_status();
 }
 
@@ -158,6 +163,8 @@ int launch_state_walk(const SsdShape& s, float* states, const float* cs, const f
 __global__ void __launch_bounds__(256)
 state_fold_kernel(const float* __restrict__ terms, const float* __restrict__ cs, const float* __restrict__ start,
                   float* __restrict__ result, int nchunks, int pn4, int seqlen, size_t total, int reverse) {
+    after_previous();
+    allow_next();
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const size_t bh = idx / pn4;
@@ -191,6 +198,8 @@ __global__ void __launch_bounds__(1024)
 state_passing_bwd_kernel(float* __restrict__ dstates, const float* __restrict__ states_start,
                          const float* __restrict__ cs, const float* __restrict__ dfinal, float* __restrict__ g_last,
                          float* __restrict__ d_initial, int nchunks, int seqlen) {
+    after_previous();
+    allow_next();
     extern __shared__ float part[];  // [min(nchunks, kPartTiles)][32]: per-warp partial dot products
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t bh = blockIdx.x;
@@ -301,6 +310,8 @@ __global__ void __launch_bounds__(256)
 dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ part, float* __restrict__ ddt,
                    float* __restrict__ dA, float* __restrict__ ddt_bias, int batch, int nchunks, int nheads, int parts,
                    int tokens, int head_blocks, int head_bits) {
+    after_previous();
+    allow_next();
     __shared__ float patch[kTile][33];
     __shared__ double red[8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -381,8 +392,8 @@ extern "C" int ssd_dt_cumsum(const SsdShape* shape, const float* dt, const float
     if (rc != SSD_OK) return rc;
     if (!dt || !A || !q || !cs) return SSD_ERR_NULL;
     const dim3 grid(shape->seqlen / kTile, (shape->nheads + 31) / 32, shape->batch);
-    dt_cumsum_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(dt, dt_bias, A, q, cs, *shape,
-                                                                               head_bits_of(shape->nheads));
+    launch_plain(dt_cumsum_kernel, grid, 256, 0, reinterpret_cast<cudaStream_t>(stream), dt, dt_bias, A, q, cs, *shape,
+                 head_bits_of(shape->nheads));
     return launch_status();
 }
 
@@ -405,8 +416,8 @@ extern "C" int ssd_state_fold(const SsdShape* shape, const float* terms, const f
     const int pn4 = shape->headdim * shape->dstate / 4;
     const size_t total = static_cast<size_t>(shape->batch) * shape->nheads * pn4;
     const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    state_fold_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        terms, cs, start, result, shape->seqlen / kTile, pn4, shape->seqlen, total, reverse != 0);
+    launch_plain(state_fold_kernel, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream), terms, cs, start, result,
+                 shape->seqlen / kTile, pn4, shape->seqlen, total, reverse != 0);
     return launch_status();
 }
 
@@ -424,8 +435,8 @@ extern "C" int ssd_state_passing_bwd(const SsdShape* shape, float* dstates, cons
     const size_t part_bytes = static_cast<size_t>(nchunks < kPartTiles ? nchunks : kPartTiles) * 32 * sizeof(float);
     const bool lng = nchunks > kPartTiles;
     auto launch = [&](auto kernel) {
-        kernel<<<blocks, 1024, part_bytes, st>>>(dstates, states_start, cs, dfinal, g_last, d_initial, nchunks,
-                                                 shape->seqlen);
+        launch_plain(kernel, blocks, 1024, part_bytes, st, dstates, states_start, cs, dfinal, g_last, d_initial,
+                     nchunks, shape->seqlen);
     };
     if (shape->dstate == 64) {
         lng ? launch(state_passing_bwd_kernel<1, true>) : launch(state_passing_bwd_kernel<1, false>);
@@ -445,9 +456,9 @@ extern "C" int ssd_dt_finalize_bias_bwd(const SsdShape* shape, const float* ddt_
     const int nchunks = shape->seqlen / kTile, head_blocks = (heads + 31) / 32;
     const int64_t blocks = static_cast<int64_t>(shape->batch) * nchunks * head_blocks + heads;
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
-    dt_finalize_kernel<<<static_cast<unsigned>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        ddt_t, dA_partial, ddt, dA, ddt_bias, shape->batch, nchunks, heads, parts, row_tokens(*shape), head_blocks,
-        head_bits_of(heads));
+    launch_plain(dt_finalize_kernel, static_cast<unsigned>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+                 ddt_t, dA_partial, ddt, dA, ddt_bias, shape->batch, nchunks, heads, parts, row_tokens(*shape),
+                 head_blocks, head_bits_of(heads));
     return launch_status();
 }
 

@@ -24,6 +24,7 @@
 // which would add up over the tiles).  Parallelism is batch x groups CTAs, so the host uses this kernel
 // only when that fills the GPU; the tile-parallel pair ssd_chunk_state + ssd_state_passing_* stays for the rest.
 #include "ssd_host.h"
+#include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
 
 namespace ssd {
@@ -86,16 +87,18 @@ chunk_state_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     // An earlier kernel or CTA gave up on a bounded wait: leave without doing work.  Thread 0 alone reads the
     // status word and the whole CTA branches on its copy after the barrier below.
     if (tid == 0) {
-        tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
         for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
         mbar_init(bar_rdy, kSsWarps);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, 256);  // product [128 x 64] + up to three running pair states
+    after_previous();
+    if (tid == 0) tmem_slot[1] = static_cast<uint32_t>(*reinterpret_cast<volatile int*>(status));
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    allow_next();
     if (tmem_slot[1] != 0) {
         if (warp == 0) tmem_dealloc(tmem, 256);
         return;
@@ -299,7 +302,8 @@ int launch_state_scan(const SsdShape& s, const float* x, const float* m, const f
     rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_scan_kernel<MODE>), smem, smem_set);
     if (rc != SSD_OK) return rc;
     const dim3 grid(s.ngroups, s.batch);
-    chunk_state_scan_kernel<MODE><<<grid, kSsLaunch, smem, stream>>>(map_x, map_m, map_st, q, cs, start, end, s, status);
+    launch_plain(chunk_state_scan_kernel<MODE>, grid, kSsLaunch, smem, stream, map_x, map_m, map_st, q, cs, start, end,
+                 s, status);
     return launch_status();
 }
 
