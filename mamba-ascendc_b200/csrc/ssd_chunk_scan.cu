@@ -11,8 +11,8 @@
 //
 // S_h is the state at the start of the tile (from the state-passing kernel).  C, B, x and S are loaded by
 // TMA straight into their operand tiles' memory and split into bf16 hi/lo in place; W is built from the CB
-// accumulator in TMEM and reuses the dead B tile.  With dstate 64 the x and S tiles are double buffered,
-// so the next head's loads are in flight while this head computes.  The state product is issued as soon
+// accumulator in TMEM and reuses the dead B tile.  The x tiles and, with dstate 64, the S tiles
+// have a ring of buffers, so the next head's loads are in flight while this head computes.  The state product is issued as soon
 // as S is split and runs under the W pass; the output tile is staged in the dead x tile and written by TMA.
 #include "ssd_decay.cuh"
 #include "ssd_host.h"
@@ -25,7 +25,9 @@ namespace {
 
 template <int N>
 struct ChunkScanSmem {
-    static constexpr int kBuf = N == 64 ? 3 : 1;                      // x / S tile buffers (a ring)
+    static constexpr int kXBuf = N == 64 ? 3 : 2;                     // x tile buffers (a ring)
+    static constexpr int kSBuf = N == 64 ? 3 : 1;                     // S tile buffers (a ring)
+    static constexpr int kRowBuf = N == 64 ? 3 : 2;                   // row sets in rotation
     static constexpr int kOffBuf = N == 64 ? 2 : 1;                   // C*S accumulators
     static constexpr uint32_t kCTile = kTile * 128 * 2 * (N / 64);    // [128 x N]: N/64 blocks of (hi | lo)
     static constexpr uint32_t kXTile = kTile * 128 * 2;               // [128 x 64] (hi | lo)
@@ -33,13 +35,14 @@ struct ChunkScanSmem {
     static constexpr uint32_t kC = 0;
     static constexpr uint32_t kB = kC + kCTile;
     static constexpr uint32_t kX = kB + kCTile;
-    static constexpr uint32_t kS = kX + kBuf * kXTile;
-    static constexpr uint32_t kRows = kS + kBuf * kSTile;
+    static constexpr uint32_t kS = kX + kXBuf * kXTile;
+    static constexpr uint32_t kRows = kS + kSBuf * kSTile;
     static constexpr uint32_t kRowSet = 2 * kTile;              // cs[128], q[128]
-    static constexpr uint32_t kBars = kRows + 3 * kRowSet * 4;  // three row sets in rotation
+    static constexpr uint32_t kBars = kRows + kRowBuf * kRowSet * 4;
     static constexpr uint32_t kTotal = kBars + 256;
 };
-static_assert(ChunkScanSmem<64>::kTotal + 1024 <= 232448 && ChunkScanSmem<128>::kTotal + 1024 <= 232448,
+// No slack for re-aligning the base: the dynamic shared memory is declared 1024-byte aligned (and checked).
+static_assert(ChunkScanSmem<64>::kTotal <= 232448 && ChunkScanSmem<128>::kTotal <= 232448,
               "output kernel exceeds the shared memory of one SM");
 
 template <int N>
@@ -49,11 +52,12 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                   const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_copy, bool copy,
                   const float* __restrict__ q, const float* __restrict__ cs, SsdShape s, int split, int* status) {
     using L = ChunkScanSmem<N>;
-    constexpr int NB = L::kBuf;
+    constexpr int NX = L::kXBuf, NS = L::kSBuf, NR = L::kRowBuf;
+    static_assert(NX > 1, "x is prepared while the iteration before is with the tensor core");
+    constexpr bool kSAhead = NS > 1;  // S too
     constexpr int NOFF = L::kOffBuf;
     constexpr int kBlocks = N / 64;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = align1024(smem_raw);
+    extern __shared__ __align__(1024) uint8_t smem[];
     float* rows = reinterpret_cast<float*>(smem + L::kRows);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
     uint64_t* full_x = bars;          // [3] x tile has landed
@@ -70,14 +74,14 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     auto bar_rs = [&](int it) { return bars + 10 + 3 * (it & 1); };  // bars[10] and bars[13]
     uint64_t* bar_rw = bars + 11;     // W and x ready
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
-    uint64_t* rows_ready = bars + 14;  // [3] the rows of an iteration are published (set it % 3)
+    uint64_t* rows_ready = bars + 14;  // [NR] the rows of an iteration are published (set it % NR)
     uint64_t* rows_free = bars + 17;   // [3] every compute warp has finished with them
     // both products of a head done, once more per S buffer for the producer warp: the compute warps may finish
     // two heads while it is busy with a store, and a waiter that misses two completions of one barrier reads
     // the parity as "not yet" for ever; the next completion on a buffer's barrier needs the S tile that the
     // producer loads after this one
     uint64_t* bar_yp = bars + 23;      // [3]
-    uint64_t* staged = bars + 20;      // [3] the output tile is staged in x buffer it % NB (an mbarrier per buffer:
+    uint64_t* staged = bars + 20;      // [3] the output tile is staged in x buffer it % NX (an mbarrier per buffer:
                                        //     the compute warps may run up to two heads ahead of the producer warp)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -92,6 +96,10 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const int total = my_tiles * heads_per_group;
     const TileWalk walk(s, static_cast<int>(gridDim.x), split);
 
+    if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need the declared alignment
+        if (tid == 0) atomicCAS(status, 0, kStatusSmemAlign);
+        return;
+    }
     if (total <= 0) return;  // no work item for this CTA: leave before anything is allocated
     // An earlier kernel or CTA gave up on a bounded wait: leave without doing work.  Thread 0 alone reads the
     // status word and the whole CTA branches on its copy after the barrier below, so that no warp is ever
@@ -147,8 +155,8 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                                                 false);
                     umma_commit(bar_cb);
                 }
-                const uint32_t xb = smem_u32(smem + L::kX + (it % NB) * L::kXTile);
-                const uint32_t sb = smem_u32(smem + L::kS + (it % NB) * L::kSTile);
+                const uint32_t xb = smem_u32(smem + L::kX + (it % NX) * L::kXTile);
+                const uint32_t sb = smem_u32(smem + L::kS + (it % NS) * L::kSTile);
                 const Operand x{xb, xb + kHalf, kTile, true};
                 const Operand st{sb, sb + kSHalf, 64, false, 2 * kSHalf};
                 mbar_wait(bar_rs(it), (ps >> (it & 1)) & 1u, status, kStatusMmaTimeout | wait_site(3, 2));
@@ -160,7 +168,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 tc_fence_after_sync();
                 issue_gemm_split_ta<kTile / 16>(tm_diag, tm_whi, tm_wlo, x, 0, make_idesc_bf16(128, 64, false, true), false);
                 umma_commit(bar_y);
-                umma_commit(&bar_yp[it % NB]);
+                umma_commit(&bar_yp[it % NS]);
                 if (++hi == heads_per_group) hi = 0;
             }
         }
@@ -169,12 +177,12 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // tile; the coordinates of the next loads are ready before the wait.
         if (warp == kThreads / 32 + 1) {
             auto load_x = [&](int it, const HeadPos& w) {
-                tma_tile_tokens(smem + L::kX + (it % NB) * L::kXTile, &map_x, &full_x[it % NB], 0, w.h, w.tok, w.b);
+                tma_tile_tokens(smem + L::kX + (it % NX) * L::kXTile, &map_x, &full_x[it % NX], 0, w.h, w.tok, w.b);
             };
             auto load_s = [&](int it, const HeadPos& w) {
-                mbar_arrive_expect_tx(&full_s[it % NB], L::kSTile);
+                mbar_arrive_expect_tx(&full_s[it % NS], L::kSTile);
                 for (int cb = 0; cb < kBlocks; ++cb)
-                    tma_tile_2d(smem + L::kS + (it % NB) * L::kSTile + cb * 2 * kSHalf, 64, &map_s, &full_s[it % NB],
+                    tma_tile_2d(smem + L::kS + (it % NS) * L::kSTile + cb * 2 * kSHalf, 64, &map_s, &full_s[it % NS],
                                 64 * cb, w.tile_index * 64, false);
             };
             auto load_cb = [&](const HeadPos& w) {  // C and B of a tile
@@ -189,15 +197,15 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             int hi = 0;
             if (lane == 0) {
                 load_cb(walk.locate(cur, 0, 0));
-                for (int it = 0; it < NB && it < total; ++it) {
+                for (int it = 0; it < NX && it < total; ++it) {
                     const HeadPos w = walk.locate(cur, 0, it);
-                    load_s(it, w);
+                    if (it < NS) load_s(it, w);
                     load_x(it, w);
                 }
             }
             uint32_t pcb = 0;
             for (int it = 0; it < total; ++it) {
-                const HeadPos w0 = walk.locate(cur, hi, 0), wn = walk.locate(cur, hi, NB);
+                const HeadPos w0 = walk.locate(cur, hi, 0), wx = walk.locate(cur, hi, NX), ws = NX == NS ? wx : walk.locate(cur, hi, NS);
                 if (hi == 0) {
                     // CB of this tile exists: B has been read and C is in tensor memory, the next tile's may land
                     const HeadPos wt = walk.locate(cur, 0, heads_per_group);
@@ -207,23 +215,23 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                     if (lane == 0 && it + heads_per_group < total) load_cb(wt);
                 }
                 // both products of this head are done: the S buffer is free again
-                mbar_wait(&bar_yp[it % NB], static_cast<uint32_t>(it / NB) & 1u, status,
+                mbar_wait(&bar_yp[it % NS], static_cast<uint32_t>(it / NS) & 1u, status,
                           kStatusMmaTimeout | wait_site(3, 10));
                 tc_fence_after_sync();
-                if (lane == 0 && it + NB < total) load_s(it + NB, wn);
+                if (lane == 0 && it + NS < total) load_s(it + NS, ws);
                 // the compute warps have staged the output tile in this head's (dead) x tile
-                mbar_wait(&staged[it % NB], static_cast<uint32_t>(it / NB) & 1u, status,
+                mbar_wait(&staged[it % NX], static_cast<uint32_t>(it / NX) & 1u, status,
                           kStatusMmaTimeout | wait_site(3, 14));
                 if (lane == 0) {
                     if (*reinterpret_cast<volatile int*>(status) == 0) {
-                        const uint8_t* stage = smem + L::kX + (it % NB) * L::kXTile;
+                        const uint8_t* stage = smem + L::kX + (it % NX) * L::kXTile;
                         tma_store_tokens(&map_out, stage, 0, w0.h, w0.tok, w0.b, s.headdim);
                         if (copy) tma_store_tokens(&map_copy, stage, 0, w0.h, w0.tok, w0.b, s.headdim);
                         tma_store_commit();
                     }
-                    if (it + NB < total) {  // then the buffer can take the next x tile that maps to it
+                    if (it + NX < total) {  // then the buffer can take the next x tile that maps to it
                         tma_store_wait_read();
-                        load_x(it + NB, wn);
+                        load_x(it + NX, wx);
                     }
                 }
                 if (++hi == heads_per_group) {
@@ -233,7 +241,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             }
             if (lane == 0) tma_store_wait_all();
         }
-        // ---- warp 18 publishes the rows (cs, q) of iteration it + 3 into set it % 3 as soon as every compute
+        // ---- warp 18 publishes the rows (cs, q) of iteration it + NR into set it % NR as soon as every compute
         // warp has finished with iteration it; the values are fetched before the wait.
         if (warp == kThreads / 32 + 2) {
             TilePos cur = walk.first(static_cast<int>(blockIdx.x));
@@ -248,23 +256,23 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                 }
             };
             auto publish = [&](int it) {
-                float* set = rows + (it % 3) * L::kRowSet;
+                float* set = rows + (it % NR) * L::kRowSet;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     set[32 * j + lane] = c[j];
                     set[kTile + 32 * j + lane] = qv[j];
                 }
-                mbar_arrive(&rows_ready[it % 3]);
+                mbar_arrive(&rows_ready[it % NR]);
             };
-            for (int it = 0; it < 3 && it < total; ++it) {
+            for (int it = 0; it < NR && it < total; ++it) {
                 fetch(walk.locate(cur, 0, it));
                 publish(it);
             }
-            for (int it = 0; it + 3 < total; ++it) {
-                fetch(walk.locate(cur, hi, 3));
-                mbar_wait(&rows_free[it % 3], static_cast<uint32_t>(it / 3) & 1u, status,
+            for (int it = 0; it + NR < total; ++it) {
+                fetch(walk.locate(cur, hi, NR));
+                mbar_wait(&rows_free[it % NR], static_cast<uint32_t>(it / NR) & 1u, status,
                           kStatusMmaTimeout | wait_site(3, 11));
-                publish(it + 3);
+                publish(it + NR);
                 if (++hi == heads_per_group) {
                     hi = 0;
                     walk.advance(cur);
@@ -275,9 +283,9 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     reg_acquire<kProducedComputeRegs>();
 
-    auto x_tile = [&](int it) { return smem + L::kX + (it % NB) * L::kXTile; };
-    auto s_tile = [&](int it) { return smem + L::kS + (it % NB) * L::kSTile; };
-    auto row_set = [&](int it) { return rows + (it % 3) * L::kRowSet; };
+    auto x_tile = [&](int it) { return smem + L::kX + (it % NX) * L::kXTile; };
+    auto s_tile = [&](int it) { return smem + L::kS + (it % NS) * L::kSTile; };
+    auto row_set = [&](int it) { return rows + (it % NR) * L::kRowSet; };
 
     uint32_t p_c = 0, p_cb = 0;
     // A tile's B is split in place; its C goes to tensor memory (row t in lane t): the thread of row t takes
@@ -319,14 +327,14 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
 
     // S and x tiles of an iteration, split in place.  The state product starts as soon as S is split.
     auto prepare_s = [&](int it) {
-        const int bi = it % NB;
+        const int bi = it % NS;
         ok = mbar_wait(&full_s[bi], (ps >> bi) & 1u, status, kStatusTmaTimeout | wait_site(3, 5)) && ok;
         ps ^= 1u << bi;
         for (int cb = 0; cb < kBlocks; ++cb) split_tile_inplace(s_tile(it) + cb * 2 * kSHalf, 64, nullptr, warp, lane);
         signal_issuer(bar_rs(it), lane);
     };
     auto prepare_x = [&](int it) {
-        const int bi = it % NB;
+        const int bi = it % NX;
         ok = mbar_wait(&full_x[bi], (px >> bi) & 1u, status, kStatusTmaTimeout | wait_site(3, 6)) && ok;
         px ^= 1u << bi;
         // The causal decay exp(cs_i - cs_j), j <= i, is factored per block of 32 columns with the block's first
@@ -334,7 +342,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         // 32 tokens) is folded, with q, into the rows of the x tile here, so that the W pass multiplies a whole
         // block of a row by ONE scalar, with no table.  A block whose decay exceeds the fast limit (or whose cs
         // increases) is left unscaled and takes one exp per element in the pass.
-        ok = mbar_wait(&rows_ready[it % 3], static_cast<uint32_t>(it / 3) & 1u, status,
+        ok = mbar_wait(&rows_ready[it % NR], static_cast<uint32_t>(it / NR) & 1u, status,
                        kStatusMmaTimeout | wait_site(3, 12)) && ok;
         const float* set = row_set(it);
         const float b0 = set[32 * cg];  // rows 8 * warp .. 8 * warp + 7 lie in block warp / 4 = cg
@@ -344,10 +352,10 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         if (span >= 0.f && span < kDecayFastLimit) fx *= __expf(b0 - set[split_row]);
         split_tile_inplace_scaled(x_tile(it), kTile, fx, warp, lane);
     };
-    // With a ring of buffers an iteration's tiles are prepared while the tensor core works on the one before it
-    // (and their loads were issued two iterations earlier); with one buffer S is prepared before the W pass and x after it (its load flies during the pass).
+    // A tile with a ring of buffers is prepared while the tensor core works on the iteration before (its load was issued a
+    // ring's length earlier); the one S buffer of dstate 128 is prepared before the W pass.
     prepare_s(0);
-    if (NB > 1) prepare_x(0);
+    prepare_x(0);
     int hi = 0;
     for (int it = 0; it < total; ++it) {
         const float* cs_s = row_set(it);
@@ -358,7 +366,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             p_cb ^= 1;
             tc_fence_after_sync();
         }
-        if (NB == 1 && it > 0) prepare_s(it);
+        if (!kSAhead && it > 0) prepare_s(it);
 
         // ---- W from CB (the previous products are complete, so W's columns are free)
         {
@@ -366,11 +374,7 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             float v[32];
             if (cg <= qr) {
                 tmem_ld32(tmem_addr(tm_cb, warp, 32 * cg), v);
-                // this row's factor for its block of 32 columns (see prepare_x); with one buffer the rows of this
-                // iteration are waited for here first
-                if (NB == 1)
-                    ok = mbar_wait(&rows_ready[it % 3], static_cast<uint32_t>(it / 3) & 1u, status,
-                                   kStatusMmaTimeout | wait_site(3, 13)) && ok;
+                // this row's factor for its block of 32 columns (see prepare_x)
                 const float c0 = cs_s[32 * cg];
                 const float span = c0 - cs_s[32 * cg + 31];
                 const float csi = cs_s[t_row];
@@ -398,13 +402,12 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             tmem_st16(tmem_addr(tm_wlo, warp, 16 * cg), wlo);
             tmem_st_wait();
         }
-        if (NB == 1) prepare_x(it);
         signal_issuer(bar_rw, lane);  // W and x of this iteration are ready
 
         // ---- while the tensor core works: the next iteration's tiles (they sit in the other buffers) and,
         //      at the end of a tile, the next tile's B
-        if (NB > 1 && more_tiles) {
-            prepare_s(it + 1);
+        if (more_tiles) {
+            if (kSAhead) prepare_s(it + 1);
             prepare_x(it + 1);
         }
         if (last_of_tile && more_tiles) split_b();
@@ -429,10 +432,10 @@ chunk_scan_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
                     make_float4(d[i] + e * o[i], d[i + 1] + e * o[i + 1], d[i + 2] + e * o[i + 2], d[i + 3] + e * o[i + 3]);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&rows_free[it % 3]);  // this warp has finished with the iteration's rows
+        if (lane == 0) mbar_arrive(&rows_free[it % NR]);  // this warp has finished with the iteration's rows
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&staged[it % NB]);  // the producer warp writes the staged tile out
+        if (lane == 0) mbar_arrive(&staged[it % NX]);  // the producer warp writes the staged tile out
         if (++hi == heads_per_group) hi = 0;
     }
     tc_fence_before_sync();
@@ -451,7 +454,7 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
     if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_out, out, s, s.nheads, s.headdim);
     if (rc == SSD_OK) rc = make_tmap_f32_tokens(&map_copy, out_copy ? out_copy : out, s, s.nheads, s.headdim);
     if (rc != SSD_OK) return rc;
-    const size_t smem = ChunkScanSmem<N>::kTotal + 1024;
+    const size_t smem = ChunkScanSmem<N>::kTotal;
     static std::atomic<uint64_t> smem_set{0};  // one per instantiation
     rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_scan_kernel<N>), smem, smem_set);
     if (rc != SSD_OK) return rc;
