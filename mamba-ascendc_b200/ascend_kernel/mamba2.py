@@ -418,6 +418,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, dt, A, B, C, D, z, dt_softplus, initial_states, dt_bias, dt_min, dt_max):
+        ctx.set_materialize_grads(False)  # an output without a gradient takes no zeros, the kernels know a null
         ctx.shape = extents_shape(x, B, A.shape[0], dt_softplus, (dt_min, dt_max))
         ctx.recompute = _save_policy == "recompute"
         ctx.has_initial = initial_states is not None
