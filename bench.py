@@ -506,7 +506,7 @@ def run_gpu_arm(args) -> None:
     for name, s0, s1 in events:
         stage_ms.setdefault(name, []).append(s0.elapsed_time(s1))
     stage_avg = {k: sum(v) / len(v) for k, v in stage_ms.items()}
-    launches = len(events) + args.steps  # the finalisation stage launches two kernels
+    launches = len(events)  # one launch per stage at this shape
 
     # ---- end to end: pinned host inputs -> device -> forward + backward -> gradients to pinned host.
     # A three-stage pipeline over steps, as a host-side caller of the API would run it: the upload of

@@ -54,7 +54,7 @@ enum {
 /* Problem shape.  `tile` is the number of tokens one CTA treats as a chunk
  * (the results do not depend on it mathematically); the kernels need
  * tile == 128 and seqlen % tile == 0.  Supported: headdim == 64,
- * dstate in {64, 128}. */
+ * dstate in {64, 128} (64 in backward); with SSD_FLAG_EXTENTS what that flag says. */
 typedef struct SsdShape {
     int32_t batch;   /* B */
     int32_t seqlen;  /* L */
@@ -76,8 +76,8 @@ const char* ssd_error_string(int code);
 /* Shape validation shared by every entry point.  Mirrors the host checks of
  * mamba_ascendc/csrc/ops/mamba2_ssd_fwd/op_host/mamba2_ssd_fwd.cpp:59-112
  * (ranks, positivity, H % G == 0, chunk > 0) and adds this library's own
- * limits: SSD_ERR_UNSUPPORTED for headdim != 64, dstate not in {64, 128}, tile != 128 or a ragged
- * seqlen; SSD_ERR_RANGE for batch or ngroups above 65535 (grid dimensions) or for
+ * limits: SSD_ERR_UNSUPPORTED for headdim != 64 or dstate not in {64, 128} (with SSD_FLAG_EXTENTS: beyond 64 and 128, or no
+ * multiples of 4), tile != 128 or a ragged seqlen; SSD_ERR_RANGE for batch or ngroups above 65535 (grid dimensions) or for
  * batch * seqlen or batch * nheads * (seqlen / tile) * headdim at or above 2^31 (TMA coordinates). */
 int ssd_check_shape(const SsdShape* shape);
 

@@ -559,6 +559,8 @@ def _short_sequence(x, B, C, D, z, initial_states) -> bool:
     n = B.shape[3]
     if not (0 < x.shape[1] <= SHORT_SEQUENCE and 0 < n <= 128 and n % 4 == 0 and min(x.shape) > 0 and B.shape[2] > 0):
         return False
+    if x.shape[0] > 65535 or B.shape[2] > 65535 or x.shape[0] * x.shape[2] * ((x.shape[3] + 63) // 64) * 64 >= 1 << 31:
+        return False  # beyond the tile kernels' range: refused there
     if torch.autograd.forward_ad._current_level >= 0:  # tangents of D and z come from the framework's operations
         return False
     return not any(t is not None and t.data_ptr() & 15 for t in (B, C, initial_states))

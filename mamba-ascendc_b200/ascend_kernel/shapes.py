@@ -1,7 +1,10 @@
 """Shapes beyond what the tile kernels take, reduced to calls the kernels do take.
 
-The CUDA tile kernels handle headdim P = 64, state size N = 64 (forward and backward) or N = 128 (forward
-only) and a sequence length that is a multiple of 128.  The reference API accepts any shape: its generic
+The CUDA tile kernels compute on headdim P = 64, state size N = 64 or 128 and tiles of 128 tokens, and their tile loads cut
+tensors of other sizes off in steps of four floats (``mamba2._tile_extents``).  What is left comes here: sizes that are no
+multiples of four, headdims above 64 that are no multiples of 64, state sizes above 128, and addresses that are not
+16-byte aligned.  The kernels called from here handle P = 64, N = 64 (128 without gradients) and a sequence length that
+is a multiple of 128.  The reference API accepts any shape: its generic
 kernel covers what its Cube kernels do not (``mamba2_ssd_fwd.cpp:49-136``; shape matrix
 ``benchmarks/mamba2_shape_matrix.py:129-190``: P and N from 8 to 128, ragged L).  ``run_general`` maps every
 such call onto kernel calls with exact algebra, using differentiable torch operations only, so autograd

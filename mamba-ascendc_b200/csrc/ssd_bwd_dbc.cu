@@ -665,7 +665,7 @@ extern "C" int ssd_chunk_dbc_split_bwd(const SsdShape* shape, const float* x, co
     if (sms <= 0) return SSD_ERR_LAUNCH;
     if (tiles * split > 0x7fffffff) return SSD_ERR_RANGE;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
-    launch_chained(bwd_dbc_kernel, grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream), map_x,
+    launch_tiles(tiles, bwd_dbc_kernel, grid, kLaunchThreadsGroups, smem, reinterpret_cast<cudaStream_t>(stream), map_x,
                    map_b, map_c, map_dout, map_s, map_du, map_db, map_dc, q, cs, g_last, s, split, blocks, status);
     rc = launch_status();
     if (rc != SSD_OK || split == 1) return rc;

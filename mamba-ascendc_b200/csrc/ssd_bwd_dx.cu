@@ -522,7 +522,7 @@ extern "C" int ssd_chunk_dx_bwd(const SsdShape* shape, const float* x, const flo
     auto launch = [&](auto kernel, size_t smem, std::atomic<uint64_t>& smem_set) {
         const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), smem, smem_set);
         if (r != SSD_OK) return r;
-        launch_chained(kernel, grid, kLaunchThreadsGroups, smem, st, map_b, map_c, map_dout, map_out, map_du, map_dx,
+        launch_tiles(items * split, kernel, grid, kLaunchThreadsGroups, smem, st, map_b, map_c, map_dout, map_out, map_du, map_dx,
                        map_x, q, cs, dt, dt_bias, A, g_last, ddt_t, dA_partial, dout, D, d_mode, s, split, status);
         return launch_status();
     };

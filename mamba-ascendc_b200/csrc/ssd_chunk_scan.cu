@@ -464,7 +464,7 @@ int launch_chunk_scan(const SsdShape& s, const float* x, const float* bm, const 
     const int split = choose_head_split(items, s.nheads / s.ngroups, sms, 1, 2);
     const int64_t tiles = items * split;
     const dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));  // persistent: one CTA per SM walks its share of the tiles
-    launch_chained(chunk_scan_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_b, map_c, map_s, map_out,
+    launch_tiles(tiles, chunk_scan_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_b, map_c, map_s, map_out,
                    map_copy, out_copy != nullptr, q, cs, s, split, status);
     return launch_status();
 }

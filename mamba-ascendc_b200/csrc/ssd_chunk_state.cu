@@ -453,7 +453,7 @@ int launch_chunk_state(const SsdShape& s, const float* x, const float* m, const 
         static std::atomic<uint64_t> smem_set{0};
         rc = set_max_smem_once(reinterpret_cast<const void*>(chunk_state_wide_kernel<N>), smem, smem_set);
         if (rc != SSD_OK) return rc;
-        launch_chained(chunk_state_wide_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_m, map_st, q,
+        launch_tiles(items * split, chunk_state_wide_kernel<N>, grid, kLaunchThreadsGroups, smem, stream, map_x, map_m, map_st, q,
                        cs, s, split, mode, status);
     }
     return launch_status();

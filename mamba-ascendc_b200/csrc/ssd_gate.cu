@@ -42,6 +42,10 @@ GateGrid gate_grid(long long rows, int cols, int min_rows) {
     while (g.rows_per_cta / 2 >= least && (rows + g.rows_per_cta - 1) / g.rows_per_cta * g.colblocks < kGateCtasWanted)
         g.rows_per_cta /= 2;
     g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
+    while (g.rowblocks > 65535) {  // grid.y
+        g.rows_per_cta *= 2;
+        g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
+    }
     return g;
 }
 
@@ -246,11 +250,7 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     if (!y || !out || (d_mode != 0 && (!D || !x))) return SSD_ERR_NULL;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!aligned16(y, x, z, out, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
-    GateGrid g = gate_grid(rows, cols, 1);
-    while (g.rowblocks > 65535) {
-        g.rows_per_cta *= 2;
-        g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
-    }
+    const GateGrid g = gate_grid(rows, cols, 1);
     const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
     auto launch = [&](auto kernel) {
         launch_plain(kernel, grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out,
@@ -276,7 +276,6 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     if (!z && d_mode == 0) return SSD_OK;  // nothing to do
     if (!aligned16(dout, y, x, z, dy, dz, dD_partial, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(rows, cols, kGateMinRows);
-    if (g.rowblocks > 65535) return SSD_ERR_UNSUPPORTED;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
     auto launch = [&](auto kernel) {

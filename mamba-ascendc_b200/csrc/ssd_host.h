@@ -77,12 +77,13 @@ int set_max_smem_once(const void* func, size_t bytes, std::atomic<uint64_t>& don
 // four items per group.  A split has to promise 5% to be taken.
 int choose_head_split(int64_t items, int heads_per_group, int slots, int unit, int overhead_halves);
 
-// Kernel launches.  launch_chained: programmatic stream order -- the kernel may start while the one before it in the stream is
+// Kernel launches.  Chained: programmatic stream order -- the kernel may start while the one before it in the stream is
 // still running its last CTAs, and waits (after_previous, ssd_pdl.cuh) before it touches global memory, so that its start-up
-// (launch, barriers, tensor memory) lies under the tail of that kernel.  For kernels that fill an SM with one CTA: forward of
-// [4,2048,16,64,128] 85 -> 81 us, Vision network 2540 -> 2497 us.  Not for kernels of small CTAs: placed early, they pile up on
-// the SMs that are free first and stay there (with all kernels chained, prefill went from 137 to 145 us and the training
-// step at [8,4096,32] from 1027 to 1052); those use launch_plain.
+// (launch, barriers, tensor memory) lies under the tail of that kernel.  For kernels that fill an SM with one CTA (launch_tiles):
+// forward of [4,2048,16,64,128] 82.4 -> 77.7 us, its training step 258 -> 251 us, Vision network 2571 -> 2493 us, no difference at
+// [8,4096,32,64,64] (14 work items per SM), 1% slower at [8,4096,256,64,64] (110 per SM), where it is left out.  Not for kernels
+// of small CTAs (launch_plain): placed early, they pile up on the SMs that are free first and stay there (with all
+// kernels chained, prefill went from 137 to 145 us and the training step at [8,4096,32] from 1027 to 1052).
 template <class... Expected, class... Args>
 inline void launch_config(bool chained, void (*kernel)(Expected...), dim3 grid, unsigned block, size_t smem,
                           cudaStream_t stream, Args&&... args) {
@@ -98,9 +99,12 @@ inline void launch_config(bool chained, void (*kernel)(Expected...), dim3 grid, 
     config.numAttrs = chained ? 1 : 0;
     (void)cudaLaunchKernelEx(&config, kernel, static_cast<Expected>(args)...);  // launch_status() picks an error up
 }
+constexpr int kChainedItemsPerSm = 32;
 template <class Kernel, class... Args>
-inline void launch_chained(Kernel kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {
-    launch_config(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+inline void launch_tiles(int64_t items, Kernel kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t stream,
+                         Args&&... args) {
+    launch_config(items <= int64_t(kChainedItemsPerSm) * sm_count(), kernel, grid, block, smem, stream,
+                  std::forward<Args>(args)...);
 }
 template <class Kernel, class... Args>
 inline void launch_plain(Kernel kernel, dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args&&... args) {

@@ -321,7 +321,7 @@ extern "C" int ssd_linear_fwd(const float* x, const float* w, const float* resid
     auto launch = [&](auto kernel, int b) {
         const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), lin_smem_bytes(b), smem_set[b - 1]);
         if (r != SSD_OK) return r;
-        launch_chained(kernel, dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(b), st,
+        launch_tiles(row_tiles * items, kernel, dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(b), st,
                        map_x, map_w, a, status);
         return launch_status();
     };

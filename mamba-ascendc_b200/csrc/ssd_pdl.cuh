@@ -1,5 +1,5 @@
-// Device side of launch_chained (ssd_host.h).  Every kernel calls both, in every thread (the first returns at once in a kernel
-// launched plainly):
+// Device side of chained launches (launch_tiles, ssd_host.h).  Every kernel calls both, in every thread (the first returns at once in a kernel
+// launched without chaining):
 //
 //   after_previous()  before any access to global memory: returns when the kernel before it in the stream has finished and its
 //                     writes are visible.  Each kernel waits itself, so that its end implies the end of all before it.
