@@ -566,7 +566,7 @@ def _short_sequence(x, B, C, D, z, initial_states) -> bool:
     return not any(t is not None and t.data_ptr() & 15 for t in (B, C, initial_states))
 
 
-def _tile_extents(x, B, C, D, z, initial_states) -> bool:
+def _tile_extents(x, B, C, D, z, initial_states, grad: bool = False) -> bool:
     """Whether the tile kernels read and write the caller's tensors as they are: their tile loads and stores cut a tile off
     at the end of a sequence, of a head's channels and of the state's columns, in steps of four floats from 16-byte
     aligned addresses.  What this leaves (other headdims and state sizes) is padded or cut into blocks by shapes.py."""
@@ -575,8 +575,8 @@ def _tile_extents(x, B, C, D, z, initial_states) -> bool:
         return False
     if torch.autograd.forward_ad._current_level >= 0 and (p != 64 or x.shape[1] % TILE):
         return False  # tangents of D and z come from the framework's operations
-    if p == 64 and x.shape[1] % TILE == 0 and n in (64, 128):
-        return True  # the kernels' own sizes: nothing to fall back to
+    if p == 64 and x.shape[1] % TILE == 0 and (n == 64 or (n == 128 and not grad)):
+        return True  # the kernels' own sizes, which nothing pads or copies: unaligned addresses are refused
     return not any(t is not None and t.data_ptr() & 15 for t in (x, B, C, D, z, initial_states))
 
 
@@ -654,7 +654,7 @@ def mamba2_ssd_fwd(
             out, final = recurrent_forward(x, dt, A, B, C, bool(dt_softplus), return_final_state, initial_states, dt_bias,
                                            lim, D, z)
             return (out, final) if return_final_state else out
-        if _tile_extents(x, B, C, D, z, initial_states):
+        if _tile_extents(x, B, C, D, z, initial_states, grad_anywhere):
             return _tile_call(x, dt, A, B, C, D, z, dt_bias, bool(dt_softplus), lim, initial_states, return_final_state,
                               grad_anywhere)
         # any other headdim and state size, unaligned addresses: see shapes.py
