@@ -546,12 +546,13 @@ def _device_guard(device: torch.device):
 
 
 # Longest sequence that takes the recurrence kernel instead of the tile kernels (which treat 128 tokens at a time and so
-# cost the same for 1 token as for 128).  Device time of both, us, with D, z and an initial state:
-#   [batch, heads, P, N, G]     1 token      16 tokens    64 tokens    100 tokens
-#   [ 1,   4, 64,  64, 1]     3.4 /  47     8.7 /  47     29 /  47     45 /   47
-#   [16,  24, 64, 128, 1]     7.0 / 165      26 / 180     90 / 198    139 /  192
-#   [64, 128, 64,  64, 8]      49 / 397     208 / 516    753 / 875   1171 / 1083
-SHORT_SEQUENCE = 64
+# cost almost the same for 1 token as for 128).  Device time of both, us, with D, z and an initial state:
+#   [batch, heads, P, N, G]    16 tokens    32 tokens    48 tokens    64 tokens
+#   [ 1,   4, 64,  64, 1]     8.6 /  22     15 /  22     22 /  22     29 /  24
+#   [16,  24, 64, 128, 1]      26 /  58     48 /  59     70 /  59     91 /  59
+#   [ 8,  32, 64, 128, 1]      18 /  46     32 /  45     46 /  46     60 /  46
+#   [64, 128, 64,  64, 8]     212 / 456    391 / 487    570 / 516    753 / 539
+SHORT_SEQUENCE = 32
 
 
 def _short_sequence(x, B, C, D, z, initial_states) -> bool:
