@@ -77,15 +77,27 @@ def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: 
     return out
 
 
+def _plain_projection(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
+    """Whether ``layer(x)`` (+ residual) is what ssd_linear_fwd computes from these tensors: widths and shapes that fit, one
+    device, contiguous fp32.  Whatever does not fit is for the layer to take or to refuse."""
+    if type(layer) is not nn.Linear or layer.bias is not None or layer.weight.dim() != 2 or x.dim() < 1:
+        return False
+    w = layer.weight
+    n, k = w.shape
+    if x.shape[-1] != k or (residual is not None and residual.shape != (*x.shape[:-1], n)):
+        return False
+    if any(t.device != x.device or t.dtype != torch.float32 or not t.is_contiguous()
+           for t in (x, w, residual) if t is not None):
+        return False
+    return (not torch.is_autocast_enabled() and torch.get_float32_matmul_precision() == "highest" and
+            not (layer._forward_hooks or layer._forward_pre_hooks or _global_hooks()))
+
+
 def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``layer(x)`` (+ residual).  A plain bias-free fp32 projection in inference runs as ``ssd_linear_fwd`` (tensor cores at
     fp32 accuracy); anything else about the layer, the precision the caller chose or the sizes goes to the layer itself."""
-    capi = _kernels()
-    if (type(layer) is nn.Linear and layer.bias is None and _fast(x) and x.is_contiguous() and x.data_ptr() % 16 == 0 and
-            layer.weight.dtype == torch.float32 and layer.weight.is_contiguous() and layer.weight.is_cuda and
-            not torch.is_autocast_enabled() and torch.get_float32_matmul_precision() == "highest" and
-            not (layer._forward_hooks or layer._forward_pre_hooks or _global_hooks()) and
-            (residual is None or (residual.is_contiguous() and residual.dtype == torch.float32))):
+    if _fast(x) and _plain_projection(layer, x, residual) and x.data_ptr() % 16 == 0:
+        capi = _kernels()
         n, k = layer.weight.shape
         rows = x.numel() // k if k else 0
         if capi.lib.ssd_linear_pays(rows, n, k):

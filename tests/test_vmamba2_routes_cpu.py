@@ -1,0 +1,35 @@
+"""Which projections of the Vision block run as the library's own kernel, which takes bare pointers: decided by the layer and
+its tensors alone, so that tensors on the CPU stand in.  What is not taken goes to the layer."""
+import pytest
+import torch
+
+from ascend_kernel import vmamba2 as V
+
+
+def _layer(n=96, k=64, **kw):
+    return torch.nn.Linear(k, n, bias=False, **kw)
+
+
+@pytest.mark.parametrize("shape,residual,taken", [
+    ((3, 5, 64), None, True), ((64,), None, True), ((3, 5, 64), (3, 5, 96), True),
+    ((3, 5, 128), None, False),          # twice the layer's width: twice the rows
+    ((3, 5, 32), None, False),           # half of it
+    ((3, 5, 64), (96,), False),          # a residual that the framework would broadcast
+    ((3, 5, 64), (3, 1, 96), False),
+    ((3, 5, 64), (5, 3, 96), False),
+])
+def test_widths_and_residuals_that_fit(shape, residual, taken):
+    r = None if residual is None else torch.zeros(residual)
+    assert V._plain_projection(_layer(), torch.zeros(shape), r) is taken
+
+
+def test_a_width_that_does_not_fit_is_refused_by_the_layer():
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        V._linear(_layer(), torch.zeros(3, 128))
+
+
+@pytest.mark.parametrize("where", ["weight", "x", "residual"])
+def test_tensors_of_different_devices_are_left_to_the_layer(where):
+    dev = lambda name: "meta" if name == where else "cpu"  # noqa: E731
+    x, r = torch.zeros(3, 64, device=dev("x")), torch.zeros(3, 96, device=dev("residual"))
+    assert not V._plain_projection(_layer(device=dev("weight")), x, r)
