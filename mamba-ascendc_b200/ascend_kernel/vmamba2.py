@@ -89,7 +89,8 @@ def _plain_projection(layer: nn.Module, x: torch.Tensor, residual: Optional[torc
     if any(t.device != x.device or t.dtype != torch.float32 or not t.is_contiguous()
            for t in (x, w, residual) if t is not None):
         return False
-    return (not torch.is_autocast_enabled() and torch.get_float32_matmul_precision() == "highest" and
+    # (torch.get_float32_matmul_precision raises once a program has set the policy per backend)
+    return (not torch.is_autocast_enabled() and torch.backends.cuda.matmul.fp32_precision in ("none", "ieee") and
             not (layer._forward_hooks or layer._forward_pre_hooks or _global_hooks()))
 
 

@@ -33,3 +33,36 @@ def test_tensors_of_different_devices_are_left_to_the_layer(where):
     dev = lambda name: "meta" if name == where else "cpu"  # noqa: E731
     x, r = torch.zeros(3, 64, device=dev("x")), torch.zeros(3, 96, device=dev("residual"))
     assert not V._plain_projection(_layer(device=dev("weight")), x, r)
+
+
+@pytest.mark.parametrize("value,taken", [("ieee", True), ("none", True), ("tf32", False)])
+def test_the_precision_policy_of_either_interface_is_kept(value, taken):
+    matmul = torch.backends.cuda.matmul
+    before = matmul.fp32_precision
+    try:
+        matmul.fp32_precision = value
+        assert V._plain_projection(_layer(), torch.zeros(3, 64), None) is taken
+    finally:
+        matmul.fp32_precision = before
+    try:
+        torch.set_float32_matmul_precision("high")
+        assert not V._plain_projection(_layer(), torch.zeros(3, 64), None)
+    finally:
+        torch.set_float32_matmul_precision("highest")
+        matmul.fp32_precision = before
+
+
+def test_autocast_and_hooks_are_left_to_the_layer():
+    layer, x = _layer(), torch.zeros(3, 64)
+    try:
+        torch.set_autocast_enabled("cuda", True)
+        assert not V._plain_projection(layer, x, None)
+    finally:
+        torch.set_autocast_enabled("cuda", False)
+    handle = layer.register_forward_pre_hook(lambda *a: None)
+    assert not V._plain_projection(layer, x, None)
+    handle.remove()
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert not V._plain_projection(layer, x, None)
+    handle.remove()
+    assert V._plain_projection(layer, x, None)
