@@ -78,11 +78,15 @@ def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: 
 
 
 def _plain_projection(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
-    """Whether ``layer(x)`` (+ residual) is what ssd_linear_fwd computes from these tensors: widths and shapes that fit, one
-    device, contiguous fp32.  Whatever does not fit is for the layer to take or to refuse."""
-    if type(layer) is not nn.Linear or layer.bias is not None or layer.weight.dim() != 2 or x.dim() < 1:
-        return False
+    """Whether ``layer(x)`` (+ residual) is what ssd_linear_fwd computes from these tensors: plain tensors whose widths and
+    shapes fit, one device, contiguous fp32.  Whatever does not fit is for the layer to take or to refuse."""
     w = layer.weight
+    if type(layer) is not nn.Linear or "forward" in layer.__dict__ or layer.bias is not None or w.dim() != 2 or x.dim() < 1:
+        return False
+    # a subclass, or a tensor inside a function transform, need not have a storage of its own
+    if torch._C._are_functorch_transforms_active() or any(type(t) not in (torch.Tensor, nn.Parameter)
+                                                          for t in (x, w, residual) if t is not None):
+        return False
     n, k = w.shape
     if x.shape[-1] != k or (residual is not None and residual.shape != (*x.shape[:-1], n)):
         return False

@@ -66,3 +66,29 @@ def test_autocast_and_hooks_are_left_to_the_layer():
     assert not V._plain_projection(layer, x, None)
     handle.remove()
     assert V._plain_projection(layer, x, None)
+
+
+class _Wrapped(torch.Tensor):
+    """A tensor subclass, as quantisation and sharding libraries put in place of a weight."""
+
+
+def test_weights_and_inputs_without_storage_of_their_own_are_left_to_the_layer():
+    layer, x = _layer(), torch.zeros(3, 64)
+    layer.weight = torch.nn.Parameter(torch.zeros(96, 64).as_subclass(_Wrapped))
+    assert not V._plain_projection(layer, x, None)
+    assert not V._plain_projection(_layer(), x.as_subclass(_Wrapped), None)
+    assert not V._plain_projection(_layer(), x, torch.zeros(3, 96).as_subclass(_Wrapped))
+    taken, layer = [], _layer()
+
+    def of_one(row):
+        taken.append(V._plain_projection(layer, row, None))
+        return row
+
+    torch.func.vmap(of_one)(x)
+    assert taken == [False]
+
+
+def test_a_replaced_forward_is_kept():
+    layer = _layer()
+    layer.forward = lambda x: x
+    assert not V._plain_projection(layer, torch.zeros(3, 64), None)
