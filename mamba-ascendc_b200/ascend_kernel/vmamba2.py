@@ -119,6 +119,13 @@ def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] 
     return y if residual is None else residual + y
 
 
+def _per_head(t: torch.Tensor, device: torch.device, heads: int) -> bool:
+    """Whether the block kernels can read ``t`` as one fp32 value per head.  Other parameters stay with the framework and the
+    SSD call, which take or refuse them."""
+    return (type(t) in (torch.Tensor, nn.Parameter) and t.device == device and t.dtype == torch.float32 and
+            t.shape == (heads,) and t.is_contiguous())
+
+
 def _global_hooks() -> bool:
     m = torch.nn.modules.module
     return bool(m._global_forward_hooks or m._global_forward_pre_hooks)
@@ -161,8 +168,7 @@ class Mamba2Block(nn.Module):
         b, l, _ = u.shape
         d_in, g, n, h, p = cfg.d_inner, cfg.ngroups, cfg.d_state, cfg.nheads, cfg.headdim
         zxbcdt = _linear(self.in_proj, self.norm(u))
-        if (_fast(zxbcdt) and zxbcdt.is_contiguous() and cfg.d_conv == 4 and d_in <= 512 and
-                all(t.dtype == torch.float32 and t.is_contiguous() for t in (self.A_log, self.D))):
+        if _fast(zxbcdt) and zxbcdt.is_contiguous() and cfg.d_conv == 4 and d_in <= 512:
             return _linear(self.out_proj, self._fused_inner(zxbcdt, b, l), residual=u)
         z, xbc, dt = torch.split(zxbcdt, [d_in, d_in + 2 * g * n, h], dim=-1)
         xbc = F.silu(self.conv1d(xbc.transpose(1, 2))[..., :l].transpose(1, 2))
@@ -186,17 +192,25 @@ class Mamba2Block(nn.Module):
         cm = torch.empty(b, l, g, n, device=dev, dtype=torch.float32)
         w = self.conv1d.weight.view(-1, cfg.d_conv)
         bias = self.conv1d.bias
-        dt = torch.empty(b, l, h, device=dev, dtype=torch.float32)
-        A = torch.empty(h, device=dev, dtype=torch.float32)
+        if _per_head(self.A_log, dev, h):  # formed in the same launch, as is the copy of dt
+            dt = torch.empty(b, l, h, device=dev, dtype=torch.float32)
+            A = torch.empty(h, device=dev, dtype=torch.float32)
+            per_head = (self.A_log.data_ptr(), dt.data_ptr(), A.data_ptr(), h)
+        else:
+            dt, A = zxbcdt[..., 2 * d_in + 2 * g * n:].contiguous(), -torch.exp(self.A_log)
+            per_head = (None, None, None, 0)
+        a_log, dt_out, a_out, heads = per_head
         capi.check(capi.lib.ssd_block_conv_split_fwd(zxbcdt.data_ptr() + 4 * d_in, width, w.data_ptr(),
-                                                     None if bias is None else bias.data_ptr(), self.A_log.data_ptr(),
-                                                     x.data_ptr(), bm.data_ptr(), cm.data_ptr(), dt.data_ptr(),
-                                                     A.data_ptr(), b, l, d_in, g * n, h,
+                                                     None if bias is None else bias.data_ptr(), a_log, x.data_ptr(),
+                                                     bm.data_ptr(), cm.data_ptr(), dt_out, a_out, b, l, d_in, g * n, heads,
                                                      torch.cuda.current_stream().cuda_stream), "vmamba2_conv1d")
-        # the skip connection is added where the gated norm reads y anyway
-        y = self.ssd_fn(x, dt, A, bm, cm, cfg.chunk_size, dt_bias=self.dt_bias, dt_softplus=True).contiguous()
+        # a skip connection per head is added where the gated norm reads y anyway
+        skip = _per_head(self.D, dev, h)
+        y = self.ssd_fn(x, dt, A, bm, cm, cfg.chunk_size, D=None if skip else self.D, dt_bias=self.dt_bias,
+                        dt_softplus=True).contiguous()
         return _rmsnorm_kernel(y.data_ptr(), d_in, zxbcdt.data_ptr(), width, self.out_norm.weight, self.out_norm.eps,
-                               b * l, d_in, x.data_ptr(), self.D.data_ptr(), p).view(b, l, d_in)
+                               b * l, d_in, x.data_ptr() if skip else None, self.D.data_ptr() if skip else None,
+                               p).view(b, l, d_in)
 
 
 class VisionMamba2(nn.Module):

@@ -100,3 +100,29 @@ def test_fused_block_kernels_match_the_framework_operations():
     # shape errors come back as codes, nothing is launched
     assert _capi.lib.ssd_block_rmsnorm_fwd(y.data_ptr(), 8, None, 0, w.data_ptr(), out.data_ptr(), rows, d_in, 1e-5, st) == -2
     assert _capi.lib.ssd_block_rmsnorm_fwd(y.data_ptr(), 1024, None, 0, w.data_ptr(), out.data_ptr(), rows, 1024, 1e-5, st) == -3
+
+
+@pytest.mark.gpu
+def test_block_parameters_that_the_kernels_do_not_read():
+    """D per channel and a strided A_log go through the SSD call and the framework as before; a parameter left on the CPU
+    is an error."""
+    from ascend_kernel.vmamba2 import VisionMamba2, VisionMamba2Config
+
+    torch.manual_seed(3)
+    dev = torch.device("cuda:0")
+    net = VisionMamba2(VisionMamba2Config(image_size=320, depth=2, num_classes=16)).to(dev)
+    img = torch.randn(2, 3, 320, 320, device=dev)
+    blk = net.blocks[0]
+    blk.D = torch.nn.Parameter(torch.randn(6, 64, device=dev))
+    blk.A_log = torch.nn.Parameter(torch.rand(12, device=dev)[::2])
+    with torch.no_grad():
+        fused = net(img)
+    with torch.enable_grad():
+        plain = net(img).detach()
+    assert ((fused - plain).norm() / plain.norm()).item() < 1e-5
+    for name in ("D", "A_log"):
+        kept = getattr(blk, name)
+        setattr(blk, name, torch.nn.Parameter(torch.ones(6)))
+        with torch.no_grad(), pytest.raises(RuntimeError, match="must be a CUDA tensor"):
+            net(img)
+        setattr(blk, name, kept)

@@ -92,3 +92,13 @@ def test_a_replaced_forward_is_kept():
     layer = _layer()
     layer.forward = lambda x: x
     assert not V._plain_projection(layer, torch.zeros(3, 64), None)
+
+
+@pytest.mark.parametrize("t,taken", [
+    (torch.ones(6), True), (torch.nn.Parameter(torch.ones(6)), True),
+    (torch.ones(6, 64), False), (torch.ones(1), False), (torch.ones(()), False), (torch.ones(12)[::2], False),
+    (torch.ones(6, dtype=torch.float64), False), (torch.ones(6, device="meta"), False),
+    (torch.ones(6).as_subclass(_Wrapped), False),
+])
+def test_per_head_parameters_that_the_block_kernels_read(t, taken):
+    assert V._per_head(t, torch.device("cpu"), 6) is taken
