@@ -67,13 +67,19 @@ def _fast(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dtype == torch.float32 and not torch.is_grad_enabled() and _kernels() is not None
 
 
+def _launch(name: str, device: torch.device, fn: Callable, *args) -> None:
+    """``fn(*args, stream)`` on the tensors' device, which need not be the current one, and its current stream."""
+    from .mamba2 import _device_guard
+
+    with _device_guard(device):
+        _kernels().check(fn(*args, torch.cuda.current_stream().cuda_stream), name)
+
+
 def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: torch.Tensor, eps: float, rows: int,
                     d: int, skip=None, D=None, headdim: int = 0) -> torch.Tensor:
-    capi = _kernels()
     out = torch.empty(rows, d, device=weight.device, dtype=torch.float32)
-    capi.check(capi.lib.ssd_block_skip_rmsnorm_fwd(x2d, x_stride, skip, D, headdim, z, z_stride, weight.data_ptr(),
-                                                   out.data_ptr(), rows, d, eps,
-                                                   torch.cuda.current_stream().cuda_stream), "vmamba2_rmsnorm")
+    _launch("vmamba2_rmsnorm", weight.device, _kernels().lib.ssd_block_skip_rmsnorm_fwd, x2d, x_stride, skip, D, headdim, z,
+            z_stride, weight.data_ptr(), out.data_ptr(), rows, d, eps)
     return out
 
 
@@ -110,10 +116,9 @@ def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] 
 
             work = torch.empty(capi.lib.ssd_linear_work_bytes(n, k), device=x.device, dtype=torch.uint8)
             out = torch.empty(*x.shape[:-1], n, device=x.device, dtype=torch.float32)
-            capi.check(capi.lib.ssd_linear_fwd(x.data_ptr(), layer.weight.data_ptr(),
-                                               None if residual is None else residual.data_ptr(), out.data_ptr(), rows, n,
-                                               k, work.data_ptr(), _status(x.device).data_ptr(),
-                                               torch.cuda.current_stream().cuda_stream), "vmamba2_linear")
+            _launch("vmamba2_linear", x.device, capi.lib.ssd_linear_fwd, x.data_ptr(), layer.weight.data_ptr(),
+                    None if residual is None else residual.data_ptr(), out.data_ptr(), rows, n, k, work.data_ptr(),
+                    _status(x.device).data_ptr())
             return out
     y = layer(x)
     return y if residual is None else residual + y
@@ -183,7 +188,7 @@ class Mamba2Block(nn.Module):
     def _fused_inner(self, zxbcdt: torch.Tensor, b: int, l: int) -> torch.Tensor:
         """conv1d + SiLU + split, SSD, gated norm on the fused kernels; z, xBC and dt are read as column slices of
         the in_proj output where they lie."""
-        cfg, capi = self.cfg, _kernels()
+        cfg = self.cfg
         d_in, g, n, h, p = cfg.d_inner, cfg.ngroups, cfg.d_state, cfg.nheads, cfg.headdim
         width = zxbcdt.shape[-1]
         dev = zxbcdt.device
@@ -195,15 +200,13 @@ class Mamba2Block(nn.Module):
         if _per_head(self.A_log, dev, h):  # formed in the same launch, as is the copy of dt
             dt = torch.empty(b, l, h, device=dev, dtype=torch.float32)
             A = torch.empty(h, device=dev, dtype=torch.float32)
-            per_head = (self.A_log.data_ptr(), dt.data_ptr(), A.data_ptr(), h)
+            a_log, dt_out, a_out, heads = self.A_log.data_ptr(), dt.data_ptr(), A.data_ptr(), h
         else:
             dt, A = zxbcdt[..., 2 * d_in + 2 * g * n:].contiguous(), -torch.exp(self.A_log)
-            per_head = (None, None, None, 0)
-        a_log, dt_out, a_out, heads = per_head
-        capi.check(capi.lib.ssd_block_conv_split_fwd(zxbcdt.data_ptr() + 4 * d_in, width, w.data_ptr(),
-                                                     None if bias is None else bias.data_ptr(), a_log, x.data_ptr(),
-                                                     bm.data_ptr(), cm.data_ptr(), dt_out, a_out, b, l, d_in, g * n, heads,
-                                                     torch.cuda.current_stream().cuda_stream), "vmamba2_conv1d")
+            a_log, dt_out, a_out, heads = None, None, None, 0
+        _launch("vmamba2_conv1d", dev, _kernels().lib.ssd_block_conv_split_fwd, zxbcdt.data_ptr() + 4 * d_in, width,
+                w.data_ptr(), None if bias is None else bias.data_ptr(), a_log, x.data_ptr(), bm.data_ptr(), cm.data_ptr(),
+                dt_out, a_out, b, l, d_in, g * n, heads)
         # a skip connection per head is added where the gated norm reads y anyway
         skip = _per_head(self.D, dev, h)
         y = self.ssd_fn(x, dt, A, bm, cm, cfg.chunk_size, D=None if skip else self.D, dt_bias=self.dt_bias,

@@ -102,3 +102,26 @@ def test_a_replaced_forward_is_kept():
 ])
 def test_per_head_parameters_that_the_block_kernels_read(t, taken):
     assert V._per_head(t, torch.device("cpu"), 6) is taken
+
+
+def test_kernels_run_on_the_device_and_stream_of_their_tensors(monkeypatch):
+    import contextlib
+    from types import SimpleNamespace
+
+    from ascend_kernel import mamba2 as M
+
+    current = ["cuda:0"]
+
+    @contextlib.contextmanager
+    def guard(device):
+        before, current[0] = current[0], str(device)
+        yield
+        current[0] = before
+
+    monkeypatch.setattr(M, "_device_guard", guard)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream="stream of " + current[0]))
+    calls = []
+    V._launch("norm", torch.device("cuda:1"), lambda *a: calls.append(a) or 0, 7)
+    assert calls == [(7, "stream of cuda:1")] and current == ["cuda:0"]
+    with pytest.raises(RuntimeError):
+        V._launch("norm", torch.device("cuda:1"), lambda *a: -3)
