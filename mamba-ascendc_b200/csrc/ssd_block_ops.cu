@@ -122,14 +122,15 @@ struct ConvArgs {
 };
 
 __global__ void __launch_bounds__(128)
-block_conv_silu_kernel(const ConvArgs a) {
+block_conv_silu_kernel(const ConvArgs a, unsigned channel_blocks) {
     after_previous();
     allow_next();
     const int channels = a.d_in + 2 * a.gn;
-    const int c = blockIdx.x * 128 + threadIdx.x;
+    const unsigned token_block = blockIdx.x / channel_blocks;  // in one dimension: as many tokens as an int counts
+    const int c = (blockIdx.x - token_block * channel_blocks) * 128 + threadIdx.x;
     if (c >= channels + a.heads) return;
-    const int t0 = blockIdx.y * kConvTokens;
-    const long long b = blockIdx.z;
+    const int t0 = token_block * kConvTokens;
+    const long long b = blockIdx.y;
     const float* src = a.xbc + (b * a.seqlen) * a.row_stride + c;
     float in[kConvTokens + 3];  // inputs from three tokens back on
 #pragma unroll
@@ -147,7 +148,7 @@ block_conv_silu_kernel(const ConvArgs a) {
         dst = a.c_out, width = a.gn, col = c - a.d_in - a.gn;
     } else {
         dst = a.dt_out, width = a.heads, col = c - channels;
-        if (blockIdx.y == 0 && blockIdx.z == 0) a.a_out[col] = -expf(a.a_log[col]);
+        if (token_block == 0 && b == 0) a.a_out[col] = -expf(a.a_log[col]);
     }
     dst += (b * a.seqlen) * width + col;
     const int n = min(kConvTokens, a.seqlen - t0);
@@ -203,10 +204,13 @@ extern "C" int ssd_block_conv_split_fwd(const float* xbc, long long row_stride, 
     if (!xbc || !weight || !x_out || !b_out || !c_out || (heads > 0 && (!a_log || !dt_out || !a_out))) return SSD_ERR_NULL;
     if (batch <= 0 || seqlen <= 0 || d_in <= 0 || gn <= 0 || heads < 0 || row_stride < d_in + 2 * gn + heads)
         return SSD_ERR_SHAPE;
-    if (batch > 65535 || (seqlen + kConvTokens - 1) / kConvTokens > 65535) return SSD_ERR_RANGE;
+    const long long channel_blocks = (static_cast<long long>(d_in) + 2ll * gn + heads + 127) / 128;
+    const long long blocks = channel_blocks * ((static_cast<long long>(seqlen) + kConvTokens - 1) / kConvTokens);
+    if (batch > 65535 || seqlen > 0x7fffffff - 2 * kConvTokens || blocks > 0x7fffffff) return SSD_ERR_RANGE;
     const ConvArgs a{xbc, weight, bias, a_log, x_out, b_out, c_out, dt_out, a_out, row_stride, seqlen, d_in, gn, heads};
-    const dim3 grid((d_in + 2 * gn + heads + 127) / 128, (seqlen + kConvTokens - 1) / kConvTokens, batch);
-    launch_plain(block_conv_silu_kernel, grid, 128, 0, reinterpret_cast<cudaStream_t>(stream), a);
+    const dim3 grid(static_cast<unsigned>(blocks), batch);
+    launch_plain(block_conv_silu_kernel, grid, 128, 0, reinterpret_cast<cudaStream_t>(stream), a,
+                 static_cast<unsigned>(channel_blocks));
     return launch_status();
 }
 

@@ -126,3 +126,25 @@ def test_block_parameters_that_the_kernels_do_not_read():
         with torch.no_grad(), pytest.raises(RuntimeError, match="must be a CUDA tensor"):
             net(img)
         setattr(blk, name, kept)
+
+
+@pytest.mark.gpu
+def test_convolution_of_more_than_a_million_tokens():
+    import torch.nn.functional as F
+
+    from ascend_kernel import _capi
+
+    dev = torch.device("cuda:0")
+    l, d_in, gn, heads = (1 << 20) + 33, 3, 2, 2  # more blocks of tokens than one grid dimension of 65535 holds
+    channels = d_in + 2 * gn
+    wide = torch.randn(1, l, channels + heads, device=dev)
+    weight, bias, a_log = torch.randn(channels, 1, 4, device=dev), torch.randn(channels, device=dev), torch.randn(heads, device=dev)
+    x, b, c, dt, a = (torch.empty(s, device=dev) for s in ((1, l, d_in), (1, l, gn), (1, l, gn), (1, l, heads), (heads,)))
+    _capi.check(_capi.lib.ssd_block_conv_split_fwd(
+        wide.data_ptr(), channels + heads, weight.data_ptr(), bias.data_ptr(), a_log.data_ptr(), x.data_ptr(), b.data_ptr(),
+        c.data_ptr(), dt.data_ptr(), a.data_ptr(), 1, l, d_in, gn, heads, torch.cuda.current_stream().cuda_stream), "conv")
+    src = F.pad(wide[..., :channels].double(), (0, 0, 3, 0))
+    w = weight.double()[:, 0]
+    want = F.silu(sum(src[:, k:k + l] * w[:, k] for k in range(4)) + bias.double())
+    assert torch.allclose(torch.cat([x, b, c], dim=-1).double(), want, rtol=1e-5, atol=1e-5)
+    assert torch.equal(dt, wide[..., channels:]) and torch.allclose(a, -a_log.exp())
