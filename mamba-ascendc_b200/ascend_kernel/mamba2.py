@@ -555,6 +555,17 @@ def _device_guard(device: torch.device):
 SHORT_SEQUENCE = 32
 
 
+def _own_sizes(x, B, grad: bool) -> bool:
+    """The kernels' own sizes, which nothing pads, copies or cuts off."""
+    return x.shape[3] == 64 and x.shape[1] % TILE == 0 and (B.shape[3] == 64 or (B.shape[3] == 128 and not grad))
+
+
+def _in_transform() -> bool:
+    """Whether forward-mode derivatives or a function transform (vmap, grad, jvp) are being taken, which see framework
+    operations only.  Away from the kernels' own sizes D and z are then applied by such operations."""
+    return torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+
+
 def _short_sequence(x, B, C, D, z, initial_states) -> bool:
     """Whether a call without gradients runs as one recurrence launch (ssd_recurrent_fwd)."""
     n = B.shape[3]
@@ -562,7 +573,7 @@ def _short_sequence(x, B, C, D, z, initial_states) -> bool:
         return False
     if x.shape[0] > 65535 or B.shape[2] > 65535 or x.shape[0] * x.shape[2] * ((x.shape[3] + 63) // 64) * 64 >= 1 << 31:
         return False  # beyond the tile kernels' range: refused there
-    if torch.autograd.forward_ad._current_level >= 0:  # tangents of D and z come from the framework's operations
+    if _in_transform():
         return False
     return not any(t is not None and t.data_ptr() & 15 for t in (B, C, initial_states))
 
@@ -574,10 +585,10 @@ def _tile_extents(x, B, C, D, z, initial_states, grad: bool = False) -> bool:
     p, n = x.shape[3], B.shape[3]
     if min(x.shape) <= 0 or min(B.shape) <= 0 or n % 4 or n > 128 or p > 1024 or (p % 64 if p > 64 else p % 4):
         return False
-    if torch.autograd.forward_ad._current_level >= 0 and (p != 64 or x.shape[1] % TILE):
-        return False  # tangents of D and z come from the framework's operations
-    if p == 64 and x.shape[1] % TILE == 0 and (n == 64 or (n == 128 and not grad)):
-        return True  # the kernels' own sizes, which nothing pads or copies: unaligned addresses are refused
+    if _own_sizes(x, B, grad):
+        return True  # unaligned addresses are refused
+    if _in_transform():
+        return False
     return not any(t is not None and t.data_ptr() & 15 for t in (x, B, C, D, z, initial_states))
 
 

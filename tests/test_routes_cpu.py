@@ -44,3 +44,30 @@ def test_sizes_of_the_recurrence():
     assert not taken(1, 2, 2, 64, 1, 132) and not taken(1, 2, 2, 64, 1, 64, "B") and not taken(0, 2, 2, 64, 1, 64)
     x = torch.empty(65536, 1, 1, 1)  # a batch beyond the range of the tile kernels is refused there
     assert not M._short_sequence(x, torch.empty(65536, 1, 1, 4), torch.empty(65536, 1, 1, 4), None, None, None)
+
+
+@pytest.mark.parametrize("l,p,n,grad,taken", [
+    (128, 64, 64, False, True), (128, 64, 64, True, True), (128, 64, 128, False, True),  # always without the framework
+    (128, 64, 128, True, False), (128, 64, 32, False, False), (128, 64, 96, False, False), (128, 64, 32, True, False),
+    (200, 64, 64, False, False), (128, 32, 64, False, False), (128, 128, 64, False, False),
+])
+def test_derivatives_of_the_framework_epilogue(l, p, n, grad, taken):
+    """Under forward-mode derivatives and function transforms D and z stay framework operations wherever they were."""
+    t = _tensors(1, l, 2, p, 1, n)
+    assert M._tile_extents(**t, grad=grad)
+    seen = []
+
+    def inside(z):
+        seen.append(M._tile_extents(**dict(t, z=z), grad=grad))
+        s = _tensors(1, 4, 2, p, 1, n)
+        seen.append(M._short_sequence(s["x"], s["B"], s["C"], s["D"], s["z"], s["initial_states"]))
+        return z.sum()
+
+    with torch.autograd.forward_ad.dual_level():
+        inside(torch.autograd.forward_ad.make_dual(t["z"], t["z"]))
+    torch.func.jvp(inside, (t["z"],), (t["z"],))
+    assert seen == [taken, False] * 2
+    if not taken:
+        torch.func.vmap(inside)(t["z"][None])
+        torch.func.grad(inside)(t["z"])
+        assert seen == [False] * 8

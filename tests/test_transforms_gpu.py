@@ -1,0 +1,47 @@
+"""Derivatives that the framework takes of the D skip connection and the z gate, at sizes where these are framework
+operations under a transform: forward mode, vmap and function gradients, against the closed form on the SSD output.
+
+Tolerance: both sides start from the same SSD output, up to the fp32 rounding of the element-wise operations: 1e-5."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(2, 256, 3, 64, 32, 1), (1, 128, 2, 64, 96, 2), (1, 200, 2, 64, 64, 1), (2, 5, 2, 64, 64, 1), (1, 128, 2, 32, 64, 1)]
+
+
+def _case(shape):
+    from ascend_kernel import mamba2_ssd_fwd
+
+    b, l, h, p, n, g = shape
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    x, dt, A, B, C = rnd(b, l, h, p), rnd(b, l, h).abs(), -rnd(h).abs(), rnd(b, l, g, n), rnd(b, l, g, n)
+    call = lambda D, z: mamba2_ssd_fwd(x, dt, A, B, C, 64, D=D, z=z, dt_softplus=True)  # noqa: E731
+    y = call(None, None)
+
+    def closed(D, z):
+        return (y + x * D.view(1, 1, -1, 1)) * F.silu(z)
+
+    return call, closed, rnd(h), rnd(b, l, h, p), rnd(h), rnd(b, l, h, p)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_transforms_of_the_skip_connection_and_the_gate(shape):
+    import torch.autograd.forward_ad as fwd
+
+    call, closed, D, z, tD, tz = _case(shape)
+    want = torch.func.jvp(closed, (D, z), (tD, tz))
+    close = lambda a, b: ((a - b).norm() <= 1e-5 * b.norm()).item()  # noqa: E731
+    with torch.no_grad(), fwd.dual_level():
+        out = fwd.unpack_dual(call(fwd.make_dual(D, tD), fwd.make_dual(z, tz)))
+        assert out.tangent is not None and close(out.primal, want[0]) and close(out.tangent, want[1])
+    with torch.no_grad():
+        got = torch.func.jvp(call, (D, z), (tD, tz))
+        assert close(got[0], want[0]) and close(got[1], want[1])
+        stack = torch.stack([D, tD]), torch.stack([z, tz])
+        assert close(torch.func.vmap(call)(*stack), torch.func.vmap(closed)(*stack))
+    for arg in (0, 1):
+        got, ref = (torch.func.grad(lambda *a: fn(*a).sum(), argnums=arg)(D, z) for fn in (call, closed))
+        assert close(got, ref)
