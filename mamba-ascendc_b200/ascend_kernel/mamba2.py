@@ -343,6 +343,31 @@ def gate_backward(dout, y, x, B, D, z, heads: Optional[int] = None):
     return dy, dz, dD
 
 
+def _per_channel(D, x, heads: int):
+    """D for x [B,L,heads * parts,64 or less] (parts > 1: several heads of x for each of D[H])."""
+    if D is None or D.dim() == 2:
+        return D
+    return D.repeat_interleave(x.shape[2] // heads).unsqueeze(-1) if x.shape[2] != heads else D.unsqueeze(-1)
+
+
+def _epilogue(y, x, D, z, heads: int):
+    """out = (y + D .* x) .* silu(z) as framework operations."""
+    out = y if D is None else y + x * _per_channel(D, x, heads)
+    return out if z is None else out * torch.nn.functional.silu(z)
+
+
+def _epilogue_gradients(dout, y, x, D, z, heads: int):
+    """(dz, dD) of the epilogue as framework operations; y and x are constants."""
+    dy, dz, dD = dout, None, None
+    if z is not None:
+        s = torch.sigmoid(z)
+        dy, dz = dout * (z * s), dout * _epilogue(y, x, D, None, heads) * (s * (1 + z * (1 - s)))
+    if D is not None:
+        dD = (dy * x).sum(dim=(0, 1))
+        dD = dD if D.dim() == 2 else dD.reshape(heads, -1).sum(-1)
+    return dz, dD
+
+
 # ----------------------------------------------------------------------------- whole calls
 # The stages of one direction as one foreign call (ssd_forward, ssd_backward).  While stage_events collects, the same
 # stages are launched one by one with events around them.
@@ -425,33 +450,64 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         # Without an epilogue the output is what backward needs.  At the kernels' own sizes it is saved itself, so that
         # changing it in place is an error in backward; elsewhere the caller may change it, and a copy is saved.
         own_sizes = x.shape[3] == 64 and B.shape[3] == 64 and x.shape[1] % TILE == 0 and x.shape[2] == A.shape[0]
-        copy = D is None and z is None and not ctx.recompute and not own_sizes
+        gated = D is not None or z is not None
+        ctx.differentiable = gated and not own_sizes  # see differentiable_backward
+        ctx.options = (dt_softplus, dt_min, dt_max)
+        copy = not gated and not ctx.recompute and not own_sizes
         out, final, y, work = forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, ctx.shape, True, copy=copy)
+        start = initial_states if ctx.recompute or ctx.differentiable else None
         if ctx.recompute:  # inputs only; y, q, cs and the tile-start states are rebuilt in backward
-            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, initial_states)
+            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start)
         else:
-            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, y, *work)
+            ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start, y, *work)
         return out, final
 
     @staticmethod
     def backward(ctx, dout, dfinal):
-        if ctx.recompute:
-            x, dt, A, B, C, dt_bias, D, z, initial_states = ctx.saved_tensors
-        else:
-            x, dt, A, B, C, dt_bias, D, z, y, *work = ctx.saved_tensors
+        x, dt, A, B, C, dt_bias, D, z, initial_states, *rest = ctx.saved_tensors
+        y, work = (rest[0], rest[1:]) if rest else (None, None)
         if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
             dout = torch.zeros_like(x)
-        dout = _aligned(dout)
-        if dfinal is not None:
-            dfinal = _aligned(dfinal)
+        alone = not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9))  # D and z alone need gradients
+        again = ctx.differentiable and (torch.is_grad_enabled() or (alone and torch._C._are_functorch_transforms_active()))
+        if again and not alone:
+            return _Mamba2SsdAutograd.differentiable_backward(ctx, dout, dfinal)
+        if not again:
+            dout = _aligned(dout)
+            if dfinal is not None:
+                dfinal = _aligned(dfinal)
         with _device_guard(x.device):
-            if ctx.recompute:
+            if y is None:
                 y, _, _, work = forward_call(x, dt, A, B, C, None, None, dt_bias, initial_states, ctx.shape, False)
-            if not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9)):  # D and z alone
+            if again:
+                dz, dD = _epilogue_gradients(dout, y, x, D, z, A.shape[0])
+                return None, None, None, None, None, dD, dz, None, None, None, None, None
+            if alone:
                 _, dz, dD = gate_backward(dout, y, x, B, D, z, A.shape[0])
                 return None, None, None, None, None, dD, dz, None, None, None, None, None
             dx, ddt, dA, dB, dC, dD, dz, dinit, dbias = backward_call(x, dt, A, B, C, D, z, dt_bias, y, work, dout, dfinal,
                                                                       ctx.shape, ctx.has_initial)
+        return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
+
+
+    @staticmethod
+    def differentiable_backward(ctx, dout, dfinal):
+        """Gradients that are differentiated again (create_graph).  The kernels' gradients are constants to autograd.  Away
+        from the kernels' own sizes D and z are nevertheless differentiable any number of times, as framework
+        operations around the plain node; so the call is made again in that form and its gradients are taken."""
+        inputs = list(ctx.saved_tensors[:9])  # x, dt, A, B, C, dt_bias, D, z, initial_states
+        x, dt, A, B, C, dt_bias, D, z, start = aliases = [None if t is None else t.view_as(t) for t in inputs]
+        softplus, lo, hi = ctx.options
+        y, final = _Mamba2SsdAutograd.apply(x, dt, A, B, C, None, None, softplus, start, dt_bias, lo, hi)
+        outputs, upstream = [_epilogue(y, x, D, z, A.shape[0])], [dout]
+        if dfinal is not None:
+            outputs, upstream = outputs + [final], upstream + [dfinal]
+        wanted = [i for i, k in enumerate((0, 1, 2, 3, 4, 9, 5, 6, 8)) if ctx.needs_input_grad[k]]
+        grads = [None] * 9
+        for i, g in zip(wanted, torch.autograd.grad(outputs, [aliases[i] for i in wanted], upstream, create_graph=True,
+                                                    allow_unused=True)):
+            grads[i] = g
+        dx, ddt, dA, dB, dC, dbias, dD, dz, dinit = grads
         return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
 
 
@@ -673,10 +729,7 @@ def mamba2_ssd_fwd(
         out, final = run_general(core, x, dt, A, B, C, initial_states, dt_bias, needs_grad)
         # D skip connection and z gate (ssd_reference.py:300-318) as element-wise epilogue; under autograd
         # their gradients (dD, dz and the extra term of dx) come from these same operations
-        if D is not None:
-            out = out + x * (D.view(1, 1, -1, 1) if D.dim() == 1 else D.view(1, 1, *D.shape))
-        if z is not None:
-            out = out * torch.nn.functional.silu(z)
+        out = _epilogue(out, x, D, z, x.shape[2])
     if return_final_state:
         return out, final
     return out

@@ -45,3 +45,41 @@ def test_transforms_of_the_skip_connection_and_the_gate(shape):
     for arg in (0, 1):
         got, ref = (torch.func.grad(lambda *a: fn(*a).sum(), argnums=arg)(D, z) for fn in (call, closed))
         assert close(got, ref)
+
+
+@pytest.mark.parametrize("policy", ["save", "recompute"])
+@pytest.mark.parametrize("alone", [False, True])
+@pytest.mark.parametrize("shape", [(2, 256, 3, 64, 32, 1), (1, 200, 2, 64, 64, 1), (1, 128, 2, 64, 128, 1), (1, 130, 2, 128, 64, 1)])
+def test_gradients_that_are_differentiated_again(shape, alone, policy):
+    """create_graph at sizes other than the kernels' own: D and z as around the plain call."""
+    import ascend_kernel as ak
+
+    b, l, h, p, n, g = shape
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    t = [rnd(b, l, h, p), rnd(b, l, h).abs(), -rnd(h).abs(), rnd(b, l, g, n), rnd(b, l, g, n)]
+    D, z, start, bias, up = rnd(h), rnd(b, l, h, p), rnd(b, h, p, n), 0.1 * rnd(h), rnd(b, l, h, p)
+    inputs = [D, z, up] if alone else [*t, D, z, start, bias, up]
+    for v in inputs:
+        v.requires_grad_(True)
+    weights = [rnd(*v.shape) for v in inputs[:-1]]
+
+    def second(fused):
+        kw = dict(dt_bias=bias, initial_states=start, dt_softplus=True)
+        out = ak.mamba2_ssd_fwd(*t, 64, **(dict(kw, D=D, z=z) if fused else kw))
+        if not fused:
+            out = (out + t[0] * D.view(1, 1, -1, 1)) * F.silu(z)
+        first = torch.autograd.grad(out, inputs[:-1], up, create_graph=True)
+        return first + torch.autograd.grad(sum((w * v).sum() for w, v in zip(weights, first)), inputs, allow_unused=True)
+
+    previous = ak.set_save_policy(policy)
+    try:
+        for got, want in zip(second(True), second(False)):
+            assert (got is None) == (want is None)
+            assert got is None or ((got - want).norm() <= 1e-5 * want.norm()).item()
+        if alone:
+            ups = torch.stack([up, 2 * up]).detach()
+            batched = torch.autograd.grad(ak.mamba2_ssd_fwd(*t, 64, D=D, z=z, dt_softplus=True), [D, z], ups, is_grads_batched=True)
+            assert all(torch.allclose(v[1], 2 * v[0], rtol=1e-5, atol=1e-6 * v.abs().max().item()) for v in batched)
+    finally:
+        ak.set_save_policy(previous)
