@@ -356,6 +356,11 @@ def _epilogue(y, x, D, z, heads: int):
     return out if z is None else out * torch.nn.functional.silu(z)
 
 
+def _is_batched(t: torch.Tensor) -> bool:
+    """A gradient under vmap, or one of several taken at once (is_grads_batched)."""
+    return torch._C._functorch.is_legacy_batchedtensor(t) or torch._C._functorch.is_functorch_wrapped_tensor(t)
+
+
 def _epilogue_gradients(dout, y, x, D, z, heads: int):
     """(dz, dD) of the epilogue as framework operations; y and x are constants."""
     dy, dz, dD = dout, None, None
@@ -469,7 +474,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
             dout = torch.zeros_like(x)
         alone = not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9))  # D and z alone need gradients
-        again = ctx.differentiable and (torch.is_grad_enabled() or (alone and torch._C._are_functorch_transforms_active()))
+        again = ctx.differentiable and (torch.is_grad_enabled() or (alone and _is_batched(dout)))
         if again and not alone:
             return _Mamba2SsdAutograd.differentiable_backward(ctx, dout, dfinal)
         if not again:
