@@ -273,8 +273,8 @@ int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const float* y, 
 int ssd_block_rmsnorm_fwd(const float* x, long long x_stride, const float* z, long long z_stride, const float* w,
                           float* out, long long rows, int d, float eps, ssd_stream_t stream);
 /* out[rows,cols] = x[rows,k] * w[cols,k]^T (+ residual[rows,cols], null = none): the block's projections at fp32 accuracy on the
- * tensor cores (three bf16 parts per operand).  k is a multiple of 64, x 16-byte aligned, inputs finite (an infinity comes
- * out as NaN); `work` has ssd_linear_work_bytes() bytes, 16-byte aligned (0: k is not taken). */
+ * tensor cores (three bf16 parts per operand).  k is a multiple of 64, x 16-byte aligned; infinities and NaN come out as in
+ * fp32; `work` has ssd_linear_work_bytes() bytes, 16-byte aligned (0: k is not taken). */
 size_t ssd_linear_work_bytes(int cols, int k);
 int ssd_linear_pays(long long rows, int cols, int k); /* 1 where the sizes are taken and large enough to gain */
 int ssd_linear_fwd(const float* x, const float* w, const float* residual, float* out, long long rows, int cols, int k,

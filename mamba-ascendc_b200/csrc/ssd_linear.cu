@@ -6,18 +6,21 @@
 //
 //     hi*lo + mid*mid + lo*hi   (2^-16)      hi*mid + mid*hi   (2^-8)      hi*hi
 //
-// smallest first, because the tensor core truncates where it adds to the fp32 accumulator: only the K/16 hi*hi additions
-// meet a sum of full size.  Error against 64 bits, normal operands, relative 2-norm: K = 192 1.6e-7 (the library's fp32
-// kernel: 2.5e-7), K = 384 3.2e-7 (3.5e-7).
+// The tensor core truncates where it adds to its fp32 accumulator, which is a bias on sums of one sign and grows with the
+// number of additions of full size.  So an accumulator holds 64 columns of K only, smallest products first: four additions
+// of full size.  It is then added to the running sum in registers, rounded to nearest.
 //
 // One CTA = 128 rows x a run of 96-column tiles.  x goes to tensor memory once (three parts of up to 192 columns of K: 288
-// columns; two 96-column accumulators take 192 of the rest, so a tile is written out under the next one's
-// products); w arrives by TMA from its split copy, one tile of all parts per stage, two stages.  K beyond 192 is
-// taken in chunks: first the small products of every chunk, then hi*hi of every chunk, so that the order above holds for
-// the whole sum; the chunks of x but the last are converted twice.  The issue of the products bounds a tile (72 of them at K =
-// 192, 3.5 us); before the first, a pass loads and converts its chunk of x (3 to 5 us).
-// [16384,192] x [902,192]: 41 us (132 in the library); [16384,384] x [192,384] + residual: 25 us (65).  Measured and dropped:
-// 64-column tiles in three stages (46 and 30 us), CTAs starting at different tiles (no change).
+// columns; two 96-column accumulators take 192 of the rest, so that one is read out under the other's products); w arrives by
+// TMA from its split copy, one tile of all parts per stage, two stages.  K beyond 192 is taken in equal chunks of up
+// to 192 (the last one filled up with zeros by the loads), with the sums of two tiles kept in registers.  The issue of the products
+// bounds a tile (72 of them at K = 192, 3.5 us); before the first, a chunk of x is loaded and converted (3 to 5 us).
+//
+// [16384,192] x [902,192]: 50 us from cold caches (139 in the library), [16384,384] x [192,384]: 36 (66).  Error against 64
+// bits, relative 2-norm, operands of both signs / of one sign (the library's fp32 kernel in brackets): K = 192 8.6e-8 / 9.2e-8
+// (2.5e-7 / 2.1e-7), K = 384 9.2e-8 / 9.4e-8 (3.5e-7 / 2.9e-7), K = 1536 1.2e-7 / 1.1e-7 (7.0e-7 / 5.8e-7).  With one accumulator
+// for all of K it was 1.8e-7 / 2.7e-7, 3.5e-7 / 6.1e-7 and 1.5e-6 / 3.7e-6.  Measured and dropped: 64-column tiles in three
+// stages, CTAs starting at different tiles.
 #include "ssd_host.h"
 #include "ssd_pdl.cuh"
 #include "ssd_tile.cuh"
@@ -29,7 +32,7 @@ namespace {
 constexpr int kLinCols = 96;                              // columns of a tile
 constexpr int kLinMaxBlocks = 3;                          // 64-column blocks of K per chunk
 constexpr uint32_t kLinBox = kLinCols * 128;              // one part of one block: [96 x 64] bf16
-constexpr int kLinWarps = 8;                              // convert x (two warps per 32 rows), write the result (four per tile)
+constexpr int kLinWarps = 8;                              // convert x, add up and write the result (two warps per 32 rows)
 constexpr int kLinThreads = kLinWarps * 32 + 64;          // and the issuing and the producer warp
 constexpr int kLinPatchCols = 8;
 constexpr uint32_t kLinPatch = 32 * (kLinPatchCols + 1) * sizeof(float);  // per warp: 32 rows x 8 columns on their way out
@@ -48,9 +51,33 @@ __host__ __device__ constexpr uint32_t lin_smem_bytes(int blocks) {
 static_assert(lin_smem_bytes(kLinMaxBlocks) <= 232448, "projection kernel exceeds the shared memory of one SM");
 static_assert(128 * 128 * 2 <= 3 * kLinBox, "a block of x lands in the stage of a block of w");
 
-// v = hi + mid + lo, bf16 each, for finite v (up to the largest bf16, 3.39e38)
+// v = hi + mid + lo, bf16 each.  An infinity becomes (+-1, 0, +-inf): its lo part meets only the other operand's hi part,
+// which has that operand's sign and is zero with it, so the sum is the infinity or NaN that fp32 gives (an infinity minus itself
+// would be NaN, and an infinite hi part would meet mid and lo parts of either sign).
+__device__ __forceinline__ void split3(float v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const uint32_t sign = __float_as_uint(v) >> 16 & 0x8000u, magnitude = __float_as_uint(v) & 0x7FFFFFFFu;
+    if (magnitude >= 0x7F800000u) {
+        hi = magnitude == 0x7F800000u ? sign | 0x3F80u : 0x7FC0u;
+        mid = 0;
+        lo = magnitude == 0x7F800000u ? sign | 0x7F80u : 0u;
+        return;
+    }
+    hi = magnitude >= 0x7F7F8000u ? sign | 0x7F7Fu : pack_bf16x2(v, 0.f) & 0xFFFFu;  // the largest bf16 instead of an infinity
+    const float rest = v - __uint_as_float(hi << 16);
+    mid = pack_bf16x2(rest, 0.f) & 0xFFFFu;
+    lo = pack_bf16x2(rest - __uint_as_float(mid << 16), 0.f) & 0xFFFFu;
+}
 __device__ __forceinline__ void split3_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = pack_bf16x2(a, b);
+    if ((hi & 0x7F80u) == 0x7F80u || (hi & 0x7F800000u) == 0x7F800000u) {
+        uint32_t h, m, l;
+        split3(a, hi, mid, lo);
+        split3(b, h, m, l);
+        hi |= h << 16;
+        mid |= m << 16;
+        lo |= l << 16;
+        return;
+    }
     const float a1 = a - __uint_as_float(hi << 16), b1 = b - __uint_as_float(hi & 0xFFFF0000u);
     mid = pack_bf16x2(a1, b1);
     lo = pack_bf16x2(a1 - __uint_as_float(mid << 16), b1 - __uint_as_float(mid & 0xFFFF0000u));
@@ -72,7 +99,8 @@ linear_split_kernel(const float* __restrict__ w, uint32_t* __restrict__ parts, i
 }
 
 // BLOCKS: 64-column blocks of K per chunk, a compile-time number, so that the issuing thread pays one addition per product.
-template <int BLOCKS>
+// HELD: tiles whose sums a CTA keeps at once; 2 with several chunks of K, which are the outer loop (a CTA then has no more tiles).
+template <int BLOCKS, int HELD>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const LinearArgs a,
               int* status) {
@@ -93,12 +121,7 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     const int row0 = blockIdx.x * 128;
     const int tile0 = blockIdx.y * a.tiles_per_item;
     const int ntiles = min(a.tiles_per_item, a.tiles - tile0);
-    const int passes = 2 * a.chunks - 1;
-    // pass -> chunk, and which products it forms
-    auto chunk_of = [&](int pass) { return pass < a.chunks ? pass : 2 * a.chunks - 2 - pass; };
-    auto has_small = [&](int pass) { return pass < a.chunks; };
-    auto has_main = [&](int pass) { return pass >= a.chunks - 1; };
-    // tiles that go through a stage in one pass
+    // tiles that go through a stage in the pass over one chunk
     auto per_pass = [&](int st) { return (ntiles + 1 - st) >> 1; };
 
     if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need the declared alignment
@@ -112,7 +135,7 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             mbar_init(&full_w[i], 1);
             mbar_init(&done[i], 1);
             mbar_init(&acc_ready[i], 1);
-            mbar_init(&acc_free[i], 4);
+            mbar_init(&acc_free[i], kLinWarps);
         }
         fence_mbar_init();
     }
@@ -136,36 +159,38 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     if (warp == kLinWarps) {  // ---- issues the products
         if (lane == 0) {
             const uint32_t idesc = make_idesc_bf16(128, kLinCols, false, false);
-            for (int pass = 0; pass < passes; ++pass) {
+            int sum = 0;  // accumulators so far
+            for (int pass = 0; pass < a.chunks; ++pass) {
                 mbar_wait(x_ready, pass & 1, status, kStatusMmaTimeout | wait_site(7, 1));
                 for (int t = 0; t < ntiles; ++t) {
                     const int st = t & 1;
                     mbar_wait(&full_w[st], (pass * per_pass(st) + (t >> 1)) & 1, status, kStatusMmaTimeout | wait_site(7, 2));
-                    if (pass == 0 && t >= 2)  // its previous tile has been read
-                        mbar_wait(&acc_free[st], ((t >> 1) - 1) & 1, status, kStatusMmaTimeout | wait_site(7, 3));
-                    tc_fence_after_sync();
-                    const uint32_t acc = tmem + st * kLinCols;
                     const uint32_t base = smem_u32(smem) + st * stage_bytes;
-                    uint32_t accumulate = pass > 0 ? 1u : 0u;
-                    auto product = [&](int xp, int wp) {
-                        const uint64_t w0 = operand_desc0(base + wp * blocks * kLinBox, kLinBox, false);
 #pragma unroll
-                        for (int s = 0; s < 4 * blocks; ++s) {
-                            umma_bf16_ta(acc, tm_x + xp * part_cols + 8u * s, w0 + (kstep_offset(kLinBox, false, s) >> 4), idesc,
-                                         accumulate);
-                            accumulate = 1u;
-                        }
-                    };
-                    if (has_small(pass)) {
+                    for (int blk = 0; blk < blocks; ++blk, ++sum) {
+                        if (sum >= 2)  // what it held before has been read
+                            mbar_wait(&acc_free[sum & 1], ((sum >> 1) - 1) & 1, status, kStatusMmaTimeout | wait_site(7, 3));
+                        tc_fence_after_sync();
+                        const uint32_t acc = tmem + (sum & 1) * kLinCols;
+                        uint32_t accumulate = 0u;
+                        auto product = [&](int xp, int wp) {
+                            const uint64_t w0 = operand_desc0(base + wp * blocks * kLinBox, kLinBox, false);
+#pragma unroll
+                            for (int s = 4 * blk; s < 4 * blk + 4; ++s) {
+                                umma_bf16_ta(acc, tm_x + xp * part_cols + 8u * s, w0 + (kstep_offset(kLinBox, false, s) >> 4), idesc,
+                                             accumulate);
+                                accumulate = 1u;
+                            }
+                        };
                         product(0, 2);
                         product(1, 1);
                         product(2, 0);
                         product(0, 1);
                         product(1, 0);
+                        product(0, 0);
+                        umma_commit(&acc_ready[sum & 1]);
                     }
-                    if (has_main(pass)) product(0, 0);
                     umma_commit(&done[st]);
-                    if (pass == passes - 1) umma_commit(&acc_ready[st]);
                 }
             }
         }
@@ -174,8 +199,8 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             auto stage_idle = [&](int st, int loads) {  // the products of the last of its `loads` tiles so far are done
                 if (loads > 0) mbar_wait(&done[st], (loads - 1) & 1, status, kStatusMmaTimeout | wait_site(7, 4));
             };
-            for (int pass = 0; pass < passes; ++pass) {
-                const int k0 = chunk_of(pass) * blocks * 64;
+            for (int pass = 0; pass < a.chunks; ++pass) {
+                const int k0 = pass * blocks * 64;
                 auto load_w = [&](int t) {
                     const int st = t & 1;
                     mbar_arrive_expect_tx(&full_w[st], stage_bytes);
@@ -199,59 +224,116 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             }
         }
     } else {  // ---- convert x, write the result
-        const int quarter = warp & 3, half = warp >> 2;
+        const int quarter = warp & 3, half = warp >> 2;  // 32 rows; every other slab of x, half the columns of a tile
+        constexpr int kCols = kLinCols / 2;
         const int out_row = row0 + quarter * 32;
         float* patch = patches + warp * 32 * (kLinPatchCols + 1);
-        for (int pass = 0; pass < passes; ++pass) {
+        float sums[HELD][kCols];  // this thread's row
+        auto clear = [&]() {
+#pragma unroll
+            for (int i = 0; i < HELD * kCols; ++i) sums[i / kCols][i % kCols] = 0.f;
+        };
+        if constexpr (HELD > 1) clear();
+        int sum = 0;  // accumulators so far
+        auto add_up = [&](float* total) {
+            const int acc = sum & 1;
+            ok = mbar_wait(&acc_ready[acc], (sum >> 1) & 1, status, kStatusMmaTimeout | wait_site(7, 7)) && ok;
+            tc_fence_after_sync();
+            constexpr int kAtOnce = HELD == 1 ? kCols : 16;  // with two tiles held the registers do not take more
+#pragma unroll
+            for (int c0 = 0; c0 < kCols; c0 += kAtOnce) {
+                float v[kAtOnce];
+#pragma unroll
+                for (int c = 0; c < kAtOnce; c += 16)
+                    tmem_ld16(tmem_addr(tmem + acc * kLinCols, warp, half * kCols + c0 + c), v + c);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < kAtOnce; ++i) total[c0 + i] += v[i];
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_free[acc]);
+            ++sum;
+        };
+        auto write_tile = [&](const float* total, int t) {  // eight columns at a time, turned so that a row is contiguous
+            const int col = (tile0 + t) * kLinCols + half * kCols + (lane & 7), r0 = lane >> 3;
+            const size_t o = static_cast<size_t>(out_row + r0) * a.cols + col;
+            // of this thread's rows r0, r0 + 4, ... those that exist
+            const int rows = ok ? static_cast<int>(max(0ll, min(8ll, (a.rows - out_row - r0 + 3) / 4))) : 0;
+            auto inside = [&](int c0, int i) { return i < rows && col + c0 < a.cols; };
+            constexpr int kPatches = kCols / kLinPatchCols, kAtOnce = HELD == 1 ? kPatches : 2;  // residual loads in flight together
+#pragma unroll
+            for (int j0 = 0; j0 < kPatches; j0 += kAtOnce) {
+                float add[kAtOnce][8];
+#pragma unroll
+                for (int j = 0; j < kAtOnce; ++j)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int c0 = (j0 + j) * kLinPatchCols;
+                        add[j][i] = a.residual != nullptr && inside(c0, i) ? a.residual[o + c0 + static_cast<size_t>(4 * i) * a.cols] : 0.f;
+                    }
+#pragma unroll
+                for (int j = 0; j < kAtOnce; ++j) {
+                    const int c0 = (j0 + j) * kLinPatchCols;
+#pragma unroll
+                    for (int i = 0; i < kLinPatchCols; ++i) patch[lane * (kLinPatchCols + 1) + i] = total[c0 + i];
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (inside(c0, i))
+                            a.out[o + c0 + static_cast<size_t>(4 * i) * a.cols] =
+                                patch[(r0 + 4 * i) * (kLinPatchCols + 1) + (lane & 7)] + add[j][i];
+                    __syncwarp();
+                }
+            }
+        };
+        for (int pass = 0; pass < a.chunks; ++pass) {
             ok = mbar_wait(full_x, pass & 1, status, kStatusTmaTimeout | wait_site(7, 6)) && ok;
             tc_fence_after_sync();
 #pragma unroll 1
             for (int slab = half; slab < 2 * blocks; slab += 2) {
                 const uint8_t* src = smem + stage_bytes + slab * kSlabBytes;
-                uint32_t hi[16], mid[16], lo[16];
+                constexpr int kPairs = HELD == 1 ? 16 : 8;  // split together
+#pragma unroll 1
+                for (int first = 0; first < 16; first += kPairs) {
+                    uint32_t hi[kPairs], mid[kPairs], lo[kPairs];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const float4 f = *reinterpret_cast<const float4*>(src + swz(quarter * 32 + lane, c));
-                    split3_pair(f.x, f.y, hi[2 * c], mid[2 * c], lo[2 * c]);
-                    split3_pair(f.z, f.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
+                    for (int c = 0; c < kPairs / 2; ++c) {
+                        const float4 f = *reinterpret_cast<const float4*>(src + swz(quarter * 32 + lane, first / 2 + c));
+                        split3_pair(f.x, f.y, hi[2 * c], mid[2 * c], lo[2 * c]);
+                        split3_pair(f.z, f.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
+                    }
+                    auto store = [&](uint32_t part, const uint32_t* v) {
+                        const uint32_t at = tmem_addr(tm_x + part * part_cols, warp, 16 * slab + first);
+                        if constexpr (kPairs == 16) tmem_st16(at, v);
+                        else tmem_st8(at, v);
+                    };
+                    store(0, hi);
+                    store(1, mid);
+                    store(2, lo);
                 }
-                tmem_st16(tmem_addr(tm_x, warp, 16 * slab), hi);
-                tmem_st16(tmem_addr(tm_x + part_cols, warp, 16 * slab), mid);
-                tmem_st16(tmem_addr(tm_x + 2 * part_cols, warp, 16 * slab), lo);
             }
             tmem_st_wait();
             signal_issuer(x_ready, lane);
-        }
-        for (int t = half; t < ntiles; t += 2) {  // one accumulator each
-            const int st = half;
-            ok = mbar_wait(&acc_ready[st], (t >> 1) & 1, status, kStatusMmaTimeout | wait_site(7, 7)) && ok;
-            tc_fence_after_sync();
-#pragma unroll 1
-            for (int c0 = 0; c0 < kLinCols; c0 += kLinPatchCols) {
-                float v[kLinPatchCols], add[kLinPatchCols];
-                const int col = (tile0 + t) * kLinCols + c0 + (lane & 7), r0 = lane >> 3;
-                const size_t o = static_cast<size_t>(out_row + r0) * a.cols + col;
-                const bool inside = col < a.cols && ok;
+            if constexpr (HELD == 1) {
+                for (int t = 0; t < ntiles; ++t) {
+                    clear();
 #pragma unroll
-                for (int i = 0; i < 8; ++i)  // rows r0, r0 + 4, ...
-                    add[i] = a.residual != nullptr && inside && out_row + r0 + 4 * i < a.rows
-                                 ? a.residual[o + static_cast<size_t>(4 * i) * a.cols] : 0.f;
-                tmem_ld8(tmem_addr(tmem + st * kLinCols, warp, c0), v);
-                tmem_ld_wait();
+                    for (int blk = 0; blk < blocks; ++blk) add_up(sums[0]);
+                    write_tile(sums[0], t);
+                }
+            } else {
 #pragma unroll
-                for (int i = 0; i < kLinPatchCols; ++i) patch[lane * (kLinPatchCols + 1) + i] = v[i];
-                __syncwarp();
+                for (int t = 0; t < HELD; ++t)
+                    if (t < ntiles)
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (inside && out_row + r0 + 4 * i < a.rows)
-                        a.out[o + static_cast<size_t>(4 * i) * a.cols] =
-                            patch[(r0 + 4 * i) * (kLinPatchCols + 1) + (lane & 7)] + add[i];
-                __syncwarp();
+                        for (int blk = 0; blk < blocks; ++blk) add_up(sums[t]);
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_free[st]);
         }
+        if constexpr (HELD > 1)
+#pragma unroll
+            for (int t = 0; t < HELD; ++t)
+                if (t < ntiles) write_tile(sums[t], t);
     }
     __syncwarp();
     tc_fence_before_sync();
@@ -259,12 +341,11 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// Blocks of 64 in a chunk of K: the largest that divides it, at most three; 0 if K is not made of them.
+// Chunks of K and blocks of 64 columns in a chunk: as few as hold all of K, as even as they come; 0 if K is not made of blocks.
+int linear_chunks(int k) { return k <= 0 || k % 64 != 0 ? 0 : (k / 64 + kLinMaxBlocks - 1) / kLinMaxBlocks; }
 int linear_blocks(int k) {
-    if (k <= 0 || k % 64 != 0) return 0;
-    for (int b = kLinMaxBlocks; b > 1; --b)
-        if (k / 64 % b == 0) return b;
-    return 1;
+    const int chunks = linear_chunks(k);
+    return chunks == 0 ? 0 : (k / 64 + chunks - 1) / chunks;
 }
 int linear_cols_padded(int cols) { return (cols + kLinCols - 1) / kLinCols * kLinCols; }
 
@@ -272,13 +353,15 @@ int linear_cols_padded(int cols) { return (cols + kLinCols - 1) / kLinCols * kLi
 
 }  // namespace ssd
 
-// Below these sizes the kernel's own latency (10 us for one tile, 22 us with two chunks of K) exceeds the library's time:
-// [784,192] x [902,192] 12 / 13 us, [196,192] x [902,192] 11 / 6.5; [4096,384] x [192,384] 25 / 22.
+// The kernel's own latency for one round of CTAs is 13 to 17 us with one chunk of K and 10 us more with each further one; below
+// these sizes the library's fp32 kernel takes less.  Measured over K = 64 ... 1536, 64 to 6278 columns, 200 to 16384 rows (us, this
+// kernel / the library): [1024,192] x [902,192] 17 / 17, [2048,192] x [902,192] 22 / 26, [16384,192] x [902,192] 50 / 139;
+// [2048,384] x [902,384] 34 / 41, [4096,384] x [192,384] 32 / 25; [2048,576] x [576,576] 44 / 33, [512,576] x [2438,576] 44 / 50;
+// [16384,64 to 1536] x [64,..] 0.9 of the library throughout, [16384,1024] x [192,1024] 81 / 150.  Of the sizes taken none was slower.
 extern "C" int ssd_linear_pays(long long rows, int cols, int k) {
-    const int blocks = ssd::linear_blocks(k);
-    if (rows <= 0 || cols <= 0 || blocks == 0) return 0;
-    const double work = static_cast<double>(rows) * cols * k;
-    return work >= (k == 64 * blocks ? 1.6e8 : 4e8) ? 1 : 0;
+    const int chunks = ssd::linear_chunks(k);
+    if (rows <= 0 || cols <= 0 || chunks == 0) return 0;
+    return static_cast<double>(rows) * cols * k >= 2.3e8 * chunks ? 1 : 0;
 }
 
 extern "C" size_t ssd_linear_work_bytes(int cols, int k) {
@@ -296,12 +379,12 @@ extern "C" int ssd_linear_fwd(const float* x, const float* w, const float* resid
     if (blocks == 0) return SSD_ERR_UNSUPPORTED;
     if (rows > 0x7fffffffLL - 128 || 3ll * a.cols_padded > 0x7fffffffLL) return SSD_ERR_RANGE;
     if (!aligned16(x, static_cast<const float*>(work))) return SSD_ERR_ALIGN;
-    a.chunks = k / (64 * blocks);
+    a.chunks = linear_chunks(k);
     a.tiles = a.cols_padded / kLinCols;
     const int sms = sm_count();
     if (sms <= 0) return SSD_ERR_LAUNCH;
     const int64_t row_tiles = (rows + 127) / 128;
-    // a chunked sum keeps its accumulators over all passes: at most two tiles per CTA; otherwise few row tiles are given
+    // with several chunks a CTA keeps its sums over all of them: at most two tiles; otherwise few row tiles are given
     // more CTAs along the columns
     a.tiles_per_item = a.chunks > 1 ? 2 : a.tiles / choose_head_split(row_tiles, a.tiles, sms, 1, 3);
     const int items = (a.tiles + a.tiles_per_item - 1) / a.tiles_per_item;
@@ -317,13 +400,17 @@ extern "C" int ssd_linear_fwd(const float* x, const float* w, const float* resid
                  static_cast<uint32_t*>(work), cols, a.cols_padded, k);
     rc = launch_status();
     if (rc != SSD_OK) return rc;
-    static std::atomic<uint64_t> smem_set[kLinMaxBlocks];
-    auto launch = [&](auto kernel, int b) {
-        const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), lin_smem_bytes(b), smem_set[b - 1]);
+    auto launch = [&](auto kernel, std::atomic<uint64_t>& smem_set) {
+        const int r = set_max_smem_once(reinterpret_cast<const void*>(kernel), lin_smem_bytes(blocks), smem_set);
         if (r != SSD_OK) return r;
-        launch_tiles(row_tiles * items, kernel, dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(b), st,
-                       map_x, map_w, a, status);
+        launch_tiles(row_tiles * items, kernel, dim3(static_cast<unsigned>(row_tiles), items), kLinThreads, lin_smem_bytes(blocks),
+                     st, map_x, map_w, a, status);
         return launch_status();
     };
-    return blocks == 3 ? launch(linear_kernel<3>, 3) : blocks == 2 ? launch(linear_kernel<2>, 2) : launch(linear_kernel<1>, 1);
+    static std::atomic<uint64_t> smem_set[5];
+    if (a.chunks > 1)  // 256 columns of K or more: chunks of two or three blocks
+        return blocks == 3 ? launch(linear_kernel<3, 2>, smem_set[0]) : launch(linear_kernel<2, 2>, smem_set[1]);
+    return blocks == 3   ? launch(linear_kernel<3, 1>, smem_set[2])
+           : blocks == 2 ? launch(linear_kernel<2, 1>, smem_set[3])
+                         : launch(linear_kernel<1, 1>, smem_set[4]);
 }

@@ -1,7 +1,8 @@
 """The projection kernel (three bf16 parts per operand) at the edges of its tiles, against fp64.
 
-Tolerance: the parts hold 24 bits and the dropped products are below 2^-24; the accumulator truncates on each of the
-K / 16 additions of full size, at most 2^-23 of the sum each and on average a tenth of that: 5e-7 up to K = 384, 1e-6 beyond."""
+Tolerance: the parts hold 24 bits and the dropped products are below 2^-24; an accumulator truncates on each of its four
+additions of full size, at most 2^-23 of its sum each, and the accumulators are added with rounding: 5e-7 up to K = 384, 1e-6
+beyond leave room for both."""
 import pytest
 import torch
 
@@ -58,3 +59,50 @@ def test_layers_with_hooks_or_a_lower_precision_policy_are_left_alone():
         assert torch.equal(V._linear(layer, x), layer(x)) and len(seen) == 2
         handle.remove()
     assert V._linear(layer, x).requires_grad  # with gradients: the layer
+
+
+def _run(x, w, residual=None):
+    from ascend_kernel import _capi, check_status, mamba2 as M
+
+    (rows, k), cols = x.shape, w.shape[0]
+    out = torch.full((rows, cols), float("nan"), device="cuda")
+    work = torch.empty(_capi.lib.ssd_linear_work_bytes(cols, k), device="cuda", dtype=torch.uint8)
+    _capi.check(_capi.lib.ssd_linear_fwd(x.data_ptr(), w.data_ptr(), residual.data_ptr() if residual is not None else None,
+                                         out.data_ptr(), rows, cols, k, work.data_ptr(), M._status(x.device).data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream), "linear")
+    check_status()
+    return out
+
+
+@pytest.mark.parametrize("one_sign", [False, True])
+@pytest.mark.parametrize("k", [64, 128, 192, 256, 320, 384, 448, 576, 768, 1536])
+def test_error_is_no_larger_than_that_of_an_fp32_product(k, one_sign):
+    """Against fp64, beside the framework's fp32 product of the same operands, at sizes that this kernel takes over: of both signs,
+    and of one sign, where truncated additions add up.  K over every split into chunks: whole ones, ones filled up with zeros
+    (320, 448), two to eight."""
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    x, w = (torch.randn(s, k, generator=gen, device="cuda") for s in (2100, 902))
+    if one_sign:
+        x, w = x.abs(), w.abs()
+    want = x.double() @ w.double().T
+    assert torch.backends.cuda.matmul.fp32_precision in ("none", "ieee")
+    ours, library = (((v.double() - want).norm() / want.norm()).item() for v in (_run(x, w), x @ w.T))
+    assert ours <= library, (ours, library)
+
+
+@pytest.mark.parametrize("k", [64, 256])
+def test_infinities_nan_and_the_largest_values(k):
+    inf, nan, largest = float("inf"), float("nan"), torch.finfo(torch.float32).max
+    x, w = torch.randn(140, k, device="cuda"), torch.randn(100, k, device="cuda")
+    x[3, 5], x[4, 6], x[5, 7], x[5, 8], x[6, 9] = inf, -inf, inf, -inf, nan
+    w[7, 5], w[8, 5], w[9, 11], w[10, 12] = inf, 0.0, -inf, nan
+    x[20, 11] = 0.0
+    x[130], x[130, 13] = 0.0, largest
+    w[:, 13] = 0.5 * torch.sign(w[:, 13])
+    got, want = _run(x, w), x.double() @ w.double().T
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.isposinf(got), torch.isposinf(want)) and torch.equal(torch.isneginf(got), torch.isneginf(want))
+    finite = torch.isfinite(want)
+    assert finite[130, :7].all() and ((got[130, :7].double() - want[130, :7]).abs() <= 1e-6 * want[130, :7].abs()).all()
+    finite[130] = False
+    assert ((got.double() - want)[finite].norm() / want[finite].norm()).item() <= 5e-7
