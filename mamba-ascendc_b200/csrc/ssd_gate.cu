@@ -21,12 +21,13 @@ namespace {
 
 constexpr int kGateThreads = 256;
 constexpr int kGateUnroll = 4;        // rows of one thread in flight together
-constexpr int kGateMaxRows = 128;     // tokens per CTA in the backward pass (one dD partial per CTA and column) ...
+constexpr int kGateMaxRows = 128;     // tokens per CTA in the backward pass at most: their products are summed in fp32 ...
 constexpr int kGateCtasWanted = 1184; // ... fewer when that leaves less than eight CTAs per SM of 148, ...
 constexpr int kGateMinRows = 32;      // ... but there not so few that adding up the partials takes longer than forming them
 
 // How [rows, cols / 4] float4s are laid over CTAs: `colblocks` blocks of `ct` threads along a row, `rt` rows side by
-// side in a CTA.  ct * rt <= kGateThreads, and ct is as even a share of the row as the block count allows.
+// side in a CTA.  ct * rt <= kGateThreads, and ct is as even a share of the row as the block count allows.  Column blocks and
+// row blocks share grid.x, column blocks first, so that any number of rows keeps its blocks of at most kGateMaxRows.
 struct GateGrid {
     int ct, rt, colblocks, rows_per_cta;
     long long rowblocks;
@@ -36,16 +37,12 @@ GateGrid gate_grid(long long rows, int cols, int min_rows) {
     const int c4 = cols / 4;
     g.colblocks = (c4 + kGateThreads - 1) / kGateThreads;
     g.ct = (c4 + g.colblocks - 1) / g.colblocks;
-    g.rt = kGateThreads / g.ct;
+    g.rt = kGateThreads / g.ct < kGateMaxRows / kGateUnroll ? kGateThreads / g.ct : kGateMaxRows / kGateUnroll;
     const int least = g.rt * kGateUnroll > min_rows ? g.rt * kGateUnroll : min_rows;
-    g.rows_per_cta = kGateMaxRows > least ? kGateMaxRows : least;
+    g.rows_per_cta = kGateMaxRows;
     while (g.rows_per_cta / 2 >= least && (rows + g.rows_per_cta - 1) / g.rows_per_cta * g.colblocks < kGateCtasWanted)
         g.rows_per_cta /= 2;
     g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
-    while (g.rowblocks > 65535) {  // grid.y
-        g.rows_per_cta *= 2;
-        g.rowblocks = (rows + g.rows_per_cta - 1) / g.rows_per_cta;
-    }
     return g;
 }
 
@@ -67,14 +64,15 @@ template <bool HAS_D, bool HAS_Z>
 __global__ void __launch_bounds__(kGateThreads)
 gate_skip_fwd_kernel(const float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ D, int d_mode,
                      const float* __restrict__ z, float* __restrict__ out, long long rows, int cols, int p_dim, int ct,
-                     int rt, int rows_per_cta) {
+                     int rt, int rows_per_cta, unsigned colblocks) {
     after_previous();
     allow_next();
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
-    const int c = (blockIdx.x * ct + tx) * 4;
+    const unsigned row_block = blockIdx.x / colblocks;
+    const int c = ((blockIdx.x - row_block * colblocks) * ct + tx) * 4;
     if (c >= cols || ty >= rt) return;
     const float4 d = load_d(D, d_mode, c, p_dim);
-    const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_cta;
+    const long long r0 = static_cast<long long>(row_block) * rows_per_cta;
     const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
     for (long long r = r0 + ty; r < r1; r += kGateUnroll * rt) {
         float4 v[kGateUnroll], xv[kGateUnroll], zv[kGateUnroll];
@@ -117,14 +115,15 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y, const float* __restrict__ x,
                      const float* __restrict__ D, int d_mode, const float* __restrict__ z, float* __restrict__ dy,
                      float* __restrict__ dz, float* __restrict__ part, long long rows, int cols, int p_dim, int ct, int rt,
-                     int rows_per_cta) {
+                     int rows_per_cta, unsigned colblocks) {
     after_previous();
     allow_next();
     __shared__ float4 sums[kGateThreads];
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
-    const int c = (blockIdx.x * ct + tx) * 4;
+    const unsigned row_block = blockIdx.x / colblocks;
+    const int c = ((blockIdx.x - row_block * colblocks) * ct + tx) * 4;
     const bool active = c < cols && ty < rt;
-    const long long r0 = static_cast<long long>(blockIdx.y) * rows_per_cta;
+    const long long r0 = static_cast<long long>(row_block) * rows_per_cta;
     const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
     constexpr int kUnroll = HAS_Z ? 2 : kGateUnroll;  // four tensors a row with z: eight float4 in flight
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -185,7 +184,7 @@ gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y
             acc.z += o.z;
             acc.w += o.w;
         }
-        st4(part + static_cast<size_t>(blockIdx.y) * cols + c, acc);
+        st4(part + static_cast<size_t>(row_block) * cols + c, acc);
     }
 }
 
@@ -251,10 +250,11 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!aligned16(y, x, z, out, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(rows, cols, 1);
-    const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
+    if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
-        launch_plain(kernel, grid, kGateThreads, 0, reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out,
-                     rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta);
+        launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0,
+                     reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out, rows, cols, shape->headdim, g.ct, g.rt,
+                     g.rows_per_cta, static_cast<unsigned>(g.colblocks));
     };
     if (d_mode != 0)
         z ? launch(gate_skip_fwd_kernel<true, true>) : launch(gate_skip_fwd_kernel<true, false>);
@@ -277,10 +277,11 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     if (!aligned16(dout, y, x, z, dy, dz, dD_partial, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(rows, cols, kGateMinRows);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const dim3 grid(g.colblocks, static_cast<unsigned>(g.rowblocks));
+    if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
-        launch_plain(kernel, grid, kGateThreads, 0, st, dout, y, x, D, d_mode, z, dy, dz, dD_partial, rows, cols,
-                     shape->headdim, g.ct, g.rt, g.rows_per_cta);
+        launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0, st, dout, y, x, D, d_mode, z,
+                     dy, dz, dD_partial, rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta,
+                     static_cast<unsigned>(g.colblocks));
     };
     if (d_mode != 0)
         z ? launch(gate_skip_bwd_kernel<true, true>) : launch(gate_skip_bwd_kernel<true, false>);

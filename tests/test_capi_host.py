@@ -170,3 +170,14 @@ def test_persistent_tile_walk_matches_the_closed_form():
                 head = gi * hpg + it % hpg
                 want = (gi, head, bi * l + k * 128, (bi * h + head) * nchunks + k)
                 assert tuple(got[it]) == want, (b, l, h, g, grid, cta, it, tuple(got[it]), want)
+
+
+@pytest.mark.parametrize("h,p", [(1, 4), (1, 8), (3, 4), (1, 28), (1, 64), (6, 64), (33, 32), (256, 64), (1, 1024)])
+@pytest.mark.parametrize("b,l", [(1, 1), (1, 129), (1, 1025), (4, 4096), (2, 1 << 20), (16, 1 << 20)])
+def test_partial_sums_of_the_skip_gradient_cover_at_most_128_tokens(h, p, b, l):
+    """dD is summed in fp32 inside a block of tokens and in fp64 over the blocks: one partial per block and channel."""
+    from ascend_kernel import _capi
+
+    s = _capi.SsdShape(b, l, h, p, 64, 128, 1, 0, 0.0, 0.0, 0)
+    blocks, rest = divmod(_capi.lib.ssd_gate_partial_floats(ctypes.byref(s)), h * p)
+    assert rest == 0 and 128 * blocks >= b * l
