@@ -244,7 +244,8 @@ int ssd_dt_finalize_bias_bwd(const SsdShape* shape, const float* ddt_t, const do
  * for the D / z part of the reference's fused epilogue and gate kernels (mamba_ascendc_ops/.../
  * mamba2_ssd_state_epilogue.cpp:413-482; mamba_ascendc/csrc/ops/mamba2_ssd_bwd_gate/design.md:8-13; the
  * semantics are those of mamba_torch/ssd_reference.py:300-318).  Tensors y, x, z, out [B,L,H,P] fp32, any L,
- * P % 4 == 0; only batch, seqlen, nheads and headdim of the shape are read.
+ * P % 4 == 0; only batch, seqlen, nheads and headdim of the shape are read, and with SSD_FLAG_EXTENTS valid_len and the
+ * parts of a head, which count as one.
  *   d_mode   0: no D;  1: D[H];  2: D[H,P].        z may be null (no gate).
  * Backward: dy = dout .* silu(z), dz = dout .* (y + D .* x) .* silu'(z) (both only written when z is given;
  * without z the caller uses dout as dy), dD = sum over batch, tokens (and channels for d_mode 1) of dy .* x,

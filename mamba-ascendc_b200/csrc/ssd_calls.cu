@@ -35,16 +35,6 @@ struct ForwardWork {
     }
 };
 
-// The caller's heads: D, z and their gradients see [.., H, P] where the kernels may see `parts` heads of 64 channels.
-SsdShape gate_shape(const SsdShape& s) {
-    SsdShape g = s;
-    const int parts = head_parts(s);
-    g.seqlen = row_tokens(s);
-    g.nheads = s.nheads / parts;
-    g.headdim = s.headdim * parts;
-    return g;
-}
-
 struct BackwardWork {
     float *dstates, *g_last, *ddt_t, *dy, *gate_part, *dbc_part;
     double* dA_part;
@@ -59,8 +49,7 @@ struct BackwardWork {
         ddt_t = c.take<float>(rows * s.seqlen);
         dA_part = c.take<double>(tiles);
         dy = has_z ? c.take<float>(tokens * s.nheads * s.headdim) : nullptr;
-        const SsdShape g = gate_shape(s);
-        gate_part = has_d ? c.take<float>(ssd_gate_partial_floats(&g)) : nullptr;
+        gate_part = has_d ? c.take<float>(ssd_gate_partial_floats(&s)) : nullptr;
         split = ssd_dbc_split(&s);
         dbc_part = split > 1 ? c.take<float>(2 * tokens * s.ngroups * s.dstate * split) : nullptr;
         bytes = c.used;
@@ -115,8 +104,7 @@ extern "C" int ssd_forward(const SsdShape* shape, const SsdForwardArgs* a, int s
         rc = ssd_chunk_scan_copy_fwd(&s, a->x, a->bm, a->cm, w.states, w.q, w.cs, a->y, gated ? nullptr : a->out, a->status,
                                      stream);
     if (rc != SSD_OK || !gated) return rc;
-    const SsdShape g = gate_shape(s);
-    return ssd_gate_skip_fwd(&g, a->y, a->x, a->D, a->D ? a->d_mode : 0, a->z, a->out, stream);
+    return ssd_gate_skip_fwd(&s, a->y, a->x, a->D, a->D ? a->d_mode : 0, a->z, a->out, stream);
 }
 
 extern "C" int ssd_backward(const SsdShape* shape, const SsdBackwardArgs* a, int state_route, ssd_stream_t stream) {
@@ -132,8 +120,7 @@ extern "C" int ssd_backward(const SsdShape* shape, const SsdBackwardArgs* a, int
     const int d_mode = a->D ? a->d_mode : 0;
     const float* dy = a->dout;
     if (a->D != nullptr || a->z != nullptr) {
-        const SsdShape g = gate_shape(s);
-        rc = ssd_gate_skip_bwd(&g, a->dout, a->y, a->x, a->D, d_mode, a->z, w.dy, a->dz, w.gate_part, a->dD, stream);
+        rc = ssd_gate_skip_bwd(&s, a->dout, a->y, a->x, a->D, d_mode, a->z, w.dy, a->dz, w.gate_part, a->dD, stream);
         if (rc != SSD_OK) return rc;
         if (a->z != nullptr) dy = w.dy;
     }

@@ -219,12 +219,19 @@ __global__ void gate_dd_reduce_kernel(const float* __restrict__ part, int row_bl
     }
 }
 
-int gate_dims(const SsdShape* s, long long* rows, int* cols) {
+// The tensors as rows of `cols` values, `heads` times `p` of them (of D): with SSD_FLAG_EXTENTS the caller's tokens, and the
+// parts of a head together.
+struct GateDims {
+    long long rows;
+    int cols, heads, p;
+};
+int gate_dims(const SsdShape* s, GateDims* d) {
     if (!s) return SSD_ERR_NULL;
     if (s->batch <= 0 || s->seqlen <= 0 || s->nheads <= 0 || s->headdim <= 0) return SSD_ERR_SHAPE;
-    if (s->headdim % 4 != 0 || s->headdim > 1024) return SSD_ERR_UNSUPPORTED;
-    *rows = static_cast<long long>(s->batch) * s->seqlen;
-    *cols = s->nheads * s->headdim;
+    const int parts = head_parts(*s), tokens = row_tokens(*s);
+    if (s->nheads % parts != 0 || tokens > s->seqlen) return SSD_ERR_SHAPE;
+    if (s->headdim % 4 != 0 || s->headdim * static_cast<long long>(parts) > 1024) return SSD_ERR_UNSUPPORTED;
+    *d = GateDims{static_cast<long long>(s->batch) * tokens, s->nheads * s->headdim, s->nheads / parts, s->headdim * parts};
     return SSD_OK;
 }
 
@@ -233,27 +240,25 @@ int gate_dims(const SsdShape* s, long long* rows, int* cols) {
 }  // namespace ssd
 
 extern "C" size_t ssd_gate_partial_floats(const SsdShape* shape) {
-    long long rows = 0;
-    int cols = 0;
-    if (ssd::gate_dims(shape, &rows, &cols) != SSD_OK) return 0;
-    return static_cast<size_t>(ssd::gate_grid(rows, cols, ssd::kGateMinRows).rowblocks) * cols;
+    ssd::GateDims n;
+    if (ssd::gate_dims(shape, &n) != SSD_OK) return 0;
+    return static_cast<size_t>(ssd::gate_grid(n.rows, n.cols, ssd::kGateMinRows).rowblocks) * n.cols;
 }
 
 extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const float* x, const float* D, int d_mode,
                                  const float* z, float* out, ssd_stream_t stream) {
     using namespace ssd;
-    long long rows = 0;
-    int cols = 0;
-    const int rc = gate_dims(shape, &rows, &cols);
+    GateDims n;
+    const int rc = gate_dims(shape, &n);
     if (rc != SSD_OK) return rc;
     if (!y || !out || (d_mode != 0 && (!D || !x))) return SSD_ERR_NULL;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!aligned16(y, x, z, out, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
-    const GateGrid g = gate_grid(rows, cols, 1);
+    const GateGrid g = gate_grid(n.rows, n.cols, 1);
     if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
         launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0,
-                     reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out, rows, cols, shape->headdim, g.ct, g.rt,
+                     reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out, n.rows, n.cols, n.p, g.ct, g.rt,
                      g.rows_per_cta, static_cast<unsigned>(g.colblocks));
     };
     if (d_mode != 0)
@@ -267,20 +272,19 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
                                  int d_mode, const float* z, float* dy, float* dz, float* dD_partial, float* dD,
                                  ssd_stream_t stream) {
     using namespace ssd;
-    long long rows = 0;
-    int cols = 0;
-    const int rc = gate_dims(shape, &rows, &cols);
+    GateDims n;
+    const int rc = gate_dims(shape, &n);
     if (rc != SSD_OK) return rc;
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!dout || (z && (!y || !dy || !dz)) || (d_mode != 0 && (!D || !x || !dD_partial || !dD))) return SSD_ERR_NULL;
     if (!z && d_mode == 0) return SSD_OK;  // nothing to do
     if (!aligned16(dout, y, x, z, dy, dz, dD_partial, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
-    const GateGrid g = gate_grid(rows, cols, kGateMinRows);
+    const GateGrid g = gate_grid(n.rows, n.cols, kGateMinRows);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
         launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0, st, dout, y, x, D, d_mode, z,
-                     dy, dz, dD_partial, rows, cols, shape->headdim, g.ct, g.rt, g.rows_per_cta,
+                     dy, dz, dD_partial, n.rows, n.cols, n.p, g.ct, g.rt, g.rows_per_cta,
                      static_cast<unsigned>(g.colblocks));
     };
     if (d_mode != 0)
@@ -288,11 +292,10 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     else
         launch(gate_skip_bwd_kernel<false, true>);
     if (d_mode != 0) {
-        const int p = shape->headdim;
-        const int lanes = 1024 / p;
-        const int threads = (lanes * p + 31) / 32 * 32;
-        launch_plain(gate_dd_reduce_kernel, shape->nheads, threads, threads * sizeof(double), st, dD_partial,
-                     static_cast<int>(g.rowblocks), cols, p, d_mode, lanes, dD);
+        const int lanes = 1024 / n.p;
+        const int threads = (lanes * n.p + 31) / 32 * 32;
+        launch_plain(gate_dd_reduce_kernel, n.heads, threads, threads * sizeof(double), st, dD_partial,
+                     static_cast<int>(g.rowblocks), n.cols, n.p, d_mode, lanes, dD);
     }
     return launch_status();
 }

@@ -92,3 +92,38 @@ def test_no_stage_writes_outside_its_buffers(shape):
     got = [v["out"], v["final"], v["dx"], v["ddt"], v["dA"], v["dB"], v["dC"]]
     for gt, w, name in zip(got, want, ["out", "final", "dx", "ddt", "dA", "dB", "dC"]):
         assert O.rel_l2(gt.cpu(), w) <= 2e-3, name
+
+
+def _between_pads(shapes, dev):
+    return {name: Padded(shp, dev, torch.float64 if name == "dA_part" else torch.float32) for name, shp in shapes.items()}
+
+
+def _check_pads(bufs, status, name):
+    torch.cuda.synchronize()
+    assert status.item() == 0, name
+    broken = [bn for bn, pb in bufs.items() if not pb.intact()]
+    assert not broken, f"{name} wrote outside {broken}"
+
+
+@pytest.mark.parametrize("b,l,h,p,parts", [(2, 129, 3, 60, 1), (1, 200, 2, 64, 3), (1, 5, 1, 4, 1)])
+def test_the_gate_stays_inside_tensors_of_any_extent(b, l, h, p, parts):
+    from ascend_kernel import _capi, mamba2 as M
+
+    dev = torch.device("cuda:0")
+    hk = h * parts
+    rnd = lambda *s: torch.randn(*s, device=dev)  # noqa: E731
+    y, x, z, dout, D = rnd(b, l, hk, p), rnd(b, l, hk, p), rnd(b, l, hk, p), rnd(b, l, hk, p), rnd(h)
+    shp = M.extents_shape(x, rnd(b, l, 1, 64), h, True, (0.0, float("inf")))
+    sp, lib, st = ctypes.byref(shp), _capi.lib, torch.cuda.current_stream().cuda_stream
+    bufs = _between_pads({"out": (b, l, hk, p), "dy": (b, l, hk, p), "dz": (b, l, hk, p), "dD": (h,),
+                          "part": (lib.ssd_gate_partial_floats(sp),)}, dev)
+    v = {name: pb.view.data_ptr() for name, pb in bufs.items()}
+    status, P = torch.zeros(1, dtype=torch.int32, device=dev), torch.Tensor.data_ptr
+    _capi.check(lib.ssd_gate_skip_fwd(sp, P(y), P(x), P(D), 1, P(z), v["out"], st), "gate_fwd")
+    _check_pads(bufs, status, "gate_fwd")
+    _capi.check(lib.ssd_gate_skip_bwd(sp, P(dout), P(y), P(x), P(D), 1, P(z), v["dy"], v["dz"], v["part"], v["dD"], st), "gate_bwd")
+    _check_pads(bufs, status, "gate_bwd")
+    want = M.gate_forward(y, x, None, D, z, h)
+    assert torch.equal(bufs["out"].view, want)
+    for got, ref in zip((bufs["dy"].view, bufs["dz"].view, bufs["dD"].view), M.gate_backward(dout, y, x, None, D, z, h)):
+        assert torch.equal(got, ref)

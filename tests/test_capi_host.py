@@ -181,3 +181,17 @@ def test_partial_sums_of_the_skip_gradient_cover_at_most_128_tokens(h, p, b, l):
     s = _capi.SsdShape(b, l, h, p, 64, 128, 1, 0, 0.0, 0.0, 0)
     blocks, rest = divmod(_capi.lib.ssd_gate_partial_floats(ctypes.byref(s)), h * p)
     assert rest == 0 and 128 * blocks >= b * l
+
+
+def test_the_gate_counts_the_tokens_and_heads_of_the_callers_tensors():
+    """A shape with SSD_FLAG_EXTENTS says the same to the gate as the tensors' own sizes: partial sums of as many blocks."""
+    from ascend_kernel import _capi
+
+    for b, l, h, parts in ((4, 37856, 6, 1), (1, 1000, 3, 4), (2, 129, 2, 16), (1, 256, 2, 2)):
+        padded = -(-l // 128) * 128
+        ext = _capi.SsdShape(b, padded, h * parts, 64, 64, 128, 1, _capi.SSD_FLAG_EXTENTS | _capi.head_parts_flag(parts), 0.0, 1.0,
+                             l if l % 128 else 0)
+        own = _capi.SsdShape(b, l, h, 64 * parts, 64, 128, 1, 0, 0.0, 0.0, 0)
+        want = _capi.lib.ssd_gate_partial_floats(ctypes.byref(own))
+        assert want > 0 and _capi.lib.ssd_gate_partial_floats(ctypes.byref(ext)) == want
+        assert _capi.lib.ssd_buffer_bytes(ctypes.byref(ext), 7) == 4 * want
