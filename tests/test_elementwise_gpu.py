@@ -124,3 +124,23 @@ def test_convolution_and_split(batch, l, d_in, gn, heads):
     want = bias.double() + sum(padded[:, k:k + l] * weight[:, k].double() for k in range(4))
     assert _rel(torch.cat([x, bm, cm], -1), torch.nn.functional.silu(want)) <= REL
     assert torch.equal(dt, src[..., ch:ch + heads]) and torch.allclose(A, -torch.exp(a_log[:heads]), rtol=1e-6)
+
+
+def test_finalize_takes_a_buffer_of_any_alignment():
+    """ddt_t is the caller's own buffer in the C interface and was never asked to be 16-byte aligned."""
+    import ctypes
+
+    from ascend_kernel import _capi
+
+    b, l, h = 2, 256, 5
+    s = ctypes.byref(_capi.SsdShape(b, l, h, 64, 64, 128, 1, 1, 0.0, float("inf"), 0))
+    part = torch.randn(b, h, l // 128, device="cuda", dtype=torch.float64)
+    raw = torch.randn(b * h * l + 1, device="cuda")
+    results = []
+    for ddt_t in (raw[1:].clone(), raw[1:]):
+        ddt, dA, dbias = torch.empty(b, l, h, device="cuda"), torch.empty(h, device="cuda"), torch.empty(h, device="cuda")
+        _capi.check(_capi.lib.ssd_dt_finalize_bias_bwd(s, ddt_t.data_ptr(), part.data_ptr(), ddt.data_ptr(), dA.data_ptr(),
+                                                      dbias.data_ptr(), torch.cuda.current_stream().cuda_stream), "finalize")
+        results.append((ddt, dA, dbias))
+    assert all(torch.equal(a, c) for a, c in zip(*results))
+    assert torch.equal(results[0][0], raw[1:].view(b, h, l).transpose(1, 2))
