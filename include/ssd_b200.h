@@ -377,6 +377,7 @@ typedef struct SsdBackwardArgs {
     int32_t* status;
     int32_t d_mode;
 } SsdBackwardArgs;
+int ssd_use_state_scan(const SsdShape* shape, int state_route); /* what that choice is on the current device */
 size_t ssd_forward_work_bytes(const SsdShape* shape);
 size_t ssd_backward_work_bytes(const SsdShape* shape, int has_d, int has_z);
 int ssd_forward(const SsdShape* shape, const SsdForwardArgs* args, int state_route, ssd_stream_t stream);

@@ -110,6 +110,7 @@ SIGNATURES = {
     "ssd_linear_work_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
     "ssd_linear_pays": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]),
     "ssd_linear_fwd": (ctypes.c_int, [_p, _p, _p, _p, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, _p, _p, _p]),
+    "ssd_use_state_scan": (ctypes.c_int, [_shape_p, ctypes.c_int]),
     "ssd_forward_work_bytes": (ctypes.c_size_t, [_shape_p]),
     "ssd_backward_work_bytes": (ctypes.c_size_t, [_shape_p, ctypes.c_int, ctypes.c_int]),
     "ssd_forward": (ctypes.c_int, [_shape_p, ctypes.POINTER(SsdForwardArgs), ctypes.c_int, _p]),

@@ -153,9 +153,9 @@ def _validate(x, dt, A, B, C, chunk_size, D, z, dt_bias, dt_limit, initial_state
 # The per-tile state products and the inter-tile recurrence run either as two tile-parallel launches
 # (ssd_chunk_state + ssd_state_passing_*) or as one launch that walks each (batch, group) in tile order with
 # the running state on chip (ssd_chunk_state_scan).  The second moves 2 GiB less per pass at the H256 shape
-# but has only batch * ngroups CTAs; "auto" takes it when that is at least 1.5 x the SM count.
+# but has only batch * ngroups CTAs; "auto" leaves the choice to the library (ssd_use_state_scan).
 _state_scan = "auto"
-_sm_counts: Dict[int, int] = {}
+_ROUTES = {"auto": 0, "on": 1, "off": 2}
 
 
 def set_state_scan(mode: str) -> str:
@@ -168,15 +168,9 @@ def set_state_scan(mode: str) -> str:
 
 
 def _use_state_scan(shape: "_capi.SsdShape", device: torch.device) -> bool:
-    if _state_scan == "off" or not _capi.lib.ssd_chunk_state_scan_supported(ctypes.byref(shape)):
-        return False
-    if _state_scan == "on":
-        return True
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    sms = _sm_counts.get(idx)
-    if sms is None:
-        sms = _sm_counts[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    return 2 * shape.batch * shape.ngroups >= 3 * sms
+    """The library's own rule, for ``device``, which is the current one wherever stages are launched."""
+    with _device_guard(device):
+        return bool(_capi.lib.ssd_use_state_scan(ctypes.byref(shape), _ROUTES[_state_scan]))
 
 
 def _state_cols(shape: "_capi.SsdShape") -> int:
@@ -376,9 +370,6 @@ def _epilogue_gradients(dout, y, x, D, z, heads: int):
 # ----------------------------------------------------------------------------- whole calls
 # The stages of one direction as one foreign call (ssd_forward, ssd_backward).  While stage_events collects, the same
 # stages are launched one by one with events around them.
-_ROUTES = {"auto": 0, "on": 1, "off": 2}
-
-
 def forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, shape, want_final: bool, copy: bool = False):
     """(out, final, y, work tensors): ``y`` is the SSD output before the D / z epilogue; without one it is ``out`` itself, or
     with ``copy`` a tensor of its own."""

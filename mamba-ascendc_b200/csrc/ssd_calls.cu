@@ -56,17 +56,9 @@ struct BackwardWork {
     }
 };
 
-// The fused state kernel has batch * ngroups CTAs and takes the place of two launches where that is at least 1.5 x the SM
-// count ([8,4096,256,64], 512 chains: 0.80 ms against 1.03 ms for the pair; [8,4096,32,64], 64 chains: the pair is
-// faster, 0.13 against 0.19 ms).  route: 0 by this rule, 1 wherever the kernel takes the shape, 2 never.
-bool use_state_scan(const SsdShape& s, int route) {
-    if (route == 2 || !ssd_chunk_state_scan_supported(&s)) return false;
-    return route == 1 || 2ll * s.batch * s.ngroups >= 3ll * sm_count();
-}
-
 int run_states(const SsdShape& s, const float* x, const float* m, const float* q, const float* cs, const float* start,
                float* states, float* end, int mode, int route, int* status, ssd_stream_t st) {
-    if (use_state_scan(s, route)) return ssd_chunk_state_scan(&s, x, m, q, cs, start, states, end, mode, status, st);
+    if (ssd_use_state_scan(&s, route)) return ssd_chunk_state_scan(&s, x, m, q, cs, start, states, end, mode, status, st);
     const int rc = ssd_chunk_state(&s, x, m, q, cs, states, mode, status, st);
     if (rc != SSD_OK) return rc;
     return mode == 0 ? ssd_state_passing_fwd(&s, states, cs, start, end, st)
@@ -76,6 +68,14 @@ int run_states(const SsdShape& s, const float* x, const float* m, const float* q
 }  // namespace
 
 }  // namespace ssd
+
+// The fused state kernel has batch * ngroups CTAs and takes the place of two launches where that is at least 1.5 x the SM
+// count ([8,4096,256,64], 512 chains: 0.80 ms against 1.03 ms for the pair; [8,4096,32,64], 64 chains: the pair is
+// faster, 0.13 against 0.19 ms).
+extern "C" int ssd_use_state_scan(const SsdShape* shape, int state_route) {
+    if (state_route == 2 || !ssd_chunk_state_scan_supported(shape)) return 0;
+    return state_route == 1 || 2ll * shape->batch * shape->ngroups >= 3ll * ssd::sm_count() ? 1 : 0;
+}
 
 extern "C" size_t ssd_forward_work_bytes(const SsdShape* shape) {
     if (ssd_check_shape(shape) != SSD_OK) return 0;
