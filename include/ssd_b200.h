@@ -323,7 +323,7 @@ int ssd_forward_static(const SsdShape* shape, const float* x, const float* dt, c
 
 /* ---------------------------------------------------------------- test hooks
  *
- * The two entry points below exist for the test suite only (source: csrc/ssd_selftest.cu); a library built with
+ * The entry points ssd_selftest_* below exist for the test suite only (source: csrc/ssd_selftest.cu); a library built with
  * `build.py --product-only` does not export them. */
 
 /* Tile-level check of the tensor-core path: D[128,n] = A * B^T with K = 128,
@@ -348,6 +348,10 @@ int ssd_selftest_wait_expiry(int* status, int polls, ssd_stream_t stream);
  * with the same incremental, division-free arithmetic the kernels use.  tests/ compare it with the closed form.
  * No counterpart in the reference. */
 int ssd_selftest_tile_walk(const SsdShape* shape, int grid, int cta, int count, int* out);
+/* The same with the heads of a group dealt to `split` work items and the state columns to `blocks` (1 or 2): 6 ints each,
+ * the four above and the group and column block that the work item reads.  And the rule that chooses the split. */
+int ssd_selftest_split_walk(const SsdShape* shape, int grid, int cta, int split, int blocks, int count, int* out);
+int ssd_selftest_head_split(long long items, int heads_per_group, int slots, int unit, int overhead_halves);
 
 /* ---------------------------------------------------------------- whole calls
  *

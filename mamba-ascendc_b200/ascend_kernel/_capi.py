@@ -80,6 +80,8 @@ SIGNATURES = {
     "ssd_buffer_bytes": (ctypes.c_size_t, [_shape_p, ctypes.c_int]),
     "ssd_selftest_wait_expiry": (ctypes.c_int, [_p, ctypes.c_int, _p]),
     "ssd_selftest_tile_walk": (ctypes.c_int, [_shape_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, _p]),
+    "ssd_selftest_split_walk": (ctypes.c_int, [_shape_p] + [ctypes.c_int] * 5 + [_p]),
+    "ssd_selftest_head_split": (ctypes.c_int, [ctypes.c_longlong] + [ctypes.c_int] * 4),
     "ssd_selftest_umma": (ctypes.c_int, [_p, _p, _p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _p, _p]),
     "ssd_dt_cumsum": (ctypes.c_int, [_shape_p, _p, _p, _p, _p, _p, _p]),
     "ssd_recurrent_fwd": (ctypes.c_int, [_shape_p] + [_p] * 7 + [ctypes.c_int] + [_p] * 5),
@@ -120,7 +122,8 @@ SIGNATURES = {
 }
 
 # test-only entry points; a library built with ``build.py --product-only`` does not have them
-TEST_HOOKS = {"ssd_selftest_umma", "ssd_selftest_wait_expiry", "ssd_selftest_tile_walk"}
+TEST_HOOKS = {"ssd_selftest_umma", "ssd_selftest_wait_expiry", "ssd_selftest_tile_walk", "ssd_selftest_split_walk",
+              "ssd_selftest_head_split"}
 
 for _name, (_res, _args) in SIGNATURES.items():
     if _name in TEST_HOOKS and not hasattr(lib, _name):

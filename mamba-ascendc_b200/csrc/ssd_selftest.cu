@@ -341,3 +341,31 @@ extern "C" int ssd_selftest_tile_walk(const SsdShape* shape, int grid, int cta, 
     return SSD_OK;
 }
 
+
+// The same walk where the heads of a group are dealt to `split` work items and the state columns to `blocks`: six ints a head
+// (group of work items, head, first token, tile index, group whose B and C it reads, column block).
+extern "C" int ssd_selftest_split_walk(const SsdShape* shape, int grid, int cta, int split, int blocks, int count, int* out) {
+    using namespace ssd;
+    const int rc = ssd_check_shape(shape);
+    if (rc != SSD_OK) return rc;
+    if (!out || grid <= 0 || cta < 0 || cta >= grid || count < 0 || split < 1 || shape->nheads / shape->ngroups % split != 0 ||
+        blocks < 1 || blocks > 2)
+        return SSD_ERR_SHAPE;
+    const TileWalk walk(*shape, grid, split, blocks);
+    TilePos cur = walk.first(cta);
+    int hi = 0;
+    for (int it = 0; it < count; ++it) {
+        const HeadPos w = walk.locate(cur, hi, 0);
+        const int row[6] = {w.g, w.h, w.tok0, w.tile_index, walk.group_of(w.g), walk.column_block(w.g)};
+        for (int i = 0; i < 6; ++i) out[6 * it + i] = row[i];
+        if (++hi == walk.heads_per_group) {
+            hi = 0;
+            walk.advance(cur);
+        }
+    }
+    return SSD_OK;
+}
+
+extern "C" int ssd_selftest_head_split(long long items, int heads_per_group, int slots, int unit, int overhead_halves) {
+    return ssd::choose_head_split(items, heads_per_group, slots, unit, overhead_halves);
+}

@@ -183,6 +183,46 @@ def test_partial_sums_of_the_skip_gradient_cover_at_most_128_tokens(h, p, b, l):
     assert rest == 0 and 128 * blocks >= b * l
 
 
+@pytest.mark.parametrize("b,l,h,g", [(2, 384, 24, 2), (1, 128, 12, 1), (3, 256, 30, 5)])
+@pytest.mark.parametrize("split", [1, 2, 3, 6])
+@pytest.mark.parametrize("blocks", [1, 2])
+def test_work_items_of_a_split_group_cover_every_head_once(b, l, h, g, split, blocks):
+    """The persistent kernels' walk with the heads of a group dealt to several work items, one set per column block."""
+    from ascend_kernel import _capi
+
+    shape = _shape(b=b, l=l, h=h, g=g)
+    if (h // g) % split:
+        return
+    items, per_item, tiles = b * g * split * blocks * (l // 128), h // g // split, l // 128
+    for grid in (1, 5, items):
+        seen = {}
+        for cta in range(grid):
+            count = len(range(cta, items, grid)) * per_item
+            out = (ctypes.c_int * (6 * count))()
+            assert _capi.lib.ssd_selftest_split_walk(ctypes.byref(shape), grid, cta, split, blocks, count, out) == 0
+            for i in range(count):
+                wg, head, tok0, tile, group, block = out[6 * i:6 * i + 6]
+                bb, k = tok0 // l, tok0 % l // 128
+                assert group == head // (h // g) and tile == (bb * h + head) * tiles + k
+                assert wg // blocks // split == group and block == wg % blocks and head // per_item == wg // blocks
+                seen[bb, head, k, block] = seen.get((bb, head, k, block), 0) + 1
+        assert len(seen) == b * h * tiles * blocks and set(seen.values()) == {1}
+
+
+def test_rule_of_the_head_split():
+    from ascend_kernel import _capi
+
+    rule = _capi.lib.ssd_selftest_head_split
+    for items in (1, 3, 64, 147, 148, 149, 300, 1000, 16 * 148 - 1, 16 * 148):
+        for heads in (1, 2, 7, 12, 32):
+            for unit, overhead in ((1, 2), (1, 3), (1, 5), (2, 1)):
+                split = rule(items, heads, 148, unit, overhead)
+                cost = lambda d: -(-items * d // 148) * (2 * -(-heads // d // unit) + overhead)  # noqa: E731
+                assert split >= 1 and heads % split == 0
+                assert split == 1 or (items < 16 * 148 and items * split <= 32 * 148 and 20 * cost(split) < 19 * cost(1))
+    assert rule(320, 8, 148, 1, 2) == 2 and rule(64, 32, 148, 1, 2) > 1 and rule(1, 1, 148, 1, 2) == 1
+
+
 def test_the_gate_counts_the_tokens_and_heads_of_the_callers_tensors():
     """A shape with SSD_FLAG_EXTENTS says the same to the gate as the tensors' own sizes: partial sums of as many blocks."""
     from ascend_kernel import _capi
