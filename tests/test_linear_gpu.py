@@ -58,6 +58,14 @@ def test_layers_with_hooks_or_a_lower_precision_policy_are_left_alone():
         handle = layer.register_forward_hook(lambda *a: seen.append(1))
         assert torch.equal(V._linear(layer, x), layer(x)) and len(seen) == 2
         handle.remove()
+        matmul, before = torch.backends.cuda.matmul, torch.backends.cuda.matmul.fp32_precision
+        try:
+            matmul.fp32_precision = "tf32"
+            assert torch.equal(V._linear(layer, x), layer(x)) and not torch.equal(layer(x), plain)
+        finally:
+            matmul.fp32_precision = before
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            assert V._linear(layer, x).dtype == torch.bfloat16
     assert V._linear(layer, x).requires_grad  # with gradients: the layer
 
 

@@ -148,3 +148,39 @@ def test_convolution_of_more_than_a_million_tokens():
     want = F.silu(sum(src[:, k:k + l] * w[:, k] for k in range(4)) + bias.double())
     assert torch.allclose(torch.cat([x, b, c], dim=-1).double(), want, rtol=1e-5, atol=1e-5)
     assert torch.equal(dt, wide[..., channels:]) and torch.allclose(a, -a_log.exp())
+
+
+@pytest.mark.gpu
+def test_network_through_the_projection_kernel():
+    """Large enough, with a ragged number of rows, for both projections of a block to run as the library's own kernel."""
+    from ascend_kernel import _capi, check_status, vmamba2 as V
+
+    torch.manual_seed(4)
+    dev = torch.device("cuda:0")
+    cfg = V.VisionMamba2Config(image_size=1008, depth=2, num_classes=16)
+    rows = 2 * cfg.tokens  # 7938
+    net = V.VisionMamba2(cfg).to(dev)
+    blk = net.blocks[0]
+    layers = (blk.in_proj, blk.out_proj)
+    assert rows % 128 and all(_capi.lib.ssd_linear_pays(rows, *layer.weight.shape) for layer in layers)
+    img = torch.randn(2, 3, 1008, 1008, device=dev)
+    launched = []
+    launch = V._launch
+    V._launch = lambda name, *args: (launched.append(name), launch(name, *args))[1]
+    try:
+        with torch.no_grad():
+            fused = net(img)
+    finally:
+        V._launch = launch
+    assert launched.count("vmamba2_linear") == 2 * cfg.depth
+    with torch.enable_grad():
+        plain = net(img).detach()
+    check_status()
+    assert ((fused - plain).norm() / plain.norm()).item() < 1e-5
+    for layer in layers:  # 24-bit operands, fp32 sums: as the framework's own layer, against fp64
+        x, u = torch.randn(2, rows // 2, layer.in_features, device=dev), torch.randn(2, rows // 2, layer.out_features, device=dev)
+        with torch.no_grad():
+            got, library = V._linear(layer, x, u).double(), (layer(x) + u).double()
+        want = x.double() @ layer.weight.double().T + u.double()
+        assert (got - want).norm() <= (library - want).norm()
+    check_status()
