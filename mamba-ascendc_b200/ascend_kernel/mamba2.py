@@ -385,7 +385,8 @@ def forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, shape, want_fina
     y = torch.empty_like(x) if gated or copy else out
     sp = ctypes.byref(shape)
     lib = _capi.lib
-    work = torch.empty(lib.ssd_forward_work_bytes(sp), device=dev, dtype=torch.uint8)
+    # q, cs and the states: floats, also for saved-tensor hooks that convert what autograd keeps
+    work = torch.empty(lib.ssd_forward_work_bytes(sp) // 4, device=dev, dtype=torch.float32)
     final = (torch.empty(shape.batch, shape.nheads, shape.headdim, shape.dstate, device=dev, dtype=torch.float32)
              if want_final else None)
     args = _capi.SsdForwardArgs(
