@@ -431,6 +431,11 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t.clone() if t.data_ptr() & 15 else t
 
 
+def _epilogue_alone(ctx) -> bool:
+    """Whether of the inputs of ``_Mamba2SsdAutograd`` only D and z need gradients."""
+    return not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9))
+
+
 class _Mamba2SsdAutograd(torch.autograd.Function):
     """Counterpart of ``_Mamba2SsdAutogradM1`` (mamba2.py:1661-1838), with the D skip connection and the z gate inside the node:
     the epilogue runs as one fused pass forward and one backward (the reference fuses them into its state-epilogue and
@@ -456,6 +461,8 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         if ctx.recompute:  # inputs only; y, q, cs and the tile-start states are rebuilt in backward
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start)
         else:
+            if _epilogue_alone(ctx):  # its gradients take y only
+                work = ()
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start, y, *work)
         return out, final
 
@@ -465,7 +472,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         y, work = (rest[0], rest[1:]) if rest else (None, None)
         if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
             dout = torch.zeros_like(x)
-        alone = not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9))  # D and z alone need gradients
+        alone = _epilogue_alone(ctx)
         again = ctx.differentiable and (torch.is_grad_enabled() or (alone and _is_batched(dout)))
         if again and not alone:
             return _Mamba2SsdAutograd.differentiable_backward(ctx, dout, dfinal)

@@ -98,3 +98,18 @@ def test_saved_tensor_hooks_that_convert(shape):
         out = mamba2_ssd_fwd(*t, 64, dt_softplus=True)
     for name, got, ref in zip(("dx", "ddt", "dA", "dB", "dC"), torch.autograd.grad(out, t, up), want):
         assert ((got - ref).norm() <= (0.3 if name == "dA" else 0.03) * ref.norm()).item(), name
+
+
+def test_what_is_kept_for_gradients_of_the_epilogue_alone():
+    from ascend_kernel import SavedTensorStats, mamba2_ssd_fwd
+
+    b, l, h, p, n, g = 1, 1000, 4, 64, 128, 1
+    rnd = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    x, dt, A, B, C, z = rnd(b, l, h, p), rnd(b, l, h).abs(), -rnd(h).abs(), rnd(b, l, g, n), rnd(b, l, g, n), rnd(b, l, h, p)
+    z.requires_grad_(True)
+    stats = SavedTensorStats()
+    with stats.hooks():
+        out = mamba2_ssd_fwd(x, dt, A, B, C, 64, z=z, dt_softplus=True)
+    inputs = sum(4 * t.numel() for t in (x, dt, A, B, C, z))
+    assert stats.unique_bytes <= inputs + 4 * out.numel() + 4096  # and the output before the gate, no states
+    assert torch.isfinite(torch.autograd.grad(out.sum(), z)[0]).all()
