@@ -357,11 +357,12 @@ int linear_cols_padded(int cols) { return (cols + kLinCols - 1) / kLinCols * kLi
 // these sizes the library's fp32 kernel takes less.  Measured over K = 64 ... 1536, 64 to 6278 columns, 200 to 16384 rows (us, this
 // kernel / the library): [1024,192] x [902,192] 17 / 17, [2048,192] x [902,192] 22 / 26, [16384,192] x [902,192] 50 / 139;
 // [2048,384] x [902,384] 34 / 41, [4096,384] x [192,384] 32 / 25; [2048,576] x [576,576] 44 / 33, [512,576] x [2438,576] 44 / 50;
-// [16384,64 to 1536] x [64,..] 0.9 of the library throughout, [16384,1024] x [192,1024] 81 / 150.  Of the sizes taken none was slower.
+// [16384,1024] x [192,1024] 81 / 150.  Fewer columns than a tile's 96 were slower at every size (64 columns: 16384 rows, K = 192
+// 20 / 18, 30000 rows, K = 768 81 / 76).  Of the sizes taken none was slower.
 extern "C" int ssd_linear_pays(long long rows, int cols, int k) {
     const int chunks = ssd::linear_chunks(k);
     if (rows <= 0 || cols <= 0 || chunks == 0) return 0;
-    return static_cast<double>(rows) * cols * k >= 2.3e8 * chunks ? 1 : 0;
+    return cols >= ssd::kLinCols && static_cast<double>(rows) * cols * k >= 2.3e8 * chunks ? 1 : 0;
 }
 
 extern "C" size_t ssd_linear_work_bytes(int cols, int k) {

@@ -235,3 +235,13 @@ def test_the_gate_counts_the_tokens_and_heads_of_the_callers_tensors():
         want = _capi.lib.ssd_gate_partial_floats(ctypes.byref(own))
         assert want > 0 and _capi.lib.ssd_gate_partial_floats(ctypes.byref(ext)) == want
         assert _capi.lib.ssd_buffer_bytes(ctypes.byref(ext), 7) == 4 * want
+
+
+@pytest.mark.parametrize("rows,cols,k,pays", [
+    (16384, 902, 192, 1), (16384, 192, 384, 1), (1024, 902, 192, 0), (4096, 192, 384, 0), (2048, 902, 384, 1), (4096, 192, 768, 0),
+    (30000, 64, 768, 0), (30000, 96, 768, 1), (1024, 902, 1024, 0), (2048, 902, 1024, 1), (16384, 902, 200, 0), (0, 902, 192, 0),
+])
+def test_sizes_at_which_the_projection_kernel_pays(rows, cols, k, pays):
+    from ascend_kernel import _capi
+
+    assert _capi.lib.ssd_linear_pays(rows, cols, k) == pays
