@@ -26,6 +26,11 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+try:  # the C-ABI binding and the SSD call; None when this file is loaded on its own (no package, no CUDA library)
+    from . import _capi, mamba2 as _mamba2
+except (ImportError, ValueError):
+    _capi = _mamba2 = None
+
 
 @dataclass
 class VisionMamba2Config:
@@ -54,50 +59,44 @@ class VisionMamba2Config:
         return (self.image_size // self.patch) ** 2
 
 
-def _kernels():
-    """The C-ABI binding, or None when this module was loaded on its own (no package, no CUDA library)."""
-    try:
-        from . import _capi
-    except (ImportError, ValueError):
-        return None
-    return _capi
-
-
 def _fast(t: torch.Tensor) -> bool:
-    return t.is_cuda and t.dtype == torch.float32 and not torch.is_grad_enabled() and _kernels() is not None
+    return t.is_cuda and t.dtype == torch.float32 and not torch.is_grad_enabled() and _capi is not None
 
 
 def _launch(name: str, device: torch.device, fn: Callable, *args) -> None:
     """``fn(*args, stream)`` on the tensors' device, which need not be the current one, and its current stream."""
-    from .mamba2 import _device_guard
-
-    with _device_guard(device):
-        _kernels().check(fn(*args, torch.cuda.current_stream().cuda_stream), name)
+    with _mamba2._device_guard(device):
+        _capi.check(fn(*args, _mamba2._stream()), name)
 
 
 def _rmsnorm_kernel(x2d: torch.Tensor, x_stride: int, z, z_stride: int, weight: torch.Tensor, eps: float, rows: int,
                     d: int, skip=None, D=None, headdim: int = 0) -> torch.Tensor:
     out = torch.empty(rows, d, device=weight.device, dtype=torch.float32)
-    _launch("vmamba2_rmsnorm", weight.device, _kernels().lib.ssd_block_skip_rmsnorm_fwd, x2d, x_stride, skip, D, headdim, z,
+    _launch("vmamba2_rmsnorm", weight.device, _capi.lib.ssd_block_skip_rmsnorm_fwd, x2d, x_stride, skip, D, headdim, z,
             z_stride, weight.data_ptr(), out.data_ptr(), rows, d, eps)
     return out
+
+
+_PLAIN = (torch.Tensor, nn.Parameter)
 
 
 def _plain_projection(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor]) -> bool:
     """Whether ``layer(x)`` (+ residual) is what ssd_linear_fwd computes from these tensors: plain tensors whose widths and
     shapes fit, one device, contiguous fp32.  Whatever does not fit is for the layer to take or to refuse."""
-    w = layer.weight
-    if type(layer) is not nn.Linear or "forward" in layer.__dict__ or layer.bias is not None or w.dim() != 2 or x.dim() < 1:
+    if type(layer) is not nn.Linear or "forward" in layer.__dict__ or layer.bias is not None:
         return False
+    w = layer.weight
     # a subclass, or a tensor inside a function transform, need not have a storage of its own
-    if torch._C._are_functorch_transforms_active() or any(type(t) not in (torch.Tensor, nn.Parameter)
-                                                          for t in (x, w, residual) if t is not None):
+    if (type(x) not in _PLAIN or type(w) not in _PLAIN or w.dim() != 2 or x.dim() < 1 or
+            torch._C._are_functorch_transforms_active()):
         return False
     n, k = w.shape
-    if x.shape[-1] != k or (residual is not None and residual.shape != (*x.shape[:-1], n)):
+    device = x.device
+    if not (x.shape[-1] == k and w.device == device and x.dtype == w.dtype == torch.float32 and x.is_contiguous() and
+            w.is_contiguous()):
         return False
-    if any(t.device != x.device or t.dtype != torch.float32 or not t.is_contiguous()
-           for t in (x, w, residual) if t is not None):
+    if residual is not None and not (type(residual) in _PLAIN and residual.shape[:-1] == x.shape[:-1] and residual.shape[-1] == n and
+                                     residual.device == device and residual.dtype == torch.float32 and residual.is_contiguous()):
         return False
     # (torch.get_float32_matmul_precision raises once a program has set the policy per backend)
     return (not torch.is_autocast_enabled() and torch.backends.cuda.matmul.fp32_precision in ("none", "ieee") and
@@ -108,17 +107,15 @@ def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] 
     """``layer(x)`` (+ residual).  A plain bias-free fp32 projection in inference runs as ``ssd_linear_fwd`` (tensor cores at
     fp32 accuracy); anything else about the layer, the precision the caller chose or the sizes goes to the layer itself."""
     if _fast(x) and _plain_projection(layer, x, residual) and x.data_ptr() % 16 == 0:
-        capi = _kernels()
-        n, k = layer.weight.shape
+        w, lib = layer.weight, _capi.lib
+        n, k = w.shape
         rows = x.numel() // k if k else 0
-        if capi.lib.ssd_linear_pays(rows, n, k):
-            from .mamba2 import _status
-
-            work = torch.empty(capi.lib.ssd_linear_work_bytes(n, k), device=x.device, dtype=torch.uint8)
+        if lib.ssd_linear_pays(rows, n, k):
+            work = torch.empty(lib.ssd_linear_work_bytes(n, k), device=x.device, dtype=torch.uint8)
             out = torch.empty(*x.shape[:-1], n, device=x.device, dtype=torch.float32)
-            _launch("vmamba2_linear", x.device, capi.lib.ssd_linear_fwd, x.data_ptr(), layer.weight.data_ptr(),
+            _launch("vmamba2_linear", x.device, lib.ssd_linear_fwd, x.data_ptr(), w.data_ptr(),
                     None if residual is None else residual.data_ptr(), out.data_ptr(), rows, n, k, work.data_ptr(),
-                    _status(x.device).data_ptr())
+                    _mamba2._status(x.device).data_ptr())
             return out
     y = layer(x)
     return y if residual is None else residual + y
@@ -127,7 +124,7 @@ def _linear(layer: nn.Module, x: torch.Tensor, residual: Optional[torch.Tensor] 
 def _per_head(t: torch.Tensor, device: torch.device, heads: int) -> bool:
     """Whether the block kernels can read ``t`` as one fp32 value per head.  Other parameters stay with the framework and the
     SSD call, which take or refuse them."""
-    return (type(t) in (torch.Tensor, nn.Parameter) and t.device == device and t.dtype == torch.float32 and
+    return (type(t) in _PLAIN and t.device == device and t.dtype == torch.float32 and
             t.shape == (heads,) and t.is_contiguous())
 
 
@@ -204,7 +201,7 @@ class Mamba2Block(nn.Module):
         else:
             dt, A = zxbcdt[..., 2 * d_in + 2 * g * n:].contiguous(), -torch.exp(self.A_log)
             a_log, dt_out, a_out, heads = None, None, None, 0
-        _launch("vmamba2_conv1d", dev, _kernels().lib.ssd_block_conv_split_fwd, zxbcdt.data_ptr() + 4 * d_in, width,
+        _launch("vmamba2_conv1d", dev, _capi.lib.ssd_block_conv_split_fwd, zxbcdt.data_ptr() + 4 * d_in, width,
                 w.data_ptr(), None if bias is None else bias.data_ptr(), a_log, x.data_ptr(), bm.data_ptr(), cm.data_ptr(),
                 dt_out, a_out, b, l, d_in, g * n, heads)
         # a skip connection per head is added where the gated norm reads y anyway

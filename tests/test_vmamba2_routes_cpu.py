@@ -88,6 +88,11 @@ def test_weights_and_inputs_without_storage_of_their_own_are_left_to_the_layer()
     assert taken == [False]
 
 
+def test_other_layers_are_left_alone():
+    assert not V._plain_projection(torch.nn.Identity(), torch.zeros(3, 64), None)
+    assert not V._plain_projection(torch.nn.Linear(64, 96), torch.zeros(3, 64), None)  # with a bias
+
+
 def test_a_replaced_forward_is_kept():
     layer = _layer()
     layer.forward = lambda x: x
@@ -106,7 +111,6 @@ def test_per_head_parameters_that_the_block_kernels_read(t, taken):
 
 def test_kernels_run_on_the_device_and_stream_of_their_tensors(monkeypatch):
     import contextlib
-    from types import SimpleNamespace
 
     from ascend_kernel import mamba2 as M
 
@@ -119,7 +123,7 @@ def test_kernels_run_on_the_device_and_stream_of_their_tensors(monkeypatch):
         current[0] = before
 
     monkeypatch.setattr(M, "_device_guard", guard)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream="stream of " + current[0]))
+    monkeypatch.setattr(M, "_stream", lambda: "stream of " + current[0])
     calls = []
     V._launch("norm", torch.device("cuda:1"), lambda *a: calls.append(a) or 0, 7)
     assert calls == [(7, "stream of cuda:1")] and current == ["cuda:0"]
