@@ -113,6 +113,7 @@ int launch_norm(const NormArgs& a, cudaStream_t stream) {
 // 20 us = 3.4 TB/s; 64 tokens per thread with eight loads in flight took 33 us.  weight [C,4] (tap k multiplies the input 3-k tokens
 // back), bias [C].  Channels behind the convolved ones are dt: copied as they are.
 constexpr int kConvTokens = 16;
+constexpr int kGridY = 65535;
 
 struct ConvArgs {
     const float *xbc, *weight, *bias, *a_log;
@@ -121,16 +122,18 @@ struct ConvArgs {
     int seqlen, d_in, gn, heads;  // heads: of dt and A, 0 = neither
 };
 
+// SLICED: a sequence of more than 65535 blocks of tokens, the most that grid.y holds, is several slices of grid.z.
+template <bool SLICED>
 __global__ void __launch_bounds__(128)
-block_conv_silu_kernel(const ConvArgs a, unsigned channel_blocks) {
+block_conv_silu_kernel(const ConvArgs a, int slices) {
     after_previous();
     allow_next();
     const int channels = a.d_in + 2 * a.gn;
-    const unsigned token_block = blockIdx.x / channel_blocks;  // in one dimension: as many tokens as an int counts
-    const int c = (blockIdx.x - token_block * channel_blocks) * 128 + threadIdx.x;
+    const int c = blockIdx.x * 128 + threadIdx.x;
     if (c >= channels + a.heads) return;
-    const int t0 = token_block * kConvTokens;
-    const long long b = blockIdx.y;
+    const long long b = SLICED ? blockIdx.z / slices : blockIdx.z;
+    const int t0 = (SLICED ? blockIdx.z % slices * kGridY + blockIdx.y : blockIdx.y) * kConvTokens;
+    if (SLICED && t0 >= a.seqlen) return;
     const float* src = a.xbc + (b * a.seqlen) * a.row_stride + c;
     float in[kConvTokens + 3];  // inputs from three tokens back on
 #pragma unroll
@@ -148,7 +151,7 @@ block_conv_silu_kernel(const ConvArgs a, unsigned channel_blocks) {
         dst = a.c_out, width = a.gn, col = c - a.d_in - a.gn;
     } else {
         dst = a.dt_out, width = a.heads, col = c - channels;
-        if (token_block == 0 && b == 0) a.a_out[col] = -expf(a.a_log[col]);
+        if (blockIdx.y == 0 && blockIdx.z == 0) a.a_out[col] = -expf(a.a_log[col]);
     }
     dst += (b * a.seqlen) * width + col;
     const int n = min(kConvTokens, a.seqlen - t0);
@@ -204,13 +207,13 @@ extern "C" int ssd_block_conv_split_fwd(const float* xbc, long long row_stride, 
     if (!xbc || !weight || !x_out || !b_out || !c_out || (heads > 0 && (!a_log || !dt_out || !a_out))) return SSD_ERR_NULL;
     if (batch <= 0 || seqlen <= 0 || d_in <= 0 || gn <= 0 || heads < 0 || row_stride < d_in + 2 * gn + heads)
         return SSD_ERR_SHAPE;
-    const long long channel_blocks = (static_cast<long long>(d_in) + 2ll * gn + heads + 127) / 128;
-    const long long blocks = channel_blocks * ((static_cast<long long>(seqlen) + kConvTokens - 1) / kConvTokens);
-    if (batch > 65535 || seqlen > 0x7fffffff - 2 * kConvTokens || blocks > 0x7fffffff) return SSD_ERR_RANGE;
+    const long long token_blocks = (static_cast<long long>(seqlen) + kConvTokens - 1) / kConvTokens;
+    const int slices = static_cast<int>((token_blocks + kGridY - 1) / kGridY);
+    if (batch > 65535 / slices || seqlen > 0x7fffffff - 2 * kConvTokens * kGridY) return SSD_ERR_RANGE;
     const ConvArgs a{xbc, weight, bias, a_log, x_out, b_out, c_out, dt_out, a_out, row_stride, seqlen, d_in, gn, heads};
-    const dim3 grid(static_cast<unsigned>(blocks), batch);
-    launch_plain(block_conv_silu_kernel, grid, 128, 0, reinterpret_cast<cudaStream_t>(stream), a,
-                 static_cast<unsigned>(channel_blocks));
+    const dim3 grid((d_in + 2 * gn + heads + 127) / 128, static_cast<unsigned>(slices == 1 ? token_blocks : kGridY), batch * slices);
+    launch_plain(slices == 1 ? block_conv_silu_kernel<false> : block_conv_silu_kernel<true>, grid, 128, 0,
+                 reinterpret_cast<cudaStream_t>(stream), a, slices);
     return launch_status();
 }
 

@@ -26,11 +26,15 @@ constexpr int kGateCtasWanted = 1184; // ... fewer when that leaves less than ei
 constexpr int kGateMinRows = 32;      // ... but there not so few that adding up the partials takes longer than forming them
 
 // How [rows, cols / 4] float4s are laid over CTAs: `colblocks` blocks of `ct` threads along a row, `rt` rows side by
-// side in a CTA.  ct * rt <= kGateThreads, and ct is as even a share of the row as the block count allows.  Column blocks and
-// row blocks share grid.x, column blocks first, so that any number of rows keeps its blocks of at most kGateMaxRows.
+// side in a CTA.  ct * rt <= kGateThreads, and ct is as even a share of the row as the block count allows.  Row blocks fill
+// grid.y and, beyond 65535, grid.z, so that any number of rows keeps its blocks of at most kGateMaxRows.
 struct GateGrid {
     int ct, rt, colblocks, rows_per_cta;
     long long rowblocks;
+    dim3 grid() const {
+        const long long slices = (rowblocks + 65534) / 65535;
+        return dim3(colblocks, static_cast<unsigned>(slices == 1 ? rowblocks : 65535), static_cast<unsigned>(slices));
+    }
 };
 GateGrid gate_grid(long long rows, int cols, int min_rows) {
     GateGrid g;
@@ -64,15 +68,15 @@ template <bool HAS_D, bool HAS_Z>
 __global__ void __launch_bounds__(kGateThreads)
 gate_skip_fwd_kernel(const float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ D, int d_mode,
                      const float* __restrict__ z, float* __restrict__ out, long long rows, int cols, int p_dim, int ct,
-                     int rt, int rows_per_cta, unsigned colblocks) {
+                     int rt, int rows_per_cta) {
     after_previous();
     allow_next();
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
-    const unsigned row_block = blockIdx.x / colblocks;
-    const int c = ((blockIdx.x - row_block * colblocks) * ct + tx) * 4;
+    const long long row_block = static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y;
+    const int c = (blockIdx.x * ct + tx) * 4;
     if (c >= cols || ty >= rt) return;
     const float4 d = load_d(D, d_mode, c, p_dim);
-    const long long r0 = static_cast<long long>(row_block) * rows_per_cta;
+    const long long r0 = row_block * rows_per_cta;
     const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
     for (long long r = r0 + ty; r < r1; r += kGateUnroll * rt) {
         float4 v[kGateUnroll], xv[kGateUnroll], zv[kGateUnroll];
@@ -115,15 +119,15 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_skip_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ y, const float* __restrict__ x,
                      const float* __restrict__ D, int d_mode, const float* __restrict__ z, float* __restrict__ dy,
                      float* __restrict__ dz, float* __restrict__ part, long long rows, int cols, int p_dim, int ct, int rt,
-                     int rows_per_cta, unsigned colblocks) {
+                     int rows_per_cta) {
     after_previous();
     allow_next();
     __shared__ float4 sums[kGateThreads];
     const int tx = threadIdx.x % ct, ty = threadIdx.x / ct;
-    const unsigned row_block = blockIdx.x / colblocks;
-    const int c = ((blockIdx.x - row_block * colblocks) * ct + tx) * 4;
-    const bool active = c < cols && ty < rt;
-    const long long r0 = static_cast<long long>(row_block) * rows_per_cta;
+    const long long row_block = static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y;
+    const int c = (blockIdx.x * ct + tx) * 4;
+    const bool active = c < cols && ty < rt && row_block * rows_per_cta < rows;
+    const long long r0 = row_block * rows_per_cta;
     const long long r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
     constexpr int kUnroll = HAS_Z ? 2 : kGateUnroll;  // four tensors a row with z: eight float4 in flight
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -255,11 +259,10 @@ extern "C" int ssd_gate_skip_fwd(const SsdShape* shape, const float* y, const fl
     if (d_mode < 0 || d_mode > 2) return SSD_ERR_SHAPE;
     if (!aligned16(y, x, z, out, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(n.rows, n.cols, 1);
-    if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
-        launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0,
+        launch_plain(kernel, g.grid(), kGateThreads, 0,
                      reinterpret_cast<cudaStream_t>(stream), y, x, D, d_mode, z, out, n.rows, n.cols, n.p, g.ct, g.rt,
-                     g.rows_per_cta, static_cast<unsigned>(g.colblocks));
+                     g.rows_per_cta);
     };
     if (d_mode != 0)
         z ? launch(gate_skip_fwd_kernel<true, true>) : launch(gate_skip_fwd_kernel<true, false>);
@@ -281,11 +284,9 @@ extern "C" int ssd_gate_skip_bwd(const SsdShape* shape, const float* dout, const
     if (!aligned16(dout, y, x, z, dy, dz, dD_partial, d_mode == 2 ? D : nullptr)) return SSD_ERR_ALIGN;
     const GateGrid g = gate_grid(n.rows, n.cols, kGateMinRows);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (g.rowblocks * g.colblocks > 0x7fffffff) return SSD_ERR_RANGE;
     auto launch = [&](auto kernel) {
-        launch_plain(kernel, static_cast<unsigned>(g.rowblocks * g.colblocks), kGateThreads, 0, st, dout, y, x, D, d_mode, z,
-                     dy, dz, dD_partial, n.rows, n.cols, n.p, g.ct, g.rt, g.rows_per_cta,
-                     static_cast<unsigned>(g.colblocks));
+        launch_plain(kernel, g.grid(), kGateThreads, 0, st, dout, y, x, D, d_mode, z,
+                     dy, dz, dD_partial, n.rows, n.cols, n.p, g.ct, g.rt, g.rows_per_cta);
     };
     if (d_mode != 0)
         z ? launch(gate_skip_bwd_kernel<true, true>) : launch(gate_skip_bwd_kernel<true, false>);

@@ -144,3 +144,21 @@ def test_finalize_takes_a_buffer_of_any_alignment():
         results.append((ddt, dA, dbias))
     assert all(torch.equal(a, c) for a, c in zip(*results))
     assert torch.equal(results[0][0], raw[1:].view(b, h, l).transpose(1, 2))
+
+
+def test_gate_with_more_row_blocks_than_one_grid_dimension_holds():
+    from ascend_kernel import mamba2 as M
+
+    b, l, h, p = 1, 65536 * 128 + 5, 1, 4
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    y, x, z, dout = (torch.randn(b, l, h, p, generator=gen, device="cuda") for _ in range(4))
+    D = torch.randn(h, p, generator=gen, device="cuda")
+    sig = torch.sigmoid(z.double())
+    pre = y.double() + x.double() * D.double()
+    assert _rel(M.gate_forward(y, x, None, D, z), pre * z.double() * sig) < REL
+    dy, dz, dD = M.gate_backward(dout, y, x, None, D, z)
+    want = dout.double() * z.double() * sig
+    assert _rel(dy, want) < REL
+    assert _rel(dz, dout.double() * pre * sig * (1 + z.double() * (1 - sig))) < REL
+    terms = want * x.double()
+    assert (dD.double() - terms.sum((0, 1))).norm().item() < REL * terms.norm().item()
