@@ -14,9 +14,11 @@
 // columns; two 96-column accumulators take 192 of the rest, so that one is read out under the other's products); w arrives by
 // TMA from its split copy, one tile of all parts per stage, two stages.  K beyond 192 is taken in equal chunks of up
 // to 192 (the last one filled up with zeros by the loads), with the sums of two tiles kept in registers.  The issue of the products
-// bounds a tile (72 of them at K = 192, 3.5 us); before the first, a chunk of x is loaded and converted (3 to 5 us).
+// bounds a tile (72 of them at K = 192, 3.5 us); before the first, a chunk of x is loaded (the later ones under the products of the
+// chunk before) and converted.
 //
-// [16384,192] x [902,192]: 50 us from cold caches (139 in the library), [16384,384] x [192,384]: 36 (66).  Error against 64
+// [16384,192] x [902,192]: 43 us with the split of w, 50 from cold caches (139 in the library); [16384,384] x [192,384] + residual:
+// 29, 36 (66 without the residual).  One accumulator for all of K: 45 and 27 us.  Error against 64
 // bits, relative 2-norm, operands of both signs / of one sign (the library's fp32 kernel in brackets): K = 192 8.6e-8 / 9.2e-8
 // (2.5e-7 / 2.1e-7), K = 384 9.2e-8 / 9.4e-8 (3.5e-7 / 2.9e-7), K = 1536 1.2e-7 / 1.1e-7 (7.0e-7 / 5.8e-7).  With one accumulator
 // for all of K it was 1.8e-7 / 2.7e-7, 3.5e-7 / 6.1e-7 and 1.5e-6 / 3.7e-6.  Measured and dropped: 64-column tiles in three
@@ -109,7 +111,7 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     constexpr uint32_t stage_bytes = lin_stage_bytes(blocks);
     float* patches = reinterpret_cast<float*>(smem + 2 * stage_bytes);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * stage_bytes + kLinWarps * kLinPatch);
-    uint64_t* full_x = bars;          // a chunk of x has landed (in stage 1, and every product before it is done)
+    uint64_t* full_x = bars;          // a chunk of x has landed
     uint64_t* x_ready = bars + 1;     // it is in tensor memory (per warp)
     uint64_t* full_w = bars + 2;      // [2] a tile of w has landed
     uint64_t* done = bars + 4;        // [2] the products that read a stage are done
@@ -121,8 +123,10 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     const int row0 = blockIdx.x * 128;
     const int tile0 = blockIdx.y * a.tiles_per_item;
     const int ntiles = min(a.tiles_per_item, a.tiles - tile0);
-    // tiles that go through a stage in the pass over one chunk
-    auto per_pass = [&](int st) { return (ntiles + 1 - st) >> 1; };
+    // Stage of a tile of w in the pass over a chunk of K, and the stage where that chunk of x lands on its way to tensor
+    // memory: the one of the pass before's first tile, so that it arrives under that pass's second.
+    auto stage_of = [](int pass, int t) { return (pass + t) & 1; };
+    auto x_stage = [&](int pass) { return stage_of(pass, 1); };
 
     if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need the declared alignment
         if (tid == 0) atomicCAS(status, 0, kStatusSmemAlign);
@@ -159,12 +163,14 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
     if (warp == kLinWarps) {  // ---- issues the products
         if (lane == 0) {
             const uint32_t idesc = make_idesc_bf16(128, kLinCols, false, false);
-            int sum = 0;  // accumulators so far
+            int sum = 0;          // accumulators so far
+            uint32_t parity = 0;  // of full_w, a bit per stage
             for (int pass = 0; pass < a.chunks; ++pass) {
                 mbar_wait(x_ready, pass & 1, status, kStatusMmaTimeout | wait_site(7, 1));
                 for (int t = 0; t < ntiles; ++t) {
-                    const int st = t & 1;
-                    mbar_wait(&full_w[st], (pass * per_pass(st) + (t >> 1)) & 1, status, kStatusMmaTimeout | wait_site(7, 2));
+                    const int st = stage_of(pass, t);
+                    mbar_wait(&full_w[st], (parity >> st) & 1u, status, kStatusMmaTimeout | wait_site(7, 2));
+                    parity ^= 1u << st;
                     const uint32_t base = smem_u32(smem) + st * stage_bytes;
 #pragma unroll
                     for (int blk = 0; blk < blocks; ++blk, ++sum) {
@@ -196,31 +202,32 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
         }
     } else if (warp == kLinWarps + 1) {  // ---- issues the loads
         if (lane == 0) {
-            auto stage_idle = [&](int st, int loads) {  // the products of the last of its `loads` tiles so far are done
-                if (loads > 0) mbar_wait(&done[st], (loads - 1) & 1, status, kStatusMmaTimeout | wait_site(7, 4));
+            uint32_t busy = 0, parity = 0;      // stages that products read, and the parity of done, a bit per stage
+            auto stage_idle = [&](int st) {     // the products of the tile it holds are done
+                if (((busy >> st) & 1u) == 0) return;
+                mbar_wait(&done[st], (parity >> st) & 1u, status, kStatusMmaTimeout | wait_site(7, 4));
+                parity ^= 1u << st;
+                busy ^= 1u << st;
             };
             for (int pass = 0; pass < a.chunks; ++pass) {
                 const int k0 = pass * blocks * 64;
                 auto load_w = [&](int t) {
-                    const int st = t & 1;
+                    const int st = stage_of(pass, t);
+                    stage_idle(st);
+                    busy |= 1u << st;
                     mbar_arrive_expect_tx(&full_w[st], stage_bytes);
                     for (int part = 0; part < 3; ++part)
                         for (int blk = 0; blk < blocks; ++blk)  // 64 bf16 columns seen as 32 floats
                             tma_load_2d(smem + st * stage_bytes + (part * blocks + blk) * kLinBox, &map_w, &full_w[st],
                                         (k0 + blk * 64) / 2, part * a.cols_padded + (tile0 + t) * kLinCols);
                 };
-                // both stages idle: every product of the passes before is done, x's tensor memory may be replaced too
-                stage_idle(0, pass * per_pass(0));
-                stage_idle(1, pass * per_pass(1));
+                stage_idle(x_stage(pass));
                 mbar_arrive_expect_tx(full_x, 2u * blocks * kSlabBytes);
                 for (int i = 0; i < 2 * blocks; ++i)
-                    tma_load_2d(smem + stage_bytes + i * kSlabBytes, &map_x, full_x, k0 + 32 * i, row0);
+                    tma_load_2d(smem + x_stage(pass) * stage_bytes + i * kSlabBytes, &map_x, full_x, k0 + 32 * i, row0);
                 load_w(0);
-                mbar_wait(x_ready, pass & 1, status, kStatusMmaTimeout | wait_site(7, 5));  // stage 1 has been read
-                for (int t = 1; t < ntiles; ++t) {
-                    if (t >= 2) stage_idle(t & 1, pass * per_pass(t & 1) + (t >> 1));
-                    load_w(t);
-                }
+                mbar_wait(x_ready, pass & 1, status, kStatusMmaTimeout | wait_site(7, 5));  // x has left its stage
+                for (int t = 1; t < ntiles; ++t) load_w(t);
             }
         }
     } else {  // ---- convert x, write the result
@@ -239,17 +246,12 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             const int acc = sum & 1;
             ok = mbar_wait(&acc_ready[acc], (sum >> 1) & 1, status, kStatusMmaTimeout | wait_site(7, 7)) && ok;
             tc_fence_after_sync();
-            constexpr int kAtOnce = HELD == 1 ? kCols : 16;  // with two tiles held the registers do not take more
+            float v[kCols];
 #pragma unroll
-            for (int c0 = 0; c0 < kCols; c0 += kAtOnce) {
-                float v[kAtOnce];
+            for (int c = 0; c < kCols; c += 16) tmem_ld16(tmem_addr(tmem + acc * kLinCols, warp, half * kCols + c), v + c);
+            tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < kAtOnce; c += 16)
-                    tmem_ld16(tmem_addr(tmem + acc * kLinCols, warp, half * kCols + c0 + c), v + c);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < kAtOnce; ++i) total[c0 + i] += v[i];
-            }
+            for (int i = 0; i < kCols; ++i) total[i] += v[i];
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_free[acc]);
@@ -261,7 +263,7 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             // of this thread's rows r0, r0 + 4, ... those that exist
             const int rows = ok ? static_cast<int>(max(0ll, min(8ll, (a.rows - out_row - r0 + 3) / 4))) : 0;
             auto inside = [&](int c0, int i) { return i < rows && col + c0 < a.cols; };
-            constexpr int kPatches = kCols / kLinPatchCols, kAtOnce = HELD == 1 ? kPatches : 2;  // residual loads in flight together
+            constexpr int kPatches = kCols / kLinPatchCols, kAtOnce = HELD == 1 ? kPatches : 3;  // residual loads in flight together
 #pragma unroll
             for (int j0 = 0; j0 < kPatches; j0 += kAtOnce) {
                 float add[kAtOnce][8];
@@ -288,30 +290,22 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             }
         };
         for (int pass = 0; pass < a.chunks; ++pass) {
+            // every accumulator of the pass before has been read: its products are done and x's tensor memory may be replaced
             ok = mbar_wait(full_x, pass & 1, status, kStatusTmaTimeout | wait_site(7, 6)) && ok;
             tc_fence_after_sync();
 #pragma unroll 1
             for (int slab = half; slab < 2 * blocks; slab += 2) {
-                const uint8_t* src = smem + stage_bytes + slab * kSlabBytes;
-                constexpr int kPairs = HELD == 1 ? 16 : 8;  // split together
-#pragma unroll 1
-                for (int first = 0; first < 16; first += kPairs) {
-                    uint32_t hi[kPairs], mid[kPairs], lo[kPairs];
+                const uint8_t* src = smem + x_stage(pass) * stage_bytes + slab * kSlabBytes;
+                uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
-                    for (int c = 0; c < kPairs / 2; ++c) {
-                        const float4 f = *reinterpret_cast<const float4*>(src + swz(quarter * 32 + lane, first / 2 + c));
-                        split3_pair(f.x, f.y, hi[2 * c], mid[2 * c], lo[2 * c]);
-                        split3_pair(f.z, f.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
-                    }
-                    auto store = [&](uint32_t part, const uint32_t* v) {
-                        const uint32_t at = tmem_addr(tm_x + part * part_cols, warp, 16 * slab + first);
-                        if constexpr (kPairs == 16) tmem_st16(at, v);
-                        else tmem_st8(at, v);
-                    };
-                    store(0, hi);
-                    store(1, mid);
-                    store(2, lo);
+                for (int c = 0; c < 8; ++c) {
+                    const float4 f = *reinterpret_cast<const float4*>(src + swz(quarter * 32 + lane, c));
+                    split3_pair(f.x, f.y, hi[2 * c], mid[2 * c], lo[2 * c]);
+                    split3_pair(f.z, f.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
                 }
+                tmem_st16(tmem_addr(tm_x, warp, 16 * slab), hi);
+                tmem_st16(tmem_addr(tm_x + part_cols, warp, 16 * slab), mid);
+                tmem_st16(tmem_addr(tm_x + 2 * part_cols, warp, 16 * slab), lo);
             }
             tmem_st_wait();
             signal_issuer(x_ready, lane);
@@ -325,15 +319,13 @@ linear_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
             } else {
 #pragma unroll
                 for (int t = 0; t < HELD; ++t)
-                    if (t < ntiles)
+                    if (t < ntiles) {
 #pragma unroll
                         for (int blk = 0; blk < blocks; ++blk) add_up(sums[t]);
+                        if (pass == a.chunks - 1) write_tile(sums[t], t);  // under the next tile's products
+                    }
             }
         }
-        if constexpr (HELD > 1)
-#pragma unroll
-            for (int t = 0; t < HELD; ++t)
-                if (t < ntiles) write_tile(sums[t], t);
     }
     __syncwarp();
     tc_fence_before_sync();
