@@ -433,7 +433,8 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 
 def _epilogue_alone(ctx) -> bool:
     """Whether of the inputs of ``_Mamba2SsdAutograd`` only D and z need gradients."""
-    return not any(ctx.needs_input_grad[i] for i in (0, 1, 2, 3, 4, 8, 9))
+    needs = ctx.needs_input_grad
+    return not (needs[0] or needs[1] or needs[2] or needs[3] or needs[4] or needs[8] or needs[9])
 
 
 class _Mamba2SsdAutograd(torch.autograd.Function):
@@ -452,7 +453,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         # Without an epilogue the output is what backward needs.  At the kernels' own sizes it is saved itself, so that
         # changing it in place is an error in backward; elsewhere the caller may change it, and a copy is saved.
         own_sizes = x.shape[3] == 64 and B.shape[3] == 64 and x.shape[1] % TILE == 0 and x.shape[2] == A.shape[0]
-        gated = D is not None or z is not None
+        gated, alone = D is not None or z is not None, _epilogue_alone(ctx)
         ctx.differentiable = gated and not own_sizes  # see differentiable_backward
         ctx.options = (dt_softplus, dt_min, dt_max)
         copy = not gated and not ctx.recompute and not own_sizes
@@ -461,9 +462,11 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         if ctx.recompute:  # inputs only; y, q, cs and the tile-start states are rebuilt in backward
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start)
         else:
-            if _epilogue_alone(ctx):  # its gradients take y only
+            if alone:  # its gradients take y only
                 work = ()
             ctx.save_for_backward(x, dt, A, B, C, dt_bias, D, z, start, y, *work)
+        if alone and not own_sizes:  # where D and z were framework operations the state never belonged to their graph
+            ctx.mark_non_differentiable(final)
         return out, final
 
     @staticmethod
@@ -492,7 +495,6 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
             dx, ddt, dA, dB, dC, dD, dz, dinit, dbias = backward_call(x, dt, A, B, C, D, z, dt_bias, y, work, dout, dfinal,
                                                                       ctx.shape, ctx.has_initial)
         return dx, ddt, dA, dB, dC, dD, dz, None, dinit, dbias, None, None
-
 
     @staticmethod
     def differentiable_backward(ctx, dout, dfinal):

@@ -110,7 +110,8 @@ def test_what_is_kept_for_gradients_of_the_epilogue_alone():
     z.requires_grad_(True)
     stats = SavedTensorStats()
     with stats.hooks():
-        out = mamba2_ssd_fwd(x, dt, A, B, C, 64, z=z, dt_softplus=True)
+        out, final = mamba2_ssd_fwd(x, dt, A, B, C, 64, z=z, dt_softplus=True, return_final_state=True)
+    assert out.requires_grad and not final.requires_grad  # the state does not depend on z
     inputs = sum(4 * t.numel() for t in (x, dt, A, B, C, z))
     assert stats.unique_bytes <= inputs + 4 * out.numel() + 4096  # and the output before the gate, no states
     assert torch.isfinite(torch.autograd.grad(out.sum(), z)[0]).all()
