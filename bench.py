@@ -404,8 +404,7 @@ def secondary_measurements(dev, timer, peaks) -> dict:
     sec["recompute_policy_h256"] = {"ms_per_step": ms, "saved_bytes": saved_recompute,
                                     "saved_bytes_default_policy": stats.unique_bytes}
     del out, final, leaves, inputs, step
-    # shapes outside the native kernels (reduced to them by padding and column blocks in the Python layer), each
-    # beside the native shape it is reduced to: what the reduction costs
+    # shapes other than the kernels' own sizes, each beside the nearest of those: what the smaller or cut-off tiles cost
     general = {}
     for name, shape, native in (
             ("dstate128_fwd_bwd", (4, 2048, 16, 64, 128, 128, 4), (4, 2048, 16, 64, 64, 128, 4)),

@@ -88,9 +88,9 @@ int ssd_check_shape(const SsdShape* shape);
 enum {
     SSD_BUF_Q = 0,          /* float [B,H,L]                                   */
     SSD_BUF_CS = 1,         /* float [B,H,L]                                   */
-    SSD_BUF_STATES = 2,     /* float [B,H,K,P,N]   (also the size of dstates)  */
+    SSD_BUF_STATES = 2,     /* float [B,H,K,P,N], with SSD_FLAG_EXTENTS [B,H,K,64,64 or 128] (also the size of dstates) */
     SSD_BUF_FINAL_STATE = 3,/* float [B,H,P,N]     (initial_state, dfinal, d_initial alike) */
-    SSD_BUF_G_LAST = 4,     /* float [B,H,K]                                   */
+    SSD_BUF_G_LAST = 4,     /* float [B,H,K], with SSD_FLAG_EXTENTS and dstate above 64 [2,B,H,K] */
     SSD_BUF_DDT_T = 5,      /* float [B,H,L]                                   */
     SSD_BUF_DA_PARTIAL = 6, /* double [B,H,K]                                  */
     SSD_BUF_GATE_PARTIAL = 7,/* float [ssd_gate_partial_floats()]              */
@@ -102,7 +102,7 @@ size_t ssd_buffer_bytes(const SsdShape* shape, int which);
  *
  * Internal buffers (caller-allocated fp32, K = L / tile):
  *   q, cs        [B,H,L]      q = dt after softplus/clamp; cs = inclusive in-tile cumulative sum of A*q
- *   states       [B,H,K,P,N]  chunk states U_k, turned in place into the state at the START of tile k
+ *   states       [B,H,K,P,N]  (as SSD_BUF_STATES says) chunk states U_k, turned in place into the state at the START of tile k
  *   status       one int32, zeroed by the caller once; a kernel whose bounded wait gives up stores a
  *                non-zero code there and writes no results; its low four bits say why: 1 = a TMA load did
  *                not arrive, 2 = a tensor-core product (or the hand-off to the issuing warp) did not

@@ -11,10 +11,11 @@ A plain stack, as the benchmark definition describes it: patch-16 embedding of a
 and a mean-pool + linear head.  The reference's own demo network (mamba_torch/vmamba2_network.py) is a
 different, hierarchical four-direction model; what is kept from it is the integration pattern of its
 ``SsdCore`` (:31-85): the block calls one injectable SSD function with the ``mamba2_ssd_fwd`` signature.
-The projections run on PyTorch / cuBLAS.  In inference on CUDA (no gradients) the norms and the convolution run
-as this library's fused forward kernels (``ssd_block_rmsnorm_fwd``, ``ssd_block_conv_silu_fwd``: one pass each,
-writing the SSD's inputs in place of the framework's split / transpose / copy chain); with gradients enabled, on
-CPU, or when this file is loaded without the package, the same steps run as framework operations.
+In inference on CUDA (no gradients) the norms and the convolution run as this library's fused forward kernels
+(``ssd_block_skip_rmsnorm_fwd``, ``ssd_block_conv_split_fwd``: one pass each, writing the SSD's inputs in place of the
+framework's split / transpose / copy chain), and the projections as ``ssd_linear_fwd`` where the layer is a plain one and
+the sizes are large enough (``_linear``); with gradients enabled, on CPU, or when this file is loaded without the
+package, the same steps run as framework operations.
 """
 from __future__ import annotations
 

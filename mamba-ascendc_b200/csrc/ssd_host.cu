@@ -183,8 +183,10 @@ extern "C" const char* ssd_error_string(int code) {
         case SSD_ERR_SHAPE:
             return "ssd: all dimensions must be positive, nheads must be divisible by ngroups and tile must be positive";
         case SSD_ERR_UNSUPPORTED:
-            return "ssd: unsupported problem (need headdim == 64, dstate in {64, 128}, tile == 128, seqlen % 128 == 0; "
-                   "ssd_forward_static also needs its outputs on the current device)";
+            return "ssd: unsupported problem (the tile kernels need tile == 128, seqlen % 128 == 0 and headdim == 64 with dstate "
+                   "64 or 128, or with SSD_FLAG_EXTENTS multiples of 4 up to these; the gate headdim % 4 == 0 up to 1024; the "
+                   "recurrence dstate % 4 == 0 up to 128; the projection k % 64 == 0; ssd_forward_static also needs its outputs "
+                   "on the current device)";
         case SSD_ERR_RANGE:
             return "ssd: size out of range (batch and ngroups at most 65535; batch * seqlen and the number of state rows "
                    "below 2^31)";
