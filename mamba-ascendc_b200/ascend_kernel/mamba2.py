@@ -622,10 +622,13 @@ def _own_sizes(x, B, grad: bool) -> bool:
     return x.shape[3] == 64 and x.shape[1] % TILE == 0 and (B.shape[3] == 64 or (B.shape[3] == 128 and not grad))
 
 
+_forward_ad, _transforms_active = torch.autograd.forward_ad, torch._C._are_functorch_transforms_active
+
+
 def _in_transform() -> bool:
     """Whether forward-mode derivatives or a function transform (vmap, grad, jvp) are being taken, which see framework
     operations only.  Away from the kernels' own sizes D and z are then applied by such operations."""
-    return torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+    return _forward_ad._current_level >= 0 or _transforms_active()
 
 
 def _short_sequence(x, B, C, D, z, initial_states) -> bool:

@@ -306,15 +306,18 @@ __device__ __forceinline__ double block_sum_256(double v, double* red, int tid) 
     return ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
 }
 
-// Four floats from an address that may take a 16-byte load or not (the caller's buffer, the same for the whole launch).
-__device__ __forceinline__ float4 load_quad(const float* p, bool aligned) {
-    return aligned ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+// ALIGNED: ddt_t, the caller's buffer, takes 16-byte loads.
+template <bool ALIGNED>
+__device__ __forceinline__ float4 load_quad(const float* p) {
+    if constexpr (ALIGNED) return *reinterpret_cast<const float4*>(p);
+    return make_float4(p[0], p[1], p[2], p[3]);
 }
 
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256)
 dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ part, float* __restrict__ ddt,
                    float* __restrict__ dA, float* __restrict__ ddt_bias, int batch, int nchunks, int nheads, int parts,
-                   int tokens, int head_blocks, int head_bits, bool aligned) {
+                   int tokens, int head_blocks, int head_bits) {
     after_previous();
     allow_next();
     __shared__ float patch[kTile][33];
@@ -331,9 +334,9 @@ dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ p
         for (int i = 0; i < 4; ++i)
             if (warp + 8 * i < heads) {
                 const float* src = ddt_t + (static_cast<size_t>(b) * nheads + h0 + warp + 8 * i) * parts * seqlen + k * kTile + 4 * lane;
-                v[i] = load_quad(src, aligned);
+                v[i] = load_quad<ALIGNED>(src);
                 for (int j = 1; j < parts; ++j) {
-                    const float4 o = load_quad(src + static_cast<size_t>(j) * seqlen, aligned);
+                    const float4 o = load_quad<ALIGNED>(src + static_cast<size_t>(j) * seqlen);
                     v[i].x += o.x;
                     v[i].y += o.y;
                     v[i].z += o.z;
@@ -371,7 +374,7 @@ dt_finalize_kernel(const float* __restrict__ ddt_t, const double* __restrict__ p
         const float* row = ddt_t + (static_cast<size_t>(b) * nheads + h) * parts * seqlen;
 #pragma unroll 4
         for (int i = tid; i < parts * (seqlen / 4); i += 256) {
-            const float4 f = load_quad(row + 4 * static_cast<size_t>(i), aligned);
+            const float4 f = load_quad<ALIGNED>(row + 4 * static_cast<size_t>(i));
             acc += (static_cast<double>(f.x) + f.y) + (static_cast<double>(f.z) + f.w);
         }
     }
@@ -461,9 +464,9 @@ extern "C" int ssd_dt_finalize_bias_bwd(const SsdShape* shape, const float* ddt_
     const int nchunks = shape->seqlen / kTile, head_blocks = (heads + 31) / 32;
     const int64_t blocks = static_cast<int64_t>(shape->batch) * nchunks * head_blocks + heads;
     if (blocks > 0x7fffffff) return SSD_ERR_RANGE;
-    launch_plain(dt_finalize_kernel, static_cast<unsigned>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+    launch_plain(aligned16(ddt_t) ? dt_finalize_kernel<true> : dt_finalize_kernel<false>, static_cast<unsigned>(blocks), 256, 0, reinterpret_cast<cudaStream_t>(stream),
                  ddt_t, dA_partial, ddt, dA, ddt_bias, shape->batch, nchunks, heads, parts, row_tokens(*shape),
-                 head_blocks, head_bits_of(heads), aligned16(ddt_t));
+                 head_blocks, head_bits_of(heads));
     return launch_status();
 }
 
