@@ -453,9 +453,11 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         # Without an epilogue the output is what backward needs.  At the kernels' own sizes it is saved itself, so that
         # changing it in place is an error in backward; elsewhere the caller may change it, and a copy is saved.
         own_sizes = x.shape[3] == 64 and B.shape[3] == 64 and x.shape[1] % TILE == 0 and x.shape[2] == A.shape[0]
-        gated, alone = D is not None or z is not None, _epilogue_alone(ctx)
+        gated = D is not None or z is not None
+        ctx.alone = alone = gated and _epilogue_alone(ctx)
         ctx.differentiable = gated and not own_sizes  # see differentiable_backward
-        ctx.options = (dt_softplus, dt_min, dt_max)
+        if ctx.differentiable:
+            ctx.options = (dt_softplus, dt_min, dt_max)
         copy = not gated and not ctx.recompute and not own_sizes
         out, final, y, work = forward_call(x, dt, A, B, C, D, z, dt_bias, initial_states, ctx.shape, True, copy=copy)
         start = initial_states if ctx.recompute or ctx.differentiable else None
@@ -475,7 +477,7 @@ class _Mamba2SsdAutograd(torch.autograd.Function):
         y, work = (rest[0], rest[1:]) if rest else (None, None)
         if dout is None:  # loss depends on the final state only (mamba2.py:1801-1802)
             dout = torch.zeros_like(x)
-        alone = _epilogue_alone(ctx)
+        alone = ctx.alone
         again = ctx.differentiable and (torch.is_grad_enabled() or (alone and _is_batched(dout)))
         if again and not alone:
             return _Mamba2SsdAutograd.differentiable_backward(ctx, dout, dfinal)
@@ -617,9 +619,9 @@ def _device_guard(device: torch.device):
 SHORT_SEQUENCE = 32
 
 
-def _own_sizes(x, B, grad: bool) -> bool:
+def _own_sizes(l: int, p: int, n: int, grad: bool) -> bool:
     """The kernels' own sizes, which nothing pads, copies or cuts off."""
-    return x.shape[3] == 64 and x.shape[1] % TILE == 0 and (B.shape[3] == 64 or (B.shape[3] == 128 and not grad))
+    return p == 64 and l % TILE == 0 and (n == 64 or (n == 128 and not grad))
 
 
 _forward_ad, _transforms_active = torch.autograd.forward_ad, torch._C._are_functorch_transforms_active
@@ -647,10 +649,11 @@ def _tile_extents(x, B, C, D, z, initial_states, grad: bool = False) -> bool:
     """Whether the tile kernels read and write the caller's tensors as they are: their tile loads and stores cut a tile off
     at the end of a sequence, of a head's channels and of the state's columns, in steps of four floats from 16-byte
     aligned addresses.  What this leaves (other headdims and state sizes) is padded or cut into blocks by shapes.py."""
-    p, n = x.shape[3], B.shape[3]
-    if min(x.shape) <= 0 or min(B.shape) <= 0 or n % 4 or n > 128 or p > 1024 or (p % 64 if p > 64 else p % 4):
+    sizes, state = x.shape, B.shape
+    p, n = sizes[3], state[3]
+    if min(sizes) <= 0 or min(state) <= 0 or n % 4 or n > 128 or p > 1024 or (p % 64 if p > 64 else p % 4):
         return False
-    if _own_sizes(x, B, grad):
+    if _own_sizes(sizes[1], p, n, grad):
         return True  # unaligned addresses are refused
     if _in_transform():
         return False
